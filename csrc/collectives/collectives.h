@@ -87,6 +87,9 @@ struct NormArgs {
   size_t piece_bytes;     // >= rows * hidden * sizeof(T), a multiple of 16
 };
 
+// kNormLocal outside the emulation (norm_local.cu).
+cudaError_t launch_norm_local(int rank, const NormArgs& args, int max_ctas, cudaStream_t stream);
+
 cudaError_t launch_fused_norm(const CommCtx& ctx, int algo, const NormArgs& args, int max_ctas, cudaStream_t stream);
 
 }  // namespace oob

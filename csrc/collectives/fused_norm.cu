@@ -518,6 +518,7 @@ cudaError_t dispatch_ppt(int algo, const CommCtx& ctx, int ctas, const NormArgs&
 cudaError_t launch_fused_norm(const CommCtx& ctx, int algo, const NormArgs& a, int max_ctas, cudaStream_t stream) {
   if (a.hidden % 8 != 0 || a.hidden <= 0 || a.rows < 0) return cudaErrorInvalidValue;
   if (a.dtype != kF16 && a.dtype != kBF16) return cudaErrorInvalidValue;
+  if (algo == kNormLocal && ctx.emu_table == nullptr) return launch_norm_local(ctx.rank, a, max_ctas, stream);
   const bool mc = (algo == kNormArTwoShotNvls || algo == kNormRsNvls);
   if (mc && a.x.mc == nullptr) return cudaErrorInvalidValue;
   if (algo == kNormArTwoShotNvls && a.y.mc == nullptr) return cudaErrorInvalidValue;
@@ -529,8 +530,7 @@ cudaError_t launch_fused_norm(const CommCtx& ctx, int algo, const NormArgs& a, i
   int rows = a.rows;
   if (algo >= kNormArTwoShot && !push) rows = (a.rows + ctx.world - 1) / ctx.world;
   int ctas = max_ctas < 1 ? 1 : max_ctas;
-  // Communicating launches are bounded by the barrier slots of the pad; the local one may fill the GPU
-  // (one row per CTA at a time, eight resident CTAs per SM hide the three dependent passes over a row).
+  // Communicating launches are bounded by the barrier slots of the pad; the local one (here in emulation only) is not.
   const int cap = algo == kNormLocal ? 148 * 8 : kMaxCommBlocks;
   if (ctas > cap) ctas = cap;
   if (ctas > rows) ctas = rows < 1 ? 1 : rows;

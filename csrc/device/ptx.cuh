@@ -40,6 +40,13 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// Programmatic dependent launch.  `launch_dependents` lets the next kernel of the stream be set up while this one still
+// runs; `wait` returns when every kernel this launch depends on has completed and its writes are visible (at once when
+// the launch has no such dependency).  A kernel that is launched with the attribute must pass `wait` in every CTA
+// before it touches memory that another kernel may write or still read.
+__device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Named barrier among a subset of the CTA's warps.
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
@@ -261,6 +268,13 @@ __device__ __forceinline__ void red_relaxed_sys_add(uint32_t* p, uint32_t v) {
 }
 __device__ __forceinline__ void fence_acq_rel_sys() { asm volatile("fence.acq_rel.sys;" ::: "memory"); }
 
+// A plain 128-bit load the compiler keeps where it is written: behind griddep_wait, where a load through the read-only
+// path might be moved up.
+__device__ __forceinline__ uint4 ld_v4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
 // 128-bit accesses that bypass L1 (peer data is never reused from L1).
 __device__ __forceinline__ uint4 ld_nc_v4(const void* p) {
   uint4 v;
