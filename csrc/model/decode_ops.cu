@@ -2,11 +2,11 @@
 // and grouped-query decode attention over a static cache.
 //
 // The attention kernel is bound by reading the cache once: a CTA handles one (sequence, KV head, key chunk); its
-// four warps take 32-key tiles in turn (cp.async double buffering, per-warp buffers, XOR-swizzled rows), compute
+// four warps take 16-key tiles in turn (cp.async, three stages, per-warp buffers, XOR-swizzled rows), compute
 // scores for all query heads of the KV group at once on the tensor cores (the <= 16 query heads are the M rows of
 // m16n8k16 MMAs -- too few rows for a tcgen05 tile, which needs 64), keep an online softmax per row and accumulate
-// P*V in fp32.  The warps' partial results are merged through shared memory; with several chunks per sequence a
-// second small kernel merges the chunks.
+// P*V in fp32.  The warps' partial results are merged through shared memory, those of the up to eight CTAs of a cluster
+// through distributed shared memory; only few long sequences are cut further, and a second small kernel then merges.
 //
 // Capability parity: none of these exist in the reference (it delegates the model to vLLM,
 // patches/vllm/v0.25.0/vllm/model_executor/models/qwen2.py); they make this library's own serving path a fixed
@@ -15,6 +15,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <cstdlib>
@@ -22,6 +23,7 @@
 
 #include "../api/oob.h"
 #include "../api/oob_model.h"
+#include "../device/ptx.cuh"
 #include "../runtime/errors.h"
 
 namespace oob {
@@ -53,6 +55,26 @@ struct Cvt<__half> {
   }
 };
 
+// Launches with programmatic stream serialization: the kernel's launch overlaps the tail of the one before it.
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t stream, int cluster, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 // ---------------------------------------------------------------------------------------------------------------
 // RoPE + KV-cache write
 // ---------------------------------------------------------------------------------------------------------------
@@ -61,6 +83,8 @@ template <typename T>
 __global__ void rope_kv_write_kernel(oob_rope_args_t a, long long units) {
   const int upr = a.hd / 8;  // units per head
   const int heads = a.H + 2 * a.KV;
+  ptx::griddep_launch_dependents();
+  ptx::griddep_wait();
   const long long pos_base = a.pos_dev != nullptr ? *a.pos_dev : static_cast<long long>(a.pos0);
   for (long long u = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; u < units;
        u += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -105,6 +129,8 @@ __global__ void rope_kv_write_kernel(oob_rope_args_t a, long long units) {
 template <typename T>
 __global__ void silu_mul_kernel(const T* gu, long long ld, T* out, long long units, int F) {
   const int upr = F / 8;
+  ptx::griddep_launch_dependents();
+  ptx::griddep_wait();
   for (long long u = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; u < units;
        u += static_cast<long long>(gridDim.x) * blockDim.x) {
     const long long r = u / upr;
@@ -126,14 +152,13 @@ __global__ void silu_mul_kernel(const T* gu, long long ld, T* out, long long uni
 // Decode attention
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int kHD = 128;
-constexpr int kTileKeys = 32;                      // keys per warp tile
+constexpr int kTileKeys = 16;                      // keys per warp tile: one K = 16 step of the P V product
 constexpr int kAttnWarps = 4;
 constexpr int kAttnThreads = kAttnWarps * 32;
 constexpr int kRowBytes = kHD * 2;                 // 256
-constexpr int kKvTileBytes = kTileKeys * kRowBytes;  // 8 KiB
-// Pipeline depth per warp (tiles of K and V in flight or in use): 2 by default (128 KiB per CTA), 3 with
-// OOB_ATTN_STAGES=3 (192 KiB: two tiles in flight while one is consumed).  The buffers are reused for the
-// cross-warp merge.
+constexpr int kKvTileBytes = kTileKeys * kRowBytes;  // 4 KiB
+constexpr int kMaxAttnCluster = 8;                 // portable cluster size
+// Pipeline depth per warp (tiles of K and V in flight or in use): 3 by default (96 KiB per CTA, two CTAs per SM).
 __host__ __device__ constexpr int attn_warp_buf_bytes(int stages) { return stages * 2 * kKvTileBytes; }
 __host__ __device__ constexpr int attn_smem_bytes(int stages) { return kAttnWarps * attn_warp_buf_bytes(stages); }
 constexpr int kPartialStride = kHD + 2;            // fp32 words of one partial result: 128 values, max, sum
@@ -187,33 +212,50 @@ struct AttnParams {
   int B, H, KV, G;
   long long batch_stride;
   int max_len, batch0;
-  int splits, chunk;
+  int splits;
   float scale_log2;
 };
 
-template <typename T, int STAGES>
-__global__ void __launch_bounds__(kAttnThreads, 1) attn_decode_kernel(AttnParams p) {
+template <typename T>
+__device__ __forceinline__ T to_out(float y) {
+  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+    return __float2bfloat16_rn(y);
+  } else {
+    return __float2half_rn(y);
+  }
+}
+
+__device__ __forceinline__ void attn_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_cluster_f32(uint32_t smem_addr, uint32_t rank) {
+  uint32_t a;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+
+// Grid: (splits * S, KV, B) in clusters of S along x.  The keys of one (sequence, KV head) are dealt out in 16-key tiles
+// to the splits * S CTAs from the length the kernel finds on the device, so that a cache that is mostly empty, or a
+// length just past a multiple of anything, leaves no CTA with more than one tile per warp over its share.
+template <typename T, int STAGES, int S>
+__global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams p) {
   constexpr int kWarpBufBytes = attn_warp_buf_bytes(STAGES);
+  static_assert(attn_smem_bytes(STAGES) >= (kAttnWarps + 1) * 16 * (kHD + 2) * 4, "merge buffers");
   extern __shared__ __align__(128) uint8_t attn_smem[];
-  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  const int part = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = p.G;
+  ptx::griddep_launch_dependents();
+  ptx::griddep_wait();
   int L = p.pos_dev != nullptr ? static_cast<int>(*p.pos_dev) + 1 : p.len;
   if (L > p.max_len) L = p.max_len;
   if (L < 1) L = 1;
-  const int start = split * p.chunk;
-  const int end = min(L, start + p.chunk);
+  const long long nt = (L + kTileKeys - 1) / kTileKeys;
+  const int parts = p.splits * S;
+  const int t0 = static_cast<int>(nt * part / parts), t1 = static_cast<int>(nt * (part + 1) / parts);
   const int h0 = kvh * G;
-
-  if (start >= end) {
-    // No keys in this chunk (only with splits > 1): a neutral partial.
-    if (threadIdx.x < G) {
-      float* w = p.ws + ((static_cast<long long>(b) * p.H + h0 + threadIdx.x) * p.splits + split) * kPartialStride;
-      w[kHD] = -INFINITY;
-      w[kHD + 1] = 0.f;
-    }
-    return;
-  }
 
   // ---- Q fragments (A operand, 16 x 128; rows >= G are zero) ----
   const int row0 = lane >> 2, colp = (lane & 3) * 2;
@@ -232,21 +274,17 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_decode_kernel(AttnParams
 
   const T* kbase = static_cast<const T*>(p.k) + (p.batch0 + b) * p.batch_stride + static_cast<long long>(kvh) * p.max_len * kHD;
   const T* vbase = static_cast<const T*>(p.v) + (p.batch0 + b) * p.batch_stride + static_cast<long long>(kvh) * p.max_len * kHD;
-  uint8_t* wbuf = attn_smem + warp * kWarpBufBytes;
-  const uint32_t wbuf_u32 = static_cast<uint32_t>(__cvta_generic_to_shared(wbuf));
-
-  const int ntiles_total = (end - start + kTileKeys - 1) / kTileKeys;
-  const int my_tiles = ntiles_total > warp ? (ntiles_total - warp + kAttnWarps - 1) / kAttnWarps : 0;
+  const uint32_t wbuf_u32 = static_cast<uint32_t>(__cvta_generic_to_shared(attn_smem + warp * kWarpBufBytes));
+  // The warps take the CTA's tiles in turn.
+  const int my_tiles = t1 - t0 > warp ? (t1 - t0 - warp + kAttnWarps - 1) / kAttnWarps : 0;
 
   auto issue_tile = [&](int i, int stage) {
-    const int key0 = start + (warp + i * kAttnWarps) * kTileKeys;
+    const int key0 = (t0 + warp + i * kAttnWarps) * kTileKeys;
     const uint32_t ks = wbuf_u32 + stage * 2 * kKvTileBytes, vs = ks + kKvTileBytes;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int unit = j * 32 + lane;  // 512 units of 16 bytes per tile
-      const int r = unit >> 4, c = unit & 15;
-      int key = key0 + r;
-      if (key > end - 1) key = end - 1;  // masked later; the address stays inside the written part of the cache
+    for (int j = 0; j < kKvTileBytes / 512; ++j) {
+      const int r = j * 2 + (lane >> 4), c = lane & 15;  // 16 units of 16 bytes per key row
+      const int key = min(key0 + r, L - 1);  // masked later; the address stays inside the written part of the cache
       cp_async_16(ks + kv_off(r, c), kbase + static_cast<long long>(key) * kHD + c * 8);
       cp_async_16(vs + kv_off(r, c), vbase + static_cast<long long>(key) * kHD + c * 8);
     }
@@ -264,22 +302,25 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_decode_kernel(AttnParams
     if (s < my_tiles) issue_tile(s, s);
     cp_async_commit();
   }
+  int stage = 0, fill = STAGES - 1;
   for (int i = 0; i < my_tiles; ++i) {
-    const int stage = i % STAGES;
-    if (i + STAGES - 1 < my_tiles) issue_tile(i + STAGES - 1, (i + STAGES - 1) % STAGES);
+    if (i + STAGES - 1 < my_tiles) issue_tile(i + STAGES - 1, fill);
+    if (++fill == STAGES) fill = 0;
     cp_async_commit();
     cp_async_wait<STAGES - 1>();
     __syncwarp();
-    const int key0 = start + (warp + i * kAttnWarps) * kTileKeys;
+    const int key0 = (t0 + warp + i * kAttnWarps) * kTileKeys;
     const uint32_t ks = wbuf_u32 + stage * 2 * kKvTileBytes, vs = ks + kKvTileBytes;
+    if (++stage == STAGES) stage = 0;
 
-    // ---- S = Q K^T for 32 keys ----
-    float s[4][4];
+    // ---- S = Q K^T for 16 keys ----
+    float s[2][4];
 #pragma unroll
-    for (int nb = 0; nb < 4; ++nb) {
-      s[nb][0] = s[nb][1] = s[nb][2] = s[nb][3] = 0.f;
+    for (int nb = 0; nb < 2; ++nb) s[nb][0] = s[nb][1] = s[nb][2] = s[nb][3] = 0.f;
 #pragma unroll
-      for (int kp = 0; kp < 4; ++kp) {
+    for (int kp = 0; kp < 4; ++kp) {
+#pragma unroll
+      for (int nb = 0; nb < 2; ++nb) {
         uint32_t r[4];
         ldmatrix_x4(r, ks + kv_off(nb * 8 + (lane & 7), kp * 4 + (lane >> 3)));
         mma_16816<T>(s[nb], qa[2 * kp], r[0], r[1]);
@@ -289,11 +330,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_decode_kernel(AttnParams
     // ---- mask, online softmax ----
     float tmax[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-    for (int nb = 0; nb < 4; ++nb) {
+    for (int nb = 0; nb < 2; ++nb) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int key = key0 + nb * 8 + colp + (e & 1);
-        const float v = key < end ? s[nb][e] * p.scale_log2 : -INFINITY;
+        const float v = key < L ? s[nb][e] * p.scale_log2 : -INFINITY;
         s[nb][e] = v;
         tmax[e >> 1] = fmaxf(tmax[e >> 1], v);
       }
@@ -310,7 +351,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_decode_kernel(AttnParams
       l_run[h] *= corr[h];
     }
 #pragma unroll
-    for (int nb = 0; nb < 4; ++nb) {
+    for (int nb = 0; nb < 2; ++nb) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float pv = exp2f(s[nb][e] - m_use[e >> 1]);
@@ -318,29 +359,29 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_decode_kernel(AttnParams
         l_run[e >> 1] += pv;
       }
     }
+    // After the first few tiles a new maximum is rare: the 64 products are skipped when every factor is one.
+    if (__any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f)) {
 #pragma unroll
-    for (int i2 = 0; i2 < 16; ++i2) {
-      o[i2][0] *= corr[0];
-      o[i2][1] *= corr[0];
-      o[i2][2] *= corr[1];
-      o[i2][3] *= corr[1];
+      for (int i2 = 0; i2 < 16; ++i2) {
+        o[i2][0] *= corr[0];
+        o[i2][1] *= corr[0];
+        o[i2][2] *= corr[1];
+        o[i2][3] *= corr[1];
+      }
     }
     // ---- O += P V ----
+    uint32_t pa[4];
+    pa[0] = Cvt<T>::pack(s[0][0], s[0][1]);
+    pa[1] = Cvt<T>::pack(s[0][2], s[0][3]);
+    pa[2] = Cvt<T>::pack(s[1][0], s[1][1]);
+    pa[3] = Cvt<T>::pack(s[1][2], s[1][3]);
 #pragma unroll
-    for (int kk = 0; kk < 2; ++kk) {
-      uint32_t pa[4];
-      pa[0] = Cvt<T>::pack(s[2 * kk][0], s[2 * kk][1]);
-      pa[1] = Cvt<T>::pack(s[2 * kk][2], s[2 * kk][3]);
-      pa[2] = Cvt<T>::pack(s[2 * kk + 1][0], s[2 * kk + 1][1]);
-      pa[3] = Cvt<T>::pack(s[2 * kk + 1][2], s[2 * kk + 1][3]);
-#pragma unroll
-      for (int dp = 0; dp < 8; ++dp) {
-        uint32_t r[4];
-        const int j = lane >> 3;
-        ldmatrix_x4_trans(r, vs + kv_off(kk * 16 + (j & 1) * 8 + (lane & 7), dp * 2 + (j >> 1)));
-        mma_16816<T>(o[2 * dp], pa, r[0], r[1]);
-        mma_16816<T>(o[2 * dp + 1], pa, r[2], r[3]);
-      }
+    for (int dp = 0; dp < 8; ++dp) {
+      uint32_t r[4];
+      const int j = lane >> 3;
+      ldmatrix_x4_trans(r, vs + kv_off((j & 1) * 8 + (lane & 7), dp * 2 + (j >> 1)));
+      mma_16816<T>(o[2 * dp], pa, r[0], r[1]);
+      mma_16816<T>(o[2 * dp + 1], pa, r[2], r[3]);
     }
     __syncwarp();  // every lane is done with this stage before the next iteration's copies overwrite it
   }
@@ -352,17 +393,20 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_decode_kernel(AttnParams
   }
   __syncthreads();  // all warps are done with their tile buffers: reuse shared memory for the merge
 
-  // ---- cross-warp merge: [warp][16 rows][128] fp32 values, then [warp][16] max and sum ----
+  // ---- merge over the warps: [warp][16 rows][128] fp32 values, [warp][16] max, [warp][16] sum, then the CTA's result
+  // in the same form with one "warp".  A warp or CTA without keys has max = -inf and contributes nothing.
   float* mo = reinterpret_cast<float*>(attn_smem);
   float* mm = mo + kAttnWarps * 16 * kHD;
   float* ml = mm + kAttnWarps * 16;
+  float* co = ml + kAttnWarps * 16;
+  float* cm = co + 16 * kHD;
+  float* cl = cm + 16;
 #pragma unroll
   for (int nb = 0; nb < 16; ++nb) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int row = row0 + (e >> 1) * 8, col = nb * 8 + colp + (e & 1);
-      mo[(warp * 16 + row) * kHD + col] = o[nb][e];
-    }
+    for (int h = 0; h < 2; ++h)
+      if (row0 + h * 8 < G)
+        *reinterpret_cast<float2*>(&mo[(warp * 16 + row0 + h * 8) * kHD + nb * 8 + colp]) = make_float2(o[nb][2 * h], o[nb][2 * h + 1]);
   }
   if ((lane & 3) == 0) {
     mm[warp * 16 + row0] = m_run[0];
@@ -372,6 +416,19 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_decode_kernel(AttnParams
   }
   __syncthreads();
   const int d = threadIdx.x;  // 128 threads = 128 dims
+  auto deliver = [&](int g, float acc, float m_tot, float l_tot) {
+    const long long hrow = static_cast<long long>(b) * p.H + h0 + g;
+    if (p.splits == 1) {
+      static_cast<T*>(p.out)[hrow * kHD + d] = to_out<T>(acc / l_tot);
+    } else {
+      float* w = p.ws + (hrow * p.splits + part / S) * kPartialStride;
+      w[d] = acc;
+      if (d == 0) {
+        w[kHD] = m_tot;
+        w[kHD + 1] = l_tot;
+      }
+    }
+  };
   for (int g = 0; g < G; ++g) {
     float m_tot = -INFINITY;
 #pragma unroll
@@ -384,23 +441,43 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_decode_kernel(AttnParams
       acc += f * mo[(w * 16 + g) * kHD + d];
       l_tot += f * ml[w * 16 + g];
     }
-    const long long hrow = static_cast<long long>(b) * p.H + h0 + g;
-    if (p.splits == 1) {
-      const float y = acc / l_tot;
-      T* dst = static_cast<T*>(p.out) + hrow * kHD + d;
-      if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-        *dst = __float2bfloat16_rn(y);
-      } else {
-        *dst = __float2half_rn(y);
-      }
+    if constexpr (S == 1) {
+      deliver(g, acc, m_tot, l_tot);
     } else {
-      float* w = p.ws + (hrow * p.splits + split) * kPartialStride;
-      w[d] = acc;
+      co[g * kHD + d] = acc;
       if (d == 0) {
-        w[kHD] = m_tot;
-        w[kHD + 1] = l_tot;
+        cm[g] = m_tot;
+        cl[g] = l_tot;
       }
     }
+  }
+  if constexpr (S > 1) {
+    // ---- merge over the cluster through distributed shared memory: CTA r takes query heads r, r + S, ... ----
+    const int rank = part % S;
+    const uint32_t co_a = static_cast<uint32_t>(__cvta_generic_to_shared(co));
+    const uint32_t cm_a = static_cast<uint32_t>(__cvta_generic_to_shared(cm)), cl_a = static_cast<uint32_t>(__cvta_generic_to_shared(cl));
+    attn_cluster_sync();
+    for (int g = rank; g < G; g += S) {
+      float m[S], l[S], v[S];
+#pragma unroll
+      for (int r = 0; r < S; ++r) {
+        m[r] = ld_cluster_f32(cm_a + g * 4, r);
+        l[r] = ld_cluster_f32(cl_a + g * 4, r);
+        v[r] = ld_cluster_f32(co_a + (g * kHD + d) * 4, r);
+      }
+      float m_tot = m[0];
+#pragma unroll
+      for (int r = 1; r < S; ++r) m_tot = fmaxf(m_tot, m[r]);
+      float acc = 0.f, l_tot = 0.f;
+#pragma unroll
+      for (int r = 0; r < S; ++r) {
+        const float f = m[r] == -INFINITY ? 0.f : exp2f(m[r] - m_tot);
+        acc += f * v[r];
+        l_tot += f * l[r];
+      }
+      deliver(g, acc, m_tot, l_tot);
+    }
+    attn_cluster_sync();  // the peers have read this CTA's part
   }
 }
 
@@ -409,6 +486,8 @@ template <typename T>
 __global__ void attn_combine_kernel(const float* ws, void* out, int splits) {
   const long long hrow = blockIdx.x;
   const int d = threadIdx.x;
+  ptx::griddep_launch_dependents();
+  ptx::griddep_wait();
   const float* w = ws + hrow * splits * kPartialStride;
   float m_tot = -INFINITY;
   for (int s = 0; s < splits; ++s) m_tot = fmaxf(m_tot, w[s * kPartialStride + kHD]);
@@ -420,54 +499,58 @@ __global__ void attn_combine_kernel(const float* ws, void* out, int splits) {
     acc += f * w[s * kPartialStride + d];
     l_tot += f * w[s * kPartialStride + kHD + 1];
   }
-  const float y = acc / l_tot;
-  T* dst = static_cast<T*>(out) + hrow * kHD + d;
-  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-    *dst = __float2bfloat16_rn(y);
-  } else {
-    *dst = __float2half_rn(y);
-  }
+  static_cast<T*>(out)[hrow * kHD + d] = to_out<T>(acc / l_tot);
 }
 
-int sm_count_model() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
-}
-
-template <typename T, int STAGES>
-cudaError_t launch_attn_stages(const AttnParams& p, cudaStream_t stream) {
-  static bool attr_done[64];
+template <typename T, int STAGES, int S>
+cudaError_t launch_attn_s(const AttnParams& p, cudaStream_t stream) {
+  static std::atomic<uint64_t> attr_done{0};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (!attr_done[dev & 63]) {
-    cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<T, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if (!(attr_done.load(std::memory_order_relaxed) >> (dev & 63) & 1)) {
+    cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<T, STAGES, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          attn_smem_bytes(STAGES));
     if (e != cudaSuccess) return e;
-    attr_done[dev & 63] = true;
+    attr_done.fetch_or(uint64_t(1) << (dev & 63), std::memory_order_relaxed);
   }
-  attn_decode_kernel<T, STAGES><<<dim3(p.splits, p.KV, p.B), kAttnThreads, attn_smem_bytes(STAGES), stream>>>(p);
-  return cudaGetLastError();
+  return launch_pdl(attn_decode_kernel<T, STAGES, S>, dim3(p.splits * S, p.KV, p.B), kAttnThreads, attn_smem_bytes(STAGES), stream, S, p);
 }
 
 template <typename T>
-cudaError_t launch_attn(const AttnParams& p, cudaStream_t stream) {
-  static const bool three_stages = [] {
-    const char* v = getenv("OOB_ATTN_STAGES");
-    return v != nullptr && v[0] == '3';
-  }();
-  cudaError_t e = three_stages ? launch_attn_stages<T, 3>(p, stream) : launch_attn_stages<T, 2>(p, stream);
-  if (e != cudaSuccess) return e;
-  if (p.splits > 1) {
-    attn_combine_kernel<T><<<p.B * p.H, kHD, 0, stream>>>(p.ws, p.out, p.splits);
-    e = cudaGetLastError();
+cudaError_t launch_attn(const AttnParams& p, int cluster, cudaStream_t stream) {
+  cudaError_t e;
+  switch (cluster) {
+    case 1: e = launch_attn_s<T, 3, 1>(p, stream); break;
+    case 2: e = launch_attn_s<T, 3, 2>(p, stream); break;
+    case 4: e = launch_attn_s<T, 3, 4>(p, stream); break;
+    default: e = launch_attn_s<T, 3, 8>(p, stream); break;
   }
+  if (e != cudaSuccess) return e;
+  if (p.splits > 1) e = launch_pdl(attn_combine_kernel<T>, dim3(p.B * p.H), kHD, 0, stream, 1, p.ws, p.out, p.splits);
   return e;
+}
+
+// CTAs of a cluster that share the keys of one (sequence, KV head).  Two CTAs fit an SM; while they do not fill the
+// machine a CTA streams as fast as its own loads in flight allow (8 ns per key), after that it gets its share of the memory
+// bandwidth (23 ns per key with 296 CTAs); starting a CTA and merging costs about as much as 110 keys.  What is
+// weighed is whole rounds of CTAs: 300 sequences in one piece each would run four of them alone in a second round.
+int attn_cluster_size(long long items, int len_bound) {
+  constexpr int kSlots = 2 * 148;
+  int best = 1;
+  double best_cost = 0;
+  for (int s = 1; s <= kMaxAttnCluster; s *= 2) {
+    if (s > 1 && len_bound < s * kTileKeys * kAttnWarps) break;
+    const long long ctas = items * s;
+    const long long waves = (ctas + kSlots - 1) / kSlots;
+    const double fill = ctas >= kSlots ? 1.0 : double(ctas) / kSlots;
+    const double ns_key = fill * 23.0 > 8.0 ? fill * 23.0 : 8.0;
+    const double cost = waves * (ns_key * len_bound / s + 110 * 23.0);
+    if (s == 1 || cost < best_cost) {
+      best = s;
+      best_cost = cost;
+    }
+  }
+  return best;
 }
 
 }  // namespace model
@@ -500,11 +583,8 @@ int oob_rope_kv_write(const oob_rope_args_t* a, void* stream) {
   long long blocks = (units + threads - 1) / threads;
   if (blocks > 148 * 16) blocks = 148 * 16;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (a->dtype == OOB_BF16)
-    rope_kv_write_kernel<__nv_bfloat16><<<static_cast<int>(blocks), threads, 0, s>>>(*a, units);
-  else
-    rope_kv_write_kernel<__half><<<static_cast<int>(blocks), threads, 0, s>>>(*a, units);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_pdl(a->dtype == OOB_BF16 ? rope_kv_write_kernel<__nv_bfloat16> : rope_kv_write_kernel<__half>,
+                                   dim3(static_cast<int>(blocks)), threads, 0, s, 1, *a, units);
   if (e != cudaSuccess) return cuda_fail(e, "rope_kv_write launch");
   return OOB_OK;
 }
@@ -520,27 +600,27 @@ int oob_silu_mul(int dtype, const void* gu, int64_t ld_gu, void* out, int rows, 
   long long blocks = (units + threads - 1) / threads;
   if (blocks > 148 * 16) blocks = 148 * 16;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dtype == OOB_BF16)
-    silu_mul_kernel<__nv_bfloat16><<<static_cast<int>(blocks), threads, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(gu), ld_gu, static_cast<__nv_bfloat16*>(out), units, F);
-  else
-    silu_mul_kernel<__half><<<static_cast<int>(blocks), threads, 0, s>>>(static_cast<const __half*>(gu), ld_gu,
-                                                                         static_cast<__half*>(out), units, F);
-  cudaError_t e = cudaGetLastError();
+  const dim3 grid(static_cast<int>(blocks));
+  const cudaError_t e =
+      dtype == OOB_BF16 ? launch_pdl(silu_mul_kernel<__nv_bfloat16>, grid, threads, 0, s, 1, static_cast<const __nv_bfloat16*>(gu),
+                                     ld_gu, static_cast<__nv_bfloat16*>(out), units, F)
+                        : launch_pdl(silu_mul_kernel<__half>, grid, threads, 0, s, 1, static_cast<const __half*>(gu), ld_gu,
+                                     static_cast<__half*>(out), units, F);
   if (e != cudaSuccess) return cuda_fail(e, "silu_mul launch");
   return OOB_OK;
 }
 
 int oob_attn_decode_auto_splits(int B, int KV, int len_bound) {
   if (B <= 0 || KV <= 0 || len_bound <= 0) return 1;
-  const int sms = 148;
-  const long long ctas = static_cast<long long>(B) * KV;
-  int s = static_cast<int>((2 * sms + ctas - 1) / ctas);  // aim at two CTAs' worth of work per SM
-  const int max_by_len = (len_bound + 127) / 128;          // at least one pass of the four warps per chunk
+  // A cluster of eight CTAs shares the keys of one (sequence, KV head) without touching memory; more CTAs are only worth
+  // the round trip of their partial results, and a second kernel, when few sequences are long.
+  const long long ctas = static_cast<long long>(B) * KV * kMaxAttnCluster;
+  long long s = (148 + ctas - 1) / ctas;
+  const int max_by_len = len_bound / (kMaxAttnCluster * 512);
   if (s > max_by_len) s = max_by_len;
   if (s > 32) s = 32;
   if (s < 1) s = 1;
-  return s;
+  return static_cast<int>(s);
 }
 
 uint64_t oob_attn_decode_workspace_bytes(int B, int H, int splits) {
@@ -584,13 +664,10 @@ int oob_attn_decode(const oob_attn_decode_args_t* a, void* stream) {
   p.max_len = a->max_len;
   p.batch0 = a->batch0;
   p.splits = splits;
-  // Keys per chunk: whole passes of the CTA (4 warps x 32 keys), covering `bound` keys.
-  int chunk = (bound + splits - 1) / splits;
-  chunk = (chunk + 127) / 128 * 128;
-  p.chunk = chunk;
   p.scale_log2 = a->scale * 1.4426950408889634f;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  cudaError_t e = a->dtype == OOB_BF16 ? launch_attn<__nv_bfloat16>(p, s) : launch_attn<__half>(p, s);
+  const int cluster = attn_cluster_size(static_cast<long long>(a->B) * a->KV * splits, (bound + splits - 1) / splits);
+  cudaError_t e = a->dtype == OOB_BF16 ? launch_attn<__nv_bfloat16>(p, cluster, s) : launch_attn<__half>(p, cluster, s);
   if (e != cudaSuccess) return cuda_fail(e, "attn_decode launch");
   return OOB_OK;
 }
