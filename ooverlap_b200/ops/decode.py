@@ -15,10 +15,7 @@ import torch
 
 from .. import _lib
 from ..utils.dtypes import dtype_code
-
-
-def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+from ..utils.stream import current_stream_ptr as _stream
 
 
 def rope_tables(max_len: int, head_dim: int, theta: float, device) -> tuple[torch.Tensor, torch.Tensor]:
@@ -106,7 +103,6 @@ def gemm_rope_kv_write(x: torch.Tensor, wqkv: torch.Tensor, B: int, T: int, head
     args.mode = _lib.GEMM_PLAIN
     fill_gemm_args(args, x, wqkv)
     args.C, args.ldc = q_out.data_ptr(), N  # C itself is not written; a valid aligned pointer keeps the checks uniform
-    args.skinny = -1
     args.epilogue = _lib.EPILOGUE_ROPE_KV
     args.epilogue_args = ctypes.cast(ctypes.pointer(r), ctypes.c_void_p)
     _lib.check(_lib.lib().oob_gemm(None, ctypes.byref(args), _stream()))

@@ -14,10 +14,7 @@ import torch
 from .. import _lib
 from ..utils.dtypes import dtype_code
 from ..utils.partition import partition
-
-
-def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+from ..utils.stream import current_stream_ptr as _stream
 
 
 def rmsnorm_reference(x: torch.Tensor, weight: torch.Tensor, eps: float,
@@ -47,7 +44,9 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, residual: 
     a.y_local = y.data_ptr()
     a.res_out_reg = -1
     a.res_out_local = residual_out.data_ptr() if residual_out is not None else None
-    _lib.check(_lib.lib().oob_fused_norm(None, _lib.NORM_LOCAL, ctypes.byref(a), max_ctas, _stream()))
+    rc = _lib.lib().oob_fused_norm(None, _lib.NORM_LOCAL, a, max_ctas, _stream())
+    if rc:
+        _lib.check(rc)
     return (y, residual_out) if residual is not None else y
 
 
