@@ -15,9 +15,10 @@ namespace oob {
 // gemv.cu
 bool gemv_supported(const GemmArgs& a);
 cudaError_t launch_gemv(const GemmArgs& a, int sms, cudaStream_t stream);
-// gemm_skinny.cu
-bool gemm_skinny_supported(const GemmArgs& a);
-cudaError_t launch_gemm_skinny(const GemmArgs& a, DeviceStatus* status, cudaStream_t stream, gemm_detail::TmapFn make_tmap);
+// gemm_cluster.cu
+bool gemm_cluster_supported(const GemmArgs& a);
+bool gemm_cluster_preferred(const GemmArgs& a);
+cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStream_t stream, gemm_detail::TmapFn make_tmap);
 
 namespace {
 
@@ -288,32 +289,51 @@ cudaError_t launch_gemm(const CommCtx& ctx, const GemmArgs& args, cudaStream_t s
   int dev = 0;
   cudaGetDevice(&dev);
   if (a.mode == kGemmPlain) {
-    // One to four rows: the CUDA-core streaming kernel.  By argument, or when the call leaves the choice open: for one
-    // row always, for two rows when the weight matrix is small (N x K up to 12 M elements), which is where it measured
-    // faster than the tensor-core paths on B200 (M = 1: 6.1 / 8.6 / 13.9 us against 10.6 / 14.3 / 17.2 us for
-    // 8192 x 1024, 1280 x 8192, 8192 x 3584; M = 2 on the two smaller ones: 8.0 / 11.7 against 10.4 / 14.3 us; from
-    // M = 4 on it loses everywhere).  OOB_GEMM_GEMV=0 switches the rule off, =1 widens it to every M <= 4.
+    // One row of a weight matrix up to 32 M elements: the CUDA-core streaming kernel.  Both sides measured on B200, M = 1: 8.0
+    // against 8.3 us for 1280 x 8192, 5.5 against 7.0 for 8192 x 1024, 13.5 against 14.1 for 8192 x 3584, but 26.8 against
+    // 22.6 for 7168 x 8192 and 49.4 against 46.7 for 16032 x 8192; from two rows on it loses (12.0 against 8.3, 7.5
+    // against 7.0).  OOB_GEMM_GEMV=0 switches the rule off, =1 widens it to every M <= 4.
     static const int gemv_env = [] {
       const char* v = getenv("OOB_GEMM_GEMV");
       return v == nullptr ? -1 : (v[0] == '1' ? 1 : 0);
     }();
     const bool gemv_by_shape =
-        gemv_env != 0 && (a.M == 1 || (a.M == 2 && static_cast<long long>(a.N) * a.K <= 12ll * 1000 * 1000));
+        gemv_env != 0 && a.M == 1 && static_cast<long long>(a.N) * a.K <= 32ll * 1000 * 1000;
     if (a.epilogue == 0 && gemv_supported(a) && ctx.emu_table == nullptr && a.c_emu_stride == 0 && a.splitk_ws == nullptr &&
         (a.gemv > 0 || (a.gemv == 0 && a.splits == 0 && a.skinny <= 0 && (gemv_env == 1 || gemv_by_shape))))
       return launch_gemv(a, a.max_ctas > 0 ? a.max_ctas : sm_count(), stream);
-    // The weight-streaming kernel (stream-K over 128-row weight tiles) is opt-in: measured on B200, inside a replayed
-    // decode step it is 2 - 12 % slower at M <= 16 than the 128x256 split-K tiles followed by the reduction kernel,
-    // and far slower from M = 32 on (every CTA re-reads its share of the activations, which then rivals the weight
-    // traffic).  OOB_GEMM_SKINNY=1 makes it the default for M <= 16.
-    static const bool skinny_env_on = [] {
+    // Few rows, or few tiles: the weight-streaming kernel.
+    static const bool cluster_env_off = [] {
       const char* v = getenv("OOB_GEMM_SKINNY");
-      return v != nullptr && v[0] == '1';
+      return v != nullptr && v[0] == '0';
     }();
-    if (a.epilogue == 0 && gemm_skinny_supported(a) && ctx.emu_table == nullptr && a.c_emu_stride == 0 && a.splitk_ws == nullptr &&
-        (a.skinny > 0 || (a.skinny == 0 && a.splits == 0 && a.M <= 16 && skinny_env_on)))
-      return launch_gemm_skinny(a, ctx.status, stream, make_tmap_cached);
-    const int splits = gemm_plan_splits(a.M, a.N, a.K, a.max_ctas, a.splits);
+    const bool cluster_auto = a.skinny == 0 && a.splits == 0 && a.pair <= 0 && a.stream_k <= 0 && a.splitk_reduce == 0 &&
+                              a.max_ctas == 0 && a.gemv <= 0 && !cluster_env_off && a.M <= kGemmClusterMaxRows &&
+                              gemm_cluster_preferred(a);
+    if ((a.skinny > 0 || cluster_auto) && gemm_cluster_supported(a) && ctx.emu_table == nullptr && a.c_emu_stride == 0 && a.splitk_ws == nullptr &&
+        a.order == nullptr && (a.epilogue == 0 || a.epilogue_args != nullptr))
+      return launch_gemm_cluster(a, ctx.status, stream, make_tmap_cached);
+    if (a.epilogue == kGemmEpilogueSwigluTile) {
+      if (ctx.emu_table != nullptr || a.c_emu_stride != 0 || a.epilogue_args == nullptr) return cudaErrorInvalidValue;
+      a.splits = 1;
+      return launch_gemm_pair(ctx, a, stream, make_tmap_cached, nullptr);
+    }
+    static const bool pair_env_off = [] {
+      const char* v = getenv("OOB_GEMM_PAIR");
+      return v != nullptr && v[0] == '0';
+    }();
+    int splits = gemm_plan_splits(a.M, a.N, a.K, a.max_ctas, a.splits);
+    // Nothing asked for and more than 128 rows: the two-SM kernel on narrow tiles, or with the SwiGLU in its epilogue, beats
+    // partial tiles through memory (250 x 8192 x 3584: 18.1 against 26.7 us).
+    if (splits > 1 && a.M > kTileM && a.splits == 0 && a.max_ctas == 0 && a.skinny == 0 && a.pair == 0 && a.splitk_reduce == 0 &&
+        a.splitk_ws == nullptr && ctx.emu_table == nullptr && a.c_emu_stride == 0 && !pair_env_off && a.epilogue <= 1) {
+      if (a.epilogue == 1 && a.epilogue_args != nullptr) {
+        a.epilogue = kGemmEpilogueSwigluTile;
+        a.splits = 1;
+        return launch_gemm_pair(ctx, a, stream, make_tmap_cached, nullptr);
+      }
+      if (a.epilogue == 0) splits = 1;
+    }
     a.splits = splits;
     if (a.epilogue != 0) {
       // The epilogue lives in the kernel that sums the splits: the problem has to be one that is split.
@@ -339,10 +359,6 @@ cudaError_t launch_gemm(const CommCtx& ctx, const GemmArgs& args, cudaStream_t s
       a.splitk_defer = 1;
     // Large problems go to the two-SM kernel: same tile count per SM, two thirds of the operand traffic.
     const bool pair_ok = splits == 1 && ctx.emu_table == nullptr && a.c_emu_stride == 0 && (a.max_ctas == 0 || a.max_ctas >= 2);
-    static const bool pair_env_off = [] {
-      const char* v = getenv("OOB_GEMM_PAIR");
-      return v != nullptr && v[0] == '0';
-    }();
     const bool pair_auto = a.M > kTileM && !pair_env_off;
     if (pair_ok && (a.pair > 0 || (a.pair == 0 && pair_auto))) {
       e = launch_gemm_pair(ctx, a, stream, make_tmap_cached, nullptr);

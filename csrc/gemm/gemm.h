@@ -37,6 +37,9 @@ enum TraceSlot : int {
 // All matrices are 16-bit (fp16 or bf16), A is [M, K] row-major with leading
 // dimension lda, B is [N, K] row-major (the layout of a torch Linear weight)
 // with leading dimension ldb, C is [M, N] row-major.
+constexpr int kGemmEpilogueSwigluTile = 3;
+constexpr int kGemmClusterMaxRows = 4096;  // rows the weight-streaming kernel (gemm_cluster.cu) accepts
+
 struct GemmArgs {
   int mode;
   int fmt;  // 0 = fp16, 1 = bf16
@@ -65,12 +68,14 @@ struct GemmArgs {
   // (set by launch_gemm; callers ask through splitk_reduce: 0 / 1 = second kernel, -1 = sum inside the GEMM kernel).
   int splitk_defer;
   int splitk_reduce;
-  // Plain mode, split problems only: an elementwise op applied by the kernel that sums the splits (see
-  // splitk_epilogues.cuh).  epilogue_args is a HOST pointer to the op's argument block.
-  // Plain mode, M <= 4: 1 = the CUDA-core streaming kernel (gemv.cu); 0 = by shape (M = 1, and M = 2 with a small
-  // weight matrix; OOB_GEMM_GEMV=1 widens that to every M <= 4, =0 switches it off); -1 = never.
+  // Plain mode: an elementwise op applied to the fp32 sums, for split problems (1, 2: by gemm_cluster.cu up to 256 rows, else
+  // by the kernel that sums the splits, splitk_epilogues.cuh) or any (3: gemm_cluster.cu or the two-SM kernel).
+  // epilogue_args is a HOST pointer to the op's argument block.
+  // Plain mode, M <= 4: 1 = the CUDA-core streaming kernel (gemv.cu); 0 = by shape (M = 1 with a weight matrix of up to
+  // 32 M elements; OOB_GEMM_GEMV=1 widens that to every M <= 4, =0 switches it off); -1 = never.
   int gemv;
-  int epilogue;               // 0 = none, 1 = SwiGLU (oob_gemm_epilogue_swiglu_t), 2 = RoPE + KV write (oob_rope_args_t)
+  int epilogue;               // 0 = none, 1 = SwiGLU (oob_gemm_epilogue_swiglu_t), 2 = RoPE + KV write (oob_rope_args_t),
+                              // 3 = kGemmEpilogueSwigluTile (oob_gemm_epilogue_swiglu_t)
   const void* epilogue_args;
   // 0 = the two-SM kernel (256x256 tiles on CTA pairs) when the shape suits it, 1 = always when possible,
   // -1 = never (the one-SM kernel with 128x256 tiles).  Applies to the plain GEMM and to the fused modes.
@@ -84,8 +89,7 @@ struct GemmArgs {
   // was complete in this GPU's memory (fused AR / RS: when it was published to the rank that reduces it),
   // [1] = pair << 32 | index of the tile in that pair's own sequence.  Sorting by [0] gives the completion order.
   unsigned long long* order;
-  // Plain mode, M <= 128: 1 = the weight-streaming kernel (gemm_skinny.cu), 0 / -1 = the tiled kernels (0 follows
-  // OOB_GEMM_SKINNY=1 for M <= 16).
+  // Plain mode, M <= kGemmClusterMaxRows: 1 = the weight-streaming kernel (gemm_cluster.cu), 0 = by shape, -1 = the tiled kernels.
   int skinny;
 
   // Fused modes

@@ -1,0 +1,706 @@
+// Weight-streaming tcgen05 GEMM for few rows: C[M, N] = A[M, K] * B[N, K]^T is computed as C^T = B * A^T, so the WEIGHT rows
+// fill the 128-row dimension of the tensor-core instruction and the tokens are its N dimension (16 .. 256).  This is the GEMM
+// of a decode step or of a short mixed batch: what bounds it is the time to read B once, plus whatever happens before the
+// first and after the last byte.
+//
+// A CTA goes through about one 64-element K block per 0.24 us (the chain load - multiply - release of one issuing thread each),
+// so that neither few CTAs nor long K ranges reach the memory's rate.  128-row weight tiles are therefore computed by S CTAs,
+// each over 1/S of K; a cost model on the host picks S and the token blocks.
+//
+// Split over K inside a thread-block cluster (S = 1 .. 8).  When a CTA has its partial sums it drains them from TMEM into its
+// own shared memory (the pipeline buffers, idle by then) as [token][128] fp32; after one cluster barrier each CTA reads its share
+// of the tokens from all S copies through distributed shared memory, adds them in rank order (deterministic) and writes
+// the 16-bit result.  Nothing goes through global memory and no second kernel has to be launched.
+//
+// PAIR: two CTAs of the cluster form a tensor-core pair (cta_group::2) on 256 weight rows.  Each stages its own 128 weight
+// rows and HALF of the tokens, and keeps the sums of its own rows.  From about 128 tokens on the activations, which every
+// weight tile reads again, rival the weights on the way from L2 to the SMs; a pair halves them.
+//
+// Epilogues applied to the fp32 sums before the only rounding:
+//   SwiGLU     a tile is 64 gate rows + 64 up rows of the [gate | up] weight; out = silu(gate) * up
+//   RoPE + KV  query and key heads are rotated, queries go to q_out, keys and values into the layer's cache
+//
+// Measured on B200, bf16, in a chain of launches (before: fp32 partial tiles through memory and a second kernel that sums
+// them): 16 x 7168 x 8192 22.6 us (26.5), 16 x 8192 x 3584 14.1 (18.2), 8 x 8192 x 1024 7.0 (10.6), 8 x 1280 x 8192 8.3 (14.3),
+// 64 x 7168 x 8192 24.5 (29.6), 128 x 4096 x 4096 13.2, 512 x 1280 x 8192 17.4 (21.6).
+//
+// Roles: warp 0 TMA producer, warp 1 MMA issuer (one thread each), warps 2-5 drain TMEM; all six warps take part in the
+// reduction.  A cluster handles tiles c, c + G, ... one after the other; normally the grid covers all tiles, a CTA
+// budget (max_ctas) makes G smaller.  All waits are bounded, and a CTA that gives up still meets its cluster's barriers.
+//
+// Capability parity with the reference: its stream-K GEMM instances (src/gemm/gemm_with_signal_sm90.h:238-292) and the
+// small-M end of its plain-GEMM dispatch table (src/gemm/gemm_plain_sm90_dispatch.h:19-46).
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include <atomic>
+
+#include "../api/oob.h"
+#include "../api/oob_model.h"
+#include "gemm_kernel.cuh"
+#include "gemm_pair.h"
+
+namespace oob {
+namespace gemm_cluster {
+
+using namespace gemm_detail;
+
+constexpr int kRowsW = 128;                  // weight rows of a CTA (the instruction's M)
+constexpr int kRowBytes = kTileK * 2;        // 128: one row of a stage
+constexpr int kMaxTokens = 256;              // per instruction (its N)
+constexpr int kMaxTileTokens = 384;          // per tile: what its fp32 sums leave of an SM's shared memory; more rows are cut into blocks
+constexpr int kThreadsC = 192;
+constexpr int kMaxStagesC = 12;
+constexpr int kMaxCluster = 8;               // portable cluster size
+constexpr int kCtlBytes = 256;
+constexpr int kSmemLimit = 227 * 1024;
+
+enum { kEpiPlain = 0, kEpiSwiglu = 1, kEpiRopeKv = 2 };
+
+struct CtlC {
+  uint64_t full[kMaxStagesC];
+  uint64_t empty[kMaxStagesC];
+  uint64_t tmem_full;
+  uint32_t tmem_base;
+  int abort;
+};
+static_assert(sizeof(CtlC) <= kCtlBytes, "control block");
+
+struct ParamsC {
+  int M, N, Mp;  // Mp: tokens of a tile = n_mma * nj
+  int n_mma, nj;  // instructions per K step and their N, a multiple of 16
+  int m_blocks;  // token blocks; tile t is block t % m_blocks of weight tile t / m_blocks
+  int F;         // SwiGLU: gate rows (N = 2F)
+  void* C;
+  int ldc;
+  int num_kb, num_tiles, clusters;
+  int S;  // CTAs (pairs) that share the K range of a tile
+  int stages, stage_bytes, work_bytes;  // work_bytes: pipeline buffers or partial sums, whichever is larger
+  int smem_bytes;
+  uint32_t tmem_cols;
+  bool vec_ok;  // 8-byte stores into C are aligned
+  oob_rope_args_t rope;
+};
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// The cta_group::2 forms.  A load goes into THIS CTA's shared memory and counts its bytes on the leader's barrier.
+__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tmap, uint32_t bar_cluster_addr, int32_t x, int32_t y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      :
+      : "r"(ptx::smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar_cluster_addr), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "}\n"
+      :
+      : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// Arrives on the barrier at this offset in every CTA of `mask` once all MMAs issued so far are complete.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t mask) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(ptx::smem_u32(bar)),
+      "h"(mask)
+      : "memory");
+}
+
+template <typename T>
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  if constexpr (PackTraits<T>::kDType == kBF16) {
+    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<uint32_t*>(&h);
+  } else {
+    __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<uint32_t*>(&h);
+  }
+}
+
+// Writes token `m`, output columns n .. n + 3 (SwiGLU: `v` gate sums, `u` up sums).
+template <typename T, int EPI>
+__device__ __forceinline__ void emit(const ParamsC& p, int m, int n, const float4& v, const float4& u, long long pos_base) {
+  if constexpr (EPI == kEpiSwiglu) {
+    if (n >= p.F) return;  // F % 8 == 0: the four columns are in or out together
+    *reinterpret_cast<uint2*>(static_cast<T*>(p.C) + size_t(m) * p.ldc + n) =
+        make_uint2(pack2<T>(swiglu_f32(v.x, u.x), swiglu_f32(v.y, u.y)), pack2<T>(swiglu_f32(v.z, u.z), swiglu_f32(v.w, u.w)));
+  } else if constexpr (EPI == kEpiRopeKv) {
+    const oob_rope_args_t& a = p.rope;
+    if (n >= p.N) return;  // N is a multiple of 8
+    const int hh = n / a.hd, c = n - hh * a.hd;
+    const int b = m / a.T, t = m - b * a.T;
+    long long pos = pos_base + t;
+    if (pos < 0) pos = 0;
+    if (pos > a.max_len - 1) pos = a.max_len - 1;  // the host checks the range; never index outside the tables / cache
+    float4 x = v;
+    if (hh < a.H + a.KV) {
+      const float2 cs = *reinterpret_cast<const float2*>(a.cos_table + pos * (a.hd / 2) + c / 2);
+      const float2 sn = *reinterpret_cast<const float2*>(a.sin_table + pos * (a.hd / 2) + c / 2);
+      x = make_float4(v.x * cs.x - v.y * sn.x, v.x * sn.x + v.y * cs.x, v.z * cs.y - v.w * sn.y, v.z * sn.y + v.w * cs.y);
+    }
+    T* dst;
+    if (hh < a.H) {
+      dst = static_cast<T*>(a.q_out) + (static_cast<long long>(m) * a.H + hh) * a.hd + c;
+    } else {
+      const int kvh = hh < a.H + a.KV ? hh - a.H : hh - a.H - a.KV;
+      T* cache = static_cast<T*>(hh < a.H + a.KV ? a.k_cache : a.v_cache);
+      dst = cache + (a.batch0 + b) * a.cache_batch_stride + (static_cast<long long>(kvh) * a.max_len + pos) * a.hd + c;
+    }
+    *reinterpret_cast<uint2*>(dst) = make_uint2(pack2<T>(x.x, x.y), pack2<T>(x.z, x.w));
+  } else {
+    T* dst = static_cast<T*>(p.C) + size_t(m) * p.ldc + n;
+    if (p.vec_ok && n + 4 <= p.N) {
+      *reinterpret_cast<uint2*>(dst) = make_uint2(pack2<T>(v.x, v.y), pack2<T>(v.z, v.w));
+    } else {
+      const float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (n + i < p.N) dst[i] = PackTraits<T>::from_float(f[i]);
+    }
+  }
+}
+
+// Sums the S partial copies of this CTA's share of a tile and writes them.  A unit is four output columns of a token; the
+// units are dealt out over the CTAs of the cluster, then over the threads, and TB units x S copies of independent loads are
+// in flight per thread.  `n_first`: first output column of the tile.
+template <typename T, int EPI, int S, bool PAIR>
+__device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base, int rank, int m_first, int n_first, int rows,
+                                            long long pos_base) {
+  constexpr int kParts = EPI == kEpiSwiglu ? 2 : 1;  // gate and up columns
+  constexpr int TB = S * kParts >= 8 ? 1 : (S * kParts >= 4 ? 2 : 4);
+  uint32_t base[S];
+#pragma unroll
+  for (int r = 0; r < S; ++r) base[r] = S == 1 ? smem_base : map_to_cta(smem_base, PAIR ? r * 2 + (cluster_ctarank() & 1) : r);
+  constexpr int upt = kRowsW / 4 / kParts;  // units of a token
+  const int units = rows * upt;
+  const int u1 = units * (rank + 1) / S;
+  for (int u0 = units * rank / S + int(threadIdx.x); u0 < u1; u0 += kThreadsC * TB) {
+    float4 v[TB][kParts][S];
+    int m[TB], c[TB];
+#pragma unroll
+    for (int i = 0; i < TB; ++i) {
+      const int u = u0 + i * kThreadsC < u1 ? u0 + i * kThreadsC : u0;  // past the end: re-read a live unit, result unused
+      m[i] = u / upt;
+      c[i] = (u - m[i] * upt) * 4;
+#pragma unroll
+      for (int h = 0; h < kParts; ++h)
+#pragma unroll
+        for (int r = 0; r < S; ++r) v[i][h][r] = ld_cluster_f4(base[r] + uint32_t(m[i] * kRowsW + h * (kRowsW / 2) + c[i]) * 4u);
+    }
+#pragma unroll
+    for (int i = 0; i < TB; ++i) {
+      float4 s[kParts];
+#pragma unroll
+      for (int h = 0; h < kParts; ++h) {
+        s[h] = v[i][h][0];
+#pragma unroll
+        for (int r = 1; r < S; ++r) {
+          s[h].x += v[i][h][r].x;
+          s[h].y += v[i][h][r].y;
+          s[h].z += v[i][h][r].z;
+          s[h].w += v[i][h][r].w;
+        }
+      }
+      if (u0 + i * kThreadsC < u1) emit<T, EPI>(p, m_first + m[i], n_first + c[i], s[0], s[kParts - 1], pos_base);
+    }
+  }
+}
+
+template <typename T, int EPI, bool PAIR>
+__global__ void __launch_bounds__(kThreadsC)
+    gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
+                        const __grid_constant__ ParamsC p, DeviceStatus* status) {
+  constexpr int FMT = PackTraits<T>::kDType == kBF16 ? 1 : 0;
+  extern __shared__ uint8_t smem_raw[];
+  // The same offset in every CTA of the cluster (same kernel, same dynamic shared memory base).
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  CtlC* ctl = reinterpret_cast<CtlC*>(smem + p.work_bytes);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int P = PAIR ? 2 : 1;
+  const int S = p.S;
+  const int cluster = blockIdx.x / (S * P), in_cluster = blockIdx.x - cluster * (S * P);
+  const int rank = in_cluster / P;                    // share of the K range
+  const int member = PAIR ? (in_cluster & 1) : 0;      // CTA of the pair: 0 = leader
+  const int kb0 = static_cast<int>(static_cast<long long>(p.num_kb) * rank / S);
+  const int kb1 = static_cast<int>(static_cast<long long>(p.num_kb) * (rank + 1) / S);
+
+  if (threadIdx.x == 0) {
+    ptx::prefetch_tmap(&tmap_w);
+    ptx::prefetch_tmap(&tmap_x);
+    for (int s = 0; s < p.stages; ++s) {
+      ptx::mbar_init(&ctl->full[s], 1);
+      ptx::mbar_init(&ctl->empty[s], 1);
+    }
+    ptx::mbar_init(&ctl->tmem_full, 1);
+    ctl->abort = 0;
+    ptx::mbar_fence_init();
+  }
+  if constexpr (PAIR) {
+    __syncthreads();
+    cluster_sync();  // both CTAs' barriers exist before anything can signal them
+    if (warp == 1) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ptx::smem_u32(&ctl->tmem_base)),
+                   "r"(p.tmem_cols)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+  } else if (warp == 1) {
+    ptx::tmem_alloc(&ctl->tmem_base, p.tmem_cols);
+    ptx::tmem_relinquish();
+  }
+  ptx::tc_fence_before_sync();
+  __syncthreads();
+  if constexpr (PAIR) cluster_sync();  // both CTAs hold their TMEM before the first MMA writes into it
+  ptx::tc_fence_after_sync();
+  const uint32_t tmem_base = ctl->tmem_base;
+  volatile int* abort = &ctl->abort;
+  // This CTA holds its TMEM: the next kernel may be set up beside it.  Everything below touches memory that earlier
+  // kernels wrote or still read.
+  ptx::griddep_launch_dependents();
+  ptx::griddep_wait();
+  long long pos_base = 0;
+  if constexpr (EPI == kEpiRopeKv) pos_base = p.rope.pos_dev != nullptr ? *p.rope.pos_dev : static_cast<long long>(p.rope.pos0);
+
+  int stage = 0;          // producer's / MMA issuer's position in the ring, carried from tile to tile
+  uint32_t phase = 0;
+  uint32_t tile_phase = 0;
+  constexpr int w_bytes = kRowsW * kRowBytes;
+  for (int t = cluster; t < p.num_tiles; t += p.clusters, tile_phase ^= 1) {
+    const int wide_tile = t / p.m_blocks, m_first = (t - wide_tile * p.m_blocks) * p.Mp;
+    const int tile = wide_tile * P + member;  // this CTA's 128 weight rows
+    const int w_row = EPI == kEpiSwiglu ? tile * (kRowsW / 2) : tile * kRowsW;
+    const int rows = min(p.Mp, p.M - m_first);
+    if (warp == 0) {
+      if (ptx::elect_one()) {
+        // ------------------------- TMA producer -------------------------
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!ptx::mbar_wait(&ctl->empty[stage], phase ^ 1, abort)) break;
+          uint8_t* sw = smem + stage * p.stage_bytes;
+          if constexpr (PAIR) {
+            const uint32_t full = map_to_cta(ptx::smem_u32(&ctl->full[stage]), in_cluster & ~1);
+            if (member == 0) ptx::mbar_arrive_expect_tx(&ctl->full[stage], 2 * p.stage_bytes);
+            if constexpr (EPI == kEpiSwiglu) {
+              tma_load_2d_pair(sw, &tmap_w, full, kb * kTileK, w_row);
+              tma_load_2d_pair(sw + w_bytes / 2, &tmap_w, full, kb * kTileK, p.F + w_row);
+            } else {
+              tma_load_2d_pair(sw, &tmap_w, full, kb * kTileK, w_row);
+            }
+            for (int j = 0; j < p.n_mma; ++j)
+              tma_load_2d_pair(sw + w_bytes + j * (p.nj / 2) * kRowBytes, &tmap_x, full, kb * kTileK,
+                               m_first + j * p.nj + member * (p.nj / 2));
+            if (++stage == p.stages) {
+              stage = 0;
+              phase ^= 1;
+            }
+            continue;
+          }
+          ptx::mbar_arrive_expect_tx(&ctl->full[stage], p.stage_bytes);
+          if constexpr (EPI == kEpiSwiglu) {
+            ptx::tma_load_2d(sw, &tmap_w, &ctl->full[stage], kb * kTileK, w_row);
+            ptx::tma_load_2d(sw + w_bytes / 2, &tmap_w, &ctl->full[stage], kb * kTileK, p.F + w_row);
+          } else {
+            ptx::tma_load_2d(sw, &tmap_w, &ctl->full[stage], kb * kTileK, w_row);
+          }
+          for (int j = 0; j < p.n_mma; ++j)
+            ptx::tma_load_2d(sw + w_bytes + j * p.nj * kRowBytes, &tmap_x, &ctl->full[stage], kb * kTileK, m_first + j * p.nj);
+          if (++stage == p.stages) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+    } else if (warp == 1) {
+      if (member == 0 && ptx::elect_one()) {
+        // ------------------------- MMA issuer (of the pair: the leader's) ---------------------------
+        const uint32_t idesc = ptx::umma_idesc_f16(FMT, P * kRowsW, p.nj);
+        [[maybe_unused]] const uint16_t mask = static_cast<uint16_t>(3u << in_cluster);  // both CTAs of the pair
+        bool ok = true;
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!ptx::mbar_wait(&ctl->full[stage], phase, abort)) {
+            ok = false;
+            break;
+          }
+          ptx::tc_fence_after_sync();
+          const uint32_t sw = ptx::smem_u32(smem + stage * p.stage_bytes);
+          const uint64_t da = ptx::umma_desc_kmajor_sw128(sw);
+          for (int j = 0; j < p.n_mma; ++j) {
+            const uint64_t db = ptx::umma_desc_kmajor_sw128(sw + w_bytes + j * (p.nj / P) * kRowBytes);
+#pragma unroll
+            for (int k = 0; k < kTileK / 16; ++k) {
+              const uint32_t d_tmem = tmem_base + j * p.nj;
+              const uint32_t add = (kb > kb0 || k > 0) ? 1u : 0u;
+              if constexpr (PAIR) {
+                umma_f16_pair(d_tmem, da + uint64_t(k * 2), db + uint64_t(k * 2), idesc, add);
+              } else {
+                ptx::umma_f16(d_tmem, da + uint64_t(k * 2), db + uint64_t(k * 2), idesc, add);
+              }
+            }
+          }
+          if constexpr (PAIR) {
+            umma_commit_pair(&ctl->empty[stage], mask);
+          } else {
+            ptx::umma_commit(&ctl->empty[stage]);
+          }
+          if (++stage == p.stages) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+        if (ok) {
+          if constexpr (PAIR) {
+            umma_commit_pair(&ctl->tmem_full, mask);
+          } else {
+            ptx::umma_commit(&ctl->tmem_full);
+          }
+        }
+      }
+    } else {
+      // ------------------- TMEM -> own shared memory, [token][128] fp32 -------------------
+      const int q = warp & 3;  // TMEM lane quadrant this warp may read: weight rows q * 32 ..
+      if (ptx::mbar_wait(&ctl->tmem_full, tile_phase, abort)) {
+        ptx::tc_fence_after_sync();
+        const uint32_t t_addr = tmem_base + (uint32_t(q * 32) << 16);
+        float* dst = reinterpret_cast<float*>(smem) + q * 32 + lane;
+        for (int c = 0; c * 16 < rows; ++c) {
+          uint32_t r[16];
+          ptx::tmem_ld_32x32b_x16(t_addr + c * 16, r);
+          ptx::tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) dst[(c * 16 + j) * kRowsW] = __uint_as_float(r[j]);
+        }
+      }
+    }
+    __syncwarp();
+    ptx::tc_fence_before_sync();
+    if (S * P > 1) {
+      cluster_sync();
+    } else {
+      __syncthreads();
+    }
+    const uint32_t own = ptx::smem_u32(smem);
+#define OOB_REDUCE(SS) \
+  case SS: reduce_tile<T, EPI, SS, PAIR>(p, own, rank, m_first, w_row, rows, pos_base); break;
+    switch (S) {
+      OOB_REDUCE(1) OOB_REDUCE(2) OOB_REDUCE(3) OOB_REDUCE(4)
+      default:
+        if constexpr (!PAIR) {
+          switch (S) { OOB_REDUCE(5) OOB_REDUCE(6) OOB_REDUCE(7) OOB_REDUCE(8) }
+        }
+    }
+#undef OOB_REDUCE
+    // Nobody reads this CTA's copy any more: the buffers belong to the pipeline again (or to the next kernel).
+    ptx::fence_proxy_async_all();
+    __syncwarp();
+    if (S * P > 1) {
+      cluster_sync();
+    } else {
+      __syncthreads();
+    }
+    ptx::tc_fence_after_sync();
+  }
+
+  // ---- teardown -----------------------------------------------------------
+  if (*abort != 0) {
+    if (threadIdx.x == 0) {
+      gemm_report(status, 0, kDevTimeoutMbarrier, 95);
+      const uint64_t t0 = ptx::globaltimer_ns();
+      while (ptx::globaltimer_ns() - t0 < 200000) __nanosleep(1000);  // copies in flight land before smem is released
+    }
+  }
+  __syncthreads();
+  if (warp == 1) {
+    ptx::tc_fence_after_sync();
+    if constexpr (PAIR) {
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(p.tmem_cols) : "memory");
+    } else {
+      ptx::tmem_dealloc(tmem_base, p.tmem_cols);
+    }
+  }
+}
+
+template <typename T, int EPI, bool PAIR>
+cudaError_t launch_pair(const GemmArgs& a, ParamsC& p, DeviceStatus* status, cudaStream_t stream, TmapFn make_tmap) {
+  auto kernel = gemm_cluster_kernel<T, EPI, PAIR>;
+  const int size = PAIR ? 2 * p.S : p.S;  // CTAs of a cluster
+  static std::atomic<uint64_t> attr_set_mask{0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!(attr_set_mask.load(std::memory_order_relaxed) >> (dev & 63) & 1)) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+    if (e != cudaSuccess) return e;
+    attr_set_mask.fetch_or(uint64_t(1) << (dev & 63), std::memory_order_relaxed);
+  }
+  p.clusters = p.num_tiles;
+  if (a.max_ctas > 0 && p.clusters > a.max_ctas / size) p.clusters = a.max_ctas / size;
+  if (p.clusters < 1) p.clusters = 1;
+  CUtensorMap tw, tx;
+  if (!make_tmap(&tw, a.B, a.N, a.K, a.ldb, EPI == kEpiSwiglu ? kRowsW / 2 : kRowsW)) return cudaErrorInvalidValue;
+  if (!make_tmap(&tx, a.A, a.M, a.K, a.lda, PAIR ? p.nj / 2 : p.nj)) return cudaErrorInvalidValue;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(p.clusters * size);
+  cfg.blockDim = dim3(kThreadsC);
+  cfg.dynamicSmemBytes = p.smem_bytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = size;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = size > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, tw, tx, p, status);
+}
+
+template <typename T, int EPI>
+cudaError_t launch_epi(const GemmArgs& a, ParamsC& p, bool pair, DeviceStatus* status, cudaStream_t stream, TmapFn make_tmap) {
+  return pair ? launch_pair<T, EPI, true>(a, p, status, stream, make_tmap) : launch_pair<T, EPI, false>(a, p, status, stream, make_tmap);
+}
+
+template <typename T>
+cudaError_t launch_fmt(const GemmArgs& a, ParamsC& p, bool pair, DeviceStatus* status, cudaStream_t stream, TmapFn make_tmap) {
+  switch (a.epilogue) {
+    case kEpiSwiglu:
+    case kGemmEpilogueSwigluTile: return launch_epi<T, kEpiSwiglu>(a, p, pair, status, stream, make_tmap);
+    case kEpiRopeKv: return launch_epi<T, kEpiRopeKv>(a, p, pair, status, stream, make_tmap);
+    default: return launch_epi<T, kEpiPlain>(a, p, pair, status, stream, make_tmap);
+  }
+}
+
+}  // namespace gemm_cluster
+
+namespace gemm_cluster {
+
+// How a problem is cut: token blocks, pairs, K splits.
+struct PlanC {
+  int m_blocks, n_mma, nj;
+  bool pair;
+  int S;
+  int stages, smem, per_sm;  // pipeline stages, shared memory of a CTA, CTAs that share an SM
+};
+
+// Tokens of a tile when M rows are cut into `blocks`: n_mma instructions of nj.
+void token_tile(int M, int blocks, PlanC* pl) {
+  const int rows = (M + blocks - 1) / blocks;
+  pl->n_mma = (rows + kMaxTokens - 1) / kMaxTokens;
+  pl->nj = ((rows + pl->n_mma - 1) / pl->n_mma + 15) / 16 * 16;
+  pl->m_blocks = (M + pl->n_mma * pl->nj - 1) / (pl->n_mma * pl->nj);
+}
+
+int tile_count(int N, const PlanC& pl) {
+  const int wtiles = (N + kRowsW - 1) / kRowsW;  // SwiGLU too: N / 2 columns in steps of 64
+  return (pl.pair ? (wtiles + 1) / 2 : wtiles) * pl.m_blocks;
+}
+
+uint32_t tmem_columns(int Mp) {
+  uint32_t cols = 32;
+  while (cols < uint32_t(Mp)) cols <<= 1;
+  return cols;
+}
+
+// Shared memory: as many stages as fit when the CTAs of the launch are spread over the SMs; fails when the work of one CTA
+// alone does not fit.
+bool size_cta(int N, int num_kb, int sms, PlanC* pl) {
+  const int P = pl->pair ? 2 : 1, Mp = pl->n_mma * pl->nj;
+  const int stage_bytes = (kRowsW + Mp / P) * kRowBytes;
+  const int fixed = 1024 + kCtlBytes;
+  const int partial = Mp * kRowsW * 4 + fixed;
+  const int kb_per = (num_kb + pl->S - 1) / pl->S;
+  const int tmem = int(tmem_columns(Mp));
+  // A CTA takes at least the share of an SM's shared memory that its TMEM columns are of the 512 (456 bytes a column; the
+  // other TMEM kernels of this library take all of both).  CTAs that fit an SM then always find their columns free:
+  // were one to wait for columns while its cluster waits for it, two clusters could wait for each other.
+  const int least = tmem * 456 < kSmemLimit ? tmem * 456 : kSmemLimit;
+  const int ctas = tile_count(N, *pl) * P * pl->S;
+  int k = (ctas + sms - 1) / sms;
+  const int most = 512 / tmem < 4 ? 512 / tmem : 4;
+  if (k > most) k = most;
+  for (; k >= 1; --k) {
+    const int share = 228 * 1024 / k - 1024;
+    const int budget = share < kSmemLimit ? share : kSmemLimit;
+    int stages = (budget - fixed) / stage_bytes;
+    if (stages > kMaxStagesC) stages = kMaxStagesC;
+    if (stages > kb_per) stages = kb_per;
+    if (stages < 2 && stages < kb_per && k > 1) continue;
+    if (stages < 1) stages = 1;
+    int smem = stages * stage_bytes + fixed;
+    if (smem < partial) smem = partial;
+    if (smem < least) smem = least;
+    if (smem > kSmemLimit || k * (smem + 1024) > 228 * 1024) continue;
+    pl->stages = stages;
+    pl->smem = smem;
+    pl->per_sm = k;
+    return true;
+  }
+  return false;
+}
+
+// Clusters of `size` CTAs that run at once with `per_sm` CTAs on an SM.  A cluster lives in one GPC (about 18 SMs on this
+// part, some have fewer).
+int cluster_slots(int sms, int size, int per_sm) {
+  if (size <= 2) return sms * per_sm / size;
+  if (size > 4 && per_sm == 1) return size == 8 ? 12 : 16;
+  return 8 * (18 * per_sm / size);
+}
+
+// Microseconds a plan takes, fitted to sweeps on B200: rounds of clusters, each as long as its K blocks at the pace of one
+// CTA or of the tensor cores of an SM (2 x tokens cycles a block), at the memory's rate for the weights or at L2's for all
+// operands, whichever is slowest; then draining the sums, reading the other CTAs' sums, and the fixed cost of a launch.
+double plan_cost(int N, int num_kb, int sms, const PlanC& pl) {
+  const int P = pl.pair ? 2 : 1, Mp = pl.n_mma * pl.nj, size = P * pl.S;
+  const int clusters = tile_count(N, pl), slots = cluster_slots(sms, size, pl.per_sm);
+  const int rounds = (clusters + slots - 1) / slots;
+  const double live = double(clusters < slots ? clusters : slots) * size;  // CTAs at once
+  const double share = live > sms ? live / sms : 1.0;
+  const double kb = double((num_kb + pl.S - 1) / pl.S);
+  const double w = kRowsW * kRowBytes, x = double(Mp) / P * kRowBytes;
+  double t = kb * (0.235 + 0.0002 * Mp);
+  const double mma = share * kb * 2.0 * Mp / 1850.0, l2 = live * kb * (w + x) / 11.5e6, hbm = live * kb * w / pl.m_blocks / 6.4e6;
+  if (mma > t) t = mma;
+  if (l2 > t) t = l2;
+  if (hbm > t) t = hbm;
+  t += 0.015 * Mp + live * Mp * kRowsW * 4.0 * (pl.S - 1) / pl.S / 3.0e6;
+  return rounds * t + (rounds - 1) * 2.0 + (size > 1 ? 3.8 : 3.4) + 0.08 * (pl.S - 1);
+}
+
+// The cheapest cut of a problem.  `fix_s` > 0 fixes the K split, `pair` is as in GemmArgs.
+bool plan(int M, int N, int K, int sms, int pair, int fix_s, PlanC* out, double* cost) {
+  const int num_kb = (K + kTileK - 1) / kTileK;
+  if (N <= kRowsW) pair = -1;  // one weight tile is no pair
+  bool found = false;
+  int last = 0;
+  for (int blocks = (M + kMaxTileTokens - 1) / kMaxTileTokens; blocks <= (M + 127) / 128; ++blocks) {
+    PlanC pl{};
+    token_tile(M, blocks, &pl);
+    const int Mp = pl.n_mma * pl.nj;
+    if (Mp == last) continue;
+    last = Mp;
+    for (int two = 0; two < 2; ++two) {
+      pl.pair = two != 0;
+      if (two ? pair < 0 || (pair == 0 && Mp <= 128) : pair > 0) continue;
+      for (pl.S = 1; pl.S <= kMaxCluster / (two ? 2 : 1); ++pl.S) {
+        if (fix_s > 0 ? pl.S != fix_s : (num_kb < 4 * pl.S && pl.S > 1)) continue;
+        if (!size_cta(N, num_kb, sms, &pl)) continue;
+        const double c = plan_cost(N, num_kb, sms, pl);
+        if (!found || c < *cost) {
+          found = true;
+          *out = pl;
+          *cost = c;
+        }
+      }
+    }
+  }
+  return found;
+}
+
+// Plans depend on sizes alone; the last ones of a thread are kept (a model's layers repeat a handful of shapes).
+struct Planned {
+  int M, N, K, flags;
+  bool ok;
+  PlanC pl;
+  double cost;
+};
+const Planned& planned(int M, int N, int K, int pair, int fix_s) {
+  static thread_local Planned cache[64];
+  const int flags = 1 | (pair > 0 ? 2 : pair < 0 ? 1 : 0) << 1 | fix_s << 3;
+  Planned& c = cache[(static_cast<unsigned>(M) * 2654435761u ^ static_cast<unsigned>(N) * 40503u ^ static_cast<unsigned>(K) * 97u ^
+                      static_cast<unsigned>(flags) * 7u) >> 8 & 63u];
+  if (c.M != M || c.N != N || c.K != K || c.flags != flags) {
+    c.M = M;
+    c.N = N;
+    c.K = K;
+    c.flags = flags;
+    c.ok = plan(M, N, K, sm_count(), pair, fix_s, &c.pl, &c.cost);
+  }
+  return c;
+}
+
+}  // namespace gemm_cluster
+
+bool gemm_cluster_supported(const GemmArgs& a) {
+  return a.mode == kGemmPlain && a.M >= 1 && a.M <= kGemmClusterMaxRows && a.epilogue <= kGemmEpilogueSwigluTile;
+}
+
+// Whether this kernel is expected to be faster than the persistent two-SM kernel, which overlaps a tile's epilogue with the next
+// tile and needs no sum of parts, but deals out 256-row tiles: with fewer than three rounds of those, what they leave
+// idle or compute on padding is often more than this kernel's fixed cost.  Both sides measured, bf16 on B200: 512 x 1280 x 8192
+// 17.4 here and 29.6 us there, 200 x 4096 x 4096 15.0 and 18.1, 1000 x 1280 x 8192 23.9 and 29.6; 250 x 8192 x 3584 20.7 and 18.1,
+// 512 x 8192 x 8192 54.8 and 50.9, 2048 x 2048 x 2048 22.3 and 17.2.
+bool gemm_cluster_preferred(const GemmArgs& a) {
+  using namespace gemm_cluster;
+  if (a.M <= kTileM) return true;
+  const bool swiglu = a.epilogue == kEpiSwiglu || a.epilogue == kGemmEpilogueSwigluTile;
+  const double two_sm = pair_cost_us(a.M, a.N, a.K, sm_count() / 2, swiglu);
+  if (two_sm <= 0) return false;
+  const Planned& c = planned(a.M, a.N, a.K, a.pair, 0);
+  return c.ok && c.cost < two_sm;
+}
+
+cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStream_t stream, gemm_detail::TmapFn make_tmap) {
+  using namespace gemm_cluster;
+  const bool swiglu = a.epilogue == kEpiSwiglu || a.epilogue == kGemmEpilogueSwigluTile;
+  const int num_kb = (a.K + kTileK - 1) / kTileK;
+  int fix_s = a.splits;
+  const int most = a.pair > 0 ? kMaxCluster / 2 : kMaxCluster;
+  if (fix_s > most) fix_s = most;
+  if (fix_s > num_kb) fix_s = num_kb;
+  if (a.max_ctas > 0) {  // a budget: K is split as far as asked for
+    if (fix_s == 0) fix_s = 1;
+    if (fix_s > a.max_ctas) fix_s = a.max_ctas;
+  }
+  const Planned& chosen = planned(a.M, a.N, a.K, a.max_ctas > 0 ? -1 : a.pair, fix_s);
+  if (!chosen.ok) return cudaErrorInvalidValue;
+  const PlanC pl = chosen.pl;
+  const int P = pl.pair ? 2 : 1;
+  ParamsC p{};
+  p.M = a.M;
+  p.N = a.N;
+  p.C = a.C;
+  p.ldc = a.ldc;
+  p.vec_ok = a.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(a.C) & 7) == 0;
+  p.num_kb = num_kb;
+  if (swiglu) p.F = static_cast<const oob_gemm_epilogue_swiglu_t*>(a.epilogue_args)->F;
+  if (a.epilogue == kEpiRopeKv) p.rope = *static_cast<const oob_rope_args_t*>(a.epilogue_args);
+  p.n_mma = pl.n_mma;
+  p.nj = pl.nj;
+  p.Mp = pl.n_mma * pl.nj;
+  p.m_blocks = pl.m_blocks;
+  p.S = pl.S;
+  p.num_tiles = tile_count(a.N, pl);
+  p.stage_bytes = (kRowsW + p.Mp / P) * kRowBytes;
+  p.stages = pl.stages;
+  p.smem_bytes = pl.smem;
+  p.work_bytes = pl.smem - 1024 - kCtlBytes;
+  p.work_bytes -= p.work_bytes % 16;
+  p.tmem_cols = tmem_columns(p.Mp);
+  return a.fmt == 1 ? gemm_cluster::launch_fmt<__nv_bfloat16>(a, p, pl.pair, status, stream, make_tmap)
+                    : gemm_cluster::launch_fmt<__half>(a, p, pl.pair, status, stream, make_tmap);
+}
+
+}  // namespace oob

@@ -136,6 +136,12 @@ __device__ __forceinline__ void gemm_report(DeviceStatus* s, int rank, int code,
   }
 }
 
+// silu(g) * u.  With exp(-|g|) the denominator is in [1, 2], where the fast division is good to two units of the last place.
+__device__ __forceinline__ float swiglu_f32(float g, float u) {
+  const float t = __expf(-fabsf(g));
+  return (g >= 0.f ? g : g * t) * __fdividef(u, 1.f + t);
+}
+
 template <typename T>
 __device__ __forceinline__ void cvt_store_32(char* dst, const uint32_t (&r)[32], bool full_vec, int valid_cols) {
   // r holds 32 consecutive fp32 columns of one row.
@@ -702,7 +708,7 @@ __global__ void __launch_bounds__(MODE == kGemmPlain ? kThreadsPlain : kThreadsF
   const int G = gemm_ctas;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       // ------------------------- TMA producer -------------------------
       int stage = 0;
       uint32_t phase = 0;
@@ -749,7 +755,7 @@ __global__ void __launch_bounds__(MODE == kGemmPlain ? kThreadsPlain : kThreadsF
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       // ------------------------- MMA issuer ---------------------------
       constexpr uint32_t idesc = ptx::umma_idesc_f16(FMT, kTileM, kTileN);
       int stage = 0;

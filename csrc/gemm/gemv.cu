@@ -56,6 +56,8 @@ __global__ void __launch_bounds__(kThreads) gemv_kernel(const T* __restrict__ A,
   float acc[MB];
 #pragma unroll
   for (int m = 0; m < MB; ++m) acc[m] = 0.f;
+  ptx::griddep_launch_dependents();
+  ptx::griddep_wait();
   if (n < N) {
     const T* w = B + static_cast<size_t>(n) * ldb;
     const int chunks = K / 8;  // 16-byte units of a row
@@ -75,7 +77,7 @@ __global__ void __launch_bounds__(kThreads) gemv_kernel(const T* __restrict__ A,
 #pragma unroll
           for (int m = 0; m < MB; ++m) {
             if (m < M) {
-              const uint4 xv = __ldg(reinterpret_cast<const uint4*>(A + static_cast<size_t>(m) * lda + static_cast<size_t>(cc) * 8));
+              const uint4 xv = ptx::ld_v4(A + static_cast<size_t>(m) * lda + static_cast<size_t>(cc) * 8);
               acc[m] += dot8<T>(wv[j], xv);
             }
           }
@@ -109,9 +111,17 @@ template <typename T, int MB, int KS>
 cudaError_t launch_one(const GemmArgs& a, cudaStream_t stream) {
   constexpr int kRowsPerCta = kWarps / KS;
   const int grid = (a.N + kRowsPerCta - 1) / kRowsPerCta;
-  gemv_kernel<T, MB, KS><<<grid, kThreads, 0, stream>>>(static_cast<const T*>(a.A), a.lda, static_cast<const T*>(a.B), a.ldb,
-                                                        static_cast<T*>(a.C), a.ldc, a.M, a.N, a.K);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, gemv_kernel<T, MB, KS>, static_cast<const T*>(a.A), a.lda, static_cast<const T*>(a.B), a.ldb,
+                            static_cast<T*>(a.C), a.ldc, a.M, a.N, a.K);
 }
 
 template <typename T, int MB>

@@ -1056,10 +1056,10 @@ int oob_gemm(oob_comm* c, const oob_gemm_args_t* a, void* stream) {
   if (a->epilogue != OOB_EPILOGUE_NONE) {
     if (a->mode != OOB_GEMM_PLAIN || emu) return set_error(OOB_ERR_INVALID, "epilogues apply to the plain GEMM only");
     if (a->epilogue_args == nullptr) return set_error(OOB_ERR_INVALID, "null epilogue arguments");
-    if (gemm_plan_splits(a->M, a->N, a->K, a->max_ctas, a->splits) <= 1)
+    if (a->epilogue != OOB_EPILOGUE_SWIGLU_TILE && gemm_plan_splits(a->M, a->N, a->K, a->max_ctas, a->splits) <= 1)
       return set_error(OOB_ERR_UNSUPPORTED, "the epilogue runs in the split-K sum, and this problem is not split "
                                             "(see oob_gemm_plan_splits)");
-    if (a->epilogue == OOB_EPILOGUE_SWIGLU) {
+    if (a->epilogue == OOB_EPILOGUE_SWIGLU || a->epilogue == OOB_EPILOGUE_SWIGLU_TILE) {
       const int F = static_cast<const oob_gemm_epilogue_swiglu_t*>(a->epilogue_args)->F;
       if (F <= 0 || F % 8 != 0 || a->N != 2 * F || a->ldc < F || a->ldc % 8 != 0 || a->C == nullptr)
         return set_error(OOB_ERR_INVALID, "SwiGLU epilogue: N must be 2F, F and ldc multiples of 8, ldc >= F");

@@ -15,6 +15,7 @@ import torch
 from .. import _lib
 from . import solutions
 from ..utils.dtypes import dtype_code
+from ..utils.stream import current_stream_ptr
 
 
 def _check_operands(a: torch.Tensor, b: torch.Tensor) -> None:
@@ -59,16 +60,17 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
     (bit-reproducible).  0 uses it when the idle share would exceed 3 % of the run, 1 whenever there is a remainder,
     -1 never.
 
-    ``skinny`` selects the weight-streaming kernel for ``M <= 128`` (the weight rows fill the tensor-core
-    instruction's 128-row dimension, the tokens are its narrow dimension; stream-K split, deterministic) with 1.
-    It is opt-in: measured inside a decode step the tiled split-K path is a little faster at every ``M``.
+    ``skinny`` selects the weight-streaming kernel for few rows (the weight rows fill the tensor-core instruction's
+    128-row dimension, the tokens are its other one; K is split over the CTAs of a cluster that sum their parts through
+    distributed shared memory, deterministic): 0 uses it up to 128 rows, and above where it is expected to be faster than
+    the two-SM kernel, 1 whenever it can (``splits`` then asks for that many CTAs per tile, at most 8), -1 never.
 
     ``splitk_reduce`` says where a split-K sum is taken: -1 inside the GEMM kernel (the warp that delivers the last
     partial of a 32-row quadrant), 0 or 1 in a second kernel launched right after it (faster at every ``M``).
     The order of summation, and so the result, is the same.
 
     ``gemv`` = 1 uses the CUDA-core streaming kernel for ``M <= 4`` (a warp per weight row, no tensor cores, no
-    split-K hand-off); 0 uses it where it measured faster (one row; two rows with ``N * K`` up to 12 M), -1 never."""
+    split-K hand-off); 0 uses it where it measured faster (one row, ``N * K`` up to 32 M), -1 never."""
     _check_operands(a, b)
     M, N = a.shape[0], b.shape[0]
     if out is None:
@@ -95,7 +97,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
     if order is not None:
         check_order_buffer(order, M, N)
         args.order = order.data_ptr()
-    _lib.check(_lib.lib().oob_gemm(None, ctypes.byref(args), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    rc = _lib.lib().oob_gemm(None, args, current_stream_ptr())
+    if rc:
+        _lib.check(rc)
     return out
 
 
@@ -186,9 +190,10 @@ def gemm_swiglu(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = 
                 fused: Optional[bool] = None) -> torch.Tensor:
     """``silu(a @ b[:F].T) * (a @ b[F:].T)`` for a gate/up weight ``b`` of shape [2F, K]; returns [M, F].
 
-    When the GEMM is one that is split over K (every decode-step shape), the activation is applied by the kernel
-    that sums the splits: no separate launch and no 16-bit round trip of the [M, 2F] intermediate.  Otherwise, or
-    with ``fused=False``, the GEMM is followed by the stand-alone SwiGLU kernel."""
+    The activation is applied to the fp32 sums by the kernel that has them (the weight-streaming kernel up to 256 rows,
+    the split-K sum, or the two-SM kernel's epilogue): no separate launch and no 16-bit round trip of the [M, 2F]
+    intermediate.  With ``fused=False`` the GEMM is followed by the stand-alone SwiGLU kernel.  ``fused=True`` insists on
+    a problem that is split over K (every decode-step shape) and raises otherwise."""
     from .decode import silu_mul
     _check_operands(a, b)
     M, N = a.shape[0], b.shape[0]
@@ -200,11 +205,10 @@ def gemm_swiglu(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = 
     elif out.shape != (M, F) or out.dtype != a.dtype or out.stride(1) != 1 or out.stride(0) % 8 != 0:
         raise ValueError("bad output tensor")
     can_fuse = gemm_plan_splits(M, N, a.shape[1], max_ctas=max_ctas) > 1
-    if fused is None:
-        fused = can_fuse
     if fused and not can_fuse:
         raise ValueError("this problem is not split over K, so the epilogue has no kernel to run in")
-    if not fused:
+    # One CTA is no pair: such a budget leaves the two kernels.
+    if fused is False or (not can_fuse and max_ctas == 1):
         return silu_mul(gemm(a, b, max_ctas=max_ctas), out)
     epi = _lib.SwigluEpilogue()
     epi.F = F
@@ -213,8 +217,9 @@ def gemm_swiglu(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = 
     fill_gemm_args(args, a, b)
     args.C, args.ldc = out.data_ptr(), out.stride(0)
     args.max_ctas = max_ctas
-    args.skinny = -1
-    args.epilogue = _lib.EPILOGUE_SWIGLU
+    args.epilogue = _lib.EPILOGUE_SWIGLU if can_fuse else _lib.EPILOGUE_SWIGLU_TILE
     args.epilogue_args = ctypes.cast(ctypes.pointer(epi), ctypes.c_void_p)
-    _lib.check(_lib.lib().oob_gemm(None, ctypes.byref(args), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    rc = _lib.lib().oob_gemm(None, args, current_stream_ptr())
+    if rc:
+        _lib.check(rc)
     return out

@@ -1,0 +1,95 @@
+"""The weight-streaming GEMM (K split inside a cluster) at the edges of its tiles, and the SwiGLU epilogue of the two-SM
+kernel, against fp32 PyTorch and against the tiled kernels on the forms of operands that both accept."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+EPS = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}  # one rounding of the result
+
+
+def _operands(M, N, K, dtype, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed + M * 7 + N * 3 + K)
+    return (torch.randn(M, K, device="cuda", generator=g).to(dtype),
+            (torch.randn(N, K, device="cuda", generator=g) / K ** 0.5).to(dtype))
+
+
+def _check(got, a, b, dtype):
+    """One rounding to the output type plus K fp32 roundings of the running sum (each at most 2^-23 of the sum of
+    magnitudes, whatever the order)."""
+    ref = a.double() @ b.double().t()
+    bound = EPS[dtype] * ref.abs() + a.shape[1] * 2.0 ** -23 * (a.double().abs() @ b.double().abs().t()) + 2.0 ** -24
+    assert ((got.double() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape", [(1, 8, 8), (15, 127, 64), (16, 128, 72), (17, 129, 1096), (31, 1001, 520), (64, 1280, 8192),
+                                   (127, 2048, 136), (128, 7168, 256), (129, 200, 2056), (255, 4104, 640), (256, 1000, 4096)])
+@pytest.mark.parametrize("splits,pair", [(0, 0), (1, -1), (2, -1), (4, -1), (8, -1), (1, 1), (2, 1), (4, 1)])
+def test_cluster_gemm_edges(shape, splits, pair, dtype):
+    from ooverlap_b200.ops import gemm
+    M, N, K = shape
+    a, b = _operands(M, N, K, dtype)
+    c = gemm(a, b, skinny=1, splits=splits, pair=pair)
+    again = gemm(a, b, skinny=1, splits=splits, pair=pair)
+    torch.cuda.synchronize()
+    _check(c, a, b, dtype)
+    assert torch.equal(c, again)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape", [(3, 520, 1032), (40, 264, 520), (200, 1000, 72)])
+def test_default_route_equals_tiled_route_on_strided_operands(shape, dtype):
+    from ooverlap_b200.ops import gemm
+    M, N, K = shape
+    wide_a, wide_b = _operands(M + 2, N + 3, K + 16, dtype, seed=5)
+    a, b = wide_a[1:M + 1, 8:K + 8], wide_b[2:N + 2, 8:K + 8]
+    for pad, off in ((0, 0), (8, 8), (5, 8)):  # row strides that are and are not multiples of 8 elements
+        out = torch.full((M, N + pad + off), 7.0, device="cuda", dtype=dtype)
+        got = gemm(a, b, out=out[:, off:off + N])
+        tiled = gemm(a, b, skinny=-1, gemv=-1)
+        torch.cuda.synchronize()
+        _check(got, a, b, dtype)
+        _check(tiled, a, b, dtype)
+        assert (out[:, :off] == 7.0).all() and (out[:, off + N:] == 7.0).all()
+
+
+def test_kernels_follow_one_another_without_gaps_in_order():
+    """A chain of dependent launches whose set-up overlaps the kernel before: every link must see the link before it."""
+    from ooverlap_b200.ops import gemm, rmsnorm, silu_mul
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(24, 512, device="cuda", generator=g).bfloat16()
+    w1 = (torch.randn(1024, 512, device="cuda", generator=g) / 512 ** 0.5).bfloat16()
+    w2 = (torch.randn(512, 512, device="cuda", generator=g) / 512 ** 0.5).bfloat16()
+    nw = torch.ones(512, device="cuda").bfloat16()
+
+    def chain(h, sync):
+        r = h
+        for _ in range(20):
+            h, r = rmsnorm(gemm(silu_mul(gemm(h, w1)), w2), nw, 1e-5, r)
+            if sync:
+                torch.cuda.synchronize()
+        return h, r
+
+    ref = chain(x, True)
+    for _ in range(3):
+        got = chain(x, False)
+        torch.cuda.synchronize()
+        assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,F,K", [(1, 8, 64), (70, 72, 200), (256, 14336, 512), (257, 9480, 264), (1030, 4744, 1032), (2048, 8192, 256),
+                                   (4096, 3584, 2048)])
+def test_swiglu_in_the_tile_epilogue(M, F, K, dtype):
+    from ooverlap_b200.ops import gemm_swiglu
+    a, b = _operands(M, 2 * F, K, dtype)
+    got = gemm_swiglu(a, b)
+    torch.cuda.synchronize()
+    gu = a.double() @ b.double().t()
+    ref = torch.nn.functional.silu(gu[:, :F]) * gu[:, F:]
+    # fp32 sums, then one rounding; the derivative of silu(g) * u is at most 1.1 |u| + |g| and the quotient and __expf add
+    # a few parts in 2^22
+    sum_err = K * 2.0 ** -23 * (a.double().abs() @ b.double().abs().t())
+    bound = (EPS[dtype] + 2.0 ** -18) * ref.abs() + 1.1 * gu[:, F:].abs() * sum_err[:, :F] + gu[:, :F].abs() * sum_err[:, F:] + 2.0 ** -24
+    assert ((got.double() - ref).abs() <= bound).all()

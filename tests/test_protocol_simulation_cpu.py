@@ -18,7 +18,7 @@ role; every ``yield`` is a point where any other role may run) and executed unde
                               from call to call, and the restart of the call numbers by recover()
                               (csrc/collectives/allreduce_ll.cu)
 * last-arriver split-K sum    per-quadrant arrival counter re-armed by the CTA that completes it
-                              (csrc/gemm/gemm_kernel.cuh, csrc/gemm/gemm_skinny.cu)
+                              (csrc/gemm/gemm_kernel.cuh)
 
 What is checked: no role waits forever, every unit of work is done exactly once and only after its inputs were
 complete, and every counter is back at its initial value when a launch ends, so the next launch (run here back to
