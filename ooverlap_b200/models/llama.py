@@ -2,9 +2,9 @@
 
 Every linear layer is this library's tcgen05 GEMM; each transformer layer has two row-parallel projections
 (``o_proj`` and ``down_proj``) whose all-reduce is fused with the residual add and the following RMSNorm, i.e. 160
-all-reduces per token step for the 80-layer 70B configuration.  A decode step of a layer is nine kernels of this
-library: QKV GEMM, RoPE + KV-cache write, grouped-query decode attention over the static cache (head size 128),
-output GEMM, all-reduce + residual + RMSNorm, gate/up GEMM, SwiGLU, down GEMM, all-reduce + residual + RMSNorm.
+all-reduces per token step for the 80-layer 70B configuration.  A decode step of a layer is seven kernels of this
+library: QKV GEMM with RoPE + KV-cache write, grouped-query decode attention over the static cache (head size 128),
+output GEMM, all-reduce + residual + RMSNorm, gate/up GEMM with SwiGLU, down GEMM, all-reduce + residual + RMSNorm.
 Prefill attention uses PyTorch's causal ``scaled_dot_product_attention`` (the reference has no attention kernels;
 it only replaces the tensor-parallel communication of a served model).  The decode step has static shapes (the
 position is a device tensor) and is replayed from one CUDA graph.
@@ -111,9 +111,9 @@ class LlamaTP:
         self.rope_cos, self.rope_sin = ang.cos().to(dtype), ang.sin().to(dtype)  # [max_len, hd/2]
         if backend == "ours":
             self.rope_cos32, self.rope_sin32 = rope_tables(max_len, hd, cfg.rope_theta, self.device)
-        # RoPE + cache write and SwiGLU applied by the kernel that sums the K splits of the preceding GEMM (two
-        # launches fewer per layer in a decode step).  Off unless OOB_FUSED_EPILOGUES=1.
-        self.fused_epilogues = backend == "ours" and env_flag("OOB_FUSED_EPILOGUES", False)
+        # RoPE + cache write and SwiGLU applied to the fp32 sums by the preceding GEMM (two launches fewer per layer in
+        # a decode step, and no 16-bit round trip of the gate/up product).  OOB_FUSED_EPILOGUES=0 turns it off.
+        self.fused_epilogues = backend == "ours" and env_flag("OOB_FUSED_EPILOGUES", True)
         # Prefill: row-parallel projections of at least OOB_PREFILL_CHUNK_MIN_ROWS tokens are computed in
         # OOB_PREFILL_CHUNKS slabs whose all-reduce + norm overlaps the next slab's GEMM (1 = off).
         self.prefill_chunks = max(1, env_int("OOB_PREFILL_CHUNKS", 1)) if backend == "ours" else 1
