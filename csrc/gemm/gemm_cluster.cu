@@ -3,8 +3,7 @@
 // of a decode step or of a short mixed batch: what bounds it is the time to read B once, plus whatever happens before the
 // first and after the last byte.
 //
-// A CTA goes through about one 64-element K block per 0.24 us (the chain load - multiply - release of one issuing thread each),
-// so that neither few CTAs nor long K ranges reach the memory's rate.  128-row weight tiles are therefore computed by S CTAs,
+// A CTA goes through 64 elements of K in 0.17 - 0.27 us (the chain load - multiply - release of its issuing threads), so that neither few CTAs nor long K ranges reach the memory's rate.  128-row weight tiles are therefore computed by S CTAs,
 // each over 1/S of K; a cost model on the host picks S and the token blocks.
 //
 // Split over K inside a thread-block cluster (S = 1 .. 8).  When a CTA has its partial sums it drains them from TMEM into its
@@ -21,11 +20,11 @@
 //   RoPE + KV  query and key heads are rotated, queries go to q_out, keys and values into the layer's cache
 //
 // Measured on B200, bf16, in a chain of launches (before: fp32 partial tiles through memory and a second kernel that sums
-// them): 16 x 7168 x 8192 22.6 us (26.5), 16 x 8192 x 3584 14.1 (18.2), 8 x 8192 x 1024 7.0 (10.6), 8 x 1280 x 8192 8.3 (14.3),
-// 64 x 7168 x 8192 24.5 (29.6), 128 x 4096 x 4096 13.2, 512 x 1280 x 8192 17.4 (21.6).
+// them): 16 x 7168 x 8192 23.1 us (26.5), 16 x 8192 x 3584 13.3 (18.2), 8 x 8192 x 1024 6.9 (10.6), 8 x 1280 x 8192 7.8 (14.3),
+// 64 x 7168 x 8192 24.4 (29.6), 128 x 4096 x 4096 13.4, 512 x 1280 x 8192 17.4 (21.6).
 //
-// Roles: warp 0 TMA producer, warp 1 MMA issuer (one thread each), warps 2-5 drain TMEM; all six warps take part in the
-// reduction.  A cluster handles tiles c, c + G, ... one after the other; normally the grid covers all tiles, a CTA
+// Roles: warp 0 loads weights, warp 1 issues the MMAs, warp 2 loads activations (one thread each), warps 2-5 drain TMEM; all six
+// warps take part in the reduction.  A cluster handles tiles c, c + G, ... one after the other; normally the grid covers all tiles, a CTA
 // budget (max_ctas) makes G smaller.  All waits are bounded, and a CTA that gives up still meets its cluster's barriers.
 //
 // Capability parity with the reference: its stream-K GEMM instances (src/gemm/gemm_with_signal_sm90.h:238-292) and the
@@ -49,6 +48,10 @@ constexpr int kRowsW = 128;                  // weight rows of a CTA (the instru
 constexpr int kRowBytes = kTileK * 2;        // 128: one row of a stage
 constexpr int kMaxTokens = 256;              // per instruction (its N)
 constexpr int kMaxTileTokens = 384;          // per tile: what its fp32 sums leave of an SM's shared memory; more rows are cut into blocks
+// Up to this many tokens a stage holds 128 elements of K: half the waits and commits per byte (one CTA, 16 tokens: 0.17 us per
+// 64 elements instead of 0.24; 64 tokens: 0.20 instead of 0.25).  With more tokens it would leave too few stages
+// (128 x 7168 x 8192 27.1 us with 64 elements and 27.6 with 128, 128 x 8192 x 3584 split four ways 17.6 and 22.8).
+constexpr int kWideTokens = 64;
 constexpr int kThreadsC = 192;
 constexpr int kMaxStagesC = 12;
 constexpr int kMaxCluster = 8;               // portable cluster size
@@ -73,7 +76,8 @@ struct ParamsC {
   int F;         // SwiGLU: gate rows (N = 2F)
   void* C;
   int ldc;
-  int num_kb, num_tiles, clusters;
+  int num_kb, num_tiles, clusters;  // num_kb: pipeline stages' worth of K (sub * 64 elements each)
+  int sub;
   int S;  // CTAs (pairs) that share the K range of a tile
   int stages, stage_bytes, work_bytes;  // work_bytes: pipeline buffers or partial sums, whichever is larger
   int smem_bytes;
@@ -129,6 +133,19 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t mask) {
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(ptx::smem_u32(bar)),
       "h"(mask)
       : "memory");
+}
+
+template <bool PAIR>
+__device__ __forceinline__ void load_box(void* smem_dst, const void* tmap, uint32_t bar, int32_t x, int32_t y) {
+  if constexpr (PAIR) {
+    tma_load_2d_pair(smem_dst, tmap, bar, x, y);
+  } else {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        :
+        : "r"(ptx::smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(x), "r"(y)
+        : "memory");
+  }
 }
 
 template <typename T>
@@ -231,7 +248,8 @@ __device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base
   }
 }
 
-template <typename T, int EPI, bool PAIR>
+// SUB: 64-element boxes of K in a pipeline stage.
+template <typename T, int EPI, bool PAIR, int SUB>
 __global__ void __launch_bounds__(kThreadsC)
     gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                         const __grid_constant__ ParamsC p, DeviceStatus* status) {
@@ -253,7 +271,7 @@ __global__ void __launch_bounds__(kThreadsC)
     ptx::prefetch_tmap(&tmap_w);
     ptx::prefetch_tmap(&tmap_x);
     for (int s = 0; s < p.stages; ++s) {
-      ptx::mbar_init(&ctl->full[s], 1);
+      ptx::mbar_init(&ctl->full[s], 2);  // two producers
       ptx::mbar_init(&ctl->empty[s], 1);
     }
     ptx::mbar_init(&ctl->tmem_full, 1);
@@ -289,52 +307,46 @@ __global__ void __launch_bounds__(kThreadsC)
   int stage = 0;          // producer's / MMA issuer's position in the ring, carried from tile to tile
   uint32_t phase = 0;
   uint32_t tile_phase = 0;
-  constexpr int w_bytes = kRowsW * kRowBytes;
+  constexpr int w_bytes = kRowsW * kRowBytes;       // a stage holds SUB boxes of weights, then SUB of activations
+  const int x_bytes = SUB * (p.Mp / P) * kRowBytes;
   for (int t = cluster; t < p.num_tiles; t += p.clusters, tile_phase ^= 1) {
     const int wide_tile = t / p.m_blocks, m_first = (t - wide_tile * p.m_blocks) * p.Mp;
     const int tile = wide_tile * P + member;  // this CTA's 128 weight rows
     const int w_row = EPI == kEpiSwiglu ? tile * (kRowsW / 2) : tile * kRowsW;
     const int rows = min(p.Mp, p.M - m_first);
-    if (warp == 0) {
+    if (warp == 0 || warp == 2) {
       if (ptx::elect_one()) {
-        // ------------------------- TMA producer -------------------------
+        // ------------------------- TMA producers: warp 0 the weights, warp 2 the activations -------------------------
+        const bool weights = warp == 0;
+        const uint32_t bytes = P * (weights ? SUB * w_bytes : x_bytes);
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!ptx::mbar_wait(&ctl->empty[stage], phase ^ 1, abort)) break;
           uint8_t* sw = smem + stage * p.stage_bytes;
-          if constexpr (PAIR) {
-            const uint32_t full = map_to_cta(ptx::smem_u32(&ctl->full[stage]), in_cluster & ~1);
-            if (member == 0) ptx::mbar_arrive_expect_tx(&ctl->full[stage], 2 * p.stage_bytes);
-            if constexpr (EPI == kEpiSwiglu) {
-              tma_load_2d_pair(sw, &tmap_w, full, kb * kTileK, w_row);
-              tma_load_2d_pair(sw + w_bytes / 2, &tmap_w, full, kb * kTileK, p.F + w_row);
+          // The bytes of both CTAs of a pair are counted on the leader's barrier.
+          if (member == 0) ptx::mbar_arrive_expect_tx(&ctl->full[stage], bytes);
+          uint32_t full = ptx::smem_u32(&ctl->full[stage]);
+          if constexpr (PAIR) full = map_to_cta(full, in_cluster & ~1);
+#pragma unroll
+          for (int h = 0; h < SUB; ++h) {
+            const int k = (kb * SUB + h) * kTileK;  // past K: the box is filled with zeros
+            if (weights) {
+              load_box<PAIR>(sw + h * w_bytes, &tmap_w, full, k, w_row);
+              if constexpr (EPI == kEpiSwiglu) load_box<PAIR>(sw + h * w_bytes + w_bytes / 2, &tmap_w, full, k, p.F + w_row);
             } else {
-              tma_load_2d_pair(sw, &tmap_w, full, kb * kTileK, w_row);
+              for (int j = 0; j < p.n_mma; ++j)
+                load_box<PAIR>(sw + SUB * w_bytes + h * (x_bytes / SUB) + j * (p.nj / P) * kRowBytes, &tmap_x, full, k,
+                               m_first + j * p.nj + member * (p.nj / P));
             }
-            for (int j = 0; j < p.n_mma; ++j)
-              tma_load_2d_pair(sw + w_bytes + j * (p.nj / 2) * kRowBytes, &tmap_x, full, kb * kTileK,
-                               m_first + j * p.nj + member * (p.nj / 2));
-            if (++stage == p.stages) {
-              stage = 0;
-              phase ^= 1;
-            }
-            continue;
           }
-          ptx::mbar_arrive_expect_tx(&ctl->full[stage], p.stage_bytes);
-          if constexpr (EPI == kEpiSwiglu) {
-            ptx::tma_load_2d(sw, &tmap_w, &ctl->full[stage], kb * kTileK, w_row);
-            ptx::tma_load_2d(sw + w_bytes / 2, &tmap_w, &ctl->full[stage], kb * kTileK, p.F + w_row);
-          } else {
-            ptx::tma_load_2d(sw, &tmap_w, &ctl->full[stage], kb * kTileK, w_row);
-          }
-          for (int j = 0; j < p.n_mma; ++j)
-            ptx::tma_load_2d(sw + w_bytes + j * p.nj * kRowBytes, &tmap_x, &ctl->full[stage], kb * kTileK, m_first + j * p.nj);
           if (++stage == p.stages) {
             stage = 0;
             phase ^= 1;
           }
         }
       }
-    } else if (warp == 1) {
+      __syncwarp();
+    }
+    if (warp == 1) {
       if (member == 0 && ptx::elect_one()) {
         // ------------------------- MMA issuer (of the pair: the leader's) ---------------------------
         const uint32_t idesc = ptx::umma_idesc_f16(FMT, P * kRowsW, p.nj);
@@ -347,17 +359,20 @@ __global__ void __launch_bounds__(kThreadsC)
           }
           ptx::tc_fence_after_sync();
           const uint32_t sw = ptx::smem_u32(smem + stage * p.stage_bytes);
-          const uint64_t da = ptx::umma_desc_kmajor_sw128(sw);
-          for (int j = 0; j < p.n_mma; ++j) {
-            const uint64_t db = ptx::umma_desc_kmajor_sw128(sw + w_bytes + j * (p.nj / P) * kRowBytes);
 #pragma unroll
-            for (int k = 0; k < kTileK / 16; ++k) {
+          for (int h = 0; h < SUB; ++h) {
+            const uint64_t da = ptx::umma_desc_kmajor_sw128(sw + h * w_bytes);
+            for (int j = 0; j < p.n_mma; ++j) {
+              const uint64_t db = ptx::umma_desc_kmajor_sw128(sw + SUB * w_bytes + h * (x_bytes / SUB) + j * (p.nj / P) * kRowBytes);
               const uint32_t d_tmem = tmem_base + j * p.nj;
-              const uint32_t add = (kb > kb0 || k > 0) ? 1u : 0u;
-              if constexpr (PAIR) {
-                umma_f16_pair(d_tmem, da + uint64_t(k * 2), db + uint64_t(k * 2), idesc, add);
-              } else {
-                ptx::umma_f16(d_tmem, da + uint64_t(k * 2), db + uint64_t(k * 2), idesc, add);
+#pragma unroll
+              for (int k = 0; k < kTileK / 16; ++k) {
+                const uint32_t add = (kb > kb0 || h > 0 || k > 0) ? 1u : 0u;
+                if constexpr (PAIR) {
+                  umma_f16_pair(d_tmem, da + uint64_t(k * 2), db + uint64_t(k * 2), idesc, add);
+                } else {
+                  ptx::umma_f16(d_tmem, da + uint64_t(k * 2), db + uint64_t(k * 2), idesc, add);
+                }
               }
             }
           }
@@ -379,7 +394,7 @@ __global__ void __launch_bounds__(kThreadsC)
           }
         }
       }
-    } else {
+    } else if (warp >= 2) {
       // ------------------- TMEM -> own shared memory, [token][128] fp32 -------------------
       const int q = warp & 3;  // TMEM lane quadrant this warp may read: weight rows q * 32 ..
       if (ptx::mbar_wait(&ctl->tmem_full, tile_phase, abort)) {
@@ -443,9 +458,9 @@ __global__ void __launch_bounds__(kThreadsC)
   }
 }
 
-template <typename T, int EPI, bool PAIR>
+template <typename T, int EPI, bool PAIR, int SUB>
 cudaError_t launch_pair(const GemmArgs& a, ParamsC& p, DeviceStatus* status, cudaStream_t stream, TmapFn make_tmap) {
-  auto kernel = gemm_cluster_kernel<T, EPI, PAIR>;
+  auto kernel = gemm_cluster_kernel<T, EPI, PAIR, SUB>;
   const int size = PAIR ? 2 * p.S : p.S;  // CTAs of a cluster
   static std::atomic<uint64_t> attr_set_mask{0};
   int dev = 0;
@@ -480,7 +495,9 @@ cudaError_t launch_pair(const GemmArgs& a, ParamsC& p, DeviceStatus* status, cud
 
 template <typename T, int EPI>
 cudaError_t launch_epi(const GemmArgs& a, ParamsC& p, bool pair, DeviceStatus* status, cudaStream_t stream, TmapFn make_tmap) {
-  return pair ? launch_pair<T, EPI, true>(a, p, status, stream, make_tmap) : launch_pair<T, EPI, false>(a, p, status, stream, make_tmap);
+  if (pair) return launch_pair<T, EPI, true, 1>(a, p, status, stream, make_tmap);
+  return p.sub == 2 ? launch_pair<T, EPI, false, 2>(a, p, status, stream, make_tmap)
+                    : launch_pair<T, EPI, false, 1>(a, p, status, stream, make_tmap);
 }
 
 template <typename T>
@@ -500,6 +517,7 @@ namespace gemm_cluster {
 // How a problem is cut: token blocks, pairs, K splits.
 struct PlanC {
   int m_blocks, n_mma, nj;
+  int sub;  // 64-element boxes of K in a stage
   bool pair;
   int S;
   int stages, smem, per_sm;  // pipeline stages, shared memory of a CTA, CTAs that share an SM
@@ -528,10 +546,12 @@ uint32_t tmem_columns(int Mp) {
 // alone does not fit.
 bool size_cta(int N, int num_kb, int sms, PlanC* pl) {
   const int P = pl->pair ? 2 : 1, Mp = pl->n_mma * pl->nj;
-  const int stage_bytes = (kRowsW + Mp / P) * kRowBytes;
+  const int stage_bytes = pl->sub * (kRowsW + Mp / P) * kRowBytes;
   const int fixed = 1024 + kCtlBytes;
   const int partial = Mp * kRowsW * 4 + fixed;
-  const int kb_per = (num_kb + pl->S - 1) / pl->S;
+  const int steps = (num_kb + pl->sub - 1) / pl->sub;
+  if (steps < pl->S) return false;
+  const int kb_per = (steps + pl->S - 1) / pl->S;
   const int tmem = int(tmem_columns(Mp));
   // A CTA takes at least the share of an SM's shared memory that its TMEM columns are of the 512 (456 bytes a column; the
   // other TMEM kernels of this library take all of both).  CTAs that fit an SM then always find their columns free:
@@ -580,13 +600,13 @@ double plan_cost(int N, int num_kb, int sms, const PlanC& pl) {
   const double share = live > sms ? live / sms : 1.0;
   const double kb = double((num_kb + pl.S - 1) / pl.S);
   const double w = kRowsW * kRowBytes, x = double(Mp) / P * kRowBytes;
-  double t = kb * (0.235 + 0.0002 * Mp);
+  double t = kb * (pl.sub == 2 ? 0.165 + 0.0005 * Mp : 0.235 + 0.0002 * Mp);
   const double mma = share * kb * 2.0 * Mp / 1850.0, l2 = live * kb * (w + x) / 11.5e6, hbm = live * kb * w / pl.m_blocks / 6.4e6;
   if (mma > t) t = mma;
   if (l2 > t) t = l2;
   if (hbm > t) t = hbm;
   t += 0.015 * Mp + live * Mp * kRowsW * 4.0 * (pl.S - 1) / pl.S / 3.0e6;
-  return rounds * t + (rounds - 1) * 2.0 + (size > 1 ? 3.8 : 3.4) + 0.08 * (pl.S - 1);
+  return rounds * t + (rounds - 1) * 2.0 + (size > 1 ? 3.8 : 3.4) + (size == 8 && Mp > 128 ? 2.0 : 0.0) + 0.08 * (pl.S - 1);
 }
 
 // The cheapest cut of a problem.  `fix_s` > 0 fixes the K split, `pair` is as in GemmArgs.
@@ -604,6 +624,7 @@ bool plan(int M, int N, int K, int sms, int pair, int fix_s, PlanC* out, double*
     for (int two = 0; two < 2; ++two) {
       pl.pair = two != 0;
       if (two ? pair < 0 || (pair == 0 && Mp <= 128) : pair > 0) continue;
+      pl.sub = !two && Mp <= kWideTokens && num_kb >= 2 * kMaxCluster ? 2 : 1;
       for (pl.S = 1; pl.S <= kMaxCluster / (two ? 2 : 1); ++pl.S) {
         if (fix_s > 0 ? pl.S != fix_s : (num_kb < 4 * pl.S && pl.S > 1)) continue;
         if (!size_cta(N, num_kb, sms, &pl)) continue;
@@ -684,7 +705,8 @@ cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStr
   p.C = a.C;
   p.ldc = a.ldc;
   p.vec_ok = a.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(a.C) & 7) == 0;
-  p.num_kb = num_kb;
+  p.sub = pl.sub;
+  p.num_kb = (num_kb + pl.sub - 1) / pl.sub;
   if (swiglu) p.F = static_cast<const oob_gemm_epilogue_swiglu_t*>(a.epilogue_args)->F;
   if (a.epilogue == kEpiRopeKv) p.rope = *static_cast<const oob_rope_args_t*>(a.epilogue_args);
   p.n_mma = pl.n_mma;
@@ -693,7 +715,7 @@ cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStr
   p.m_blocks = pl.m_blocks;
   p.S = pl.S;
   p.num_tiles = tile_count(a.N, pl);
-  p.stage_bytes = (kRowsW + p.Mp / P) * kRowBytes;
+  p.stage_bytes = pl.sub * (kRowsW + p.Mp / P) * kRowBytes;
   p.stages = pl.stages;
   p.smem_bytes = pl.smem;
   p.work_bytes = pl.smem - 1024 - kCtlBytes;
