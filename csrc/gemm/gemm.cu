@@ -65,7 +65,7 @@ bool make_tmap_cached(CUtensorMap* out, const void* p, uint64_t rows, uint64_t c
 }
 
 // Library-owned scratch.  One split-K workspace per device, shared by every launch on that device: GEMMs that use it
-// (split problems, the weight-streaming kernel) must not overlap on the GPU, i.e. they run on one stream or are
+// (problems split through memory) must not overlap on the GPU, i.e. they run on one stream or are
 // ordered by events; the same holds for the stream-K workspace of the two-SM kernel.  A workspace that has been handed
 // out is never freed or moved (a CUDA graph captured earlier keeps launching with its address): when a larger one is
 // needed a new block is allocated and the old one stays alive.  Nothing can be allocated while the stream is being
@@ -190,12 +190,6 @@ cudaError_t launch_fmt(const CommCtx& ctx, const GemmArgs& a, cudaStream_t strea
 }
 
 }  // namespace
-
-cudaError_t gemm_library_workspace(size_t bytes, cudaStream_t stream, void** out) {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  return ensure_splitk(dev, bytes, stream, out);
-}
 
 cudaError_t gemm_reserve_splitk(size_t bytes) {
   int dev = 0;

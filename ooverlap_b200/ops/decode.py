@@ -3,7 +3,7 @@ attention over a static cache.
 
 Capability parity: the reference leaves the model's own ops to vLLM
 (patches/vllm/v0.25.0/vllm/model_executor/models/qwen2.py); this library's serving path needs them so that one
-decode step is a fixed sequence of kernels (nine per transformer layer) that a CUDA graph replays.
+decode step is a fixed sequence of kernels (seven per transformer layer) that a CUDA graph replays.
 """
 from __future__ import annotations
 
@@ -77,8 +77,8 @@ def gemm_rope_kv_write(x: torch.Tensor, wqkv: torch.Tensor, B: int, T: int, head
                        batch0: int = 0, q_out: Optional[torch.Tensor] = None, fused: Optional[bool] = None) -> torch.Tensor:
     """``rope_kv_write(x @ wqkv.T, ...)``: the QKV projection followed by the rotation and the cache write.
 
-    When the GEMM is one that is split over K (every decode-step shape), rotation and cache write are done by the
-    kernel that sums the splits, from the fp32 sums; otherwise (or with ``fused=False``) the GEMM is followed by
+    When the GEMM is one that is split over K (every decode-step shape), rotation and cache write are done from the fp32
+    sums by the kernel that has them (the weight-streaming kernel, or the one that sums the splits); otherwise (or with ``fused=False``) the GEMM is followed by
     :func:`rope_kv_write`.  Returns the rotated queries, [B*T, heads * hd]."""
     from .gemm import _check_operands, fill_gemm_args, gemm, gemm_plan_splits
     _check_operands(x, wqkv)
