@@ -123,18 +123,6 @@ def silu_mul(gu: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tens
     return out
 
 
-_workspaces: dict = {}
-
-
-def _workspace(device, nbytes: int) -> torch.Tensor:
-    key = (device.type, device.index)
-    ws = _workspaces.get(key)
-    if ws is None or ws.numel() * 4 < nbytes:
-        ws = torch.empty(max(nbytes, 1 << 20) // 4 + 1, dtype=torch.float32, device=device)
-        _workspaces[key] = ws
-    return ws
-
-
 def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, pos, *, batch0: int = 0,
                 scale: Optional[float] = None, out: Optional[torch.Tensor] = None, splits: int = 0,
                 len_bound: int = 0) -> torch.Tensor:
@@ -173,11 +161,12 @@ def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, p
         a.pos_dev, a.len = None, int(pos) + 1
     a.scale = scale if scale is not None else 1.0 / math.sqrt(hd)
     a.splits, a.len_bound = splits, bound
+    ws = None
     if splits > 1:
-        ws = _workspace(q.device, lib.oob_attn_decode_workspace_bytes(B, H, splits))
-        a.workspace = ws.data_ptr()
-    else:
-        a.workspace = None
+        # Of this call alone, in stream order (and in the graph's pool under capture): a workspace shared by calls would be
+        # written by two streams at once, and one that a later call outgrows would be freed under a captured graph.
+        ws = torch.empty(lib.oob_attn_decode_workspace_bytes(B, H, splits), dtype=torch.uint8, device=q.device)
+    a.workspace = ws.data_ptr() if ws is not None else None
     _lib.check(lib.oob_attn_decode(ctypes.byref(a), _stream()))
     return out
 
