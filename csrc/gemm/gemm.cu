@@ -296,6 +296,12 @@ cudaError_t launch_gemm(const CommCtx& ctx, const GemmArgs& args, cudaStream_t s
     if (a.epilogue == 0 && gemv_supported(a) && ctx.emu_table == nullptr && a.c_emu_stride == 0 && a.splitk_ws == nullptr &&
         (a.gemv > 0 || (a.gemv == 0 && a.splits == 0 && a.skinny <= 0 && (gemv_env == 1 || gemv_by_shape))))
       return launch_gemv(a, a.max_ctas > 0 ? a.max_ctas : sm_count(), stream);
+    // OOB_GEMM_PAIR=0 stands for pair = -1 in every call that leaves the choice open.
+    static const bool pair_env_off = [] {
+      const char* v = getenv("OOB_GEMM_PAIR");
+      return v != nullptr && v[0] == '0';
+    }();
+    if (a.pair == 0 && pair_env_off) a.pair = -1;
     // Few rows, or few tiles: the weight-streaming kernel.
     static const bool cluster_env_off = [] {
       const char* v = getenv("OOB_GEMM_SKINNY");
@@ -307,27 +313,30 @@ cudaError_t launch_gemm(const CommCtx& ctx, const GemmArgs& args, cudaStream_t s
     if ((a.skinny > 0 || cluster_auto) && gemm_cluster_supported(a) && ctx.emu_table == nullptr && a.c_emu_stride == 0 && a.splitk_ws == nullptr &&
         a.order == nullptr && (a.epilogue == 0 || a.epilogue_args != nullptr))
       return launch_gemm_cluster(a, ctx.status, stream, make_tmap_cached);
-    if (a.epilogue == kGemmEpilogueSwigluTile) {
-      if (ctx.emu_table != nullptr || a.c_emu_stride != 0 || a.epilogue_args == nullptr) return cudaErrorInvalidValue;
-      a.splits = 1;
-      return launch_gemm_pair(ctx, a, stream, make_tmap_cached, nullptr);
-    }
-    static const bool pair_env_off = [] {
-      const char* v = getenv("OOB_GEMM_PAIR");
-      return v != nullptr && v[0] == '0';
-    }();
+    // More than 128 rows: the two-SM kernel on narrow tiles, or with the SwiGLU in its epilogue, beats partial tiles through
+    // memory (250 x 8192 x 3584: 18.1 against 26.7 us) where nothing was asked for.  SwiGLU in the tile epilogue has no other
+    // tiled kernel: without the two-SM kernel (forbidden, no pair in the budget or none that fits the device) the sum of a
+    // split problem applies it, and an unsplit one is refused.
     int splits = gemm_plan_splits(a.M, a.N, a.K, a.max_ctas, a.splits);
-    // Nothing asked for and more than 128 rows: the two-SM kernel on narrow tiles, or with the SwiGLU in its epilogue, beats
-    // partial tiles through memory (250 x 8192 x 3584: 18.1 against 26.7 us).
-    if (splits > 1 && a.M > kTileM && a.splits == 0 && a.max_ctas == 0 && a.skinny == 0 && a.pair == 0 && a.splitk_reduce == 0 &&
-        a.splitk_ws == nullptr && ctx.emu_table == nullptr && a.c_emu_stride == 0 && !pair_env_off && a.epilogue <= 1) {
-      if (a.epilogue == 1 && a.epilogue_args != nullptr) {
-        a.epilogue = kGemmEpilogueSwigluTile;
-        a.splits = 1;
-        return launch_gemm_pair(ctx, a, stream, make_tmap_cached, nullptr);
-      }
-      if (a.epilogue == 0) splits = 1;
+    const bool plain_launch = ctx.emu_table == nullptr && a.c_emu_stride == 0;
+    const bool tile_epilogue = a.epilogue == kGemmEpilogueSwigluTile;
+    if (tile_epilogue && (!plain_launch || a.epilogue_args == nullptr)) return cudaErrorInvalidValue;
+    const bool asked = a.splits != 0 || a.max_ctas != 0 || a.skinny != 0 || a.pair != 0 || a.splitk_reduce != 0;
+    const bool unsplit = splits > 1 && a.M > kTileM && !asked && a.splitk_ws == nullptr && plain_launch && a.epilogue <= 1;
+    if ((tile_epilogue && a.pair >= 0 && (a.max_ctas == 0 || a.max_ctas >= 2)) ||
+        (unsplit && a.epilogue == 1 && a.epilogue_args != nullptr)) {
+      GemmArgs t = a;
+      t.epilogue = kGemmEpilogueSwigluTile;
+      t.splits = 1;
+      e = launch_gemm_pair(ctx, t, stream, make_tmap_cached, nullptr);
+      if (e != cudaErrorNotSupported) return e;
+      cudaGetLastError();
     }
+    if (tile_epilogue) {
+      if (splits <= 1) return cudaErrorNotSupported;
+      a.epilogue = 1;
+    }
+    if (unsplit && a.epilogue == 0) splits = 1;
     a.splits = splits;
     if (a.epilogue != 0) {
       // The epilogue lives in the kernel that sums the splits: the problem has to be one that is split.
@@ -352,9 +361,8 @@ cudaError_t launch_gemm(const CommCtx& ctx, const GemmArgs& args, cudaStream_t s
         (a.epilogue != 0 || a.splitk_reduce > 0 || (a.splitk_reduce == 0 && a.M >= splitk_reduce_min_rows)))
       a.splitk_defer = 1;
     // Large problems go to the two-SM kernel: same tile count per SM, two thirds of the operand traffic.
-    const bool pair_ok = splits == 1 && ctx.emu_table == nullptr && a.c_emu_stride == 0 && (a.max_ctas == 0 || a.max_ctas >= 2);
-    const bool pair_auto = a.M > kTileM && !pair_env_off;
-    if (pair_ok && (a.pair > 0 || (a.pair == 0 && pair_auto))) {
+    const bool pair_ok = splits == 1 && plain_launch && (a.max_ctas == 0 || a.max_ctas >= 2);
+    if (pair_ok && (a.pair > 0 || (a.pair == 0 && a.M > kTileM))) {
       e = launch_gemm_pair(ctx, a, stream, make_tmap_cached, nullptr);
       if (e != cudaErrorNotSupported) return e;
       cudaGetLastError();

@@ -1113,6 +1113,11 @@ int oob_gemm(oob_comm* c, const oob_gemm_args_t* a, void* stream) {
     return set_error(OOB_ERR_UNSUPPORTED, "this GEMM needs a larger scratch workspace and the stream is being captured: "
                                           "call oob_gemm_reserve_workspace before the capture");
   }
+  if (e == cudaErrorNotSupported && a->epilogue == OOB_EPILOGUE_SWIGLU_TILE) {
+    (void)cudaGetLastError();
+    return set_error(OOB_ERR_UNSUPPORTED, "no kernel applies this SwiGLU: the problem is not split over K and the two-SM kernel is "
+                                          "ruled out (OOB_GEMM_PAIR=0, pair = -1, one CTA) or does not fit the device");
+  }
   if (e != cudaSuccess) return cuda_fail(e, "GEMM launch");
   return OOB_OK;
 }

@@ -207,8 +207,7 @@ def gemm_swiglu(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = 
     can_fuse = gemm_plan_splits(M, N, a.shape[1], max_ctas=max_ctas) > 1
     if fused and not can_fuse:
         raise ValueError("this problem is not split over K, so the epilogue has no kernel to run in")
-    # One CTA is no pair: such a budget leaves the two kernels.
-    if fused is False or (not can_fuse and max_ctas == 1):
+    if fused is False:
         return silu_mul(gemm(a, b, max_ctas=max_ctas), out)
     epi = _lib.SwigluEpilogue()
     epi.F = F
@@ -220,6 +219,8 @@ def gemm_swiglu(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = 
     args.epilogue = _lib.EPILOGUE_SWIGLU if can_fuse else _lib.EPILOGUE_SWIGLU_TILE
     args.epilogue_args = ctypes.cast(ctypes.pointer(epi), ctypes.c_void_p)
     rc = _lib.lib().oob_gemm(None, args, current_stream_ptr())
+    if rc == _lib.ERR_UNSUPPORTED and not can_fuse:  # no kernel that has the sums may or can apply it: two kernels
+        return silu_mul(gemm(a, b, max_ctas=max_ctas), out)
     if rc:
         _lib.check(rc)
     return out

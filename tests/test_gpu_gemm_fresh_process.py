@@ -36,3 +36,44 @@ torch.cuda.synchronize()
 ref = a.float() @ b.float().t()
 assert (out.float() - ref).abs().max().item() <= 2e-2 * max(1.0, ref.abs().max().item())
 """)
+
+
+@pytest.mark.parametrize("M,F,K", [(2048, 2048, 512), (4224, 1024, 512), (300, 8192, 1024)])
+def test_the_switch_that_forbids_the_two_sm_kernel_holds_for_swiglu(M, F, K):
+    """OOB_GEMM_PAIR=0 (and no weight-streaming kernel): an unsplit gate/up projection is a one-SM GEMM and the
+    stand-alone activation."""
+    _child(f"M, F, K = {M}, {F}, {K}\n" """
+from ooverlap_b200.ops import gemm, gemm_plan_splits, gemm_swiglu, silu_mul
+a = torch.randn(M, K, device="cuda").bfloat16()
+b = (torch.randn(2 * F, K, device="cuda") / K ** 0.5).bfloat16()
+assert gemm_plan_splits(M, 2 * F, K) == 1
+got, want = gemm_swiglu(a, b), silu_mul(gemm(a, b, pair=-1, skinny=-1))
+torch.cuda.synchronize()
+assert torch.equal(got, want)
+""", OOB_GEMM_PAIR="0", OOB_GEMM_SKINNY="0")
+
+
+def test_swiglu_runs_where_no_pair_of_sms_can(monkeypatch):
+    """A device (or a budget) without the two-SM kernel: the native call refuses, the op runs two kernels instead."""
+    import torch
+    from ooverlap_b200 import _lib
+    from ooverlap_b200.ops import gemm, gemm_swiglu, silu_mul
+    real = _lib.lib()
+
+    class NoPair:
+        def __getattr__(self, name):
+            return getattr(real, name)
+
+        def oob_gemm(self, comm, args, stream):
+            a = getattr(args, "_obj", args)
+            return _lib.ERR_UNSUPPORTED if a.epilogue == _lib.EPILOGUE_SWIGLU_TILE else real.oob_gemm(comm, args, stream)
+
+    a = torch.randn(2048, 512, device="cuda").bfloat16()
+    b = (torch.randn(4096, 512, device="cuda") / 22).bfloat16()
+    want = silu_mul(gemm(a, b))
+    one = gemm_swiglu(a, b, max_ctas=1)  # one CTA is no pair
+    monkeypatch.setattr(_lib, "lib", lambda: NoPair())
+    got = gemm_swiglu(a, b)
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    assert torch.equal(one, silu_mul(gemm(a, b, max_ctas=1)))
