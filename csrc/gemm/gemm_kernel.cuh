@@ -38,6 +38,7 @@
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include "../device/activation.cuh"
 #include "../device/reduce.cuh"
 #include "../device/sync.cuh"
 #include "gemm.h"
@@ -134,12 +135,6 @@ __device__ __forceinline__ void gemm_report(DeviceStatus* s, int rank, int code,
     s->where = where;
     __threadfence_system();
   }
-}
-
-// silu(g) * u.  With exp(-|g|) the denominator is in [1, 2], where the fast division is good to two units of the last place.
-__device__ __forceinline__ float swiglu_f32(float g, float u) {
-  const float t = __expf(-fabsf(g));
-  return (g >= 0.f ? g : g * t) * __fdividef(u, 1.f + t);
 }
 
 template <typename T>

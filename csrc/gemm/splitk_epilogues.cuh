@@ -64,7 +64,7 @@ __global__ void splitk_reduce_swiglu_kernel(const float* __restrict__ partials, 
     splitk_sum8(partials, m, j, tiles_n, splits, g);
     splitk_sum8(partials, m, F + j, tiles_n, splits, u);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) o[e] = g[e] / (1.f + __expf(-g[e])) * u[e];
+    for (int e = 0; e < 8; ++e) o[e] = swiglu_f32(g[e], u[e]);
     *reinterpret_cast<uint4*>(out + static_cast<size_t>(m) * ld_out + j) = pack8<T>(o);
   }
 }

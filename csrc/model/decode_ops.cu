@@ -23,6 +23,7 @@
 
 #include "../api/oob.h"
 #include "../api/oob_model.h"
+#include "../device/activation.cuh"
 #include "../device/ptx.cuh"
 #include "../runtime/errors.h"
 
@@ -142,7 +143,7 @@ __global__ void silu_mul_kernel(const T* gu, long long ld, T* out, long long uni
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const float2 x = Cvt<T>::unpack(gw[i]), y = Cvt<T>::unpack(vw[i]);
-      o[i] = Cvt<T>::pack(x.x / (1.f + __expf(-x.x)) * y.x, x.y / (1.f + __expf(-x.y)) * y.y);
+      o[i] = Cvt<T>::pack(swiglu_f32(x.x, y.x), swiglu_f32(x.y, y.y));
     }
     *reinterpret_cast<uint4*>(out + r * static_cast<long long>(F) + c * 8) = make_uint4(o[0], o[1], o[2], o[3]);
   }

@@ -93,3 +93,20 @@ def test_swiglu_in_the_tile_epilogue(M, F, K, dtype):
     sum_err = K * 2.0 ** -23 * (a.double().abs() @ b.double().abs().t())
     bound = (EPS[dtype] + 2.0 ** -18) * ref.abs() + 1.1 * gu[:, F:].abs() * sum_err[:, :F] + gu[:, :F].abs() * sum_err[:, F:] + 2.0 ** -24
     assert ((got.double() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,F", [(64, 4096), (200, 2048), (512, 8192), (2048, 4096)])
+def test_swiglu_is_one_formula_whatever_kernel_applies_it(M, F, dtype):
+    """Rows of A that pick one column of B make every sum exact, so that the fused kernels see the very values that the
+    stand-alone activation reads back; then the same formula gives the same bits."""
+    from ooverlap_b200.ops import gemm, gemm_swiglu, silu_mul
+    K = max(M, 512)
+    g = torch.Generator(device="cuda").manual_seed(M + F)
+    a = torch.eye(M, K, device="cuda").to(dtype)
+    b = (torch.randn(2 * F, K, device="cuda", generator=g) * 3).to(dtype)
+    b[:F, :4] = torch.tensor([0.0, -80.0, -1000.0, 1000.0], device="cuda", dtype=dtype)
+    got, want = gemm_swiglu(a, b), silu_mul(gemm(a, b))
+    torch.cuda.synchronize()
+    assert torch.equal(gemm(a, b), b.t()[:M].contiguous())
+    assert torch.equal(got, want)
