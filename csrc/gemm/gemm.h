@@ -22,7 +22,7 @@ constexpr int kTileBytes = kTileM * kTileN * 2;  // one 16-bit output tile
 
 // Layout of one CTA's trace record (GemmArgs::trace).
 enum TraceSlot : int {
-  kTraceStart = 0,       // kernel entry
+  kTraceStart = 0,       // kernel entry; plain two-SM launches: when the kernels before this one are complete
   kTraceGemmDone = 1,    // GEMM CTAs: all tiles computed and stored / pushed
   kTraceFirstReady = 2,  // communication role: first work item became ready; GEMM CTAs of the two-SM fused kernel:
                          // the last tile has left the epilogue (its publication may still be under way)
