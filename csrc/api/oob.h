@@ -199,7 +199,8 @@ typedef struct {
   int use_nvls; /* fused modes: 0 = peer loads/stores only, non-zero = NVLS multimem when the heap has it */
   int splits;   /* plain mode: K splits per tile; 0 = chosen from the shape, 1 = off */
   int no_join;  /* fused AR / RS: 1 = only the dedicated communication CTAs reduce */
-  void* trace;  /* optional device buffer, 8 x uint64 per CTA: globaltimer stamps of the kernel's phases */
+  void* trace;  /* optional device buffer, 8 x uint64 per CTA: globaltimer stamps of the kernel's phases (tiled kernels: a
+                   traced plain GEMM does not take the weight-streaming kernel by itself) */
   int pair;     /* 0 = two-SM kernel (CTA pairs, 256x256 tiles) when the shape suits it, 1 = whenever possible,
                    -1 = never; plain and fused modes (fused GEMM->AR on pairs reduces C in place and ignores partial_*) */
   int splitk_reduce; /* split-K: 0 / 1 = separate reduction kernel, -1 = sum inside the GEMM kernel */

@@ -302,13 +302,14 @@ cudaError_t launch_gemm(const CommCtx& ctx, const GemmArgs& args, cudaStream_t s
       return v != nullptr && v[0] == '0';
     }();
     if (a.pair == 0 && pair_env_off) a.pair = -1;
-    // Few rows, or few tiles: the weight-streaming kernel.
+    // Few rows, or few tiles: the weight-streaming kernel.  It writes no trace, and its grid is not bounded by the SM count as
+    // the records of a trace buffer are: a traced GEMM runs on the tiled kernels.
     static const bool cluster_env_off = [] {
       const char* v = getenv("OOB_GEMM_SKINNY");
       return v != nullptr && v[0] == '0';
     }();
     const bool cluster_auto = a.skinny == 0 && a.splits == 0 && a.pair <= 0 && a.stream_k <= 0 && a.splitk_reduce == 0 &&
-                              a.max_ctas == 0 && a.gemv <= 0 && !cluster_env_off && a.M <= kGemmClusterMaxRows &&
+                              a.max_ctas == 0 && a.gemv <= 0 && a.trace == nullptr && !cluster_env_off && a.M <= kGemmClusterMaxRows &&
                               gemm_cluster_preferred(a);
     if ((a.skinny > 0 || cluster_auto) && gemm_cluster_supported(a) && ctx.emu_table == nullptr && a.c_emu_stride == 0 && a.splitk_ws == nullptr &&
         a.order == nullptr && (a.epilogue == 0 || a.epilogue_args != nullptr))

@@ -34,3 +34,18 @@ def test_stamps_of_a_gemm_start_after_the_kernel_before_it():
         # The clock that is stamped advances in steps of up to 1 us.
         assert int(start[start > 0].min()) >= int(end.max()) - 1000
         assert (after[:, END] >= after[:, GEMM_DONE]).all() and (after[:, GEMM_DONE] >= after[:, START]).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 7168, 8192), (16, 1024, 2048), (128, 1280, 8192), (200, 1280, 8192)])
+def test_small_gemm_is_traced(M, N, K):
+    a = torch.randn(M, K, device="cuda").bfloat16()
+    b = (torch.randn(N, K, device="cuda") / K ** 0.5).bfloat16()
+    c = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    trace = torch.zeros(148 + 64, 8, dtype=torch.int64, device="cuda")
+    _launch(a, b, c, trace)
+    torch.cuda.synchronize()
+    ref = a.float() @ b.float().t()
+    assert (c.float() - ref).abs().max().item() <= 2e-2 * max(1.0, ref.abs().max().item())
+    used = trace[:, START] > 0
+    assert int(used.sum()) > 0 and (trace[used][:, GEMM_DONE] >= trace[used][:, START]).all()
+    assert not trace[148:].any()  # one record per CTA, at most one CTA per SM
