@@ -278,6 +278,10 @@ int oob_pad_counter_count(void);
  * pair of the tile.  Returns the item count, -1 when cap is too small. */
 int oob_test_pair_schedule(int mode, int M, int N, int K, int pairs, int stream_k, int world, int rank, int* out, int cap);
 
+/* Test hook: the local norm of oob_fused_norm(NULL, OOB_NORM_LOCAL, ...) whose waits for the rows of its ring run out at
+ * once, so that every row takes the way of a row that arrives late. */
+int oob_test_norm_late_rows(const oob_norm_args_t* a, int max_ctas, void* stream);
+
 /* Test hook: waits on a flag that nobody sets, with the communicator's
  * timeout, and reports through the status block (bounded-wait self test). */
 int oob_test_bounded_wait(oob_comm* c, void* stream);

@@ -87,8 +87,8 @@ struct NormArgs {
   size_t piece_bytes;     // >= rows * hidden * sizeof(T), a multiple of 16
 };
 
-// kNormLocal outside the emulation (norm_local.cu).
-cudaError_t launch_norm_local(int rank, const NormArgs& args, int max_ctas, cudaStream_t stream);
+// kNormLocal outside the emulation (norm_local.cu).  `polls` bounds a wait for a row of its ring.
+cudaError_t launch_norm_local(int rank, const NormArgs& args, int max_ctas, cudaStream_t stream, uint32_t polls = 1u << 24);
 
 cudaError_t launch_fused_norm(const CommCtx& ctx, int algo, const NormArgs& args, int max_ctas, cudaStream_t stream);
 

@@ -6,7 +6,8 @@
 //     issues them), so the loads of the next rows are in flight while a row is summed, scaled and written.  The old form (plain
 //     loads, three block barriers per row, loads of a row issued only when the row before was done) kept too little in
 //     flight.  One block barrier per row: it publishes the warps' partial sums (two sets, alternating) and
-//     frees the row's buffer at the same time.
+//     frees the row's buffer at the same time.  A wait that runs out costs the ring, not the rows: from there on the block
+//     reads rows with plain loads, and leaves when its copies have landed.
 //   * few rows (a decode step): one row per CTA, all loads issued at once; what counts is latency.
 // fp32 sums; the normalisation sees the residual stream as it is stored (rounded).
 // Measured on B200, bf16 with residual: 16384 x 8192 in 182.5 us (5.9 TB/s; 280.4 us before), 4096 x 8192 in 47.6 us,
@@ -37,6 +38,7 @@ struct LocalNorm {
   int rows, hidden;
   float eps;
   int stages;
+  uint32_t polls;  // of a wait for a row
 };
 
 __device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -115,8 +117,12 @@ __global__ void __launch_bounds__(kThreadsN) norm_stream_kernel(const __grid_con
   __syncthreads();
   int stage = 0, set = 0;
   uint32_t phase = 0;
+  bool ring = true;  // the same in every thread
+  long long late_row = -1;
+  int late_stage = 0;
+  uint32_t late_phase = 0;
   for (long long row = blockIdx.x; row < a.rows; row += gridDim.x) {
-    const bool landed = ptx::mbar_wait(&full[stage], phase, abort);
+    const bool landed = ring && ptx::mbar_wait(&full[stage], phase, abort, a.polls);
     const uint8_t* src = smem + size_t(stage) * stage_bytes;
     const size_t off = size_t(row) * row_bytes;
     float v[PPT][8];
@@ -132,11 +138,32 @@ __global__ void __launch_bounds__(kThreadsN) norm_stream_kernel(const __grid_con
           ss += take_pack<T>(a, xv, rv, off + size_t(p) * 16, v[j]);
         }
       }
+    } else {
+      // A thread reads only what it writes itself (in place: the packs of this row), so one that saw its row land and
+      // one that did not can work side by side.
+#pragma unroll
+      for (int j = 0; j < PPT; ++j) {
+        const int p = threadIdx.x + j * kThreadsN;
+        if (p < packs) {
+          const uint4 xv = ptx::ld_v4(a.x + off + size_t(p) * 16);
+          uint4 rv = xv;
+          if (a.res != nullptr) rv = ptx::ld_v4(a.res + off + size_t(p) * 16);
+          ss += take_pack<T>(a, xv, rv, off + size_t(p) * 16, v[j]);
+        }
+      }
     }
     ss = warp_sum(ss);
     if ((threadIdx.x & 31) == 0) part[set][warp] = ss;
-    if (!__syncthreads_and(landed)) break;  // a copy never landed: the whole block gives up
-    if (threadIdx.x == 0) {
+    const bool all_landed = __syncthreads_and(landed);
+    if (ring && !all_landed) {
+      ring = false;
+      if (threadIdx.x == 0) {  // the copies in flight: this row's and those of the next rows
+        late_row = row;
+        late_stage = stage;
+        late_phase = phase;
+      }
+    }
+    if (ring && threadIdx.x == 0) {
       const long long next = row + static_cast<long long>(a.stages) * gridDim.x;
       if (next < a.rows) issue(next, stage);
     }
@@ -161,9 +188,15 @@ __global__ void __launch_bounds__(kThreadsN) norm_stream_kernel(const __grid_con
       phase ^= 1;
     }
   }
-  if (*abort != 0) {  // copies in flight land before shared memory is released
-    const uint64_t t0 = ptx::globaltimer_ns();
-    while (ptx::globaltimer_ns() - t0 < 200000) __nanosleep(1000);
+  if (late_row >= 0) {  // copies in flight land before shared memory is released
+    int gave_up = 0;
+    for (int s = 0; s < a.stages && late_row < a.rows; ++s, late_row += gridDim.x) {
+      ptx::mbar_wait(&full[late_stage], late_phase, &gave_up);
+      if (++late_stage == a.stages) {
+        late_stage = 0;
+        late_phase ^= 1;
+      }
+    }
   }
 }
 
@@ -243,7 +276,8 @@ cudaError_t launch_stream(LocalNorm n, int max_ctas, cudaStream_t stream) {
     attr_set.fetch_or(uint64_t(1) << (dev & 63), std::memory_order_relaxed);
   }
   const int stage_bytes = n.hidden * 2 * (n.res != nullptr ? 2 : 1);
-  // Three rows of the ring in at most 110 KiB, so that at least two CTAs share an SM.
+  // Three rows of the ring, or two, in at most 110 KiB, so that two CTAs share an SM.  Two rows it is in any case: from 13832
+  // elements with a residual on they leave room for one CTA only.
   n.stages = 110 * 1024 / stage_bytes;
   if (n.stages > 3) n.stages = 3;
   if (n.stages < 2) n.stages = 2;
@@ -277,7 +311,7 @@ cudaError_t dispatch(const LocalNorm& n, int max_ctas, cudaStream_t stream) {
 
 }  // namespace
 
-cudaError_t launch_norm_local(int rank, const NormArgs& a, int max_ctas, cudaStream_t stream) {
+cudaError_t launch_norm_local(int rank, const NormArgs& a, int max_ctas, cudaStream_t stream, uint32_t polls) {
   if (a.hidden > 8 * 8 * kThreadsN) return cudaErrorInvalidValue;  // 16384
   LocalNorm n{};
   n.x = static_cast<const char*>(a.x.p[rank]);
@@ -288,6 +322,7 @@ cudaError_t launch_norm_local(int rank, const NormArgs& a, int max_ctas, cudaStr
   n.rows = a.rows;
   n.hidden = a.hidden;
   n.eps = a.eps;
+  n.polls = polls;
   if (a.rows == 0) return cudaSuccess;
   if (max_ctas < 1) max_ctas = 1;
   return a.dtype == kF16 ? dispatch<__half>(n, max_ctas, stream) : dispatch<__nv_bfloat16>(n, max_ctas, stream);

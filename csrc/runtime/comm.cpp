@@ -941,22 +941,40 @@ int oob_all_to_all(oob_comm* c, int dtype, int out_reg, uint64_t out_off, const 
   return OOB_OK;
 }
 
+// Local normalisation needs no communicator: x_off carries the address of x.
+static int local_norm_args(int algo, const oob_norm_args_t* a, NormArgs* n) {
+  if (algo != OOB_NORM_LOCAL) return set_error(OOB_ERR_INVALID, "fused norm algorithms need a communicator");
+  if (a->weight == nullptr || a->y_local == nullptr || (a->x_off & 15)) return set_error(OOB_ERR_INVALID, "bad argument");
+  n->dtype = a->dtype;
+  n->rows = a->rows;
+  n->hidden = a->hidden;
+  n->eps = a->eps;
+  n->x.p[0] = reinterpret_cast<void*>(static_cast<uintptr_t>(a->x_off));
+  n->residual = a->residual;
+  n->weight = a->weight;
+  n->y_local = a->y_local;
+  n->res_out_local = a->res_out_local;
+  return OOB_OK;
+}
+
+int oob_test_norm_late_rows(const oob_norm_args_t* a, int max_ctas, void* stream) {
+  if (a == nullptr) return set_error(OOB_ERR_INVALID, "null argument");
+  NormArgs n{};
+  int rc = local_norm_args(OOB_NORM_LOCAL, a, &n);
+  if (rc != OOB_OK) return rc;
+  if (a->hidden <= 0 || a->hidden % 8 != 0 || a->rows < 0 || (a->dtype != OOB_F16 && a->dtype != OOB_BF16))
+    return set_error(OOB_ERR_INVALID, "bad shape");
+  cudaError_t e = launch_norm_local(0, n, max_ctas > 0 ? max_ctas : 148 * 8, static_cast<cudaStream_t>(stream), 0);
+  if (e != cudaSuccess) return cuda_fail(e, "rmsnorm launch");
+  return OOB_OK;
+}
+
 int oob_fused_norm(oob_comm* c, int algo, const oob_norm_args_t* a, int max_ctas, void* stream) {
   if (a == nullptr) return set_error(OOB_ERR_INVALID, "null argument");
   if (c == nullptr) {
-    // Local normalisation needs no communicator: x_off carries the address of x.
-    if (algo != OOB_NORM_LOCAL) return set_error(OOB_ERR_INVALID, "fused norm algorithms need a communicator");
-    if (a->weight == nullptr || a->y_local == nullptr || (a->x_off & 15)) return set_error(OOB_ERR_INVALID, "bad argument");
     NormArgs n{};
-    n.dtype = a->dtype;
-    n.rows = a->rows;
-    n.hidden = a->hidden;
-    n.eps = a->eps;
-    n.x.p[0] = reinterpret_cast<void*>(static_cast<uintptr_t>(a->x_off));
-    n.residual = a->residual;
-    n.weight = a->weight;
-    n.y_local = a->y_local;
-    n.res_out_local = a->res_out_local;
+    int rc = local_norm_args(algo, a, &n);
+    if (rc != OOB_OK) return rc;
     CommCtx ctx{};
     ctx.world = 1;
     ctx.rank = 0;

@@ -158,6 +158,7 @@ def _declare(lib) -> None:
     lib.oob_topology_json.argtypes = [c_char_p, c_uint64, c_int]
     lib.oob_topology_describe.argtypes = [c_char_p, c_uint64, c_uint, POINTER(c_int), c_int]
     lib.oob_test_bounded_wait.argtypes = [P, P]
+    lib.oob_test_norm_late_rows.argtypes = [POINTER(NormArgs), c_int, P]
     lib.oob_bootstrap_create.argtypes = [c_int, c_int, c_char_p, c_int, POINTER(P)]
     lib.oob_bootstrap_destroy.argtypes = [P]
     lib.oob_bootstrap_allgather.argtypes = [P, P, P, c_uint64]

@@ -35,3 +35,27 @@ def test_rmsnorm_in_place():
         rmsnorm(x, w, 1e-5, r, out=x, residual_out=r)
         torch.cuda.synchronize()
         assert torch.equal(r, r_ref) and ((x.float() - y_ref.float()).abs() <= 2.0 ** -7 * y_ref.float().abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("rows,hidden,residual,max_ctas", [(297, 2056, True, 0), (700, 4104, False, 0), (1000, 8192, True, 0),
+                                                           (300, 16384, True, 0), (2500, 3072, True, 5)])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_rows_that_arrive_too_late_are_still_normalised(rows, hidden, residual, max_ctas, in_place):
+    """A wait of the streaming kernel that runs out (here: at once) must not lose a row."""
+    from ooverlap_b200 import _lib
+    from ooverlap_b200.ops import rmsnorm
+    x = torch.randn(rows, hidden, device="cuda").bfloat16()
+    r = torch.randn_like(x) if residual else None
+    w = (1 + 0.1 * torch.randn(hidden, device="cuda")).bfloat16()
+    want = rmsnorm(x, w, 1e-5, r)
+    want = want if residual else (want,)
+    y = x if in_place else torch.full_like(x, float("nan"))
+    ro = (r if in_place else torch.full_like(x, float("nan"))) if residual else None
+    a = _lib.NormArgs()
+    a.dtype, a.rows, a.hidden, a.eps = _lib.BF16, rows, hidden, 1e-5
+    a.x_reg, a.x_off, a.weight, a.y_local, a.res_out_reg = 0, x.data_ptr(), w.data_ptr(), y.data_ptr(), -1
+    a.residual = r.data_ptr() if residual else None
+    a.res_out_local = ro.data_ptr() if residual else None
+    _lib.check(_lib.lib().oob_test_norm_late_rows(a, max_ctas, torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert torch.equal(y, want[0]) and (not residual or torch.equal(ro, want[1]))
