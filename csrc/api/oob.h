@@ -277,6 +277,8 @@ int oob_pad_counter_count(void);
  * whole tiles, -2 for the part that starts a tile: its pair owns the tile and parks nothing), parts of the tile, first
  * pair of the tile.  Returns the item count, -1 when cap is too small. */
 int oob_test_pair_schedule(int mode, int M, int N, int K, int pairs, int stream_k, int world, int rank, int* out, int cap);
+/* Columns of the tiles of that schedule (rows: 256). */
+int oob_test_pair_tile_columns(int mode, int M, int N, int K, int pairs, int stream_k);
 
 /* Test hook: the local norm of oob_fused_norm(NULL, OOB_NORM_LOCAL, ...) whose waits for the rows of its ring run out at
  * once, so that every row takes the way of a row that arrives late. */

@@ -147,6 +147,13 @@ void pair_streamk_plan(int tiles, int pairs, int num_kb, int* sk_tiles, int* sk_
 // 23.3 at 256, 2048 x 8192 x 8192 182 at 224 and 193 with the tail, 2048 x 2048 x 2048 17.2 at 256 and 25.7 with the tail;
 // 4096 x 7168 x 8192 305 with the tail and 310 at 224.
 int pair_tile_columns(int M, int N, int num_kb, int pairs, bool stream_k);
+// How a problem is cut into tiles on `pairs` pairs.  `order`: a tile-order record is written.
+struct PairCut {
+  int tile_n;  // columns of a tile
+  int tiles;
+  int sk_tiles, sk_pairs;  // stream-K tail (256-column tiles), both 0 without one
+};
+PairCut pair_cut(int mode, int M, int N, int K, int pairs, int stream_k, bool swiglu, bool emulated, bool order);
 // Microseconds the two-SM kernel is expected to take (plain, or with the SwiGLU epilogue); 0 beyond three rounds of tiles.
 double pair_cost_us(int M, int N, int K, int pairs, bool swiglu);
 

@@ -1163,6 +1163,11 @@ int oob_test_pair_schedule(int mode, int M, int N, int K, int pairs, int stream_
   return pair_schedule_dump(mode, M, N, K, pairs, stream_k, world, rank, out, cap);
 }
 
+int oob_test_pair_tile_columns(int mode, int M, int N, int K, int pairs, int stream_k) {
+  if (M <= 0 || N <= 0 || K <= 0 || pairs < 1) return -1;
+  return pair_cut(mode, M, N, K, pairs, stream_k, false, false, false).tile_n;
+}
+
 uint64_t oob_gemm_splitk_bytes(int M, int N, int K, int max_ctas, int splits) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   return gemm_splitk_bytes(M, N, K, max_ctas, splits);

@@ -1,4 +1,4 @@
-"""Work schedule of the two-SM GEMM (whole tiles round robin + stream-K tail), enumerated on the host through the
+"""Work schedule of the two-SM GEMM (whole tiles round robin, of 256 columns or fewer, or a stream-K tail), enumerated on the host through the
 test hook ``oob_test_pair_schedule`` (the kernel runs the same code on the device).
 
 Checked for many shapes and pair counts: every (tile, K block) is computed exactly once; a pair parks at most one
@@ -22,8 +22,13 @@ def schedule(mode, M, N, K, pairs, stream_k, world=1, rank=0):
     return [tuple(buf[i * 9:(i + 1) * 9]) for i in range(n)]
 
 
+def columns(mode, M, N, K, pairs, stream_k):
+    return _lib.lib().oob_test_pair_tile_columns(mode, M, N, K, pairs, stream_k)
+
+
 SHAPES = [(512, 8192, 8192), (2048, 8192, 8192), (8192, 8192, 8192), (4096, 3584, 8192), (4096, 8192, 3584),
-          (300, 520, 1024), (256, 256, 64), (1024, 1024, 4096), (2304, 768, 2048), (128 * 9, 256 * 5, 8192)]
+          (300, 520, 1024), (256, 256, 64), (1024, 1024, 4096), (2304, 768, 2048), (128 * 9, 256 * 5, 8192),
+          (250, 8192, 3584), (1037, 4104, 2056), (2048, 2048, 2048), (129, 40, 72)]
 
 
 @pytest.mark.parametrize("pairs", [74, 70, 66, 7, 3, 2, 1])
@@ -31,7 +36,9 @@ SHAPES = [(512, 8192, 8192), (2048, 8192, 8192), (8192, 8192, 8192), (4096, 3584
 def test_every_k_block_of_every_tile_is_computed_once(pairs, stream_k):
     for M, N, K in SHAPES:
         items = schedule(PLAIN, M, N, K, pairs, stream_k)
-        tm, tn, nkb = (M + 255) // 256, (N + 255) // 256, (K + 63) // 64
+        width = columns(PLAIN, M, N, K, pairs, stream_k)
+        assert width % 32 == 0 and 128 <= width <= 256 and (width == 256 or stream_k <= 0)
+        tm, tn, nkb = (M + 255) // 256, (N + width - 1) // width, (K + 63) // 64
         cover = {}
         slots = set()
         per_pair = {}
@@ -90,22 +97,33 @@ def test_stream_k_balances_the_last_wave():
             load = {}
             for p, seq, mb, nb, kb0, kb1, slot, parts, first in schedule(PLAIN, M, N, K, pairs, -1):
                 load[p] = load.get(p, 0) + kb1 - kb0
-            tiles = ((M + 255) // 256) * ((N + 255) // 256)
+            width = columns(PLAIN, M, N, K, pairs, -1)
+            tiles = ((M + 255) // 256) * ((N + width - 1) // width)
             if tiles % pairs:
                 assert max(load.values()) - min(load.get(p, 0) for p in range(pairs)) == nkb
 
 
+def _tail(mode, M, N, K, pairs=74):
+    return any(item[6] >= 0 for item in schedule(mode, M, N, K, pairs, 0))
+
+
 def test_auto_rule_picks_a_tail_only_where_it_pays():
-    # 8192^3 on 74 pairs wastes 1.2 % of the last wave: whole tiles only; 2048 rows waste 13 % and have a whole wave:
-    # tail; 512 rows are less than a wave of tiles with operands beyond L2: whole tiles (measured slower with a tail);
-    # the all-gather shape's operands fit L2: tail
-    assert all(s[6] == -1 for s in schedule(PLAIN, 8192, 8192, 8192, 74, 0))
-    assert any(s[6] >= 0 for s in schedule(PLAIN, 2048, 8192, 8192, 74, 0))
-    assert all(s[6] == -1 for s in schedule(PLAIN, 512, 8192, 8192, 74, 0))
-    assert any(s[6] >= 0 for s in schedule(PLAIN, 4096, 3584, 8192, 74, 0))
-    assert any(s[6] >= 0 for s in schedule(PLAIN, 512, 2048, 2048, 74, 0))
-    # shallow K (tensor-parallel shards) is never cut
-    assert all(s[6] == -1 for s in schedule(PLAIN, 2048, 8192, 512, 74, 0))
+    # 8192^3 on 74 pairs wastes 1.2 % of the last wave: whole tiles only
+    assert not _tail(PLAIN, 8192, 8192, 8192) and columns(PLAIN, 8192, 8192, 8192, 74, 0) == 256
+    # less than a wave of tiles with operands beyond L2: a tail measured slower, narrower tiles fill the wave
+    assert not _tail(PLAIN, 512, 8192, 8192) and columns(PLAIN, 512, 8192, 8192, 74, 0) == 224
+    # a quarter of the last wave idle and no narrower width that fills it: tail
+    assert _tail(PLAIN, 4096, 3584, 8192)
+    # few tiles, shallow K: parking and adding accumulators costs more than the idle pairs
+    assert not _tail(PLAIN, 512, 2048, 2048) and columns(PLAIN, 512, 2048, 2048, 74, 0) == 128
+    # K of a tensor-parallel shard is never cut
+    assert not _tail(PLAIN, 2048, 8192, 512)
+
+
+def test_all_gather_keeps_whole_columns_and_the_tail():
+    # the chunk flags of an all-gather count 256-column tiles: a tail is the only way to fill the last wave
+    assert _tail(AG, 4096, 3584, 8192) and _tail(AG, 2048, 8192, 8192)
+    assert all(columns(mode, M, N, K, 70, 0) == 256 for mode in (AR, RS, AG) for M, N, K in SHAPES)
 
 
 @pytest.mark.parametrize("world", [2, 4, 8])
