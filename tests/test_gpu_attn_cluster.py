@@ -25,3 +25,36 @@ def test_attention_lengths_and_clusters(B, H, KV, L, bound, splits, dtype):
     # probabilities and the result are each rounded once to the 16-bit type; values are about 1, at most about 5
     tol = 2e-2 if dtype == torch.bfloat16 else 4e-3
     assert (out.float() - ref).abs().max().item() <= tol * max(1.0, ref.abs().max().item())
+
+
+def test_split_calls_on_two_streams_and_in_a_graph():
+    """Partial results belong to their call: neither a call on another stream nor a replayed graph touches them."""
+    from ooverlap_b200.ops import attn_decode
+    g = torch.Generator(device="cuda").manual_seed(9)
+
+    def state(B):
+        return (torch.randn(B, 32, 128, device="cuda", generator=g).bfloat16(),
+                *(torch.randn(B, 8, 3000, 128, device="cuda", generator=g).bfloat16() for _ in range(2)))
+    small, other, large = state(2), state(2), state(6)
+    want = [attn_decode(*s, 2999, splits=5).clone() for s in (small, other, large)]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    got = [[], []]
+    for _ in range(20):
+        for i, s in enumerate((small, other)):
+            with torch.cuda.stream(streams[i]):
+                got[i].append(attn_decode(*s, 2999, splits=5))
+    torch.cuda.synchronize()
+    assert all(torch.equal(x, want[i]) for i in range(2) for x in got[i])
+    out = torch.empty_like(want[0])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        attn_decode(*small, 2999, splits=5, out=out)
+    assert torch.equal(attn_decode(*large, 2999, splits=5), want[2])
+    guard = [torch.full((1 << 18,), 7.0, device="cuda") for _ in range(16)]  # may land where an outgrown workspace was
+    for _ in range(3):
+        out.zero_()
+        graph.replay()
+        assert torch.equal(attn_decode(*large, 2999, splits=5), want[2])
+    torch.cuda.synchronize()
+    assert torch.equal(out, want[0]) and all((x == 7.0).all() for x in guard)
