@@ -59,6 +59,8 @@ int oob_attn_decode(const oob_attn_decode_args_t* a, void* stream);
 /* Split count oob_attn_decode picks for splits == 0. */
 int oob_attn_decode_auto_splits(int B, int KV, int len_bound);
 uint64_t oob_attn_decode_workspace_bytes(int B, int H, int splits);
+/* Test hook (host only): CTAs that share the keys of one of `items` (sequence, KV head) pairs. */
+int oob_test_attn_cluster_size(long long items, int len_bound);
 
 #pragma GCC visibility pop
 #ifdef __cplusplus
