@@ -2,13 +2,13 @@
 //
 // Bound by memory: x and the residual are read once, y and the new residual written once, and nothing is reused but the
 // norm weight.  Two kernels:
-//   * many rows: a CTA walks rows b, b + G, ...; rows arrive through a ring of bulk copies (cp.async.bulk, one thread
+//   * many long rows: a CTA walks rows b, b + G, ...; rows arrive through a ring of bulk copies (cp.async.bulk, one thread
 //     issues them), so the loads of the next rows are in flight while a row is summed, scaled and written.  The old form (plain
 //     loads, three block barriers per row, loads of a row issued only when the row before was done) kept too little in
 //     flight.  One block barrier per row: it publishes the warps' partial sums (two sets, alternating) and
 //     frees the row's buffer at the same time.  A wait that runs out costs the ring, not the rows: from there on the block
 //     reads rows with plain loads, and leaves when its copies have landed.
-//   * few rows (a decode step): one row per CTA, all loads issued at once; what counts is latency.
+//   * few rows (a decode step), or short ones: one row per CTA, all loads issued at once; what counts is latency.
 // fp32 sums; the normalisation sees the residual stream as it is stored (rounded).
 // Measured on B200, bf16 with residual: 16384 x 8192 in 182.5 us (5.9 TB/s; 280.4 us before), 4096 x 8192 in 47.6 us,
 // 1024 x 8192 in 11.0 us, 16 rows in 2.2 us as a link of a chain of launches.
@@ -76,9 +76,58 @@ __device__ __forceinline__ float take_pack(const LocalNorm& a, const uint4& xv, 
   return ss;
 }
 
+// The rows `row`, row + G, ... of a block whose ring was given up, with plain loads.  `summed`: this thread has seen the first of
+// them land, and has stored its packs of the sum where a.ro asks for it (in place, over an input), before the block learned
+// that others have not.  One pack at a time and two passes, so that it asks for no more registers than the streaming loop.
+template <typename T>
+__device__ __forceinline__ void finish_rows(const LocalNorm& a, int row, bool summed, float (*part)[kWarpsN]) {
+  using PT = PackTraits<T>;
+  const int packs = a.hidden / 8;
+  int set = 0;
+#pragma unroll 1
+  for (; row < a.rows; row += gridDim.x, set ^= 1, summed = false) {
+    const size_t off = size_t(row) * a.hidden * 2;
+    float v[8], ss = 0.f;
+#pragma unroll 1
+    for (int p = threadIdx.x; p < packs; p += kThreadsN) {
+      const size_t at = off + size_t(p) * 16;
+      LocalNorm from = a;
+      if (summed && a.ro != nullptr) {
+        from.x = a.ro;
+        from.res = nullptr;
+      }
+      const uint4 xv = ptx::ld_v4(from.x + at);
+      ss += take_pack<T>(from, xv, from.res != nullptr ? ptx::ld_v4(from.res + at) : xv, at, v);
+    }
+    ss = warp_sum(ss);
+    if ((threadIdx.x & 31) == 0) part[set][threadIdx.x >> 5] = ss;
+    __syncthreads();
+    float total = 0.f;
+#pragma unroll
+    for (int i = 0; i < kWarpsN; ++i) total += part[set][i];
+    const float scale = rsqrtf(total / float(a.hidden) + a.eps);
+#pragma unroll 1
+    for (int p = threadIdx.x; p < packs; p += kThreadsN) {
+      const size_t at = off + size_t(p) * 16;
+      float w[8];
+      PT::unpack(ptx::ld_v4(a.w + size_t(p) * 16), w);
+      PT::unpack(ptx::ld_v4((a.ro != nullptr ? a.ro : a.x) + at), v);
+      if (a.ro == nullptr && a.res != nullptr) {
+        float r[8];
+        PT::unpack(ptx::ld_v4(a.res + at), r);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] += r[i];
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = v[i] * scale * w[i];
+      ptx::st_v4(a.y + at, PT::pack(v));
+    }
+  }
+}
+
 // PPT: 16-byte packs per thread and row.
 template <typename T, int PPT>
-__global__ void __launch_bounds__(kThreadsN) norm_stream_kernel(const __grid_constant__ LocalNorm a) {
+__global__ void __launch_bounds__(kThreadsN, PPT <= 2 ? 5 : PPT <= 4 ? 3 : 1) norm_stream_kernel(const __grid_constant__ LocalNorm a) {
   using PT = PackTraits<T>;
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ uint64_t full[kMaxStagesN];
@@ -89,7 +138,7 @@ __global__ void __launch_bounds__(kThreadsN) norm_stream_kernel(const __grid_con
   const uint32_t stage_bytes = row_bytes * (a.res != nullptr ? 2 : 1);
   const int warp = threadIdx.x >> 5;
   volatile int* abort = &abort_word;
-  auto issue = [&](long long row, int stage) {
+  auto issue = [&](int row, int stage) {
     uint8_t* dst = smem + size_t(stage) * stage_bytes;
     ptx::mbar_arrive_expect_tx(&full[stage], stage_bytes);
     bulk_load(dst, a.x + size_t(row) * row_bytes, row_bytes, &full[stage]);
@@ -104,7 +153,7 @@ __global__ void __launch_bounds__(kThreadsN) norm_stream_kernel(const __grid_con
   ptx::griddep_wait();
   if (threadIdx.x == 0) {
     for (int s = 0; s < a.stages; ++s) {
-      const long long row = blockIdx.x + static_cast<long long>(s) * gridDim.x;
+      const int row = blockIdx.x + s * gridDim.x;
       if (row < a.rows) issue(row, s);
     }
   }
@@ -117,12 +166,10 @@ __global__ void __launch_bounds__(kThreadsN) norm_stream_kernel(const __grid_con
   __syncthreads();
   int stage = 0, set = 0;
   uint32_t phase = 0;
-  bool ring = true;  // the same in every thread
-  long long late_row = -1;
-  int late_stage = 0;
-  uint32_t late_phase = 0;
-  for (long long row = blockIdx.x; row < a.rows; row += gridDim.x) {
-    const bool landed = ring && ptx::mbar_wait(&full[stage], phase, abort, a.polls);
+  int row = blockIdx.x;
+  bool landed = true;
+  for (; row < a.rows; row += gridDim.x) {
+    landed = ptx::mbar_wait(&full[stage], phase, abort, a.polls);
     const uint8_t* src = smem + size_t(stage) * stage_bytes;
     const size_t off = size_t(row) * row_bytes;
     float v[PPT][8];
@@ -138,33 +185,12 @@ __global__ void __launch_bounds__(kThreadsN) norm_stream_kernel(const __grid_con
           ss += take_pack<T>(a, xv, rv, off + size_t(p) * 16, v[j]);
         }
       }
-    } else {
-      // A thread reads only what it writes itself (in place: the packs of this row), so one that saw its row land and
-      // one that did not can work side by side.
-#pragma unroll
-      for (int j = 0; j < PPT; ++j) {
-        const int p = threadIdx.x + j * kThreadsN;
-        if (p < packs) {
-          const uint4 xv = ptx::ld_v4(a.x + off + size_t(p) * 16);
-          uint4 rv = xv;
-          if (a.res != nullptr) rv = ptx::ld_v4(a.res + off + size_t(p) * 16);
-          ss += take_pack<T>(a, xv, rv, off + size_t(p) * 16, v[j]);
-        }
-      }
     }
     ss = warp_sum(ss);
     if ((threadIdx.x & 31) == 0) part[set][warp] = ss;
-    const bool all_landed = __syncthreads_and(landed);
-    if (ring && !all_landed) {
-      ring = false;
-      if (threadIdx.x == 0) {  // the copies in flight: this row's and those of the next rows
-        late_row = row;
-        late_stage = stage;
-        late_phase = phase;
-      }
-    }
-    if (ring && threadIdx.x == 0) {
-      const long long next = row + static_cast<long long>(a.stages) * gridDim.x;
+    if (!__syncthreads_and(landed)) break;  // a copy did not land in time: the same in every thread
+    if (threadIdx.x == 0) {
+      const int next = row + a.stages * int(gridDim.x);
       if (next < a.rows) issue(next, stage);
     }
     float total = 0.f;
@@ -188,13 +214,16 @@ __global__ void __launch_bounds__(kThreadsN) norm_stream_kernel(const __grid_con
       phase ^= 1;
     }
   }
-  if (late_row >= 0) {  // copies in flight land before shared memory is released
-    int gave_up = 0;
-    for (int s = 0; s < a.stages && late_row < a.rows; ++s, late_row += gridDim.x) {
-      ptx::mbar_wait(&full[late_stage], late_phase, &gave_up);
-      if (++late_stage == a.stages) {
-        late_stage = 0;
-        late_phase ^= 1;
+  if (row < a.rows) {
+    finish_rows<T>(a, row, landed, part);
+    if (threadIdx.x == 0) {  // copies in flight (this row's and the next rows') land before shared memory is released
+      int gave_up = 0;
+      for (int s = 0; s < a.stages && row < a.rows; ++s, row += gridDim.x) {
+        ptx::mbar_wait(&full[stage], phase, &gave_up);
+        if (++stage == a.stages) {
+          stage = 0;
+          phase ^= 1;
+        }
       }
     }
   }
@@ -294,10 +323,18 @@ cudaError_t launch_stream(LocalNorm n, int max_ctas, cudaStream_t stream) {
 template <typename T>
 cudaError_t dispatch(const LocalNorm& n, int max_ctas, cudaStream_t stream) {
   const int packs = n.hidden / 8;
-  // Up to two rows per SM nothing is gained by a ring: every row is in flight at once (256 x 8192: 3.6 us).
-  if (n.rows <= 2 * kSmPerGpu) {
+  // Up to two rows per SM nothing is gained by a ring: every row is in flight at once (256 x 8192: 3.6 us).  Nor is it, however
+  // many rows there are, where a row is at most one pack per thread: what a row costs then is the wait, the barrier and the
+  // copies' set-up of the ring, while CTAs of one row each overlap freely.  With and without residual, one row per CTA
+  // against the ring: 4096 x 1024 7.2 and 4.4 against 9.2 and 7.9 us, 16384 x 128 14.3 and 9.4 against 23.4 and
+  // 21.7, 16384 x 2048 44.1 and 25.5 against 45.1 and 27.6; at 16384 x 2560 the ring is ahead, 62.9 and 32.5 against 67.3 and 41.9.
+  // With a residual and very many rows of 513 - 1024 elements eight CTAs of 128 threads per SM have too little in flight: 16384 x
+  // 1024 29.7 against 27.1 (4096 x 1000 still 7.4 against 9.2).
+  const bool few_in_flight = n.res != nullptr && packs > 64 && packs <= 128 && n.rows > 8192;
+  if (n.rows <= 2 * kSmPerGpu || (packs <= kThreadsN && !few_in_flight)) {
     const int grid = n.rows < max_ctas ? n.rows : max_ctas;
     if (packs <= 128) return launch(norm_rows_kernel<T, 128, 1>, grid, 128, 0, n, stream);
+    if (packs <= 256) return launch(norm_rows_kernel<T, 256, 1>, grid, 256, 0, n, stream);
     if (packs <= 512) return launch(norm_rows_kernel<T, 512, 1>, grid, 512, 0, n, stream);
     if (packs <= 1024) return launch(norm_rows_kernel<T, 512, 2>, grid, 512, 0, n, stream);
     return launch(norm_rows_kernel<T, 512, 4>, grid, 512, 0, n, stream);

@@ -7,7 +7,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("rows,hidden", [(1, 8), (3, 1000), (296, 4104), (297, 8), (297, 2048), (600, 2056), (1000, 8192), (2500, 1024),
-                                         (300, 16384), (5, 16384)])
+                                         (300, 16384), (5, 16384), (2000, 2048), (900, 1032), (8192, 1024), (8193, 520), (8193, 1024), (9000, 1032),
+                                         (310, 2056)])
 @pytest.mark.parametrize("residual,max_ctas", [(True, 0), (False, 0), (True, 3)])
 def test_rmsnorm_rows_and_widths(rows, hidden, residual, max_ctas, dtype):
     from ooverlap_b200.ops import rmsnorm, rmsnorm_reference
