@@ -59,8 +59,9 @@ int oob_attn_decode(const oob_attn_decode_args_t* a, void* stream);
 /* Split count oob_attn_decode picks for splits == 0. */
 int oob_attn_decode_auto_splits(int B, int KV, int len_bound);
 uint64_t oob_attn_decode_workspace_bytes(int B, int H, int splits);
-/* Test hook (host only): CTAs that share the keys of one of `items` (sequence, KV head) pairs. */
-int oob_test_attn_cluster_size(long long items, int len_bound);
+/* Test hook (host only): CTAs that share the keys of one of `items` (sequence, KV head) pairs on a device that runs 296 CTAs of
+ * the kernel at once, and as many of them in clusters of 2, 4 and 8 as given. */
+int oob_test_attn_cluster_size(long long items, int len_bound, int slots2, int slots4, int slots8);
 
 #pragma GCC visibility pop
 #ifdef __cplusplus

@@ -19,6 +19,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstdlib>
+#include <mutex>
 #include <type_traits>
 
 #include "../api/oob.h"
@@ -159,9 +160,9 @@ constexpr int kAttnThreads = kAttnWarps * 32;
 constexpr int kRowBytes = kHD * 2;                 // 256
 constexpr int kKvTileBytes = kTileKeys * kRowBytes;  // 4 KiB
 constexpr int kMaxAttnCluster = 8;                 // portable cluster size
-// Pipeline depth per warp (tiles of K and V in flight or in use): 3 by default (96 KiB per CTA, two CTAs per SM).
-__host__ __device__ constexpr int attn_warp_buf_bytes(int stages) { return stages * 2 * kKvTileBytes; }
-__host__ __device__ constexpr int attn_smem_bytes(int stages) { return kAttnWarps * attn_warp_buf_bytes(stages); }
+constexpr int kAttnStages = 3;                     // tiles of K and V in flight or in use per warp (96 KiB per CTA, two per SM)
+constexpr int kWarpBufBytes = kAttnStages * 2 * kKvTileBytes;
+__host__ __device__ constexpr int attn_smem_bytes() { return kAttnWarps * kWarpBufBytes; }
 constexpr int kPartialStride = kHD + 2;            // fp32 words of one partial result: 128 values, max, sum
 
 template <typename T>
@@ -240,10 +241,10 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t smem_addr, uint32_t ran
 // Grid: (splits * S, KV, B) in clusters of S along x.  The keys of one (sequence, KV head) are dealt out in 16-key tiles
 // to the splits * S CTAs from the length the kernel finds on the device, so that a cache that is mostly empty, or a
 // length just past a multiple of anything, leaves no CTA with more than one tile per warp over its share.
-template <typename T, int STAGES, int S>
+template <typename T, int S>
 __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams p) {
-  constexpr int kWarpBufBytes = attn_warp_buf_bytes(STAGES);
-  static_assert(attn_smem_bytes(STAGES) >= (kAttnWarps + 1) * 16 * (kHD + 2) * 4, "merge buffers");
+  constexpr int STAGES = kAttnStages;
+  static_assert(attn_smem_bytes() >= (kAttnWarps + 1) * 16 * (kHD + 2) * 4, "merge buffers");
   extern __shared__ __align__(128) uint8_t attn_smem[];
   const int part = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -503,58 +504,113 @@ __global__ void attn_combine_kernel(const float* ws, void* out, int splits) {
   static_cast<T*>(out)[hrow * kHD + d] = to_out<T>(acc / l_tot);
 }
 
-template <typename T, int STAGES, int S>
+template <typename T, int S>
 cudaError_t launch_attn_s(const AttnParams& p, cudaStream_t stream) {
   static std::atomic<uint64_t> attr_done{0};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!(attr_done.load(std::memory_order_relaxed) >> (dev & 63) & 1)) {
-    cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<T, STAGES, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         attn_smem_bytes(STAGES));
+    cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         attn_smem_bytes());
     if (e != cudaSuccess) return e;
     attr_done.fetch_or(uint64_t(1) << (dev & 63), std::memory_order_relaxed);
   }
-  return launch_pdl(attn_decode_kernel<T, STAGES, S>, dim3(p.splits * S, p.KV, p.B), kAttnThreads, attn_smem_bytes(STAGES), stream, S, p);
+  return launch_pdl(attn_decode_kernel<T, S>, dim3(p.splits * S, p.KV, p.B), kAttnThreads, attn_smem_bytes(), stream, S, p);
 }
 
 template <typename T>
 cudaError_t launch_attn(const AttnParams& p, int cluster, cudaStream_t stream) {
   cudaError_t e;
   switch (cluster) {
-    case 1: e = launch_attn_s<T, 3, 1>(p, stream); break;
-    case 2: e = launch_attn_s<T, 3, 2>(p, stream); break;
-    case 4: e = launch_attn_s<T, 3, 4>(p, stream); break;
-    default: e = launch_attn_s<T, 3, 8>(p, stream); break;
+    case 1: e = launch_attn_s<T, 1>(p, stream); break;
+    case 2: e = launch_attn_s<T, 2>(p, stream); break;
+    case 4: e = launch_attn_s<T, 4>(p, stream); break;
+    default: e = launch_attn_s<T, 8>(p, stream); break;
   }
   if (e != cudaSuccess) return e;
   if (p.splits > 1) e = launch_pdl(attn_combine_kernel<T>, dim3(p.B * p.H), kHD, 0, stream, 1, p.ws, p.out, p.splits);
   return e;
 }
 
-// Nanoseconds for `items` (sequence, KV head) pairs of `len` keys with s CTAs each.  Two CTAs fit an SM; a full round of 296
-// shares the memory bandwidth (23 ns per key of a CTA), the CTAs of the last round get more of it, down to what their own
-// loads in flight allow (9 ns); starting a CTA and merging takes 2.6 us, 4.2 us in a cluster.
-double attn_cost_ns(long long items, int s, double len) {
-  constexpr int kSlots = 2 * 148;
-  const long long ctas = items * s, rounds = ctas / kSlots, rest = ctas % kSlots;
+// CTAs that run at once in clusters of 1, 2, 4 and 8.  Two fit an SM, but a cluster lives in one GPC, and how many SMs a GPC has
+// may differ from one GPU to the next: the device is asked.
+struct AttnSlots {
+  int n[4];
+};
+
+template <typename T, int S>
+int attn_slots_of() {
+  if (cudaFuncSetAttribute(attn_decode_kernel<T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem_bytes()) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(S * 2 * 148);
+  cfg.blockDim = dim3(kAttnThreads);
+  cfg.dynamicSmemBytes = attn_smem_bytes();
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = S;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, attn_decode_kernel<T, S>, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return clusters * S;
+}
+
+// The same kernel shape for both types: one answer per device.
+AttnSlots attn_slots() {
+  static std::mutex mu;
+  static AttnSlots cached[64];
+  static bool have[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> g(mu);
+  AttnSlots& s = cached[dev & 63];
+  if (!have[dev & 63]) {
+    s.n[0] = 2 * 148;
+    s.n[1] = attn_slots_of<__nv_bfloat16, 2>();
+    s.n[2] = attn_slots_of<__nv_bfloat16, 4>();
+    s.n[3] = attn_slots_of<__nv_bfloat16, 8>();
+    have[dev & 63] = true;
+  }
+  return s;
+}
+
+// Nanoseconds for `items` (sequence, KV head) pairs of `len` keys with s CTAs each, `slots` of which run at once.  A key takes a
+// CTA 8 ns where its own loads in flight are the limit and 23 ns where 296 CTAs share the memory's rate; the limits blend.
+// Starting a CTA and merging takes 2.6 us, 4.2 us in a cluster.
+double attn_cost_ns(long long items, int s, int slots, double len) {
+  slots -= slots % s;
+  const long long rounds = items * s / slots, rest = items * s % slots;
   const double keys = len / s, fixed = s > 1 ? 4200.0 : 2600.0;
-  const double last = 23.0 * rest / kSlots > 9.0 ? 23.0 * rest / kSlots : 9.0;
-  return rounds * (23.0 * keys + fixed) + (rest > 0 ? last * keys + fixed : 0.0);
+  auto ns_key = [](double ctas) {
+    const double shared = 23.0 * ctas / 296;
+    return std::cbrt(512.0 + shared * shared * shared);
+  };
+  return rounds * (ns_key(slots) * keys + fixed) + (rest > 0 ? ns_key(double(rest)) * keys + fixed : 0.0);
 }
 
 // CTAs of a cluster that share the keys of one (sequence, KV head).  The host knows a bound of the length, not the length, so a
-// size is weighed at the bound and at a quarter of it, each against one CTA: a cluster that gains little on a full cache
-// loses several times over on a short context, where all it adds is CTAs.  Timed with every size over 1057 combinations of
-// batch, heads, bound and length on B200, this choice is 1 % off the best one at full caches and 4 % over all lengths.  The
-// rule that looked at whole rounds at the bound only took four CTAs for 300 items of a 2048-key cache with 16 keys in it
-// (20.3 us, 5.6 with one) and for 600 items with 500 keys in it (68.5, 33.5).
-int attn_cluster_size(long long items, int len_bound) {
+// size is weighed at the bound and at a third of it, each against one CTA: a cluster that gains little on a full cache loses
+// several times over on a short context, where all it adds is CTAs.  Timed with every size over 1057 combinations of batch,
+// heads, bound and length on B200, this choice is 0.3 % off the best one at full caches and 4 % over all lengths.  The rule that
+// looked at whole rounds at the bound only took four CTAs for 300 items of a 2048-key cache with 16 keys in it (20.3 us, 5.6 with
+// one) and for 600 items with 500 keys in it (68.5, 33.5).
+int attn_cluster_size(long long items, int len_bound, const AttnSlots& slots) {
+  const double third = len_bound / 3.0;
+  const double one = attn_cost_ns(items, 1, slots.n[0], len_bound), one_third = attn_cost_ns(items, 1, slots.n[0], third);
   int best = 1;
   double best_cost = 2.0;
-  for (int s = 2; s <= kMaxAttnCluster; s *= 2) {
-    if (len_bound < s * 2 * kTileKeys * kAttnWarps) break;  // two tiles for every warp at least
-    const double cost = attn_cost_ns(items, s, len_bound) / attn_cost_ns(items, 1, len_bound) +
-                        attn_cost_ns(items, s, len_bound / 4.0) / attn_cost_ns(items, 1, len_bound / 4.0);
+  for (int i = 1; i < 4; ++i) {
+    const int s = 1 << i;
+    if (slots.n[i] < s || len_bound < s * kTileKeys * kAttnWarps) continue;
+    const double cost = attn_cost_ns(items, s, slots.n[i], len_bound) / one + attn_cost_ns(items, s, slots.n[i], third) / one_third;
     if (cost < best_cost) {
       best = s;
       best_cost = cost;
@@ -633,8 +689,9 @@ int oob_attn_decode_auto_splits(int B, int KV, int len_bound) {
   return static_cast<int>(s);
 }
 
-int oob_test_attn_cluster_size(long long items, int len_bound) {
-  return items > 0 && len_bound > 0 ? oob::model::attn_cluster_size(items, len_bound) : -1;
+int oob_test_attn_cluster_size(long long items, int len_bound, int slots2, int slots4, int slots8) {
+  if (items <= 0 || len_bound <= 0) return -1;
+  return oob::model::attn_cluster_size(items, len_bound, {{2 * 148, slots2, slots4, slots8}});
 }
 
 uint64_t oob_attn_decode_workspace_bytes(int B, int H, int splits) {
@@ -680,7 +737,11 @@ int oob_attn_decode(const oob_attn_decode_args_t* a, void* stream) {
   p.splits = splits;
   p.scale_log2 = a->scale * 1.4426950408889634f;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int cluster = attn_cluster_size(static_cast<long long>(a->B) * a->KV * splits, (bound + splits - 1) / splits);
+  AttnSlots slots = attn_slots();
+  // Behind a split launch waits the kernel that merges, and calls follow one another: clusters of eight that need every slot of
+  // the GPU then wait for the last ones (2 x 30000 keys on 8 KV heads 48 - 55 us in eights, 45 in fours; alone both 44).
+  if (splits > 1) slots.n[3] -= slots.n[3] / 4;
+  const int cluster = attn_cluster_size(static_cast<long long>(a->B) * a->KV * splits, (bound + splits - 1) / splits, slots);
   cudaError_t e = a->dtype == OOB_BF16 ? launch_attn<__nv_bfloat16>(p, cluster, s) : launch_attn<__half>(p, cluster, s);
   if (e != cudaSuccess) return cuda_fail(e, "attn_decode launch");
   return OOB_OK;

@@ -152,7 +152,7 @@ def _declare(lib) -> None:
     lib.oob_silu_mul.argtypes = [c_int, P, c_int64, P, c_int, c_int, P]
     lib.oob_attn_decode.argtypes = [POINTER(AttnDecodeArgs), P]
     lib.oob_attn_decode_auto_splits.argtypes = [c_int, c_int, c_int]
-    lib.oob_test_attn_cluster_size.argtypes = [ctypes.c_longlong, c_int]
+    lib.oob_test_attn_cluster_size.argtypes = [ctypes.c_longlong] + [c_int] * 4
     lib.oob_attn_decode_workspace_bytes.argtypes = [c_int, c_int, c_int]
     lib.oob_attn_decode_workspace_bytes.restype = c_uint64
     lib.oob_policy_load.argtypes = [c_char_p]
