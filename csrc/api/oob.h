@@ -209,7 +209,7 @@ typedef struct {
   int epilogue; /* plain mode: OOB_EPILOGUE_* applied to the fp32 sums.  1 and 2 are for split problems only
                    (oob_gemm_plan_splits > 1) */
   const void* epilogue_args; /* host pointer: oob_gemm_epilogue_swiglu_t or oob_rope_args_t (oob_model.h) */
-  int gemv;     /* plain mode, M <= 4: 1 = CUDA-core streaming kernel, 0 = by shape (M = 1 with N x K <= 32 M), -1 = never */
+  int gemv;     /* plain mode, M <= 4: 1 = CUDA-core streaming kernel, 0 = by shape (M = 1; M = 2 with small weights), -1 = never */
   int stream_k; /* two-SM kernel, plain and AG modes: stream-K tail; 0 = when it pays for the shape, 1 = whenever the
                    tile count leaves a remainder, -1 = never */
   void* order;  /* two-SM kernel: optional device buffer, 2 x uint64 per 128-row half of every 256x256 tile (index
@@ -219,7 +219,8 @@ typedef struct {
 #define OOB_EPILOGUE_NONE 0
 #define OOB_EPILOGUE_SWIGLU 1  /* N = 2F columns [gate | up]; C is [M, F] = silu(gate) * up */
 #define OOB_EPILOGUE_ROPE_KV 2 /* columns = (H + 2 KV) heads of hd: rotate q and k, q -> q_out, k and v -> cache; C unused */
-#define OOB_EPILOGUE_SWIGLU_TILE 3 /* as 1, for any problem: applied where a GEMM tile is written */
+#define OOB_EPILOGUE_SWIGLU_TILE 3 /* as 1, for any problem: applied where a GEMM tile is written.  OOB_ERR_UNSUPPORTED where no
+                                      kernel may (pair) or should (one row of a large weight): then oob_gemm + oob_silu_mul */
 typedef struct {
   int F;
 } oob_gemm_epilogue_swiglu_t;

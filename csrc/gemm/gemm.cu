@@ -283,16 +283,20 @@ cudaError_t launch_gemm(const CommCtx& ctx, const GemmArgs& args, cudaStream_t s
   int dev = 0;
   cudaGetDevice(&dev);
   if (a.mode == kGemmPlain) {
-    // One row of a weight matrix up to 32 M elements: the CUDA-core streaming kernel.  Both sides measured on B200, M = 1: 8.0
-    // against 8.3 us for 1280 x 8192, 5.5 against 7.0 for 8192 x 1024, 13.5 against 14.1 for 8192 x 3584, but 26.8 against
-    // 22.6 for 7168 x 8192 and 49.4 against 46.7 for 16032 x 8192; from two rows on it loses (12.0 against 8.3, 7.5
-    // against 7.0).  OOB_GEMM_GEMV=0 switches the rule off, =1 widens it to every M <= 4.
+    // The CUDA-core streaming kernel, both sides measured on B200, microseconds here and in the weight-streaming kernel.  One
+    // row: up to 32 M elements of weights (1280 x 8192 8.5 and 7.8, 8192 x 1024 5.2 and 6.6, 2048 x 2048 3.9 and 5.1), and from 48 M on
+    // where there are more 128-row tiles of them than SMs (57344 x 8192 135.5 and 160.9, 64000 x 2048 41.9 and 56.7, 24000 x 4096 32.8
+    // and 35.3; but 7168 x 8192 26.8 and 22.6, 16032 x 8192 46.0 and 43.6).  Two rows: up to 1.2 M elements (1024 x 1024 2.9 and 4.0, 256 x
+    // 4096 2.9 and 4.7; 2048 x 1024 4.6 and 4.2, 1280 x 8192 12.4 and 7.8).  OOB_GEMM_GEMV=0 switches the rule off, =1 widens it to
+    // every M <= 4.
     static const int gemv_env = [] {
       const char* v = getenv("OOB_GEMM_GEMV");
       return v == nullptr ? -1 : (v[0] == '1' ? 1 : 0);
     }();
-    const bool gemv_by_shape =
-        gemv_env != 0 && a.M == 1 && static_cast<long long>(a.N) * a.K <= 32ll * 1000 * 1000;
+    const long long weights = static_cast<long long>(a.N) * a.K;
+    const bool gemv_large = a.M == 1 && a.N > kTileM * sm_count() && weights > 48ll * 1000 * 1000;
+    const bool gemv_by_shape = gemv_env != 0 && (gemv_large || (a.M == 1 && weights <= 32ll * 1000 * 1000) ||
+                                                 (a.M == 2 && weights <= 1200ll * 1000));
     if (a.epilogue == 0 && gemv_supported(a) && ctx.emu_table == nullptr && a.c_emu_stride == 0 && a.splitk_ws == nullptr &&
         (a.gemv > 0 || (a.gemv == 0 && a.splits == 0 && a.skinny <= 0 && (gemv_env == 1 || gemv_by_shape))))
       return launch_gemv(a, a.max_ctas > 0 ? a.max_ctas : sm_count(), stream);
@@ -302,6 +306,10 @@ cudaError_t launch_gemm(const CommCtx& ctx, const GemmArgs& args, cudaStream_t s
       return v != nullptr && v[0] == '0';
     }();
     if (a.pair == 0 && pair_env_off) a.pair = -1;
+    // The activation of such a row in a kernel of its own costs less than what the streaming kernel gains.
+    if (a.epilogue == kGemmEpilogueSwigluTile && gemv_large && gemv_env != 0 && a.gemv >= 0 && a.skinny == 0 && a.splits == 0 &&
+        a.pair <= 0 && a.max_ctas == 0)
+      return cudaErrorNotSupported;
     // Few rows, or few tiles: the weight-streaming kernel.  It writes no trace, and its grid is not bounded by the SM count as
     // the records of a trace buffer are: a traced GEMM runs on the tiled kernels.
     static const bool cluster_env_off = [] {

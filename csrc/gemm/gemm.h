@@ -71,8 +71,8 @@ struct GemmArgs {
   // Plain mode: an elementwise op applied to the fp32 sums, for split problems (1, 2: by gemm_cluster.cu up to 256 rows, else
   // by the kernel that sums the splits, splitk_epilogues.cuh) or any (3: gemm_cluster.cu or the two-SM kernel).
   // epilogue_args is a HOST pointer to the op's argument block.
-  // Plain mode, M <= 4: 1 = the CUDA-core streaming kernel (gemv.cu); 0 = by shape (M = 1 with a weight matrix of up to
-  // 32 M elements; OOB_GEMM_GEMV=1 widens that to every M <= 4, =0 switches it off); -1 = never.
+  // Plain mode, M <= 4: 1 = the CUDA-core streaming kernel (gemv.cu); 0 = by shape (M = 1 and M = 2, see launch_gemm;
+  // OOB_GEMM_GEMV=1 widens that to every M <= 4, =0 switches it off); -1 = never.
   int gemv;
   int epilogue;               // 0 = none, 1 = SwiGLU (oob_gemm_epilogue_swiglu_t), 2 = RoPE + KV write (oob_rope_args_t),
                               // 3 = kGemmEpilogueSwigluTile (oob_gemm_epilogue_swiglu_t)

@@ -675,7 +675,14 @@ bool gemm_cluster_supported(const GemmArgs& a) {
 // 512 x 8192 x 8192 54.8 and 50.9, 2048 x 2048 x 2048 22.3 and 17.2.
 bool gemm_cluster_preferred(const GemmArgs& a) {
   using namespace gemm_cluster;
-  if (a.M <= kTileM) return true;
+  // Up to 128 rows the alternative is the one-SM kernel, persistent from the first tile to the last, on 256 weight rows a tile.
+  // It is the better one where there are more than two CTAs of 128 weight rows for every SM, from 49 rows on (128 x 57344 x 1024 27.9
+  // and 37.4 here, 80 x 64000 x 2048 47.3 and 61.5, 128 x 128256 x 4096 183 and 214) and, where K is long, from nine (16 x 57344 x
+  // 8192 155 and 172, 16 x 128256 x 4096 171 and 185; but 32 x 57344 x 1024 28.2 and 25.9, 16 x 64000 x 2048 62.6 and 58.9, 4 x 57344 x
+  // 8192 193 and 164).  With fewer tiles it is the worse one or equal (128 x 32768 x 4096 50.4 and 50.7, 64 x 24000 x 4096 40.2 and
+  // 38.4).  SwiGLU would need a kernel of its own behind it.
+  if (a.M <= kTileM)
+    return a.epilogue != 0 || a.M <= (a.K >= 4096 ? 8 : 48) || (a.N + kRowsW - 1) / kRowsW <= 2 * sm_count();
   const bool swiglu = a.epilogue == kEpiSwiglu || a.epilogue == kGemmEpilogueSwigluTile;
   const double two_sm = pair_cost_us(a.M, a.N, a.K, sm_count() / 2, swiglu);
   if (two_sm <= 0) return false;

@@ -1134,7 +1134,8 @@ int oob_gemm(oob_comm* c, const oob_gemm_args_t* a, void* stream) {
   if (e == cudaErrorNotSupported && a->epilogue == OOB_EPILOGUE_SWIGLU_TILE) {
     (void)cudaGetLastError();
     return set_error(OOB_ERR_UNSUPPORTED, "no kernel applies this SwiGLU: the problem is not split over K and the two-SM kernel is "
-                                          "ruled out (OOB_GEMM_PAIR=0, pair = -1, one CTA) or does not fit the device");
+                                          "ruled out (OOB_GEMM_PAIR=0, pair = -1, one CTA) or does not fit the device, or it is "
+                                          "one row of a weight that the CUDA-core kernel streams faster");
   }
   if (e != cudaSuccess) return cuda_fail(e, "GEMM launch");
   return OOB_OK;

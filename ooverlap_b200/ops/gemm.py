@@ -62,15 +62,16 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
 
     ``skinny`` selects the weight-streaming kernel for few rows (the weight rows fill the tensor-core instruction's
     128-row dimension, the tokens are its other one; K is split over the CTAs of a cluster that sum their parts through
-    distributed shared memory, deterministic): 0 uses it up to 128 rows, and above where it is expected to be faster than
-    the two-SM kernel, 1 whenever it can (``splits`` then asks for that many CTAs per tile, at most 8), -1 never.
+    distributed shared memory, deterministic): 0 uses it up to 128 rows (up to 48, or 8 where K is long, of a weight with
+    over 296 tiles of 128), and above where it is expected to be faster than the two-SM kernel, 1 whenever it can (``splits`` then asks for that many CTAs per tile, at most 8), -1 never.
 
     ``splitk_reduce`` says where a split-K sum is taken: -1 inside the GEMM kernel (the warp that delivers the last
     partial of a 32-row quadrant), 0 or 1 in a second kernel launched right after it (faster at every ``M``).
     The order of summation, and so the result, is the same.
 
     ``gemv`` = 1 uses the CUDA-core streaming kernel for ``M <= 4`` (a warp per weight row, no tensor cores, no
-    split-K hand-off); 0 uses it where it measured faster (one row, ``N * K`` up to 32 M), -1 never."""
+    split-K hand-off); 0 uses it where it measured faster (one row of a small or a very large weight,
+    two rows of a tiny one), -1 never."""
     _check_operands(a, b)
     M, N = a.shape[0], b.shape[0]
     if out is None:

@@ -43,7 +43,7 @@ def env_flag(name: str, default: bool = False) -> bool:
 #   OOB_GEMM_PAIR=0            plain GEMM: never use the two-SM kernel
 #   OOB_GEMM_SKINNY=0          plain GEMM: never use the weight-streaming kernel by default
 #   OOB_GEMM_GEMV=0 / 1        plain GEMM, CUDA-core streaming kernel: 0 = never by default, 1 = for every M <= 4
-#                              (unset: M = 1 with a weight matrix of up to 32 M elements)
+#                              (unset: one row of a small or a very large weight matrix, two rows of a tiny one)
 #   OOB_SPLITK_REDUCE_MIN_M=n  split-K: sum inside the GEMM kernel below n rows (default 1: always the second kernel)
 #   OOB_FUSED_EPILOGUES=0      model runner: RoPE + cache write and SwiGLU as kernels of their own behind the GEMM
 #   OOB_PREFILL_CHUNKS=n       model runner, prefill: row-parallel GEMM in n slabs overlapped with the all-reduce + norm

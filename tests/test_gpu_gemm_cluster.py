@@ -110,3 +110,23 @@ def test_swiglu_is_one_formula_whatever_kernel_applies_it(M, F, dtype):
     torch.cuda.synchronize()
     assert torch.equal(gemm(a, b), b.t()[:M].contiguous())
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K", [(1, 18960, 2536), (1, 18944, 2536), (1, 19008, 2520), (2, 1152, 1032), (2, 1168, 1032), (3, 1024, 1024),
+                                   (8, 38016, 4096), (9, 38016, 4096), (9, 37888, 4096), (48, 38016, 136), (49, 38016, 136),
+                                   (128, 37888, 136), (128, 40000, 136)])
+def test_default_route_at_the_edges_of_the_rules_for_few_rows(M, N, K, dtype):
+    """One row below and above 48 M weights and 148 tiles, two rows around 1.2 M weights, more than 296 tiles of weights."""
+    from ooverlap_b200.ops import gemm, gemm_swiglu
+    a, b = _operands(M, N, K, dtype)
+    c = gemm(a, b)
+    _check(c, a, b, dtype)
+    F = N // 2
+    s = gemm_swiglu(a, b)
+    torch.cuda.synchronize()
+    gu = a.double() @ b.double().t()
+    ref = torch.nn.functional.silu(gu[:, :F]) * gu[:, F:]
+    # the two-kernel route rounds gate and up to the 16-bit type first
+    tol = 4 * EPS[dtype] * ((1.1 * gu[:, F:].abs() + 1) * (gu[:, :F].abs() + 1))
+    assert ((s.double() - ref).abs() <= tol).all()
