@@ -164,8 +164,11 @@ template <typename T, int EPI>
 __device__ __forceinline__ void emit(const ParamsC& p, int m, int n, const float4& v, const float4& u, long long pos_base) {
   if constexpr (EPI == kEpiSwiglu) {
     if (n >= p.F) return;  // F % 8 == 0: the four columns are in or out together
+    uint32_t g[4] = {__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w)};
+    const uint32_t up[4] = {__float_as_uint(u.x), __float_as_uint(u.y), __float_as_uint(u.z), __float_as_uint(u.w)};
+    swiglu_n(g, up);
     *reinterpret_cast<uint2*>(static_cast<T*>(p.C) + size_t(m) * p.ldc + n) =
-        make_uint2(pack2<T>(swiglu_f32(v.x, u.x), swiglu_f32(v.y, u.y)), pack2<T>(swiglu_f32(v.z, u.z), swiglu_f32(v.w, u.w)));
+        make_uint2(pack2<T>(__uint_as_float(g[0]), __uint_as_float(g[1])), pack2<T>(__uint_as_float(g[2]), __uint_as_float(g[3])));
   } else if constexpr (EPI == kEpiRopeKv) {
     const oob_rope_args_t& a = p.rope;
     if (n >= p.N) return;  // N is a multiple of 8
