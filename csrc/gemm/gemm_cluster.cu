@@ -595,7 +595,9 @@ int cluster_slots(int sms, int size, int per_sm) {
 // Microseconds a plan takes, fitted to sweeps on B200: rounds of clusters, each as long as its K blocks at the pace of one
 // CTA or of the tensor cores of an SM (2 x tokens cycles a block), at the memory's rate for the weights or at L2's for all
 // operands, whichever is slowest; then draining the sums, reading the other CTAs' sums, and the fixed cost of a launch.
-double plan_cost(int N, int num_kb, int sms, const PlanC& pl) {
+// `ragged`: rows start off a 128-byte line, a row of a box touches two, and the pace and L2's rate are 1.45 times worse (for the
+// comparison with the two-SM kernel; the plans were swept with rows on a line).
+double plan_cost(int N, int num_kb, int sms, bool ragged, const PlanC& pl) {
   const int P = pl.pair ? 2 : 1, Mp = pl.n_mma * pl.nj, size = P * pl.S;
   const int clusters = tile_count(N, pl), slots = cluster_slots(sms, size, pl.per_sm);
   const int rounds = (clusters + slots - 1) / slots;
@@ -603,8 +605,9 @@ double plan_cost(int N, int num_kb, int sms, const PlanC& pl) {
   const double share = live > sms ? live / sms : 1.0;
   const double kb = double((num_kb + pl.S - 1) / pl.S);
   const double w = kRowsW * kRowBytes, x = double(Mp) / P * kRowBytes;
-  double t = kb * (pl.sub == 2 ? 0.165 + 0.0005 * Mp : 0.235 + 0.0002 * Mp);
-  const double mma = share * kb * 2.0 * Mp / 1850.0, l2 = live * kb * (w + x) / 11.5e6, hbm = live * kb * w / pl.m_blocks / 6.4e6;
+  const double lines = ragged ? 1.45 : 1.0;
+  double t = lines * kb * (pl.sub == 2 ? 0.165 + 0.0005 * Mp : 0.235 + 0.0002 * Mp);
+  const double mma = share * kb * 2.0 * Mp / 1850.0, l2 = lines * live * kb * (w + x) / 11.5e6, hbm = live * kb * w / pl.m_blocks / 6.4e6;
   if (mma > t) t = mma;
   if (l2 > t) t = l2;
   if (hbm > t) t = hbm;
@@ -631,7 +634,7 @@ bool plan(int M, int N, int K, int sms, int pair, int fix_s, PlanC* out, double*
       for (pl.S = 1; pl.S <= kMaxCluster / (two ? 2 : 1); ++pl.S) {
         if (fix_s > 0 ? pl.S != fix_s : (num_kb < 4 * pl.S && pl.S > 1)) continue;
         if (!size_cta(N, num_kb, sms, &pl)) continue;
-        const double c = plan_cost(N, num_kb, sms, pl);
+        const double c = plan_cost(N, num_kb, sms, false, pl);
         if (!found || c < *cost) {
           found = true;
           *out = pl;
@@ -673,7 +676,8 @@ bool gemm_cluster_supported(const GemmArgs& a) {
 
 // Whether this kernel is expected to be faster than the persistent two-SM kernel, which overlaps a tile's epilogue with the next
 // tile and needs no sum of parts, but deals out 256-row tiles: with fewer than three rounds of those, what they leave
-// idle or compute on padding is often more than this kernel's fixed cost.  Both sides measured, bf16 on B200: 512 x 1280 x 8192
+// idle or compute on padding is often more than this kernel's fixed cost.  The two models, each with a spread of 12 %, choose a
+// kernel that is 1.4 % slower than the best choice over 283 shapes, 14 % at worst (500 x 4096 x 14336).  Both sides measured, bf16 on B200: 512 x 1280 x 8192
 // 17.4 here and 29.6 us there, 200 x 4096 x 4096 15.0 and 18.1, 1000 x 1280 x 8192 23.9 and 29.6; 250 x 8192 x 3584 20.7 and 18.1,
 // 512 x 8192 x 8192 54.8 and 50.9, 2048 x 2048 x 2048 22.3 and 17.2.
 bool gemm_cluster_preferred(const GemmArgs& a) {
@@ -687,10 +691,11 @@ bool gemm_cluster_preferred(const GemmArgs& a) {
   if (a.M <= kTileM)
     return a.epilogue != 0 || a.M <= (a.K >= 4096 ? 8 : 48) || (a.N + kRowsW - 1) / kRowsW <= 2 * sm_count();
   const bool swiglu = a.epilogue == kEpiSwiglu || a.epilogue == kGemmEpilogueSwigluTile;
-  const double two_sm = pair_cost_us(a.M, a.N, a.K, sm_count() / 2, swiglu);
-  if (two_sm <= 0) return false;
+  const int pairs = sm_count() / 2;
+  if (static_cast<long long>((a.M + 2 * kTileM - 1) / (2 * kTileM)) * ((a.N + kTileN - 1) / kTileN) > 3ll * pairs) return false;
+  const double two_sm = pair_cut(kGemmPlain, a.M, a.N, a.K, pairs, a.stream_k, swiglu, false, false).us;
   const Planned& c = planned(a.M, a.N, a.K, a.pair, 0);
-  return c.ok && c.cost < two_sm;
+  return c.ok && plan_cost(a.N, (a.K + kTileK - 1) / kTileK, sm_count(), a.K % kTileK != 0, c.pl) < two_sm;
 }
 
 cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStream_t stream, gemm_detail::TmapFn make_tmap) {

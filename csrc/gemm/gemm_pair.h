@@ -141,21 +141,18 @@ int pair_streamk_auto(int tiles, int pairs, int num_kb, long long operand_bytes)
 // that share it; both 0 when a tail is not possible.
 void pair_streamk_plan(int tiles, int pairs, int num_kb, int* sk_tiles, int* sk_pairs);
 
-// Columns of a plain GEMM's tiles (a multiple of 32 in 128 .. 256) when another width than 256, or whole tiles instead of a
-// stream-K tail (`stream_k`: one is planned), leave the pairs less idle; 0 = stay with 256 and the tail.  Both sides measured,
-// bf16: 512 x 8192 x 8192 50.9 us at 224 columns (74 tiles) and 52.8 - 61 at 256 (64 tiles), 250 x 8192 x 3584 18.1 at 128 and
-// 23.3 at 256, 2048 x 8192 x 8192 182 at 224 and 193 with the tail, 2048 x 2048 x 2048 17.2 at 256 and 25.7 with the tail;
-// 4096 x 7168 x 8192 305 with the tail and 310 at 224.
-int pair_tile_columns(int M, int N, int num_kb, int pairs, bool stream_k);
-// How a problem is cut into tiles on `pairs` pairs.  `order`: a tile-order record is written.
+// How a problem is cut into tiles on `pairs` pairs: 256 columns with or without a stream-K tail or, in plain launches that do
+// not ask for a tail, narrower tiles where these are expected to be clearly faster.  `order`: a tile-order record is written.
+// Both sides measured, bf16: 512 x 8192 x 8192 50.9 us at 224 columns (74 tiles) and 52.8 - 61 at 256 (64 tiles),
+// 250 x 8192 x 3584 18.1 at 128 and 23.3 at 256, 2048 x 2048 x 2048 17.2 at 256 and 25.7 with the tail, 4096 x 7168 x 8192
+// 304 at 224, 309 with the tail and 323 at 256.
 struct PairCut {
   int tile_n;  // columns of a tile
   int tiles;
   int sk_tiles, sk_pairs;  // stream-K tail (256-column tiles), both 0 without one
+  double us;  // what it is expected to take
 };
 PairCut pair_cut(int mode, int M, int N, int K, int pairs, int stream_k, bool swiglu, bool emulated, bool order);
-// Microseconds the two-SM kernel is expected to take (plain, or with the SwiGLU epilogue); 0 beyond three rounds of tiles.
-double pair_cost_us(int M, int N, int K, int pairs, bool swiglu);
 
 // Whether the pair kernel can run this (mode, shape).
 bool gemm_pair_supported(const CommCtx& ctx, const GemmArgs& args);
