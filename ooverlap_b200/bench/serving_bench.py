@@ -109,7 +109,7 @@ def main() -> int:
                    "checksum": int(toks.sum().item()) % 1000003, "first": int(first[0, 0]),
                    # switches that change which kernels run (recorded so that lines from different runs can be told apart)
                    "switches": {k: os.environ[k] for k in ("OOB_FUSED_EPILOGUES", "OOB_PREFILL_CHUNKS", "OOB_GEMM_GEMV",
-                                                           "OOB_ATTN_STAGES", "OOB_GEMM_SKINNY", "OOB_GEMM_PAIR",
+                                                           "OOB_GEMM_SKINNY", "OOB_GEMM_PAIR",
                                                            "OOB_SPLITK_REDUCE_MIN_M") if k in os.environ}}
             lines.append(rec)
             if rank == 0:
