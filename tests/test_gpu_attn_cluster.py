@@ -21,10 +21,37 @@ def test_attention_lengths_and_clusters(B, H, KV, L, bound, splits, dtype):
     pos = torch.full((1,), L - 1, dtype=torch.long, device="cuda")
     out = attn_decode(q, kc, vc, pos, splits=splits, len_bound=bound)
     torch.cuda.synchronize()
-    ref = attn_decode_reference(q, kc, vc, L - 1)
-    # probabilities and the result are each rounded once to the 16-bit type; values are about 1, at most about 5
-    tol = 2e-2 if dtype == torch.bfloat16 else 4e-3
-    assert (out.float() - ref).abs().max().item() <= tol * max(1.0, ref.abs().max().item())
+    ref = attn_decode_reference(q, kc, vc, L - 1).view(B, H, 128)
+    # The result is rounded once.  So are the probabilities, by at most eps each and independently of one another: their
+    # errors add like sqrt(sum (p v)^2), of which eight standard deviations (eps / sqrt(3)) are allowed.
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    p = torch.softmax(torch.einsum("bhd,bhld->bhl", q.float(), kc[:, :, :L].float().repeat_interleave(H // KV, 1)) / 128 ** 0.5, -1)
+    spread = torch.einsum("bhl,bhld->bhd", p.square(), vc[:, :, :L].float().square().repeat_interleave(H // KV, 1)).sqrt()
+    assert ((out.float().view(B, H, 128) - ref).abs() <= eps * ref.abs() + (8 * eps / 3 ** 0.5 + 1e-5) * spread + 1e-6).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,H,KV,L,bound,splits", [
+    (1, 8, 1, 1, 0, 0), (1, 16, 1, 17, 0, 0), (2, 8, 2, 63, 0, 1), (1, 8, 1, 65, 4096, 0), (1, 8, 1, 2047, 0, 0), (3, 8, 1, 4097, 0, 0),
+    (33, 8, 1, 515, 0, 0), (70, 8, 1, 300, 0, 0), (150, 8, 1, 129, 0, 0), (2, 24, 3, 1000, 0, 5), (1, 4, 1, 40, 0, 7), (1, 8, 8, 4112, 0, 3)])
+def test_every_key_counts_once(B, H, KV, L, bound, splits, dtype):
+    """Equal scores, and one key per dimension with a value of one: the result is 1 / L there and zero elsewhere, exactly."""
+    from ooverlap_b200.ops import attn_decode
+    max_len = 4112
+    q = torch.zeros(B, H, 128, device="cuda", dtype=dtype)
+    kc = torch.randn(B, KV, max_len, 128, device="cuda").to(dtype)
+    kc[:, :, L:] = float("nan")
+    vc = torch.zeros_like(kc)
+    vc[:, :, L:] = float("nan")
+    pos = torch.full((1,), L - 1, dtype=torch.long, device="cuda")
+    one = torch.full((128,), 1.0 / L, device="cuda", dtype=torch.float32).to(dtype)
+    for base in range(0, L, 128):
+        n = min(128, L - base)
+        i = torch.arange(n, device="cuda")
+        vc[:, :, base + i, i] = 1
+        out = attn_decode(q, kc, vc, pos, splits=splits, len_bound=bound).view(B, H, 128)
+        assert (out[:, :, :n] == one[:n]).all() and (out[:, :, n:] == 0).all(), base
+        vc[:, :, base + i, i] = 0
 
 
 def test_split_calls_on_two_streams_and_in_a_graph():

@@ -48,10 +48,12 @@ def _rope_ref(x, cos, sin):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("B,T,H,KV,hd,K,pos,dev_pos", [(2, 1, 8, 1, 128, 8192, 37, True), (64, 1, 8, 1, 128, 8192, 5, True),
-                                                        (3, 4, 4, 2, 64, 1024, 9, False)])
+                                                        (3, 4, 4, 2, 64, 1024, 9, False), (2, 100, 8, 1, 128, 8192, 3, False),
+                                                        (3, 100, 4, 2, 64, 1024, 0, True), (1, 512, 8, 1, 128, 8192, 7, True),
+                                                        (4, 250, 8, 1, 128, 8192, 11, False), (5, 201, 8, 2, 64, 2056, 1, True)])
 def test_gemm_rope_kv_write(B, T, H, KV, hd, K, pos, dev_pos, dtype):
     from ooverlap_b200.ops import gemm_plan_splits, gemm_rope_kv_write, rope_tables
-    max_len, batch0 = 96, 1
+    max_len, batch0 = max(96, pos + T + 5), 1
     N = (H + 2 * KV) * hd
     assert gemm_plan_splits(B * T, N, K) > 1
     g = torch.Generator(device="cuda").manual_seed(B * 100 + T)

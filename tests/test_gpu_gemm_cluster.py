@@ -38,6 +38,38 @@ def test_cluster_gemm_edges(shape, splits, pair, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape,splits,pair", [
+    ((16, 300, 520), 3, -1), ((100, 264, 1032), 5, -1), ((64, 1280, 2056), 6, -1), ((130, 200, 4096), 7, -1), ((512, 1280, 8192), 3, 1),
+    ((257, 392, 520), 0, 0), ((257, 264, 520), 3, 1), ((383, 520, 264), 0, -1), ((383, 392, 1032), 2, 1), ((384, 264, 136), 1, 1),
+    ((385, 264, 520), 0, 0), ((385, 1000, 520), 7, -1), ((1000, 520, 1096), 3, 1), ((1000, 264, 520), 0, 0), ((4095, 136, 264), 0, 0),
+    ((4096, 392, 520), 4, -1), ((4096, 264, 520), 4, 1)])
+def test_cluster_gemm_token_blocks_and_odd_splits(shape, splits, pair, dtype):
+    """Two instructions per tile (257 - 384 tokens), several token blocks with a ragged last one, splits that are no power of two."""
+    from ooverlap_b200.ops import gemm
+    M, N, K = shape
+    a, b = _operands(M, N, K, dtype)
+    c = gemm(a, b, skinny=1, splits=splits, pair=pair)
+    again = gemm(a, b, skinny=1, splits=splits, pair=pair)
+    torch.cuda.synchronize()
+    _check(c, a, b, dtype)
+    assert torch.equal(c, again)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape", [(17, 1290, 1032), (64, 1280, 2056), (200, 1000, 520), (300, 1288, 264), (1000, 640, 520)])
+@pytest.mark.parametrize("splits,max_ctas", [(1, 3), (2, 4), (2, 7), (3, 6), (4, 4), (8, 8)])
+def test_cluster_takes_several_tiles_one_after_the_other(shape, splits, max_ctas, dtype):
+    """A budget leaves fewer clusters than tiles: shared memory, TMEM and the ring's phases are used again after the parts were
+    read through distributed shared memory."""
+    from ooverlap_b200.ops import gemm
+    M, N, K = shape
+    a, b = _operands(M, N, K, dtype)
+    c = gemm(a, b, skinny=1, splits=splits, max_ctas=max_ctas)
+    torch.cuda.synchronize()
+    _check(c, a, b, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("shape", [(3, 520, 1032), (40, 264, 520), (200, 1000, 72)])
 def test_default_route_equals_tiled_route_on_strided_operands(shape, dtype):
     from ooverlap_b200.ops import gemm
