@@ -51,8 +51,8 @@ typedef struct {
   const int64_t* pos_dev; /* device scalar: index of the newest key; context length = *pos_dev + 1.  NULL = len */
   int len;
   float scale;        /* softmax scale (1/sqrt(128) for standard attention) */
-  int splits;         /* CTAs per (sequence, KV head) along the keys; 0 = choose from B * KV and len_bound */
-  int len_bound;      /* upper bound of the context length for this launch (sizes the key chunks); 0 = max_len */
+  int splits;         /* clusters of CTAs per (sequence, KV head) along the keys; 0 = choose from B * KV and len_bound */
+  int len_bound;      /* upper bound of the context length for this launch (chooses clusters and splits); 0 = max_len */
   float* workspace;   /* fp32, oob_attn_decode_workspace_bytes(B, H, splits) bytes; may be NULL when splits == 1 */
 } oob_attn_decode_args_t;
 int oob_attn_decode(const oob_attn_decode_args_t* a, void* stream);

@@ -34,12 +34,12 @@ enum TraceSlot : int {
   kTraceWords = 8
 };
 
-// All matrices are 16-bit (fp16 or bf16), A is [M, K] row-major with leading
-// dimension lda, B is [N, K] row-major (the layout of a torch Linear weight)
-// with leading dimension ldb, C is [M, N] row-major.
 constexpr int kGemmEpilogueSwigluTile = 3;
 constexpr int kGemmClusterMaxRows = 4096;  // rows the weight-streaming kernel (gemm_cluster.cu) accepts
 
+// All matrices are 16-bit (fp16 or bf16), A is [M, K] row-major with leading
+// dimension lda, B is [N, K] row-major (the layout of a torch Linear weight)
+// with leading dimension ldb, C is [M, N] row-major.
 struct GemmArgs {
   int mode;
   int fmt;  // 0 = fp16, 1 = bf16
@@ -68,21 +68,21 @@ struct GemmArgs {
   // (set by launch_gemm; callers ask through splitk_reduce: 0 / 1 = second kernel, -1 = sum inside the GEMM kernel).
   int splitk_defer;
   int splitk_reduce;
-  // Plain mode: an elementwise op applied to the fp32 sums, for split problems (1, 2: by gemm_cluster.cu up to 256 rows, else
-  // by the kernel that sums the splits, splitk_epilogues.cuh) or any (3: gemm_cluster.cu or the two-SM kernel).
-  // epilogue_args is a HOST pointer to the op's argument block.
   // Plain mode, M <= 4: 1 = the CUDA-core streaming kernel (gemv.cu); 0 = by shape (M = 1 and M = 2, see launch_gemm;
   // OOB_GEMM_GEMV=1 widens that to every M <= 4, =0 switches it off); -1 = never.
   int gemv;
-  int epilogue;               // 0 = none, 1 = SwiGLU (oob_gemm_epilogue_swiglu_t), 2 = RoPE + KV write (oob_rope_args_t),
-                              // 3 = kGemmEpilogueSwigluTile (oob_gemm_epilogue_swiglu_t)
+  // Plain mode: an elementwise op applied to the fp32 sums by the kernel that has them: 0 = none, 1 = SwiGLU
+  // (oob_gemm_epilogue_swiglu_t) and 2 = RoPE + KV write (oob_rope_args_t) for split problems, 3 = kGemmEpilogueSwigluTile
+  // (oob_gemm_epilogue_swiglu_t) for any.  gemm_cluster.cu applies all of them, the two-SM kernel SwiGLU, the kernel that sums
+  // K splits (splitk_epilogues.cuh) the first two.  epilogue_args is a HOST pointer to the op's argument block.
+  int epilogue;
   const void* epilogue_args;
-  // 0 = the two-SM kernel (256x256 tiles on CTA pairs) when the shape suits it, 1 = always when possible,
-  // -1 = never (the one-SM kernel with 128x256 tiles).  Applies to the plain GEMM and to the fused modes.
+  // 0 = the two-SM kernel (256x256 or narrower tiles on CTA pairs) when the shape suits it, 1 = always when possible,
+  // -1 = never (the one-SM kernel with 128x256 tiles, or the weight-streaming kernel without CTA pairs).  Applies to the plain GEMM and to the fused modes.
   int pair;
   // Two-SM kernel, plain and AG modes: stream-K tail (the last wave and the remainder are cut along K so that no
-  // pair idles; partial accumulators meet in a library-owned workspace).  0 = when it pays for the shape, 1 = whenever
-  // the tile count leaves a remainder, -1 = never.
+  // pair idles; partial accumulators meet in a library-owned workspace).  0 = when it is expected to pay for the shape, against
+  // whole tiles and, in plain mode, narrower ones (pair_cut); 1 = whenever the tile count leaves a remainder, -1 = never.
   int stream_k;
   // Two-SM kernel, every mode: optional tile-order record.  Two 64-bit words per 128-row half of every 256x256 tile,
   // indexed 2 * (tile's number in the schedule) + (CTA of the pair): [0] globaltimer nanoseconds at which the half

@@ -3,8 +3,9 @@
 // of a decode step or of a short mixed batch: what bounds it is the time to read B once, plus whatever happens before the
 // first and after the last byte.
 //
-// A CTA goes through 64 elements of K in 0.17 - 0.27 us (the chain load - multiply - release of its issuing threads), so that neither few CTAs nor long K ranges reach the memory's rate.  128-row weight tiles are therefore computed by S CTAs,
-// each over 1/S of K; a cost model on the host picks S and the token blocks.
+// A CTA goes through 64 elements of K in 0.17 - 0.27 us (the chain load - multiply - release of its issuing threads), so that
+// neither few CTAs nor long K ranges reach the memory's rate.  128-row weight tiles are therefore computed by S CTAs, each over 1/S
+// of K; a cost model on the host picks S and the token blocks.
 //
 // Split over K inside a thread-block cluster (S = 1 .. 8).  When a CTA has its partial sums it drains them from TMEM into its
 // own shared memory (the pipeline buffers, idle by then) as [token][128] fp32; after one cluster barrier each CTA reads its share

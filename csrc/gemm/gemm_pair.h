@@ -23,7 +23,7 @@ struct PairPlan {
   int sk_tiles;    // tiles of the stream-K tail, 0 = every tile is computed whole by one pair
   int sk_pairs;    // pairs that share the tail
   void* sk_ws;     // stream-K workspace (flags + slots), null without a tail
-  int tile_n;      // columns of a tile: 256 except in plain launches without a tail (pair_tile_columns)
+  int tile_n;      // columns of a tile: 256 except in plain launches without a tail (pair_cut)
 };
 
 // ---- schedule (host and device: the host side exists for tests of the enumeration) ------------------------------
@@ -133,9 +133,10 @@ struct ItemIter {
 
 }  // namespace gemm_pair
 
-// 1 when a stream-K tail pays for `tiles` 256x256 tiles on `pairs` pairs with `num_kb` K blocks per tile: the last
+// 1 when a stream-K tail may pay for `tiles` 256x256 tiles on `pairs` pairs with `num_kb` K blocks per tile: the last
 // wave would leave pairs idle for more than 3 % of the run, K is deep enough to cut, and the operands (`operand_bytes`
-// of A and B together) are small enough for L2 to make up for the lost lockstep of the pairs.
+// of A and B together) are small enough for L2 to make up for the lost lockstep of the pairs.  A plain launch then still weighs
+// it against whole and narrower tiles (pair_cut).
 int pair_streamk_auto(int tiles, int pairs, int num_kb, long long operand_bytes);
 // Size of the tail (one wave + remainder, or everything when there is less than a wave) and the number of pairs
 // that share it; both 0 when a tail is not possible.

@@ -496,7 +496,7 @@ __global__ void attn_combine_kernel(const float* ws, void* out, int splits) {
   float acc = 0.f, l_tot = 0.f;
   for (int s = 0; s < splits; ++s) {
     const float ms = w[s * kPartialStride + kHD];
-    if (ms == -INFINITY) continue;  // empty chunk: its values were never written
+    if (ms == -INFINITY) continue;  // a part without keys
     const float f = exp2f(ms - m_tot);
     acc += f * w[s * kPartialStride + d];
     l_tot += f * w[s * kPartialStride + kHD + 1];

@@ -77,9 +77,9 @@ def gemm_rope_kv_write(x: torch.Tensor, wqkv: torch.Tensor, B: int, T: int, head
                        batch0: int = 0, q_out: Optional[torch.Tensor] = None, fused: Optional[bool] = None) -> torch.Tensor:
     """``rope_kv_write(x @ wqkv.T, ...)``: the QKV projection followed by the rotation and the cache write.
 
-    When the GEMM is one that is split over K (every decode-step shape), rotation and cache write are done from the fp32
-    sums by the kernel that has them (the weight-streaming kernel, or the one that sums the splits); otherwise (or with ``fused=False``) the GEMM is followed by
-    :func:`rope_kv_write`.  Returns the rotated queries, [B*T, heads * hd]."""
+    When the GEMM is one that the tiled kernels would split over K (every decode-step shape), rotation and cache write are
+    done from the fp32 sums by the kernel that has them (the weight-streaming kernel, or the one that sums the splits);
+    otherwise (or with ``fused=False``) the GEMM is followed by :func:`rope_kv_write`.  Returns the rotated queries, [B*T, heads * hd]."""
     from .gemm import _check_operands, fill_gemm_args, gemm, gemm_plan_splits
     _check_operands(x, wqkv)
     M, N, K = x.shape[0], wqkv.shape[0], x.shape[1]
@@ -130,8 +130,9 @@ def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, p
     [batch, kv_heads, max_len, 128] and keys ``0 .. pos`` of sequences ``batch0 .. batch0 + B - 1`` are attended
     (``pos``: int or one-element device ``int64`` tensor, the index of the newest key).  Returns [B, heads * 128].
 
-    ``splits`` CTAs share the keys of one (sequence, KV head); 0 picks the count from ``B * kv_heads`` and
-    ``len_bound`` (an upper bound of the context length of this and any replayed launch; default ``max_len``)."""
+    The CTAs of a cluster share the keys of one (sequence, KV head) by the length found on the device; ``splits`` > 1 adds
+    that many clusters, whose results a second kernel merges.  0 picks both from ``B * kv_heads`` and ``len_bound`` (an
+    upper bound of the context length of this and any replayed launch; default ``max_len``)."""
     if q.dim() != 3 or q.shape[2] != 128 or not q.is_contiguous():
         raise ValueError("q must be a contiguous [B, heads, 128] tensor")
     B, H, hd = q.shape

@@ -47,23 +47,24 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
     it was stored and ``pair << 32 | index in the pair's sequence``; see :func:`tile_order`.
 
     ``splits`` > 1 splits K over that many CTAs per output tile (fp32 partials in the library's workspace,
-    summed in split order); 0 picks a split from the shape (small-M problems that would otherwise leave most
-    SMs idle), 1 turns it off.
+    summed in split order), 1 turns it off; 0 leaves it to the kernel that the shape takes (few rows or few tiles: the
+    weight-streaming kernel, else the two-SM kernel; the tiled kernels split by shape where both are ruled out).
 
-    ``pair`` selects the two-SM kernel (256x256 tiles computed by CTA pairs with ``tcgen05.mma.cta_group::2``; each
-    CTA stages half of the B block): 0 uses it for unsplit problems with more than 128 rows, 1 whenever the problem
-    is unsplit, -1 never.
+    ``pair`` selects the two-SM kernel (tiles of 256 rows and 128 to 256 columns computed by CTA pairs with
+    ``tcgen05.mma.cta_group::2``; each CTA stages half of the B block): 0 uses it for problems with more than 128 rows that
+    the weight-streaming kernel is not expected to compute faster, 1 whenever the problem is unsplit, -1 never.
 
     ``stream_k`` (two-SM kernel): when the tile count is not a multiple of the pair count, the last wave and the
     remainder are cut along K into equal ranges, one per pair, so that no pair idles; pairs that compute part of a tile
     park fp32 accumulators in a library-owned workspace and the part that arrives last sums them in pair order
-    (bit-reproducible).  0 uses it when the idle share would exceed 3 % of the run, 1 whenever there is a remainder,
-    -1 never.
+    (bit-reproducible).  0 uses it when the idle share would exceed 3 % of the run and neither whole tiles nor narrower
+    ones are expected to be faster, 1 whenever there is a remainder, -1 never.
 
     ``skinny`` selects the weight-streaming kernel for few rows (the weight rows fill the tensor-core instruction's
     128-row dimension, the tokens are its other one; K is split over the CTAs of a cluster that sum their parts through
     distributed shared memory, deterministic): 0 uses it up to 128 rows (up to 48, or 8 where K is long, of a weight with
-    over 296 tiles of 128), and above where it is expected to be faster than the two-SM kernel, 1 whenever it can (``splits`` then asks for that many CTAs per tile, at most 8), -1 never.
+    over 296 tiles of 128), and above where it is expected to be faster than the two-SM kernel, 1 whenever it can
+    (``splits`` then asks for that many CTAs per tile, at most 8), -1 never.
 
     ``splitk_reduce`` says where a split-K sum is taken: -1 inside the GEMM kernel (the warp that delivers the last
     partial of a 32-row quadrant), 0 or 1 in a second kernel launched right after it (faster at every ``M``).
@@ -183,7 +184,7 @@ def splitk_workspace_bytes(M: int, N: int, K: int, *, max_ctas: int = 0, splits:
 
 
 def gemm_plan_splits(M: int, N: int, K: int, *, max_ctas: int = 0, splits: int = 0) -> int:
-    """Number of K splits :func:`gemm` uses for this shape (1 = the problem is not split)."""
+    """Number of K splits the tiled kernels use for this shape (1 = the problem is not split)."""
     return int(_lib.lib().oob_gemm_plan_splits(M, N, K, max_ctas, splits))
 
 
@@ -191,10 +192,11 @@ def gemm_swiglu(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = 
                 fused: Optional[bool] = None) -> torch.Tensor:
     """``silu(a @ b[:F].T) * (a @ b[F:].T)`` for a gate/up weight ``b`` of shape [2F, K]; returns [M, F].
 
-    The activation is applied to the fp32 sums by the kernel that has them (the weight-streaming kernel up to 256 rows,
-    the split-K sum, or the two-SM kernel's epilogue): no separate launch and no 16-bit round trip of the [M, 2F]
-    intermediate.  With ``fused=False`` the GEMM is followed by the stand-alone SwiGLU kernel.  ``fused=True`` insists on
-    a problem that is split over K (every decode-step shape) and raises otherwise."""
+    The activation is applied to the fp32 sums by the kernel that has them (the weight-streaming kernel, the two-SM kernel's
+    epilogue or the split-K sum): no separate launch and no 16-bit round trip of the [M, 2F] intermediate.  Where none of
+    them may run (``OOB_GEMM_PAIR=0``, one CTA), for one row of a large weight, and with ``fused=False`` the GEMM is followed
+    by the stand-alone SwiGLU kernel.  ``fused=True`` insists on a problem that the tiled kernels would split over K (every
+    decode-step shape) and raises otherwise."""
     from .decode import silu_mul
     _check_operands(a, b)
     M, N = a.shape[0], b.shape[0]
