@@ -603,6 +603,9 @@ double attn_cost_ns(long long items, int s, int slots, double len) {
 // looked at whole rounds at the bound only took four CTAs for 300 items of a 2048-key cache with 16 keys in it (20.3 us, 5.6 with
 // one) and for 600 items with 500 keys in it (68.5, 33.5).
 int attn_cluster_size(long long items, int len_bound, const AttnSlots& slots) {
+  // With a CTA for every SM the memory is busy: clusters gained 8 % at most on full caches (192 items of 8192 keys 119 us in fours, 129)
+  // and lost up to 2.5 times on short contexts (150 items, 100 of 8192 keys 11.4 in pairs, 6.1).
+  if (items > 148) return 1;
   const double third = len_bound / 3.0;
   const double one = attn_cost_ns(items, 1, slots.n[0], len_bound), one_third = attn_cost_ns(items, 1, slots.n[0], third);
   int best = 1;

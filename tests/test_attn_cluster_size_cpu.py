@@ -8,8 +8,8 @@ def size(items, bound, slots=(296, 264, 256)):
     return _lib.lib().oob_test_attn_cluster_size(items, bound, *slots)
 
 
-@pytest.mark.parametrize("bound", [64, 128, 512, 2048])
-@pytest.mark.parametrize("items", [150, 256, 296, 300, 512, 600, 2048])
+@pytest.mark.parametrize("bound", [64, 128, 512, 2048, 4096, 8192, 32768])
+@pytest.mark.parametrize("items", [149, 150, 256, 296, 300, 512, 600, 2048])
 def test_a_batch_that_fills_the_gpu_gets_one_cta_each(items, bound):
     """More CTAs gain at most a few per cent on a full cache and cost several times the time on a short context."""
     assert size(items, bound) == 1
