@@ -223,7 +223,8 @@ def gemm_swiglu(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = 
     args.epilogue_args = ctypes.cast(ctypes.pointer(epi), ctypes.c_void_p)
     rc = _lib.lib().oob_gemm(None, args, current_stream_ptr())
     if rc == _lib.ERR_UNSUPPORTED and not can_fuse:  # no kernel that has the sums may or can apply it: two kernels
-        return silu_mul(gemm(a, b, max_ctas=max_ctas), out)
+        dense = silu_mul(gemm(a, b, max_ctas=max_ctas), out if out.is_contiguous() else None)
+        return out if dense is out else out.copy_(dense)
     if rc:
         _lib.check(rc)
     return out

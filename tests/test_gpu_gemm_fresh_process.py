@@ -74,6 +74,9 @@ def test_swiglu_runs_where_no_pair_of_sms_can(monkeypatch):
     one = gemm_swiglu(a, b, max_ctas=1)  # one CTA is no pair
     monkeypatch.setattr(_lib, "lib", lambda: NoPair())
     got = gemm_swiglu(a, b)
+    wide = torch.zeros(2048, 2048 + 16, device="cuda", dtype=torch.bfloat16)
+    strided = gemm_swiglu(a, b, out=wide[:, 8:2056])
     torch.cuda.synchronize()
-    assert torch.equal(got, want)
+    assert torch.equal(got, want) and torch.equal(strided, want) and strided.data_ptr() == wide[:, 8:].data_ptr()
+    assert not wide[:, :8].any() and not wide[:, 2056:].any()
     assert torch.equal(one, silu_mul(gemm(a, b, max_ctas=1)))
