@@ -678,9 +678,10 @@ bool gemm_cluster_supported(const GemmArgs& a) {
 // Whether this kernel is expected to be faster than the persistent two-SM kernel, which overlaps a tile's epilogue with the next
 // tile and needs no sum of parts, but deals out 256-row tiles: with fewer than three rounds of those, what they leave
 // idle or compute on padding is often more than this kernel's fixed cost.  The two models, each with a spread of 12 %, choose a
-// kernel that is 1.4 % slower than the best choice over 283 shapes, 14 % at worst (500 x 4096 x 14336).  Both sides measured, bf16 on B200: 512 x 1280 x 8192
-// 17.4 here and 29.6 us there, 200 x 4096 x 4096 15.0 and 18.1, 1000 x 1280 x 8192 23.9 and 29.6; 250 x 8192 x 3584 20.7 and 18.1,
-// 512 x 8192 x 8192 54.8 and 50.9, 2048 x 2048 x 2048 22.3 and 17.2.
+// kernel that is 1.5 % slower than the best choice on average over 283 shapes, 18 % at worst (512 x 2048 x 2048).  Both sides
+// measured, bf16 on B200: 512 x 1280 x 8192 17.4 here and 29.6 us there, 200 x 4096 x 4096 15.0 and 18.1, 1000 x 1280 x 8192 23.9 and
+// 29.6, 1037 x 4104 x 2056 26.4 and 28.7; 250 x 8192 x 3584 20.7 and 18.1, 512 x 8192 x 8192 54.8 and 50.9, 2048 x 2048 x 2048 22.3 and
+// 17.2.
 bool gemm_cluster_preferred(const GemmArgs& a) {
   using namespace gemm_cluster;
   // Up to 128 rows the alternative is the one-SM kernel, persistent from the first tile to the last, on 256 weight rows a tile.
