@@ -215,6 +215,8 @@ typedef struct {
   void* order;  /* two-SM kernel: optional device buffer, 2 x uint64 per 128-row half of every 256x256 tile (index
                    2 * tile's number in the schedule + CTA of the pair): [0] globaltimer ns at which the half was
                    complete (fused AR / RS: published to its reducer), [1] = pair << 32 | index in the pair's sequence */
+  int b_static; /* plain mode: 1 = nothing that this call could overtake writes B (weights): the kernel may read B while the
+                   kernel before it on the stream still runs.  0 = B may be that kernel's output */
 } oob_gemm_args_t;
 #define OOB_EPILOGUE_NONE 0
 #define OOB_EPILOGUE_SWIGLU 1  /* N = 2F columns [gate | up]; C is [M, F] = silu(gate) * up */

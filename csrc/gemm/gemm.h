@@ -91,6 +91,9 @@ struct GemmArgs {
   unsigned long long* order;
   // Plain mode, M <= kGemmClusterMaxRows: 1 = the weight-streaming kernel (gemm_cluster.cu), 0 = by shape, -1 = the tiled kernels.
   int skinny;
+  // Plain mode: 1 = B is a weight that no kernel the launch may overlap writes; the weight-streaming kernel then starts to load it
+  // before the kernels it depends on are done.
+  int b_static;
 
   // Fused modes
   PeerPtrs partial;     // AR / RS: per-owner staging of partial tiles, registered; see oob_gemm_partial_bytes

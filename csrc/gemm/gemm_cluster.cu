@@ -84,6 +84,7 @@ struct ParamsC {
   int smem_bytes;
   uint32_t tmem_cols;
   bool vec_ok;  // 8-byte stores into C are aligned
+  bool w_static;  // the weights may be loaded before the kernels this one depends on are done
   oob_rope_args_t rope;
 };
 
@@ -304,9 +305,14 @@ __global__ void __launch_bounds__(kThreadsC)
   // This CTA holds its TMEM: the next kernel may be set up beside it.  Everything below touches memory that earlier
   // kernels wrote or still read.
   ptx::griddep_launch_dependents();
-  ptx::griddep_wait();
+  // Static weights are not behind that wait: their warp fills the ring at once, and waits when it has loaded its first tile.
+  bool waited = !(p.w_static && warp == 0);
+  if (waited) ptx::griddep_wait();
   long long pos_base = 0;
-  if constexpr (EPI == kEpiRopeKv) pos_base = p.rope.pos_dev != nullptr ? *p.rope.pos_dev : static_cast<long long>(p.rope.pos0);
+  auto load_pos = [&]() { return p.rope.pos_dev != nullptr ? *p.rope.pos_dev : static_cast<long long>(p.rope.pos0); };
+  if constexpr (EPI == kEpiRopeKv) {
+    if (waited) pos_base = load_pos();
+  }
 
   int stage = 0;          // producer's / MMA issuer's position in the ring, carried from tile to tile
   uint32_t phase = 0;
@@ -349,6 +355,11 @@ __global__ void __launch_bounds__(kThreadsC)
         }
       }
       __syncwarp();
+      if (!waited) {  // the results below go where earlier kernels may still read
+        ptx::griddep_wait();
+        waited = true;
+        if constexpr (EPI == kEpiRopeKv) pos_base = load_pos();
+      }
     }
     if (warp == 1) {
       if (member == 0 && ptx::elect_one()) {
@@ -721,6 +732,7 @@ cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStr
   p.N = a.N;
   p.C = a.C;
   p.ldc = a.ldc;
+  p.w_static = a.b_static != 0;
   p.vec_ok = a.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(a.C) & 7) == 0;
   p.sub = pl.sub;
   p.num_kb = (num_kb + pl.sub - 1) / pl.sub;

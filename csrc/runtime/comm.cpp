@@ -1069,6 +1069,7 @@ int oob_gemm(oob_comm* c, const oob_gemm_args_t* a, void* stream) {
   g.gemv = a->gemv;
   g.stream_k = a->stream_k;
   g.order = static_cast<unsigned long long*>(a->order);
+  g.b_static = a->b_static;
   g.epilogue = a->epilogue;
   g.epilogue_args = a->epilogue_args;
   if (a->epilogue != OOB_EPILOGUE_NONE) {

@@ -24,7 +24,7 @@ import torch
 import torch.nn.functional as F
 
 from ..ops import (attn_decode, fused_allreduce_rmsnorm, gemm, gemm_rope_kv_write, gemm_swiglu, rmsnorm, rope_kv_write,
-                   rope_tables, silu_mul)
+                   rope_tables, silu_mul, static_weights)
 from ..utils.config import env_flag, env_int
 from ..utils.tracing import nvtx_range
 
@@ -185,6 +185,8 @@ class LlamaTP:
         return y, h
 
     # --------------------------------------------------------------- forward
+    # The embedding lookup, which no other kernel overlaps, stands between whatever wrote the weights and the first GEMM.
+    @static_weights()
     def forward(self, tokens: torch.Tensor, pos, attn_mask: Optional[torch.Tensor] = None, batch0: int = 0):
         """tokens: [B, T].  Prefill: ``pos`` is the int start position (0) and attention is causal over the chunk.
         Decode: T == 1, ``pos`` is a device LongTensor of shape [1] and ``attn_mask`` masks the unused tail of
@@ -301,7 +303,8 @@ class LlamaTP:
         def step():
             mask.index_fill_(3, pos, 0.0)
             hs = self.forward(cur, pos, attn_mask=mask)
-            nxt.copy_(self.greedy_token(hs))
+            with static_weights():
+                nxt.copy_(self.greedy_token(hs))
             cur.copy_(nxt.view(B, 1))
             pos.add_(1)
 

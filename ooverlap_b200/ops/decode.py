@@ -80,7 +80,7 @@ def gemm_rope_kv_write(x: torch.Tensor, wqkv: torch.Tensor, B: int, T: int, head
     When the GEMM is one that the tiled kernels would split over K (every decode-step shape), rotation and cache write are
     done from the fp32 sums by the kernel that has them (the weight-streaming kernel, or the one that sums the splits);
     otherwise (or with ``fused=False``) the GEMM is followed by :func:`rope_kv_write`.  Returns the rotated queries, [B*T, heads * hd]."""
-    from .gemm import _check_operands, fill_gemm_args, gemm, gemm_plan_splits
+    from .gemm import _check_operands, _scope, fill_gemm_args, gemm, gemm_plan_splits
     _check_operands(x, wqkv)
     M, N, K = x.shape[0], wqkv.shape[0], x.shape[1]
     if M != B * T:
@@ -103,6 +103,7 @@ def gemm_rope_kv_write(x: torch.Tensor, wqkv: torch.Tensor, B: int, T: int, head
     args.mode = _lib.GEMM_PLAIN
     fill_gemm_args(args, x, wqkv)
     args.C, args.ldc = q_out.data_ptr(), N  # C itself is not written; a valid aligned pointer keeps the checks uniform
+    args.b_static = _scope.static_b
     args.epilogue = _lib.EPILOGUE_ROPE_KV
     args.epilogue_args = ctypes.cast(ctypes.pointer(r), ctypes.c_void_p)
     _lib.check(_lib.lib().oob_gemm(None, ctypes.byref(args), _stream()))

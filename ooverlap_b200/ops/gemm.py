@@ -7,7 +7,9 @@ generated CUTLASS instances.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
+import threading
 from typing import Optional
 
 import torch
@@ -16,6 +18,27 @@ from .. import _lib
 from . import solutions
 from ..utils.dtypes import dtype_code
 from ..utils.stream import current_stream_ptr
+
+
+class _Scope(threading.local):
+    static_b = False
+
+
+_scope = _Scope()
+
+
+@contextlib.contextmanager
+def static_weights():
+    """GEMMs that this thread launches in this block take their ``b`` to be a weight: neither the kernel before the call on the
+    stream nor, in a chain of this library's kernels, one of those before it writes ``b``.  The weight-streaming kernel then
+    loads its first weights while the kernel before it still runs.  Elsewhere ``b`` may be any tensor, also the result of
+    the call just before."""
+    before = _scope.static_b
+    _scope.static_b = True
+    try:
+        yield
+    finally:
+        _scope.static_b = before
 
 
 def _check_operands(a: torch.Tensor, b: torch.Tensor) -> None:
@@ -96,6 +119,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
     args.splitk_reduce = splitk_reduce
     args.gemv = gemv
     args.stream_k = stream_k
+    args.b_static = _scope.static_b
     if order is not None:
         check_order_buffer(order, M, N)
         args.order = order.data_ptr()
@@ -219,6 +243,7 @@ def gemm_swiglu(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = 
     fill_gemm_args(args, a, b)
     args.C, args.ldc = out.data_ptr(), out.stride(0)
     args.max_ctas = max_ctas
+    args.b_static = _scope.static_b
     args.epilogue = _lib.EPILOGUE_SWIGLU if can_fuse else _lib.EPILOGUE_SWIGLU_TILE
     args.epilogue_args = ctypes.cast(ctypes.pointer(epi), ctypes.c_void_p)
     rc = _lib.lib().oob_gemm(None, args, current_stream_ptr())

@@ -1,0 +1,69 @@
+"""GEMMs whose weights may be loaded ahead of the kernel before them: the same bits as without the promise, and without the
+promise an operand that the kernel before has just written."""
+import pytest
+import torch
+
+from ooverlap_b200.ops import gemm, gemm_rope_kv_write, gemm_swiglu, rmsnorm, rope_tables, static_weights
+from ooverlap_b200.ops.gemm import _scope
+
+pytestmark = pytest.mark.gpu
+
+
+def _chain(x, w, b, t, heads, kv, kc, vc, cos, sin, pos):
+    """Norm -> QKV + cache write -> norm -> gate/up -> down, every GEMM right behind another kernel of this library."""
+    h = rmsnorm(x, w["n"], 1e-5)
+    q = gemm_rope_kv_write(h, w["qkv"], b, t, heads, kv, kc, vc, cos, sin, pos)
+    y, r = rmsnorm(gemm(q, w["o"]), w["n"], 1e-5, x)
+    return q, r, gemm(gemm_swiglu(y, w["gu"]), w["d"])
+
+
+# one stage per CTA; several; more K than the ring holds (wide and narrow stages); two token blocks on CTA pairs
+@pytest.mark.parametrize("rows,hidden,ffn", [(1, 512, 256), (16, 1024, 520), (64, 4096, 1024), (100, 4096, 1024), (250, 2048, 1024)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_same_bits_with_weights_loaded_ahead(rows, hidden, ffn, dtype):
+    torch.manual_seed(0)
+    heads, kv, hd, max_len = 4, 2, 128, 64
+
+    def w(n, k):
+        return (torch.randn(n, k, device="cuda") / k ** 0.5).to(dtype)
+
+    ws = {"n": torch.ones(hidden, device="cuda", dtype=dtype), "qkv": w((heads + 2 * kv) * hd, hidden), "o": w(hidden, heads * hd),
+          "gu": w(2 * ffn, hidden), "d": w(hidden, ffn)}
+    x = torch.randn(rows, hidden, device="cuda").to(dtype)
+    cos, sin = rope_tables(max_len, hd, 10000.0, "cuda")
+    pos = torch.full((1,), 7, dtype=torch.long, device="cuda")
+    out = []
+    for ahead in (False, True):
+        kc = torch.zeros(rows, kv, max_len, hd, device="cuda", dtype=dtype)
+        vc = torch.zeros_like(kc)
+        if ahead:
+            with static_weights():
+                res = [_chain(x, ws, rows, 1, heads, kv, kc, vc, cos, sin, pos) for _ in range(3)][-1]
+        else:
+            res = _chain(x, ws, rows, 1, heads, kv, kc, vc, cos, sin, pos)
+        out.append((*res, kc, vc))
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
+
+
+def test_without_the_promise_b_may_be_the_result_of_the_call_before():
+    torch.manual_seed(1)
+    x = torch.randn(4096, 512, device="cuda").bfloat16()
+    y = (torch.randn(2048, 512, device="cuda") / 512 ** 0.5).bfloat16()
+    a = torch.randn(16, 2048, device="cuda").bfloat16()
+    b = torch.empty(4096, 2048, device="cuda", dtype=torch.bfloat16)
+    for _ in range(5):
+        b.fill_(float("nan"))
+        gemm(x, y, out=b)
+        got = gemm(a, b)
+        want = a.double() @ b.double().t()
+        assert (got.double() - want).norm() < 4e-3 * want.norm()
+
+
+def test_the_promise_ends_with_its_block():
+    assert not _scope.static_b
+    with pytest.raises(RuntimeError):
+        with static_weights():
+            assert _scope.static_b
+            raise RuntimeError
+    assert not _scope.static_b
