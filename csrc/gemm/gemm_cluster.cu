@@ -34,6 +34,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "../api/oob.h"
 #include "../api/oob_model.h"
@@ -91,6 +92,9 @@ struct ParamsC {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The two halves of cluster_sync.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
@@ -161,9 +165,32 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
   }
 }
 
+// Where a unit of a query, key or value head goes, and the rotation it gets.
+struct RopeUnit {
+  float2 cs, sn;
+  long long pos;
+  int hh, c, b;
+};
+__device__ __forceinline__ RopeUnit rope_unit(const ParamsC& p, int m, int n, long long pos_base) {
+  const oob_rope_args_t& a = p.rope;
+  RopeUnit r;
+  r.hh = n / a.hd;
+  r.c = n - r.hh * a.hd;
+  r.b = m / a.T;
+  r.pos = pos_base + (m - r.b * a.T);
+  if (r.pos < 0) r.pos = 0;
+  if (r.pos > a.max_len - 1) r.pos = a.max_len - 1;  // the host checks the range; never index outside the tables / cache
+  r.cs = r.sn = make_float2(0.f, 0.f);
+  if (r.hh < a.H + a.KV) {
+    r.cs = *reinterpret_cast<const float2*>(a.cos_table + r.pos * (a.hd / 2) + r.c / 2);
+    r.sn = *reinterpret_cast<const float2*>(a.sin_table + r.pos * (a.hd / 2) + r.c / 2);
+  }
+  return r;
+}
+
 // Writes token `m`, output columns n .. n + 3 (SwiGLU: `v` gate sums, `u` up sums).
 template <typename T, int EPI>
-__device__ __forceinline__ void emit(const ParamsC& p, int m, int n, const float4& v, const float4& u, long long pos_base) {
+__device__ __forceinline__ void emit(const ParamsC& p, int m, int n, const float4& v, const float4& u, const RopeUnit& r) {
   if constexpr (EPI == kEpiSwiglu) {
     if (n >= p.F) return;  // F % 8 == 0: the four columns are in or out together
     uint32_t g[4] = {__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w)};
@@ -174,24 +201,17 @@ __device__ __forceinline__ void emit(const ParamsC& p, int m, int n, const float
   } else if constexpr (EPI == kEpiRopeKv) {
     const oob_rope_args_t& a = p.rope;
     if (n >= p.N) return;  // N is a multiple of 8
-    const int hh = n / a.hd, c = n - hh * a.hd;
-    const int b = m / a.T, t = m - b * a.T;
-    long long pos = pos_base + t;
-    if (pos < 0) pos = 0;
-    if (pos > a.max_len - 1) pos = a.max_len - 1;  // the host checks the range; never index outside the tables / cache
     float4 x = v;
-    if (hh < a.H + a.KV) {
-      const float2 cs = *reinterpret_cast<const float2*>(a.cos_table + pos * (a.hd / 2) + c / 2);
-      const float2 sn = *reinterpret_cast<const float2*>(a.sin_table + pos * (a.hd / 2) + c / 2);
-      x = make_float4(v.x * cs.x - v.y * sn.x, v.x * sn.x + v.y * cs.x, v.z * cs.y - v.w * sn.y, v.z * sn.y + v.w * cs.y);
-    }
+    if (r.hh < a.H + a.KV)
+      x = make_float4(v.x * r.cs.x - v.y * r.sn.x, v.x * r.sn.x + v.y * r.cs.x, v.z * r.cs.y - v.w * r.sn.y,
+                      v.z * r.sn.y + v.w * r.cs.y);
     T* dst;
-    if (hh < a.H) {
-      dst = static_cast<T*>(a.q_out) + (static_cast<long long>(m) * a.H + hh) * a.hd + c;
+    if (r.hh < a.H) {
+      dst = static_cast<T*>(a.q_out) + (static_cast<long long>(m) * a.H + r.hh) * a.hd + r.c;
     } else {
-      const int kvh = hh < a.H + a.KV ? hh - a.H : hh - a.H - a.KV;
-      T* cache = static_cast<T*>(hh < a.H + a.KV ? a.k_cache : a.v_cache);
-      dst = cache + (a.batch0 + b) * a.cache_batch_stride + (static_cast<long long>(kvh) * a.max_len + pos) * a.hd + c;
+      const int kvh = r.hh < a.H + a.KV ? r.hh - a.H : r.hh - a.H - a.KV;
+      T* cache = static_cast<T*>(r.hh < a.H + a.KV ? a.k_cache : a.v_cache);
+      dst = cache + (a.batch0 + r.b) * a.cache_batch_stride + (static_cast<long long>(kvh) * a.max_len + r.pos) * a.hd + r.c;
     }
     *reinterpret_cast<uint2*>(dst) = make_uint2(pack2<T>(x.x, x.y), pack2<T>(x.z, x.w));
   } else {
@@ -210,9 +230,11 @@ __device__ __forceinline__ void emit(const ParamsC& p, int m, int n, const float
 // Sums the S partial copies of this CTA's share of a tile and writes them.  A unit is four output columns of a token; the
 // units are dealt out over the CTAs of the cluster, then over the threads, and TB units x S copies of independent loads are
 // in flight per thread.  `n_first`: first output column of the tile.
-template <typename T, int EPI, int S, bool PAIR>
+// All threads of the CTA call `read_done` together, once, when the last copies have been read and before the last results are
+// written: the cluster barrier behind it would otherwise wait for those stores (0.6 us).
+template <typename T, int EPI, int S, bool PAIR, typename F>
 __device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base, int rank, int m_first, int n_first, int rows,
-                                            long long pos_base) {
+                                            long long pos_base, F read_done) {
   constexpr int kParts = EPI == kEpiSwiglu ? 2 : 1;  // gate and up columns
   constexpr int TB = S * kParts >= 8 ? 1 : (S * kParts >= 4 ? 2 : 4);
   uint32_t base[S];
@@ -220,37 +242,45 @@ __device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base
   for (int r = 0; r < S; ++r) base[r] = S == 1 ? smem_base : map_to_cta(smem_base, PAIR ? r * 2 + (cluster_ctarank() & 1) : r);
   constexpr int upt = kRowsW / 4 / kParts;  // units of a token
   const int units = rows * upt;
-  const int u1 = units * (rank + 1) / S;
-  for (int u0 = units * rank / S + int(threadIdx.x); u0 < u1; u0 += kThreadsC * TB) {
+  const int u_first = units * rank / S, u1 = units * (rank + 1) / S;
+  const int turns = (u1 - u_first + kThreadsC * TB - 1) / (kThreadsC * TB);  // the same for all threads
+  for (int turn = 0; turn < turns; ++turn) {
+    const int u0 = u_first + turn * kThreadsC * TB + int(threadIdx.x);
     float4 v[TB][kParts][S];
+    RopeUnit rope[TB];
     int m[TB], c[TB];
 #pragma unroll
     for (int i = 0; i < TB; ++i) {
-      const int u = u0 + i * kThreadsC < u1 ? u0 + i * kThreadsC : u0;  // past the end: re-read a live unit, result unused
+      const int u = u0 + i * kThreadsC < u1 ? u0 + i * kThreadsC : u_first;  // past the end: re-read a live unit, result unused
       m[i] = u / upt;
       c[i] = (u - m[i] * upt) * 4;
+      if constexpr (EPI == kEpiRopeKv) rope[i] = rope_unit(p, m_first + m[i], n_first + c[i], pos_base);
 #pragma unroll
       for (int h = 0; h < kParts; ++h)
 #pragma unroll
         for (int r = 0; r < S; ++r) v[i][h][r] = ld_cluster_f4(base[r] + uint32_t(m[i] * kRowsW + h * (kRowsW / 2) + c[i]) * 4u);
     }
+    float4 s[TB][kParts];
 #pragma unroll
     for (int i = 0; i < TB; ++i) {
-      float4 s[kParts];
 #pragma unroll
       for (int h = 0; h < kParts; ++h) {
-        s[h] = v[i][h][0];
+        s[i][h] = v[i][h][0];
 #pragma unroll
         for (int r = 1; r < S; ++r) {
-          s[h].x += v[i][h][r].x;
-          s[h].y += v[i][h][r].y;
-          s[h].z += v[i][h][r].z;
-          s[h].w += v[i][h][r].w;
+          s[i][h].x += v[i][h][r].x;
+          s[i][h].y += v[i][h][r].y;
+          s[i][h].z += v[i][h][r].z;
+          s[i][h].w += v[i][h][r].w;
         }
       }
-      if (u0 + i * kThreadsC < u1) emit<T, EPI>(p, m_first + m[i], n_first + c[i], s[0], s[kParts - 1], pos_base);
     }
+    if (turn + 1 == turns) read_done();
+#pragma unroll
+    for (int i = 0; i < TB; ++i)
+      if (u0 + i * kThreadsC < u1) emit<T, EPI>(p, m_first + m[i], n_first + c[i], s[i][0], s[i][kParts - 1], rope[i]);
   }
+  if (turns == 0) read_done();
 }
 
 // SUB: 64-element boxes of K in a pipeline stage.
@@ -324,36 +354,53 @@ __global__ void __launch_bounds__(kThreadsC)
     const int tile = wide_tile * P + member;  // this CTA's 128 weight rows
     const int w_row = EPI == kEpiSwiglu ? tile * (kRowsW / 2) : tile * kRowsW;
     const int rows = min(p.Mp, p.M - m_first);
-    if (warp == 0 || warp == 2) {
-      if (ptx::elect_one()) {
-        // ------------------------- TMA producers: warp 0 the weights, warp 2 the activations -------------------------
-        const bool weights = warp == 0;
-        const uint32_t bytes = P * (weights ? SUB * w_bytes : x_bytes);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!ptx::mbar_wait(&ctl->empty[stage], phase ^ 1, abort)) break;
-          uint8_t* sw = smem + stage * p.stage_bytes;
-          // The bytes of both CTAs of a pair are counted on the leader's barrier.
-          if (member == 0) ptx::mbar_arrive_expect_tx(&ctl->full[stage], bytes);
-          uint32_t full = ptx::smem_u32(&ctl->full[stage]);
-          if constexpr (PAIR) full = map_to_cta(full, in_cluster & ~1);
+    using One = std::integral_constant<int, 1>;
+    using Two = std::integral_constant<int, 2>;
+    // ------------------------- TMA producers: warp 0 the weights, warp 2 the activations -------------------------
+    // Straight-line copies of the loops here and below: where the compiler cannot see which tensor map a thread takes or how
+    // many instructions it issues, 64 elements of K take a CTA 0.16 us (16 tokens) and 0.26 (128) instead of 0.107 and 0.142.
+    auto produce = [&](auto weights, auto instructions) {
+      constexpr bool W = decltype(weights)::value;
+      constexpr int NM = decltype(instructions)::value;
+      const uint32_t bytes = P * (W ? SUB * w_bytes : x_bytes);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!ptx::mbar_wait(&ctl->empty[stage], phase ^ 1, abort)) break;
+        uint8_t* sw = smem + stage * p.stage_bytes;
+        // The bytes of both CTAs of a pair are counted on the leader's barrier.
+        if (!PAIR || member == 0) ptx::mbar_arrive_expect_tx(&ctl->full[stage], bytes);
+        uint32_t full = ptx::smem_u32(&ctl->full[stage]);
+        if constexpr (PAIR) full = map_to_cta(full, in_cluster & ~1);
 #pragma unroll
-          for (int h = 0; h < SUB; ++h) {
-            const int k = (kb * SUB + h) * kTileK;  // past K: the box is filled with zeros
-            if (weights) {
-              load_box<PAIR>(sw + h * w_bytes, &tmap_w, full, k, w_row);
-              if constexpr (EPI == kEpiSwiglu) load_box<PAIR>(sw + h * w_bytes + w_bytes / 2, &tmap_w, full, k, p.F + w_row);
-            } else {
-              for (int j = 0; j < p.n_mma; ++j)
-                load_box<PAIR>(sw + SUB * w_bytes + h * (x_bytes / SUB) + j * (p.nj / P) * kRowBytes, &tmap_x, full, k,
-                               m_first + j * p.nj + member * (p.nj / P));
-            }
-          }
-          if (++stage == p.stages) {
-            stage = 0;
-            phase ^= 1;
+        for (int h = 0; h < SUB; ++h) {
+          const int k = (kb * SUB + h) * kTileK;  // past K: the box is filled with zeros
+          if constexpr (W) {
+            load_box<PAIR>(sw + h * w_bytes, &tmap_w, full, k, w_row);
+            if constexpr (EPI == kEpiSwiglu) load_box<PAIR>(sw + h * w_bytes + w_bytes / 2, &tmap_w, full, k, p.F + w_row);
+          } else {
+            uint8_t* sx = sw + SUB * w_bytes + h * (x_bytes / SUB);
+#pragma unroll
+            for (int j = 0; j < NM; ++j)
+              load_box<PAIR>(sx + j * (p.nj / P) * kRowBytes, &tmap_x, full, k, m_first + j * p.nj + member * (p.nj / P));
           }
         }
+        if (++stage == p.stages) {
+          stage = 0;
+          phase ^= 1;
+        }
       }
+    };
+    if (warp == 0) {
+      if (ptx::elect_one()) produce(std::true_type{}, One{});
+    } else if (warp == 2) {
+      if (ptx::elect_one()) {
+        if (SUB == 1 && p.n_mma == 2) {  // a wide stage holds one instruction's tokens
+          produce(std::false_type{}, Two{});
+        } else {
+          produce(std::false_type{}, One{});
+        }
+      }
+    }
+    if (warp == 0 || warp == 2) {
       __syncwarp();
       if (!waited) {  // the results below go where earlier kernels may still read
         ptx::griddep_wait();
@@ -367,39 +414,51 @@ __global__ void __launch_bounds__(kThreadsC)
         const uint32_t idesc = ptx::umma_idesc_f16(FMT, P * kRowsW, p.nj);
         [[maybe_unused]] const uint16_t mask = static_cast<uint16_t>(3u << in_cluster);  // both CTAs of the pair
         bool ok = true;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!ptx::mbar_wait(&ctl->full[stage], phase, abort)) {
-            ok = false;
-            break;
-          }
-          ptx::tc_fence_after_sync();
-          const uint32_t sw = ptx::smem_u32(smem + stage * p.stage_bytes);
+        auto multiply = [&](auto instructions) {
+          constexpr int NM = decltype(instructions)::value;
+          bool ready = false;  // seen while the stage before was worked on
+          for (int kb = kb0; kb < kb1; ++kb) {
+            if (!ready && !ptx::mbar_wait(&ctl->full[stage], phase, abort)) {
+              ok = false;
+              break;
+            }
+            ptx::tc_fence_after_sync();
+            const uint32_t sw = ptx::smem_u32(smem + stage * p.stage_bytes);
+            uint64_t* empty = &ctl->empty[stage];
+            if (++stage == p.stages) {
+              stage = 0;
+              phase ^= 1;
+            }
+            ready = kb + 1 < kb1 && ptx::mbar_test_wait(&ctl->full[stage], phase);
 #pragma unroll
-          for (int h = 0; h < SUB; ++h) {
-            const uint64_t da = ptx::umma_desc_kmajor_sw128(sw + h * w_bytes);
-            for (int j = 0; j < p.n_mma; ++j) {
-              const uint64_t db = ptx::umma_desc_kmajor_sw128(sw + SUB * w_bytes + h * (x_bytes / SUB) + j * (p.nj / P) * kRowBytes);
-              const uint32_t d_tmem = tmem_base + j * p.nj;
+            for (int h = 0; h < SUB; ++h) {
+              const uint64_t da = ptx::umma_desc_kmajor_sw128(sw + h * w_bytes);
 #pragma unroll
-              for (int k = 0; k < kTileK / 16; ++k) {
-                const uint32_t add = (kb > kb0 || h > 0 || k > 0) ? 1u : 0u;
-                if constexpr (PAIR) {
-                  umma_f16_pair(d_tmem, da + uint64_t(k * 2), db + uint64_t(k * 2), idesc, add);
-                } else {
-                  ptx::umma_f16(d_tmem, da + uint64_t(k * 2), db + uint64_t(k * 2), idesc, add);
+              for (int j = 0; j < NM; ++j) {
+                const uint64_t db = ptx::umma_desc_kmajor_sw128(sw + SUB * w_bytes + h * (x_bytes / SUB) + j * (p.nj / P) * kRowBytes);
+                const uint32_t d_tmem = tmem_base + j * p.nj;
+#pragma unroll
+                for (int k = 0; k < kTileK / 16; ++k) {
+                  const uint32_t add = (kb > kb0 || h > 0 || k > 0) ? 1u : 0u;
+                  if constexpr (PAIR) {
+                    umma_f16_pair(d_tmem, da + uint64_t(k * 2), db + uint64_t(k * 2), idesc, add);
+                  } else {
+                    ptx::umma_f16(d_tmem, da + uint64_t(k * 2), db + uint64_t(k * 2), idesc, add);
+                  }
                 }
               }
             }
+            if constexpr (PAIR) {
+              umma_commit_pair(empty, mask);
+            } else {
+              ptx::umma_commit(empty);
+            }
           }
-          if constexpr (PAIR) {
-            umma_commit_pair(&ctl->empty[stage], mask);
-          } else {
-            ptx::umma_commit(&ctl->empty[stage]);
-          }
-          if (++stage == p.stages) {
-            stage = 0;
-            phase ^= 1;
-          }
+        };
+        if (SUB == 1 && p.n_mma == 2) {
+          multiply(Two{});
+        } else {
+          multiply(One{});
         }
         if (ok) {
           if constexpr (PAIR) {
@@ -433,8 +492,15 @@ __global__ void __launch_bounds__(kThreadsC)
       __syncthreads();
     }
     const uint32_t own = ptx::smem_u32(smem);
+    // Nobody reads this CTA's copy any more: the buffers belong to the pipeline again (or to the next kernel).
+    const bool last_tile = t + p.clusters >= p.num_tiles;
+    auto read_done = [&]() {
+      if (!last_tile) ptx::fence_proxy_async_all();
+      __syncwarp();
+      if (S * P > 1) cluster_arrive();
+    };
 #define OOB_REDUCE(SS) \
-  case SS: reduce_tile<T, EPI, SS, PAIR>(p, own, rank, m_first, w_row, rows, pos_base); break;
+  case SS: reduce_tile<T, EPI, SS, PAIR>(p, own, rank, m_first, w_row, rows, pos_base, read_done); break;
     switch (S) {
       OOB_REDUCE(1) OOB_REDUCE(2) OOB_REDUCE(3) OOB_REDUCE(4)
       default:
@@ -443,11 +509,9 @@ __global__ void __launch_bounds__(kThreadsC)
         }
     }
 #undef OOB_REDUCE
-    // Nobody reads this CTA's copy any more: the buffers belong to the pipeline again (or to the next kernel).
-    ptx::fence_proxy_async_all();
     __syncwarp();
     if (S * P > 1) {
-      cluster_sync();
+      cluster_wait();
     } else {
       __syncthreads();
     }
