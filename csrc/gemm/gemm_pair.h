@@ -13,7 +13,8 @@ namespace gemm_pair {
 // accumulator (256x256 fp32), so the size depends on the pair count only.
 constexpr int kSkMaxPairs = 80;               // >= 74 pairs of a 148-SM part
 constexpr int kSkMaxTiles = 2 * kSkMaxPairs;  // tiles of a tail
-constexpr size_t kSkFlagBytes = 8192;         // kSkMaxTiles x 2 CTAs x 4 warps x 4 bytes, rounded up
+constexpr int kSkWarps = 8;                   // epilogue warps of a CTA that park and add
+constexpr size_t kSkFlagBytes = 16384;        // kSkMaxTiles x 2 CTAs x kSkWarps x 4 bytes, rounded up
 constexpr size_t kSkSlotBytes = size_t(256) * 256 * 4;
 constexpr size_t kSkWorkspaceBytes = kSkFlagBytes + size_t(kSkMaxPairs) * kSkSlotBytes;
 
@@ -23,7 +24,8 @@ struct PairPlan {
   int sk_tiles;    // tiles of the stream-K tail, 0 = every tile is computed whole by one pair
   int sk_pairs;    // pairs that share the tail
   void* sk_ws;     // stream-K workspace (flags + slots), null without a tail
-  int tile_n;      // columns of a tile: 256 except in plain launches without a tail (pair_cut)
+  int tile_n;      // columns of an accumulator: 256 except in plain launches without a tail (pair_cut)
+  int joined;      // accumulators of a tile: a tile is joined * tile_n columns wide
 };
 
 // ---- schedule (host and device: the host side exists for tests of the enumeration) ------------------------------
@@ -143,12 +145,15 @@ int pair_streamk_auto(int tiles, int pairs, int num_kb, long long operand_bytes)
 void pair_streamk_plan(int tiles, int pairs, int num_kb, int* sk_tiles, int* sk_pairs);
 
 // How a problem is cut into tiles on `pairs` pairs: 256 columns with or without a stream-K tail or, in plain launches that do
-// not ask for a tail, narrower tiles where these are expected to be clearly faster.  `order`: a tile-order record is written.
-// Both sides measured, bf16: 512 x 8192 x 8192 50.9 us at 224 columns (74 tiles) and 52.8 - 61 at 256 (64 tiles),
-// 250 x 8192 x 3584 18.1 at 128 and 23.3 at 256, 2048 x 2048 x 2048 17.2 at 256 and 25.7 with the tail, 4096 x 7168 x 8192
-// 304 at 224, 309 with the tail and 323 at 256.
+// not ask for a tail, another width where it is expected to be faster.  Up to 256 columns the two accumulators alternate between
+// tiles; a wider tile takes both at once, which brings fewer operand bytes per product and leaves the drain of a tile to be
+// waited for.  `order`: a tile-order record is written.
+// Both sides measured, bf16: 512 x 8192 x 8192 51 us at 224 columns (74 tiles) and 52 at 256 (64 tiles), 4096 x 1280 x 8192 60.3 at
+// 320 and 82 at 256 (75.6 with a tail), 1037 x 4104 x 2056 23.0 at 320 and 28.5 at 160, 768 x 7168 x 8192 64.7 at 320 and 68.3 at 160,
+// 2048 x 2048 x 2048 17.5 at 256 and 31 with a tail, 4096 x 3584 x 8192 163.7 at 160, 164.6 with a tail and 174.9 at 256.
 struct PairCut {
-  int tile_n;  // columns of a tile
+  int tile_n;  // columns of an accumulator
+  int joined;  // accumulators of a tile
   int tiles;
   int sk_tiles, sk_pairs;  // stream-K tail (256-column tiles), both 0 without one
   double us;  // what it is expected to take
