@@ -668,12 +668,21 @@ int cluster_slots(int sms, int size, int per_sm) {
   return 8 * (18 * per_sm / size);
 }
 
-// Microseconds a plan takes, fitted to sweeps on B200: rounds of clusters, each as long as its K blocks at the pace of one
-// CTA or of the tensor cores of an SM (2 x tokens cycles a block), at the memory's rate for the weights or at L2's for all
-// operands, whichever is slowest; then draining the sums, reading the other CTAs' sums, and the fixed cost of a launch.
-// `ragged`: rows start off a 128-byte line, a row of a box touches two, and the pace and L2's rate are 1.45 times worse (for the
-// comparison with the two-SM kernel; the plans were swept with rows on a line).
-double plan_cost(int N, int num_kb, int sms, bool ragged, const PlanC& pl) {
+// Microseconds a plan takes: rounds of clusters, each as long as its K blocks at the pace of one CTA or of the tensor cores of an
+// SM (cycles a block grow with the tokens), at the memory's rate for the weights or at L2's for all operands, whichever is
+// slowest; then draining the sums, reading the other CTAs' sums, and the fixed cost of a launch.  `ragged`: rows start off a
+// 128-byte line, and a row of a box touches two.
+// The constants are fitted to timings for the choice they make, so that one need not be the rate that it stands for.  Up to 128 rows to
+// 16000 timings of every K split (1930 shapes of 3 - 128 rows, N and K of 512 - 8192): 3.3 % off the best plan on average, 4.8 % with
+// the other set.  Above, the set against which the two-SM kernel is weighed.
+struct CostC {
+  double wide, wide_tokens, pace, pace_tokens, mma, l2, hbm, drain, reduce, round, alone, cluster, eight, split, ragged;
+};
+constexpr CostC kFewRows = {0.153, 0.00061, 0.17, 0.00028, 1140.0, 11.8e6, 6.4e6, 0.0117, 2.84e6, 1.85, 2.52, 3.06, 2.6, 0.105, 1.29};
+constexpr CostC kMoreRows = {0.165, 0.0005, 0.235, 0.0002, 1850.0, 11.5e6, 6.4e6, 0.015, 3.0e6, 2.0, 3.4, 3.8, 2.0, 0.08, 1.45};
+
+double plan_cost(int M, int N, int num_kb, int sms, bool ragged, const PlanC& pl) {
+  const CostC& c = M <= kTileM ? kFewRows : kMoreRows;
   const int P = pl.pair ? 2 : 1, Mp = pl.n_mma * pl.nj, size = P * pl.S;
   const int clusters = tile_count(N, pl), slots = cluster_slots(sms, size, pl.per_sm);
   const int rounds = (clusters + slots - 1) / slots;
@@ -681,18 +690,27 @@ double plan_cost(int N, int num_kb, int sms, bool ragged, const PlanC& pl) {
   const double share = live > sms ? live / sms : 1.0;
   const double kb = double((num_kb + pl.S - 1) / pl.S);
   const double w = kRowsW * kRowBytes, x = double(Mp) / P * kRowBytes;
-  const double lines = ragged ? 1.45 : 1.0;
-  double t = lines * kb * (pl.sub == 2 ? 0.165 + 0.0005 * Mp : 0.235 + 0.0002 * Mp);
-  const double mma = share * kb * 2.0 * Mp / 1850.0, l2 = lines * live * kb * (w + x) / 11.5e6, hbm = live * kb * w / pl.m_blocks / 6.4e6;
+  const double lines = ragged ? c.ragged : 1.0;
+  double t = lines * kb * (pl.sub == 2 ? c.wide + c.wide_tokens * Mp : c.pace + c.pace_tokens * Mp);
+  const double mma = share * kb * 2.0 * Mp / c.mma, l2 = lines * live * kb * (w + x) / c.l2, hbm = live * kb * w / pl.m_blocks / c.hbm;
   if (mma > t) t = mma;
   if (l2 > t) t = l2;
   if (hbm > t) t = hbm;
-  t += 0.015 * Mp + live * Mp * kRowsW * 4.0 * (pl.S - 1) / pl.S / 3.0e6;
-  return rounds * t + (rounds - 1) * 2.0 + (size > 1 ? 3.8 : 3.4) + (size == 8 && Mp > 128 ? 2.0 : 0.0) + 0.08 * (pl.S - 1);
+  t += c.drain * Mp + live * Mp * kRowsW * 4.0 * (pl.S - 1) / pl.S / c.reduce;
+  return rounds * t + (rounds - 1) * c.round + (size > 1 ? c.cluster : c.alone) + (size == 8 && Mp > 128 ? c.eight : 0.0) +
+         c.split * (pl.S - 1);
 }
 
-// The cheapest cut of a problem.  `fix_s` > 0 fixes the K split, `pair` is as in GemmArgs.
-bool plan(int M, int N, int K, int sms, int pair, int fix_s, PlanC* out, double* cost) {
+// What static weights save: the rings are filled while the kernel before ends.  Plans with more CTAs hold more (32 x 8192 x 3584 in a
+// decode step 13.3 us on 128 CTAs, 14.3 on 64, which were taken for faster).
+double ring_us(int N, int num_kb, int sms, const PlanC& pl) {
+  const int clusters = tile_count(N, pl), size = (pl.pair ? 2 : 1) * pl.S, slots = cluster_slots(sms, size, pl.per_sm);
+  const double live = double(clusters < slots ? clusters : slots) * size;
+  return live * pl.stages * pl.sub * kRowsW * kRowBytes / 6.05e6;
+}
+
+// The cheapest cut of a problem.  `fix_s` > 0 fixes the K split, `pair` is as in GemmArgs; `ahead`: static weights.
+bool plan(int M, int N, int K, int sms, int pair, int fix_s, bool ahead, PlanC* out, double* cost) {
   const int num_kb = (K + kTileK - 1) / kTileK;
   if (N <= kRowsW) pair = -1;  // one weight tile is no pair
   bool found = false;
@@ -710,7 +728,9 @@ bool plan(int M, int N, int K, int sms, int pair, int fix_s, PlanC* out, double*
       for (pl.S = 1; pl.S <= kMaxCluster / (two ? 2 : 1); ++pl.S) {
         if (fix_s > 0 ? pl.S != fix_s : (num_kb < 4 * pl.S && pl.S > 1)) continue;
         if (!size_cta(N, num_kb, sms, &pl)) continue;
-        const double c = plan_cost(N, num_kb, sms, false, pl);
+        // (with more rows the plans are compared as if rows started on a line: the set was fitted so)
+        double c = plan_cost(M, N, num_kb, sms, M <= kTileM && K % kTileK != 0, pl);
+        if (ahead) c -= ring_us(N, num_kb, sms, pl);
         if (!found || c < *cost) {
           found = true;
           *out = pl;
@@ -729,9 +749,9 @@ struct Planned {
   PlanC pl;
   double cost;
 };
-const Planned& planned(int M, int N, int K, int pair, int fix_s) {
+const Planned& planned(int M, int N, int K, int pair, int fix_s, bool ahead) {
   static thread_local Planned cache[64];
-  const int flags = 1 | (pair > 0 ? 2 : pair < 0 ? 1 : 0) << 1 | fix_s << 3;
+  const int flags = 1 | (pair > 0 ? 2 : pair < 0 ? 1 : 0) << 1 | (ahead ? 1 : 0) << 3 | fix_s << 4;
   Planned& c = cache[(static_cast<unsigned>(M) * 2654435761u ^ static_cast<unsigned>(N) * 40503u ^ static_cast<unsigned>(K) * 97u ^
                       static_cast<unsigned>(flags) * 7u) >> 8 & 63u];
   if (c.M != M || c.N != N || c.K != K || c.flags != flags) {
@@ -739,7 +759,7 @@ const Planned& planned(int M, int N, int K, int pair, int fix_s) {
     c.N = N;
     c.K = K;
     c.flags = flags;
-    c.ok = plan(M, N, K, sm_count(), pair, fix_s, &c.pl, &c.cost);
+    c.ok = plan(M, N, K, sm_count(), pair, fix_s, ahead, &c.pl, &c.cost);
   }
   return c;
 }
@@ -752,11 +772,11 @@ bool gemm_cluster_supported(const GemmArgs& a) {
 
 // Whether this kernel is expected to be faster than the persistent two-SM kernel, which overlaps a tile's epilogue with the next
 // tile and needs no sum of parts, but deals out 256-row tiles: with fewer than three rounds of those, what they leave
-// idle or compute on padding is often more than this kernel's fixed cost.  The two models, each with a spread of 12 %, choose a
-// kernel that is 1.5 % slower than the best choice on average over 283 shapes, 18 % at worst (512 x 2048 x 2048).  Both sides
-// measured, bf16 on B200: 512 x 1280 x 8192 17.4 here and 29.6 us there, 200 x 4096 x 4096 15.0 and 18.1, 1000 x 1280 x 8192 23.9 and
-// 29.6, 1037 x 4104 x 2056 26.4 and 28.7; 250 x 8192 x 3584 20.7 and 18.1, 512 x 8192 x 8192 54.8 and 50.9, 2048 x 2048 x 2048 22.3 and
-// 17.2.
+// idle or compute on padding is often more than this kernel's fixed cost.  Its estimate is taken a tenth lower,
+// which fits its present pace: over 1611 shapes of more than 128 rows the choice is then 3.1 % slower than the best one on average.
+// Both sides measured, bf16 on B200: 512 x 1280 x 8192 17.4 here and 29.6 us there, 200 x 4096 x 4096 15.0 and 18.1, 512 x 2048 x 2048
+// 12.0 and 11.9; 1037 x 4104 x 2056 27.2 and 23.0, 768 x 7168 x 8192 71.5 and 64.7, 512 x 8192 x 8192 53.8 and 51.0, 2048 x 2048 x 2048
+// 20.5 and 17.5.
 bool gemm_cluster_preferred(const GemmArgs& a) {
   using namespace gemm_cluster;
   // Up to 128 rows the alternative is the one-SM kernel, persistent from the first tile to the last, on 256 weight rows a tile.
@@ -771,8 +791,8 @@ bool gemm_cluster_preferred(const GemmArgs& a) {
   const int pairs = sm_count() / 2;
   if (static_cast<long long>((a.M + 2 * kTileM - 1) / (2 * kTileM)) * ((a.N + kTileN - 1) / kTileN) > 3ll * pairs) return false;
   const double two_sm = pair_cut(kGemmPlain, a.M, a.N, a.K, pairs, a.stream_k, swiglu, false, false).us;
-  const Planned& c = planned(a.M, a.N, a.K, a.pair, 0);
-  return c.ok && plan_cost(a.N, (a.K + kTileK - 1) / kTileK, sm_count(), a.K % kTileK != 0, c.pl) < two_sm;
+  const Planned& c = planned(a.M, a.N, a.K, a.pair, 0, false);
+  return c.ok && 0.9 * plan_cost(a.M, a.N, (a.K + kTileK - 1) / kTileK, sm_count(), a.K % kTileK != 0, c.pl) < two_sm;
 }
 
 cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStream_t stream, gemm_detail::TmapFn make_tmap) {
@@ -787,7 +807,7 @@ cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStr
     if (fix_s == 0) fix_s = 1;
     if (fix_s > a.max_ctas) fix_s = a.max_ctas;
   }
-  const Planned& chosen = planned(a.M, a.N, a.K, a.max_ctas > 0 ? -1 : a.pair, fix_s);
+  const Planned& chosen = planned(a.M, a.N, a.K, a.max_ctas > 0 ? -1 : a.pair, fix_s, a.b_static != 0);
   if (!chosen.ok) return cudaErrorInvalidValue;
   const PlanC pl = chosen.pl;
   const int P = pl.pair ? 2 : 1;

@@ -1,5 +1,7 @@
-"""GEMMs whose weights may be loaded ahead of the kernel before them: the same bits as without the promise, and without the
-promise an operand that the kernel before has just written."""
+"""GEMMs whose weights may be loaded ahead of the kernel before them: the results of calls without the promise, the same bits each
+time, and without the promise an operand that the kernel before has just written."""
+import contextlib
+
 import pytest
 import torch
 
@@ -20,7 +22,7 @@ def _chain(x, w, b, t, heads, kv, kc, vc, cos, sin, pos):
 # one stage per CTA; several; more K than the ring holds (wide and narrow stages); two token blocks on CTA pairs
 @pytest.mark.parametrize("rows,hidden,ffn", [(1, 512, 256), (16, 1024, 520), (64, 4096, 1024), (100, 4096, 1024), (250, 2048, 1024)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-def test_same_bits_with_weights_loaded_ahead(rows, hidden, ffn, dtype):
+def test_weights_loaded_ahead(rows, hidden, ffn, dtype):
     torch.manual_seed(0)
     heads, kv, hd, max_len = 4, 2, 128, 64
 
@@ -33,17 +35,18 @@ def test_same_bits_with_weights_loaded_ahead(rows, hidden, ffn, dtype):
     cos, sin = rope_tables(max_len, hd, 10000.0, "cuda")
     pos = torch.full((1,), 7, dtype=torch.long, device="cuda")
     out = []
-    for ahead in (False, True):
+    for ahead in (False, True, True, True):
         kc = torch.zeros(rows, kv, max_len, hd, device="cuda", dtype=dtype)
         vc = torch.zeros_like(kc)
-        if ahead:
-            with static_weights():
-                res = [_chain(x, ws, rows, 1, heads, kv, kc, vc, cos, sin, pos) for _ in range(3)][-1]
-        else:
-            res = _chain(x, ws, rows, 1, heads, kv, kc, vc, cos, sin, pos)
-        out.append((*res, kc, vc))
-    for a, b in zip(*out):
-        assert torch.equal(a, b)
+        with static_weights() if ahead else contextlib.nullcontext():
+            out.append((*_chain(x, ws, rows, 1, heads, kv, kc, vc, cos, sin, pos), kc, vc))
+    for again in out[2:]:
+        assert all(torch.equal(a, b) for a, b in zip(out[1], again))
+    # K may be split differently: sums of fp32 in another order, which now and then round to the neighbouring 16-bit value; four
+    # 16-bit steps lie between x and the last result.
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for a, b in zip(out[0], out[1]):
+        assert (a.double() - b.double()).norm() <= 4 * eps * a.double().norm()
 
 
 def test_without_the_promise_b_may_be_the_result_of_the_call_before():
