@@ -12,6 +12,7 @@ Capability parity: the reference exposes its C++ through two pybind11 modules
 from __future__ import annotations
 
 import ctypes
+import struct
 import threading
 from ctypes import (POINTER, Structure, byref, c_char_p, c_float, c_int, c_int64, c_uint, c_uint64, c_void_p)
 
@@ -105,6 +106,19 @@ _lib = None
 
 
 def _declare(lib) -> None:
+def packer(structure) -> struct.Struct:
+    """The same layout for ``struct.pack``, which fills all fields in one step: what a call of a microsecond-sized kernel takes on the
+    host counts."""
+    codes = {c_int: "i", c_float: "f", c_uint64: "Q", c_int64: "q", c_void_p: "P"}
+    return struct.Struct("@" + "".join(codes[t] for _, t in structure._fields_) + "0P")
+
+
+NORM_ARGS = packer(NormArgs)
+# GemmArgs: the fields every plain call sets, and the rest with nothing asked for, with and without static weights.
+GEMM_HEAD = struct.Struct("@iiiiiPiPiPi")
+GEMM_TAIL = bytes(ctypes.sizeof(GemmArgs) - GEMM_HEAD.size)
+GEMM_TAIL_STATIC = bytes(GemmArgs(b_static=1))[GEMM_HEAD.size:]
+
     P = c_void_p
     lib.oob_last_error.restype = c_char_p
     lib.oob_version.restype = c_char_p
@@ -142,6 +156,8 @@ def _declare(lib) -> None:
     lib.oob_pad_counter_offset.argtypes = []
     lib.oob_pad_counter_count.argtypes = []
     lib.oob_gemm_counters_needed.argtypes = [c_int, c_int, c_int, c_int]
+    lib.packed_fused_norm = ctypes.CFUNCTYPE(c_int, P, c_int, c_char_p, c_int, P)(("oob_fused_norm", lib))
+    lib.packed_gemm = ctypes.CFUNCTYPE(c_int, P, c_char_p, P)(("oob_gemm", lib))
     lib.oob_test_pair_schedule.argtypes = [c_int] * 8 + [POINTER(c_int), c_int]
     lib.oob_test_pair_tile_columns.argtypes = [c_int] * 6
     lib.oob_gemm_reserve_workspace.argtypes = [c_uint64]

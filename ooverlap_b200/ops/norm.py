@@ -36,15 +36,11 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, residual: 
     y = out if out is not None else torch.empty_like(x)
     if residual is not None and residual_out is None:
         residual_out = torch.empty_like(x)
-    a = _lib.NormArgs()
-    a.dtype, a.rows, a.hidden, a.eps = dtype_code(x.dtype), rows, hidden, eps
-    a.x_reg, a.x_off = 0, x.data_ptr()  # no communicator: x_off carries the address
-    a.residual = residual.data_ptr() if residual is not None else None
-    a.weight = weight.data_ptr()
-    a.y_local = y.data_ptr()
-    a.res_out_reg = -1
-    a.res_out_local = residual_out.data_ptr() if residual_out is not None else None
-    rc = _lib.lib().oob_fused_norm(None, _lib.NORM_LOCAL, a, max_ctas, _stream())
+    # Fields in the order of the structure.  No communicator: x_off carries the address.
+    a = _lib.NORM_ARGS.pack(dtype_code(x.dtype), rows, hidden, eps, 0, x.data_ptr(), residual.data_ptr() if residual is not None else 0,
+                            weight.data_ptr(), 0, 0, y.data_ptr(), -1, 0, residual_out.data_ptr() if residual_out is not None else 0,
+                            0, 0, 0, 0)
+    rc = _lib.lib().packed_fused_norm(None, _lib.NORM_LOCAL, a, max_ctas, _stream())
     if rc:
         _lib.check(rc)
     return (y, residual_out) if residual is not None else y
