@@ -217,12 +217,25 @@ typedef struct {
                    complete (fused AR / RS: published to its reducer), [1] = pair << 32 | index in the pair's sequence */
   int b_static; /* plain mode: 1 = nothing that this call could overtake writes B (weights): the kernel may read B while the
                    kernel before it on the stream still runs.  0 = B may be that kernel's output */
+  const float* row_ssq; /* plain mode, M <= 128: row m of the product is multiplied by 1 / sqrt(s / K + row_eps), s = the sum over
+                           row_parts of row_ssq[part * M + m] (the sums that OOB_EPILOGUE_ADD writes); null = not */
+  int row_parts;
+  float row_eps;
 } oob_gemm_args_t;
 #define OOB_EPILOGUE_NONE 0
 #define OOB_EPILOGUE_SWIGLU 1  /* N = 2F columns [gate | up]; C is [M, F] = silu(gate) * up */
 #define OOB_EPILOGUE_ROPE_KV 2 /* columns = (H + 2 KV) heads of hd: rotate q and k, q -> q_out, k and v -> cache; C unused */
 #define OOB_EPILOGUE_SWIGLU_TILE 3 /* as 1, for any problem: applied where a GEMM tile is written.  OOB_ERR_UNSUPPORTED where no
                                       kernel may (pair) or should (one row of a large weight): then oob_gemm + oob_silu_mul */
+#define OOB_EPILOGUE_ADD 4 /* M <= 128, N % 8 == 0: C = round(A B^T) + residual, scaled_out = C * norm_weight, and per 128 columns the
+                              sums of the squares of C's rows.  OOB_ERR_UNSUPPORTED where the weight-streaming kernel may not run */
+typedef struct {
+  const void* residual;    /* [M, N], row stride ld_residual (a multiple of 4 elements, 8-byte aligned) */
+  int ld_residual;
+  const void* norm_weight; /* [N] */
+  void* scaled_out;        /* [M, N], dense */
+  float* ssq;              /* [ceil(N / 128), M] */
+} oob_gemm_epilogue_add_t;
 typedef struct {
   int F;
 } oob_gemm_epilogue_swiglu_t;
@@ -280,7 +293,7 @@ int oob_pad_counter_count(void);
  * whole tiles, -2 for the part that starts a tile: its pair owns the tile and parks nothing), parts of the tile, first
  * pair of the tile.  Returns the item count, -1 when cap is too small. */
 int oob_test_pair_schedule(int mode, int M, int N, int K, int pairs, int stream_k, int world, int rank, int* out, int cap);
-/* Columns of the tiles of that schedule (rows: 256). */
+/* Columns of an accumulator of that schedule (rows: 256); a pair may take two neighbouring ones in one item. */
 int oob_test_pair_tile_columns(int mode, int M, int N, int K, int pairs, int stream_k);
 
 /* Test hook: the local norm of oob_fused_norm(NULL, OOB_NORM_LOCAL, ...) whose waits for the rows of its ring run out at

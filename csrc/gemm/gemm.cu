@@ -283,6 +283,26 @@ cudaError_t launch_gemm(const CommCtx& ctx, const GemmArgs& args, cudaStream_t s
   int dev = 0;
   cudaGetDevice(&dev);
   if (a.mode == kGemmPlain) {
+    static const bool cluster_env_off = [] {
+      const char* v = getenv("OOB_GEMM_SKINNY");
+      return v != nullptr && v[0] == '0';
+    }();
+    // What the weight-streaming kernel alone can do.
+    if (a.epilogue == kGemmEpilogueAdd || a.row_ssq != nullptr) {
+      if (a.epilogue != 0 && a.epilogue_args == nullptr) return cudaErrorInvalidValue;
+      if (a.row_ssq != nullptr && a.row_parts < 1) return cudaErrorInvalidValue;
+      if (a.epilogue == kGemmEpilogueAdd) {
+        const auto& add = *static_cast<const oob_gemm_epilogue_add_t*>(a.epilogue_args);
+        const uintptr_t align = reinterpret_cast<uintptr_t>(add.residual) | reinterpret_cast<uintptr_t>(add.norm_weight) |
+                                reinterpret_cast<uintptr_t>(add.scaled_out) | reinterpret_cast<uintptr_t>(a.C);
+        if (add.residual == nullptr || add.norm_weight == nullptr || add.scaled_out == nullptr || add.ssq == nullptr || (align & 7) ||
+            a.N % 8 != 0 || a.ldc % 4 != 0 || add.ld_residual % 4 != 0)
+          return cudaErrorInvalidValue;
+      }
+      if (cluster_env_off || a.skinny < 0 || a.pair > 0 || !gemm_cluster_supported(a) || ctx.emu_table != nullptr || a.c_emu_stride != 0)
+        return cudaErrorNotSupported;
+      return launch_gemm_cluster(a, ctx.status, stream, make_tmap_cached);
+    }
     // The CUDA-core streaming kernel, both sides measured on B200, microseconds here and in the weight-streaming kernel.  One
     // row: up to 32 M elements of weights (1280 x 8192 8.5 and 7.8, 8192 x 1024 5.2 and 6.6, 2048 x 2048 3.9 and 5.1), and from 48 M on
     // where there are more 128-row tiles of them than SMs (57344 x 8192 135.5 and 160.9, 64000 x 2048 41.9 and 56.7, 24000 x 4096 32.8
@@ -312,10 +332,6 @@ cudaError_t launch_gemm(const CommCtx& ctx, const GemmArgs& args, cudaStream_t s
       return cudaErrorNotSupported;
     // Few rows, or few tiles: the weight-streaming kernel.  It writes no trace, and its grid is not bounded by the SM count as
     // the records of a trace buffer are: a traced GEMM runs on the tiled kernels.
-    static const bool cluster_env_off = [] {
-      const char* v = getenv("OOB_GEMM_SKINNY");
-      return v != nullptr && v[0] == '0';
-    }();
     const bool cluster_auto = a.skinny == 0 && a.splits == 0 && a.pair <= 0 && a.stream_k <= 0 && a.splitk_reduce == 0 &&
                               a.max_ctas == 0 && a.gemv <= 0 && a.trace == nullptr && !cluster_env_off && a.M <= kGemmClusterMaxRows &&
                               gemm_cluster_preferred(a);

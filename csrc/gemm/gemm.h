@@ -35,6 +35,7 @@ enum TraceSlot : int {
 };
 
 constexpr int kGemmEpilogueSwigluTile = 3;
+constexpr int kGemmEpilogueAdd = 4;
 constexpr int kGemmClusterMaxRows = 4096;  // rows the weight-streaming kernel (gemm_cluster.cu) accepts
 
 // All matrices are 16-bit (fp16 or bf16), A is [M, K] row-major with leading
@@ -74,7 +75,7 @@ struct GemmArgs {
   // Plain mode: an elementwise op applied to the fp32 sums by the kernel that has them: 0 = none, 1 = SwiGLU
   // (oob_gemm_epilogue_swiglu_t) and 2 = RoPE + KV write (oob_rope_args_t) for split problems, 3 = kGemmEpilogueSwigluTile
   // (oob_gemm_epilogue_swiglu_t) for any.  gemm_cluster.cu applies all of them, the two-SM kernel SwiGLU, the kernel that sums
-  // K splits (splitk_epilogues.cuh) the first two.  epilogue_args is a HOST pointer to the op's argument block.
+  // K splits (splitk_epilogues.cuh) the first two.  4 = kGemmEpilogueAdd (oob_gemm_epilogue_add_t): gemm_cluster.cu, few rows.  epilogue_args is a HOST pointer to the op's argument block.
   int epilogue;
   const void* epilogue_args;
   // 0 = the two-SM kernel (256x256 or narrower tiles on CTA pairs) when the shape suits it, 1 = always when possible,
@@ -94,6 +95,11 @@ struct GemmArgs {
   // Plain mode: 1 = B is a weight that no kernel the launch may overlap writes; the weight-streaming kernel then starts to load it
   // before the kernels it depends on are done.
   int b_static;
+  // Plain mode, few rows (the weight-streaming kernel alone): row m of the product is multiplied by 1 / sqrt(s / K + row_eps), s = the
+  // sum over `row_parts` of row_ssq[part][m].  Null: not.
+  const float* row_ssq;
+  int row_parts;
+  float row_eps;
 
   // Fused modes
   PeerPtrs partial;     // AR / RS: per-owner staging of partial tiles, registered; see oob_gemm_partial_bytes

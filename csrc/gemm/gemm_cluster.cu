@@ -16,6 +16,10 @@
 // rows and HALF of the tokens, and keeps the sums of its own rows.  From about 128 tokens on the activations, which every
 // weight tile reads again, rival the weights on the way from L2 to the SMs; a pair halves them.
 //
+// RMSNorm around it (a decode step, ParamsC::row_ssq and the Add epilogue): the GEMM in front of a norm adds the residual, writes the
+// new residual stream h and h * norm weight, and each tile the sum of h^2 of its columns; the GEMM behind the norm multiplies its sums
+// by 1 / rms of their row.  No norm kernel stands between the two.
+//
 // Epilogues applied to the fp32 sums before the only rounding:
 //   SwiGLU     a tile is 64 gate rows + 64 up rows of the [gate | up] weight; out = silu(gate) * up
 //   RoPE + KV  query and key heads are rotated, queries go to q_out, keys and values into the layer's cache
@@ -57,10 +61,11 @@ constexpr int kWideTokens = 64;
 constexpr int kThreadsC = 192;
 constexpr int kMaxStagesC = 12;
 constexpr int kMaxCluster = 8;               // portable cluster size
-constexpr int kCtlBytes = 256;
+constexpr int kMaxScaledRows = 128;           // rows that may carry a sum of squares (ParamsC::row_ssq)
+constexpr int kCtlBytes = 256 + kMaxScaledRows * 4;
 constexpr int kSmemLimit = 227 * 1024;
 
-enum { kEpiPlain = 0, kEpiSwiglu = 1, kEpiRopeKv = 2 };
+enum { kEpiPlain = 0, kEpiSwiglu = 1, kEpiRopeKv = 2, kEpiAdd = 3 };
 
 struct CtlC {
   uint64_t full[kMaxStagesC];
@@ -68,6 +73,7 @@ struct CtlC {
   uint64_t tmem_full;
   uint32_t tmem_base;
   int abort;
+  float scale[kMaxScaledRows];  // 1 / rms of the rows of A
 };
 static_assert(sizeof(CtlC) <= kCtlBytes, "control block");
 
@@ -87,6 +93,11 @@ struct ParamsC {
   bool vec_ok;  // 8-byte stores into C are aligned
   bool w_static;  // the weights may be loaded before the kernels this one depends on are done
   oob_rope_args_t rope;
+  // Rows of A that are still to be divided by their rms: its sums of squares in `row_parts` pieces, [part][M]; null: none.
+  const float* row_ssq;
+  int row_parts;
+  float row_eps, inv_k;
+  oob_gemm_epilogue_add_t add;
 };
 
 __device__ __forceinline__ void cluster_sync() {
@@ -165,6 +176,15 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
   }
 }
 
+template <typename T>
+__device__ __forceinline__ float2 unpack2(uint32_t w) {
+  if constexpr (PackTraits<T>::kDType == kBF16) {
+    return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
+  } else {
+    return __half22float2(*reinterpret_cast<const __half2*>(&w));
+  }
+}
+
 // Where a unit of a query, key or value head goes, and the rotation it gets.
 struct RopeUnit {
   float2 cs, sn;
@@ -234,7 +254,7 @@ __device__ __forceinline__ void emit(const ParamsC& p, int m, int n, const float
 // written: the cluster barrier behind it would otherwise wait for those stores (0.6 us).
 template <typename T, int EPI, int S, bool PAIR, typename F>
 __device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base, int rank, int m_first, int n_first, int rows,
-                                            long long pos_base, F read_done) {
+                                            long long pos_base, const float* scale, F read_done) {
   constexpr int kParts = EPI == kEpiSwiglu ? 2 : 1;  // gate and up columns
   constexpr int TB = S * kParts >= 8 ? 1 : (S * kParts >= 4 ? 2 : 4);
   uint32_t base[S];
@@ -242,12 +262,15 @@ __device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base
   for (int r = 0; r < S; ++r) base[r] = S == 1 ? smem_base : map_to_cta(smem_base, PAIR ? r * 2 + (cluster_ctarank() & 1) : r);
   constexpr int upt = kRowsW / 4 / kParts;  // units of a token
   const int units = rows * upt;
-  const int u_first = units * rank / S, u1 = units * (rank + 1) / S;
+  // The Add epilogue sums the squares of a token's columns in a warp: whole tokens for each CTA.
+  const int u_first = EPI == kEpiAdd ? rows * rank / S * upt : units * rank / S;
+  const int u1 = EPI == kEpiAdd ? rows * (rank + 1) / S * upt : units * (rank + 1) / S;
   const int turns = (u1 - u_first + kThreadsC * TB - 1) / (kThreadsC * TB);  // the same for all threads
   for (int turn = 0; turn < turns; ++turn) {
     const int u0 = u_first + turn * kThreadsC * TB + int(threadIdx.x);
     float4 v[TB][kParts][S];
     RopeUnit rope[TB];
+    uint2 res[TB], nw[TB];
     int m[TB], c[TB];
 #pragma unroll
     for (int i = 0; i < TB; ++i) {
@@ -255,6 +278,13 @@ __device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base
       m[i] = u / upt;
       c[i] = (u - m[i] * upt) * 4;
       if constexpr (EPI == kEpiRopeKv) rope[i] = rope_unit(p, m_first + m[i], n_first + c[i], pos_base);
+      if constexpr (EPI == kEpiAdd) {
+        res[i] = nw[i] = make_uint2(0u, 0u);
+        if (n_first + c[i] < p.N) {  // N is a multiple of 8
+          res[i] = *reinterpret_cast<const uint2*>(static_cast<const T*>(p.add.residual) + size_t(m_first + m[i]) * p.add.ld_residual + n_first + c[i]);
+          nw[i] = *reinterpret_cast<const uint2*>(static_cast<const T*>(p.add.norm_weight) + n_first + c[i]);
+        }
+      }
 #pragma unroll
       for (int h = 0; h < kParts; ++h)
 #pragma unroll
@@ -276,6 +306,37 @@ __device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base
       }
     }
     if (turn + 1 == turns) read_done();
+    if (p.row_ssq != nullptr) {
+#pragma unroll
+      for (int i = 0; i < TB; ++i) {
+        const float f = scale[m[i]];
+#pragma unroll
+        for (int h = 0; h < kParts; ++h) s[i][h] = make_float4(s[i][h].x * f, s[i][h].y * f, s[i][h].z * f, s[i][h].w * f);
+      }
+    }
+    if constexpr (EPI == kEpiAdd) {
+#pragma unroll
+      for (int i = 0; i < TB; ++i) {
+        if (u0 + i * kThreadsC >= u1) continue;  // all lanes of a warp together
+        const int row = m_first + m[i], n = n_first + c[i];
+        float ss = 0.f;
+        if (n < p.N) {
+          // The product is rounded before the sum, as the norm kernel would read it.
+          const float2 o0 = unpack2<T>(pack2<T>(s[i][0].x, s[i][0].y)), o1 = unpack2<T>(pack2<T>(s[i][0].z, s[i][0].w));
+          const float2 r0 = unpack2<T>(res[i].x), r1 = unpack2<T>(res[i].y), w0 = unpack2<T>(nw[i].x), w1 = unpack2<T>(nw[i].y);
+          const uint2 hw = make_uint2(pack2<T>(o0.x + r0.x, o0.y + r0.y), pack2<T>(o1.x + r1.x, o1.y + r1.y));
+          const float2 h0 = unpack2<T>(hw.x), h1 = unpack2<T>(hw.y);
+          *reinterpret_cast<uint2*>(static_cast<T*>(p.C) + size_t(row) * p.ldc + n) = hw;
+          *reinterpret_cast<uint2*>(static_cast<T*>(p.add.scaled_out) + size_t(row) * p.N + n) =
+              make_uint2(pack2<T>(h0.x * w0.x, h0.y * w0.y), pack2<T>(h1.x * w1.x, h1.y * w1.y));
+          ss = h0.x * h0.x + h0.y * h0.y + h1.x * h1.x + h1.y * h1.y;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if ((threadIdx.x & 31) == 0) p.add.ssq[size_t(n_first / kRowsW) * p.M + row] = ss;
+      }
+      continue;
+    }
 #pragma unroll
     for (int i = 0; i < TB; ++i)
       if (u0 + i * kThreadsC < u1) emit<T, EPI>(p, m_first + m[i], n_first + c[i], s[i][0], s[i][kParts - 1], rope[i]);
@@ -342,6 +403,15 @@ __global__ void __launch_bounds__(kThreadsC)
   auto load_pos = [&]() { return p.rope.pos_dev != nullptr ? *p.rope.pos_dev : static_cast<long long>(p.rope.pos0); };
   if constexpr (EPI == kEpiRopeKv) {
     if (waited) pos_base = load_pos();
+  }
+
+  if (warp >= 3 && p.row_ssq != nullptr) {  // at most kMaxScaledRows rows: one token block
+    for (int m = threadIdx.x - 96; m < p.M; m += 96) {
+      float ss = 0.f;
+#pragma unroll 8
+      for (int i = 0; i < p.row_parts; ++i) ss += p.row_ssq[size_t(i) * p.M + m];
+      ctl->scale[m] = rsqrtf(ss * p.inv_k + p.row_eps);
+    }
   }
 
   int stage = 0;          // producer's / MMA issuer's position in the ring, carried from tile to tile
@@ -500,7 +570,7 @@ __global__ void __launch_bounds__(kThreadsC)
       if (S * P > 1) cluster_arrive();
     };
 #define OOB_REDUCE(SS) \
-  case SS: reduce_tile<T, EPI, SS, PAIR>(p, own, rank, m_first, w_row, rows, pos_base, read_done); break;
+  case SS: reduce_tile<T, EPI, SS, PAIR>(p, own, rank, m_first, w_row, rows, pos_base, ctl->scale, read_done); break;
     switch (S) {
       OOB_REDUCE(1) OOB_REDUCE(2) OOB_REDUCE(3) OOB_REDUCE(4)
       default:
@@ -585,6 +655,7 @@ cudaError_t launch_fmt(const GemmArgs& a, ParamsC& p, bool pair, DeviceStatus* s
     case kEpiSwiglu:
     case kGemmEpilogueSwigluTile: return launch_epi<T, kEpiSwiglu>(a, p, pair, status, stream, make_tmap);
     case kEpiRopeKv: return launch_epi<T, kEpiRopeKv>(a, p, pair, status, stream, make_tmap);
+    case kGemmEpilogueAdd: return launch_epi<T, kEpiAdd>(a, p, pair, status, stream, make_tmap);
     default: return launch_epi<T, kEpiPlain>(a, p, pair, status, stream, make_tmap);
   }
 }
@@ -767,7 +838,8 @@ const Planned& planned(int M, int N, int K, int pair, int fix_s, bool ahead) {
 }  // namespace gemm_cluster
 
 bool gemm_cluster_supported(const GemmArgs& a) {
-  return a.mode == kGemmPlain && a.M >= 1 && a.M <= kGemmClusterMaxRows && a.epilogue <= kGemmEpilogueSwigluTile;
+  return a.mode == kGemmPlain && a.M >= 1 && a.M <= kGemmClusterMaxRows && a.epilogue <= kGemmEpilogueAdd &&
+         ((a.row_ssq == nullptr && a.epilogue != kGemmEpilogueAdd) || a.M <= gemm_cluster::kMaxScaledRows);
 }
 
 // Whether this kernel is expected to be faster than the persistent two-SM kernel, which overlaps a tile's epilogue with the next
@@ -821,6 +893,11 @@ cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStr
   p.sub = pl.sub;
   p.num_kb = (num_kb + pl.sub - 1) / pl.sub;
   if (swiglu) p.F = static_cast<const oob_gemm_epilogue_swiglu_t*>(a.epilogue_args)->F;
+  if (a.epilogue == kGemmEpilogueAdd) p.add = *static_cast<const oob_gemm_epilogue_add_t*>(a.epilogue_args);
+  p.row_ssq = a.row_ssq;
+  p.row_parts = a.row_parts;
+  p.row_eps = a.row_eps;
+  p.inv_k = 1.f / static_cast<float>(a.K);
   if (a.epilogue == kEpiRopeKv) p.rope = *static_cast<const oob_rope_args_t*>(a.epilogue_args);
   p.n_mma = pl.n_mma;
   p.nj = pl.nj;

@@ -1070,12 +1070,15 @@ int oob_gemm(oob_comm* c, const oob_gemm_args_t* a, void* stream) {
   g.stream_k = a->stream_k;
   g.order = static_cast<unsigned long long*>(a->order);
   g.b_static = a->b_static;
+  g.row_ssq = a->row_ssq;
+  g.row_parts = a->row_parts;
+  g.row_eps = a->row_eps;
   g.epilogue = a->epilogue;
   g.epilogue_args = a->epilogue_args;
   if (a->epilogue != OOB_EPILOGUE_NONE) {
     if (a->mode != OOB_GEMM_PLAIN || emu) return set_error(OOB_ERR_INVALID, "epilogues apply to the plain GEMM only");
     if (a->epilogue_args == nullptr) return set_error(OOB_ERR_INVALID, "null epilogue arguments");
-    if (a->epilogue != OOB_EPILOGUE_SWIGLU_TILE && gemm_plan_splits(a->M, a->N, a->K, a->max_ctas, a->splits) <= 1)
+    if (a->epilogue != OOB_EPILOGUE_SWIGLU_TILE && a->epilogue != OOB_EPILOGUE_ADD && a->row_ssq == nullptr && gemm_plan_splits(a->M, a->N, a->K, a->max_ctas, a->splits) <= 1)
       return set_error(OOB_ERR_UNSUPPORTED, "the epilogue runs in the split-K sum, and this problem is not split "
                                             "(see oob_gemm_plan_splits)");
     if (a->epilogue == OOB_EPILOGUE_SWIGLU || a->epilogue == OOB_EPILOGUE_SWIGLU_TILE) {
@@ -1099,7 +1102,7 @@ int oob_gemm(oob_comm* c, const oob_gemm_args_t* a, void* stream) {
       if (r->pos_dev == nullptr && (r->pos0 < 0 || r->pos0 + r->T > r->max_len))
         return set_error(OOB_ERR_INVALID, "RoPE epilogue: positions outside the cache");
     } else {
-      return set_error(OOB_ERR_INVALID, "unknown epilogue");
+      if (a->epilogue != OOB_EPILOGUE_ADD) return set_error(OOB_ERR_INVALID, "unknown epilogue");
     }
   }
   g.splitk_ws = nullptr;
@@ -1131,6 +1134,11 @@ int oob_gemm(oob_comm* c, const oob_gemm_args_t* a, void* stream) {
     (void)cudaGetLastError();
     return set_error(OOB_ERR_UNSUPPORTED, "this GEMM needs a larger scratch workspace and the stream is being captured: "
                                           "call oob_gemm_reserve_workspace before the capture");
+  }
+  if (e == cudaErrorNotSupported && (a->epilogue == OOB_EPILOGUE_ADD || a->row_ssq != nullptr)) {
+    (void)cudaGetLastError();
+    return set_error(OOB_ERR_UNSUPPORTED, "row sums of squares are for the weight-streaming kernel: at most 128 rows, and neither "
+                                          "OOB_GEMM_SKINNY=0 nor an argument may rule it out");
   }
   if (e == cudaErrorNotSupported && a->epilogue == OOB_EPILOGUE_SWIGLU_TILE) {
     (void)cudaGetLastError();

@@ -36,7 +36,7 @@ AG_PUSH_P2P, AG_PUSH_NVLS, AG_PULL_P2P = 0, 1, 2
 NORM_LOCAL, NORM_AR_ONESHOT, NORM_AR_TWOSHOT, NORM_AR_TWOSHOT_NVLS, NORM_RS, NORM_RS_NVLS = range(6)
 NORM_AR_PUSH, NORM_AR_PUSH_NVLS, NORM_AR_LL = 6, 7, 8
 GEMM_PLAIN, GEMM_AR, GEMM_RS_NORM, GEMM_AG = range(4)
-EPILOGUE_NONE, EPILOGUE_SWIGLU, EPILOGUE_ROPE_KV, EPILOGUE_SWIGLU_TILE = range(4)
+EPILOGUE_NONE, EPILOGUE_SWIGLU, EPILOGUE_ROPE_KV, EPILOGUE_SWIGLU_TILE, EPILOGUE_ADD = range(5)
 FLAG_NO_NVLS, FLAG_LEGACY_IPC = 1, 2
 
 
@@ -80,7 +80,12 @@ class GemmArgs(Structure):
                 ("rs_emu_stride", c_uint64), ("a_full_reg", c_int), ("a_full_off", c_uint64), ("use_nvls", c_int),
                 ("splits", c_int), ("no_join", c_int), ("trace", c_void_p), ("pair", c_int), ("splitk_reduce", c_int), ("skinny", c_int), ("epilogue", c_int),
                 ("epilogue_args", c_void_p), ("gemv", c_int), ("stream_k", c_int), ("order", c_void_p),
-                ("b_static", c_int)]
+                ("b_static", c_int), ("row_ssq", c_void_p), ("row_parts", c_int), ("row_eps", c_float)]
+
+
+class AddEpilogue(Structure):
+    _fields_ = [("residual", c_void_p), ("ld_residual", c_int), ("norm_weight", c_void_p), ("scaled_out", c_void_p),
+                ("ssq", c_void_p)]
 
 
 class SwigluEpilogue(Structure):
@@ -101,11 +106,6 @@ class AttnDecodeArgs(Structure):
                 ("len_bound", c_int), ("workspace", c_void_p)]
 
 
-_lock = threading.Lock()
-_lib = None
-
-
-def _declare(lib) -> None:
 def packer(structure) -> struct.Struct:
     """The same layout for ``struct.pack``, which fills all fields in one step: what a call of a microsecond-sized kernel takes on the
     host counts."""
@@ -119,6 +119,11 @@ GEMM_HEAD = struct.Struct("@iiiiiPiPiPi")
 GEMM_TAIL = bytes(ctypes.sizeof(GemmArgs) - GEMM_HEAD.size)
 GEMM_TAIL_STATIC = bytes(GemmArgs(b_static=1))[GEMM_HEAD.size:]
 
+_lock = threading.Lock()
+_lib = None
+
+
+def _declare(lib) -> None:
     P = c_void_p
     lib.oob_last_error.restype = c_char_p
     lib.oob_version.restype = c_char_p
@@ -151,13 +156,13 @@ GEMM_TAIL_STATIC = bytes(GemmArgs(b_static=1))[GEMM_HEAD.size:]
     lib.oob_allreduce_ll.argtypes = [P, c_int, c_int, c_int, c_uint64, c_uint64, P, P, c_uint64, c_int, c_int, P]
     lib.oob_fused_norm.argtypes = [P, c_int, POINTER(NormArgs), c_int, P]
     lib.oob_gemm.argtypes = [P, POINTER(GemmArgs), P]
+    lib.packed_fused_norm = ctypes.CFUNCTYPE(c_int, P, c_int, c_char_p, c_int, P)(("oob_fused_norm", lib))
+    lib.packed_gemm = ctypes.CFUNCTYPE(c_int, P, c_char_p, P)(("oob_gemm", lib))
     lib.oob_gemm_plan_splits.argtypes = [c_int, c_int, c_int, c_int, c_int]
     lib.oob_pad_counter_offset.restype = c_uint64
     lib.oob_pad_counter_offset.argtypes = []
     lib.oob_pad_counter_count.argtypes = []
     lib.oob_gemm_counters_needed.argtypes = [c_int, c_int, c_int, c_int]
-    lib.packed_fused_norm = ctypes.CFUNCTYPE(c_int, P, c_int, c_char_p, c_int, P)(("oob_fused_norm", lib))
-    lib.packed_gemm = ctypes.CFUNCTYPE(c_int, P, c_char_p, P)(("oob_gemm", lib))
     lib.oob_test_pair_schedule.argtypes = [c_int] * 8 + [POINTER(c_int), c_int]
     lib.oob_test_pair_tile_columns.argtypes = [c_int] * 6
     lib.oob_gemm_reserve_workspace.argtypes = [c_uint64]

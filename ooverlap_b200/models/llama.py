@@ -23,7 +23,7 @@ from typing import Optional
 import torch
 import torch.nn.functional as F
 
-from ..ops import (attn_decode, fused_allreduce_rmsnorm, gemm, gemm_rope_kv_write, gemm_swiglu, rmsnorm, rope_kv_write,
+from ..ops import (DEFERRED_NORM_MAX_ROWS, attn_decode, fused_allreduce_rmsnorm, gemm, gemm_add_norm, gemm_rope_kv_write, gemm_swiglu, rmsnorm, rope_kv_write,
                    rope_tables, silu_mul, static_weights)
 from ..utils.config import env_flag, env_int
 from ..utils.tracing import nvtx_range
@@ -114,6 +114,12 @@ class LlamaTP:
         # RoPE + cache write and SwiGLU applied to the fp32 sums by the preceding GEMM (two launches fewer per layer in
         # a decode step, and no 16-bit round trip of the gate/up product).  OOB_FUSED_EPILOGUES=0 turns it off.
         self.fused_epilogues = backend == "ours" and env_flag("OOB_FUSED_EPILOGUES", True)
+        # One GPU, few rows: the norms between the projections are folded into them (gemm_add_norm), two launches fewer per
+        # layer.  bf16 only: the stream times the norm's weight is kept in 16 bits before it is divided by its rms, which
+        # could leave the range of fp16.  OOB_DEFERRED_NORM=0 turns it off.
+        self.deferred_norm = (self.fused_epilogues and world == 1 and dtype == torch.bfloat16 and cfg.hidden % 8 == 0
+                              and self.device.type == "cuda" and env_flag("OOB_DEFERRED_NORM", True)
+                              and env_flag("OOB_GEMM_SKINNY", True))
         # Prefill: row-parallel projections of at least OOB_PREFILL_CHUNK_MIN_ROWS tokens are computed in
         # OOB_PREFILL_CHUNKS slabs whose all-reduce + norm overlaps the next slab's GEMM (1 = off).
         self.prefill_chunks = max(1, env_int("OOB_PREFILL_CHUNKS", 1)) if backend == "ours" else 1
@@ -203,6 +209,7 @@ class LlamaTP:
         h = self.embed[tokens.reshape(-1)]  # [B*T, hidden]  residual stream
         x = self._norm(h, self.layers[0]["norm1"])
         sl = slice(batch0, batch0 + B)
+        deferred = self.deferred_norm and B * T <= DEFERRED_NORM_MAX_ROWS
         for li, layer in enumerate(self.layers):
             with nvtx_range("layer"):
                 if ours and self.fused_epilogues:
@@ -243,7 +250,10 @@ class LlamaTP:
                         self.v_cache[li, sl, :, pos:pos + T] = v
                         att = F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=True)
                     att = att.transpose(1, 2).reshape(B * T, self.h_local * hd)
-                x, h = self._row_parallel_norm(att, layer["wo"], h, layer["norm2"])
+                if deferred:
+                    x, h = gemm_add_norm(att, layer["wo"], h, layer["norm2"], cfg.eps)
+                else:
+                    x, h = self._row_parallel_norm(att, layer["wo"], h, layer["norm2"])
                 if ours and self.fused_epilogues:
                     act = gemm_swiglu(x, layer["wgu"])
                 elif ours:
@@ -253,7 +263,10 @@ class LlamaTP:
                     half = gu.shape[1] // 2
                     act = F.silu(gu[:, :half]) * gu[:, half:]
                 next_norm = self.layers[li + 1]["norm1"] if li + 1 < len(self.layers) else self.final_norm
-                x, h = self._row_parallel_norm(act, layer["wd"], h, next_norm)
+                if deferred and li + 1 < len(self.layers):
+                    x, h = gemm_add_norm(act, layer["wd"], h, next_norm, cfg.eps)
+                else:
+                    x, h = self._row_parallel_norm(act, layer["wd"], h, next_norm)
         return x
 
     def greedy_token(self, hidden_last: torch.Tensor) -> torch.Tensor:

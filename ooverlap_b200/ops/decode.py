@@ -79,8 +79,14 @@ def gemm_rope_kv_write(x: torch.Tensor, wqkv: torch.Tensor, B: int, T: int, head
 
     When the GEMM is one that the tiled kernels would split over K (every decode-step shape), rotation and cache write are
     done from the fp32 sums by the kernel that has them (the weight-streaming kernel, or the one that sums the splits);
-    otherwise (or with ``fused=False``) the GEMM is followed by :func:`rope_kv_write`.  Returns the rotated queries, [B*T, heads * hd]."""
-    from .gemm import _check_operands, _scope, fill_gemm_args, gemm, gemm_plan_splits
+    otherwise (or with ``fused=False``) the GEMM is followed by :func:`rope_kv_write`.  ``x`` may be a ``RowSums`` (see
+    ``gemm_add_norm``).  Returns the rotated queries, [B*T, heads * hd]."""
+    from .gemm import RowSums, _check_operands, _plain_args, _set_row_sums, gemm, gemm_plan_splits
+    sums = x
+    if isinstance(x, RowSums):
+        if fused is False:
+            raise ValueError("row sums need the kernel that this call rules out")
+        x = x.scaled
     _check_operands(x, wqkv)
     M, N, K = x.shape[0], wqkv.shape[0], x.shape[1]
     if M != B * T:
@@ -88,7 +94,7 @@ def gemm_rope_kv_write(x: torch.Tensor, wqkv: torch.Tensor, B: int, T: int, head
     hd = N // (heads + 2 * kv_heads)
     if hd * (heads + 2 * kv_heads) != N or hd % 8 != 0:
         raise ValueError("head geometry does not match the QKV weight")
-    can_fuse = gemm_plan_splits(M, N, K) > 1
+    can_fuse = sums is not x or gemm_plan_splits(M, N, K) > 1
     if fused is None:
         fused = can_fuse
     if fused and not can_fuse:
@@ -99,11 +105,9 @@ def gemm_rope_kv_write(x: torch.Tensor, wqkv: torch.Tensor, B: int, T: int, head
     if q_out is None:
         q_out = torch.empty((M, heads * hd), dtype=x.dtype, device=x.device)
     r = _rope_args(x.dtype, B, T, heads, kv_heads, hd, k_cache, v_cache, cos, sin, pos, batch0, q_out)
-    args = _lib.GemmArgs()
-    args.mode = _lib.GEMM_PLAIN
-    fill_gemm_args(args, x, wqkv)
-    args.C, args.ldc = q_out.data_ptr(), N  # C itself is not written; a valid aligned pointer keeps the checks uniform
-    args.b_static = _scope.static_b
+    args = _plain_args(x, wqkv, q_out)
+    args.ldc = N  # C itself is not written; a valid aligned pointer keeps the checks uniform
+    _set_row_sums(args, sums)
     args.epilogue = _lib.EPILOGUE_ROPE_KV
     args.epilogue_args = ctypes.cast(ctypes.pointer(r), ctypes.c_void_p)
     _lib.check(_lib.lib().oob_gemm(None, ctypes.byref(args), _stream()))

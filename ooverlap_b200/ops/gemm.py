@@ -10,7 +10,7 @@ from __future__ import annotations
 import contextlib
 import ctypes
 import threading
-from typing import Optional
+from typing import NamedTuple, Optional
 
 import torch
 
@@ -134,7 +134,6 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
     args.splitk_reduce = splitk_reduce
     args.gemv = gemv
     args.stream_k = stream_k
-    args.b_static = _scope.static_b
     if order is not None:
         check_order_buffer(order, M, N)
         args.order = order.data_ptr()
@@ -227,6 +226,44 @@ def gemm_plan_splits(M: int, N: int, K: int, *, max_ctas: int = 0, splits: int =
     return int(_lib.lib().oob_gemm_plan_splits(M, N, K, max_ctas, splits))
 
 
+class RowSums(NamedTuple):
+    """Sums of squares of the rows of a residual stream, one per 128 columns: the norm that is still to be applied to
+    ``scaled`` (the stream times the norm's weight) by the GEMM that reads it."""
+    scaled: torch.Tensor  # [M, hidden]
+    ssq: torch.Tensor     # [ceil(hidden / 128), M] fp32
+    eps: float
+
+
+def _set_row_sums(args: _lib.GemmArgs, x) -> None:
+    if isinstance(x, RowSums):
+        args.row_ssq, args.row_parts, args.row_eps = x.ssq.data_ptr(), x.ssq.shape[0], x.eps
+
+
+DEFERRED_NORM_MAX_ROWS = 128
+
+
+def gemm_add_norm(a: torch.Tensor, b: torch.Tensor, residual: torch.Tensor, weight: torch.Tensor, eps: float) -> tuple:
+    """The row-parallel projection in front of an RMSNorm on one GPU, for up to 128 rows: ``h = residual + a @ b.T`` and the norm of ``h``
+    as a :class:`RowSums`, which :func:`gemm_swiglu` and ``gemm_rope_kv_write`` take in place of the normalised rows.  They
+    divide by the rms after the product, where the sums are still fp32: no norm kernel runs.  Returns ``(RowSums, h)``."""
+    _check_operands(a, b)
+    M, N = a.shape[0], b.shape[0]
+    if M > DEFERRED_NORM_MAX_ROWS or N % 8 != 0:
+        raise ValueError(f"at most {DEFERRED_NORM_MAX_ROWS} rows, and columns in multiples of 8")
+    if residual.shape != (M, N) or residual.dtype != a.dtype or residual.stride(1) != 1 or residual.stride(0) % 4 != 0 \
+            or weight.shape != (N,) or weight.dtype != a.dtype or not weight.is_contiguous():
+        raise ValueError("residual must be [M, N] with unit column stride and weight [N], both of the operands' dtype")
+    h = torch.empty((M, N), dtype=a.dtype, device=a.device)
+    scaled = torch.empty_like(h)
+    ssq = torch.empty(((N + 127) // 128, M), dtype=torch.float32, device=a.device)
+    epi = _lib.AddEpilogue(residual.data_ptr(), residual.stride(0), weight.data_ptr(), scaled.data_ptr(), ssq.data_ptr())
+    args = _plain_args(a, b, h)
+    args.epilogue = _lib.EPILOGUE_ADD
+    args.epilogue_args = ctypes.cast(ctypes.pointer(epi), ctypes.c_void_p)
+    _lib.check(_lib.lib().oob_gemm(None, args, current_stream_ptr()))
+    return RowSums(scaled, ssq, eps), h
+
+
 def gemm_swiglu(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *, max_ctas: int = 0,
                 fused: Optional[bool] = None) -> torch.Tensor:
     """``silu(a @ b[:F].T) * (a @ b[F:].T)`` for a gate/up weight ``b`` of shape [2F, K]; returns [M, F].
@@ -235,8 +272,14 @@ def gemm_swiglu(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = 
     epilogue or the split-K sum): no separate launch and no 16-bit round trip of the [M, 2F] intermediate.  Where none of
     them may run (``OOB_GEMM_PAIR=0``, one CTA), for one row of a large weight, and with ``fused=False`` the GEMM is followed
     by the stand-alone SwiGLU kernel.  ``fused=True`` insists on a problem that the tiled kernels would split over K (every
-    decode-step shape) and raises otherwise."""
+    decode-step shape) and raises otherwise.  ``a`` may be a :class:`RowSums` (see
+    :func:`gemm_add_norm`)."""
     from .decode import silu_mul
+    sums = a
+    if isinstance(a, RowSums):
+        if max_ctas or fused is False:
+            raise ValueError("row sums need the kernel that this call rules out")
+        a = a.scaled
     _check_operands(a, b)
     M, N = a.shape[0], b.shape[0]
     if N % 16 != 0:
@@ -253,16 +296,13 @@ def gemm_swiglu(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = 
         return silu_mul(gemm(a, b, max_ctas=max_ctas), out)
     epi = _lib.SwigluEpilogue()
     epi.F = F
-    args = _lib.GemmArgs()
-    args.mode = _lib.GEMM_PLAIN
-    fill_gemm_args(args, a, b)
-    args.C, args.ldc = out.data_ptr(), out.stride(0)
+    args = _plain_args(a, b, out)
+    _set_row_sums(args, sums)
     args.max_ctas = max_ctas
-    args.b_static = _scope.static_b
     args.epilogue = _lib.EPILOGUE_SWIGLU if can_fuse else _lib.EPILOGUE_SWIGLU_TILE
     args.epilogue_args = ctypes.cast(ctypes.pointer(epi), ctypes.c_void_p)
     rc = _lib.lib().oob_gemm(None, args, current_stream_ptr())
-    if rc == _lib.ERR_UNSUPPORTED and not can_fuse:  # no kernel that has the sums may or can apply it: two kernels
+    if rc == _lib.ERR_UNSUPPORTED and not can_fuse and sums is a:  # no kernel that has the sums may or can apply it: two kernels
         dense = silu_mul(gemm(a, b, max_ctas=max_ctas), out if out.is_contiguous() else None)
         return out if dense is out else out.copy_(dense)
     if rc:
