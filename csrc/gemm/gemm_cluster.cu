@@ -119,7 +119,6 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
                : "memory");
   return v;
 }
-
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));

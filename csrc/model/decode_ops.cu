@@ -216,6 +216,7 @@ struct AttnParams {
   int max_len, batch0;
   int splits;
   float scale_log2;
+  bool ahead;  // the position and the keys and values before the newest may be read before the kernels this one depends on are done
 };
 
 template <typename T>
@@ -230,6 +231,9 @@ __device__ __forceinline__ T to_out(float y) {
 __device__ __forceinline__ void attn_cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The two halves of attn_cluster_sync.
+__device__ __forceinline__ void attn_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void attn_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ float ld_cluster_f32(uint32_t smem_addr, uint32_t rank) {
   uint32_t a;
   float v;
@@ -250,7 +254,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = p.G;
   ptx::griddep_launch_dependents();
-  ptx::griddep_wait();
+  if (!p.ahead) ptx::griddep_wait();
   int L = p.pos_dev != nullptr ? static_cast<int>(*p.pos_dev) + 1 : p.len;
   if (L > p.max_len) L = p.max_len;
   if (L < 1) L = 1;
@@ -258,21 +262,6 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
   const int parts = p.splits * S;
   const int t0 = static_cast<int>(nt * part / parts), t1 = static_cast<int>(nt * (part + 1) / parts);
   const int h0 = kvh * G;
-
-  // ---- Q fragments (A operand, 16 x 128; rows >= G are zero) ----
-  const int row0 = lane >> 2, colp = (lane & 3) * 2;
-  uint32_t qa[8][4];
-  {
-    const T* qb = static_cast<const T*>(p.q) + (static_cast<long long>(b) * p.H + h0) * kHD;
-#pragma unroll
-    for (int ks = 0; ks < 8; ++ks) {
-      const int c0 = ks * 16 + colp;
-      qa[ks][0] = row0 < G ? *reinterpret_cast<const uint32_t*>(qb + row0 * kHD + c0) : 0u;
-      qa[ks][1] = row0 + 8 < G ? *reinterpret_cast<const uint32_t*>(qb + (row0 + 8) * kHD + c0) : 0u;
-      qa[ks][2] = row0 < G ? *reinterpret_cast<const uint32_t*>(qb + row0 * kHD + c0 + 8) : 0u;
-      qa[ks][3] = row0 + 8 < G ? *reinterpret_cast<const uint32_t*>(qb + (row0 + 8) * kHD + c0 + 8) : 0u;
-    }
-  }
 
   const T* kbase = static_cast<const T*>(p.k) + (p.batch0 + b) * p.batch_stride + static_cast<long long>(kvh) * p.max_len * kHD;
   const T* vbase = static_cast<const T*>(p.v) + (p.batch0 + b) * p.batch_stride + static_cast<long long>(kvh) * p.max_len * kHD;
@@ -298,11 +287,35 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
 
   // One commit group per tile slot, empty when there is no tile: the group count is then the same for every warp
-  // and wait<STAGES - 1> always means "tile i has landed".
+  // and wait<STAGES - 1> always means "tile i has landed".  Ahead of the kernel before: all but the tile with the newest key, which is
+  // a warp's last one.
+  bool waited = !p.ahead;
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
-    if (s < my_tiles) issue_tile(s, s);
+    if (s < my_tiles) {
+      if (!waited && (t0 + warp + s * kAttnWarps + 1) * kTileKeys >= L) {
+        ptx::griddep_wait();
+        waited = true;
+      }
+      issue_tile(s, s);
+    }
     cp_async_commit();
+  }
+  if (!waited) ptx::griddep_wait();
+
+  // ---- Q fragments (A operand, 16 x 128; rows >= G are zero) ----
+  const int row0 = lane >> 2, colp = (lane & 3) * 2;
+  uint32_t qa[8][4];
+  {
+    const T* qb = static_cast<const T*>(p.q) + (static_cast<long long>(b) * p.H + h0) * kHD;
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+      const int c0 = ks * 16 + colp;
+      qa[ks][0] = row0 < G ? *reinterpret_cast<const uint32_t*>(qb + row0 * kHD + c0) : 0u;
+      qa[ks][1] = row0 + 8 < G ? *reinterpret_cast<const uint32_t*>(qb + (row0 + 8) * kHD + c0) : 0u;
+      qa[ks][2] = row0 < G ? *reinterpret_cast<const uint32_t*>(qb + row0 * kHD + c0 + 8) : 0u;
+      qa[ks][3] = row0 + 8 < G ? *reinterpret_cast<const uint32_t*>(qb + (row0 + 8) * kHD + c0 + 8) : 0u;
+    }
   }
   int stage = 0, fill = STAGES - 1;
   for (int i = 0; i < my_tiles; ++i) {
@@ -459,6 +472,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
     const uint32_t co_a = static_cast<uint32_t>(__cvta_generic_to_shared(co));
     const uint32_t cm_a = static_cast<uint32_t>(__cvta_generic_to_shared(cm)), cl_a = static_cast<uint32_t>(__cvta_generic_to_shared(cl));
     attn_cluster_sync();
+    if (rank >= G) attn_cluster_arrive();
     for (int g = rank; g < G; g += S) {
       float m[S], l[S], v[S];
 #pragma unroll
@@ -477,9 +491,11 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
         acc += f * v[r];
         l_tot += f * l[r];
       }
+      // All parts are read: the barrier need not wait for the stores of the last result.
+      if (g + S >= G) attn_cluster_arrive();
       deliver(g, acc, m_tot, l_tot);
     }
-    attn_cluster_sync();  // the peers have read this CTA's part
+    attn_cluster_wait();  // the peers have read this CTA's part
   }
 }
 
@@ -739,6 +755,7 @@ int oob_attn_decode(const oob_attn_decode_args_t* a, void* stream) {
   p.batch0 = a->batch0;
   p.splits = splits;
   p.scale_log2 = a->scale * 1.4426950408889634f;
+  p.ahead = a->ahead != 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   AttnSlots slots = attn_slots();
   // Behind a split launch waits the kernel that merges, and calls follow one another: clusters of eight that need every slot of

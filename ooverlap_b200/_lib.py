@@ -103,7 +103,7 @@ class AttnDecodeArgs(Structure):
     _fields_ = [("dtype", c_int), ("B", c_int), ("H", c_int), ("KV", c_int), ("q", c_void_p), ("k_cache", c_void_p),
                 ("v_cache", c_void_p), ("cache_batch_stride", c_int64), ("max_len", c_int), ("batch0", c_int),
                 ("out", c_void_p), ("pos_dev", c_void_p), ("len", c_int), ("scale", c_float), ("splits", c_int),
-                ("len_bound", c_int), ("workspace", c_void_p)]
+                ("len_bound", c_int), ("workspace", c_void_p), ("ahead", c_int)]
 
 
 def packer(structure) -> struct.Struct:

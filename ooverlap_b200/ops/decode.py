@@ -16,6 +16,7 @@ import torch
 from .. import _lib
 from ..utils.dtypes import dtype_code
 from ..utils.stream import current_stream_ptr as _stream
+from .gemm import _scope
 
 
 def rope_tables(max_len: int, head_dim: int, theta: float, device) -> tuple[torch.Tensor, torch.Tensor]:
@@ -173,6 +174,8 @@ def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, p
         # written by two streams at once, and one that a later call outgrows would be freed under a captured graph.
         ws = torch.empty(lib.oob_attn_decode_workspace_bytes(B, H, splits), dtype=torch.uint8, device=q.device)
     a.workspace = ws.data_ptr() if ws is not None else None
+    if _scope.static_b:
+        a.ahead = 1
     _lib.check(lib.oob_attn_decode(ctypes.byref(a), _stream()))
     return out
 

@@ -5,7 +5,7 @@ import contextlib
 import pytest
 import torch
 
-from ooverlap_b200.ops import gemm, gemm_rope_kv_write, gemm_swiglu, rmsnorm, rope_tables, static_weights
+from ooverlap_b200.ops import attn_decode, attn_decode_reference, gemm, gemm_rope_kv_write, gemm_swiglu, rmsnorm, rope_tables, static_weights
 from ooverlap_b200.ops.gemm import _scope
 
 pytestmark = pytest.mark.gpu
@@ -47,6 +47,33 @@ def test_weights_loaded_ahead(rows, hidden, ffn, dtype):
     eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
     for a, b in zip(out[0], out[1]):
         assert (a.double() - b.double()).norm() <= 4 * eps * a.double().norm()
+
+
+@pytest.mark.parametrize("ctx", [1, 2, 16, 17, 64, 65, 200, 1000])
+@pytest.mark.parametrize("b,heads,kv", [(1, 8, 1), (3, 16, 1), (40, 8, 2)])
+def test_cache_read_ahead_of_the_newest_key(ctx, b, heads, kv):
+    """The newest key and value come from the kernel just before; all older ones may be loaded while it runs.  Same bits."""
+    torch.manual_seed(ctx)
+    hd, max_len, hidden = 128, 1024, 512
+    x = torch.randn(b, hidden, device="cuda").bfloat16()
+    w = (torch.randn((heads + 2 * kv) * hd, hidden, device="cuda") / hidden ** 0.5).bfloat16()
+    cos, sin = rope_tables(max_len, hd, 10000.0, "cuda")
+    pos = torch.full((1,), ctx - 1, dtype=torch.long, device="cuda")
+    cache = torch.randn(2, b, kv, max_len, hd, device="cuda").bfloat16()
+    cache[:, :, :, ctx - 1:] = float("nan")  # read only once the projection has written it
+    out = []
+    for ahead in (False, True, True):
+        kc, vc = cache.clone()
+        torch.cuda.synchronize()
+        with static_weights() if ahead else contextlib.nullcontext():
+            q = gemm_rope_kv_write(x, w, b, 1, heads, kv, kc, vc, cos, sin, pos)
+        with static_weights() if ahead else contextlib.nullcontext():
+            out.append((attn_decode(q.view(b, heads, hd), kc, vc, pos), q))
+    assert torch.equal(out[1][0], out[2][0])
+    want = attn_decode_reference(out[1][1].view(b, heads, hd), kc, vc, ctx - 1)
+    assert (out[1][0].double() - want.double()).norm() < 2 * 2.0 ** -8 * want.double().norm()
+    if torch.equal(out[0][1], out[1][1]):
+        assert torch.equal(out[0][0], out[1][0])
 
 
 def test_without_the_promise_b_may_be_the_result_of_the_call_before():
