@@ -114,6 +114,8 @@ def packer(structure) -> struct.Struct:
 
 
 NORM_ARGS = packer(NormArgs)
+ROPE_ARGS = packer(RopeArgs)
+ATTN_ARGS = packer(AttnDecodeArgs)
 # GemmArgs: the fields every plain call sets, and the rest with nothing asked for, with and without static weights.
 GEMM_HEAD = struct.Struct("@iiiiiPiPiPi")
 GEMM_TAIL = bytes(ctypes.sizeof(GemmArgs) - GEMM_HEAD.size)

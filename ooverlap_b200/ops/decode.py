@@ -38,19 +38,16 @@ def _rope_args(dtype, B: int, T: int, heads: int, kv_heads: int, hd: int, k_cach
     max_len = k_cache.shape[2]
     if cos.dtype != torch.float32 or cos.shape != (max_len, hd // 2) or not cos.is_contiguous() or sin.shape != cos.shape:
         raise ValueError("cos / sin must be contiguous fp32 [max_len, hd/2] tables")
-    a = _lib.RopeArgs()
-    a.dtype, a.B, a.T, a.H, a.KV, a.hd = dtype_code(dtype), B, T, heads, kv_heads, hd
-    a.qkv, a.q_out = None, q_out.data_ptr()
-    a.k_cache, a.v_cache = k_cache.data_ptr(), v_cache.data_ptr()
-    a.cache_batch_stride, a.max_len, a.batch0 = k_cache.stride(0), max_len, batch0
-    a.cos_table, a.sin_table = cos.data_ptr(), sin.data_ptr()
     if isinstance(pos, torch.Tensor):
         if pos.dtype != torch.int64 or pos.numel() != 1 or not pos.is_cuda:
             raise ValueError("pos must be a one-element int64 CUDA tensor")
-        a.pos_dev, a.pos0 = pos.data_ptr(), 0
+        pos_dev, pos0 = pos.data_ptr(), 0
     else:
-        a.pos_dev, a.pos0 = None, int(pos)
-    return a
+        pos_dev, pos0 = 0, int(pos)
+    # Fields in the order of the structure, qkv left null.
+    return _lib.RopeArgs.from_buffer_copy(_lib.ROPE_ARGS.pack(
+        dtype_code(dtype), B, T, heads, kv_heads, hd, 0, q_out.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), k_cache.stride(0), max_len,
+        batch0, cos.data_ptr(), sin.data_ptr(), pos_dev, pos0))
 
 
 def rope_kv_write(qkv: torch.Tensor, B: int, T: int, heads: int, kv_heads: int, k_cache: torch.Tensor,
@@ -110,8 +107,8 @@ def gemm_rope_kv_write(x: torch.Tensor, wqkv: torch.Tensor, B: int, T: int, head
     args.ldc = N  # C itself is not written; a valid aligned pointer keeps the checks uniform
     _set_row_sums(args, sums)
     args.epilogue = _lib.EPILOGUE_ROPE_KV
-    args.epilogue_args = ctypes.cast(ctypes.pointer(r), ctypes.c_void_p)
-    _lib.check(_lib.lib().oob_gemm(None, ctypes.byref(args), _stream()))
+    args.epilogue_args = ctypes.addressof(r)
+    _lib.check(_lib.lib().oob_gemm(None, args, _stream()))
     return q_out
 
 
@@ -156,26 +153,22 @@ def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, p
     bound = len_bound or max_len
     if splits == 0:
         splits = lib.oob_attn_decode_auto_splits(B, KV, bound)
-    a = _lib.AttnDecodeArgs()
-    a.dtype, a.B, a.H, a.KV = dtype_code(q.dtype), B, H, KV
-    a.q, a.k_cache, a.v_cache, a.out = q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr()
-    a.cache_batch_stride, a.max_len, a.batch0 = k_cache.stride(0), max_len, batch0
     if isinstance(pos, torch.Tensor):
         if pos.dtype != torch.int64 or pos.numel() != 1 or not pos.is_cuda:
             raise ValueError("pos must be a one-element int64 CUDA tensor")
-        a.pos_dev, a.len = pos.data_ptr(), 0
+        pos_dev, length = pos.data_ptr(), 0
     else:
-        a.pos_dev, a.len = None, int(pos) + 1
-    a.scale = scale if scale is not None else 1.0 / math.sqrt(hd)
-    a.splits, a.len_bound = splits, bound
+        pos_dev, length = 0, int(pos) + 1
     ws = None
     if splits > 1:
         # Of this call alone, in stream order (and in the graph's pool under capture): a workspace shared by calls would be
         # written by two streams at once, and one that a later call outgrows would be freed under a captured graph.
         ws = torch.empty(lib.oob_attn_decode_workspace_bytes(B, H, splits), dtype=torch.uint8, device=q.device)
-    a.workspace = ws.data_ptr() if ws is not None else None
-    if _scope.static_b:
-        a.ahead = 1
+    # Fields in the order of the structure.
+    a = _lib.AttnDecodeArgs.from_buffer_copy(_lib.ATTN_ARGS.pack(
+        dtype_code(q.dtype), B, H, KV, q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), k_cache.stride(0), max_len, batch0,
+        out.data_ptr(), pos_dev, length, scale if scale is not None else 1.0 / math.sqrt(hd), splits, bound,
+        ws.data_ptr() if ws is not None else 0, _scope.static_b))
     _lib.check(lib.oob_attn_decode(ctypes.byref(a), _stream()))
     return out
 

@@ -61,14 +61,16 @@ def fill_gemm_args(args: _lib.GemmArgs, a: torch.Tensor, b: torch.Tensor) -> Non
     args.B, args.ldb = b.data_ptr(), b.stride(0)
 
 
+def _packed_plain_args(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor) -> bytes:
+    """The arguments of a call that asks for nothing, packed in one step: a third of the time of assigning them one by one (0.17 and
+    0.75 us)."""
+    return _lib.GEMM_HEAD.pack(_lib.GEMM_PLAIN, dtype_code(a.dtype), a.shape[0], b.shape[0], a.shape[1], a.data_ptr(), a.stride(0),
+                               b.data_ptr(), b.stride(0), out.data_ptr(), out.stride(0)
+                               ) + (_lib.GEMM_TAIL_STATIC if _scope.static_b else _lib.GEMM_TAIL)
+
+
 def _plain_args(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor) -> _lib.GemmArgs:
-    args = _lib.GemmArgs()
-    args.mode = _lib.GEMM_PLAIN
-    fill_gemm_args(args, a, b)
-    args.C, args.ldc = out.data_ptr(), out.stride(0)
-    if _scope.static_b:
-        args.b_static = 1
-    return args
+    return _lib.GemmArgs.from_buffer_copy(_packed_plain_args(a, b, out))
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *, max_ctas: int = 0,
@@ -120,10 +122,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
             splits, pair, skinny = int(sol.get("splits", 0)), int(sol.get("pair", 0)), int(sol.get("skinny", 0))
             gemv, stream_k = int(sol.get("gemv", 0)), int(sol.get("stream_k", 0))
     if order is None and not (splits or pair or skinny or splitk_reduce or gemv or stream_k or max_ctas):
-        # Packed in one step: a third of the time of assigning the fields one by one (0.17 and 0.75 us).
-        args = _lib.GEMM_HEAD.pack(_lib.GEMM_PLAIN, dtype_code(a.dtype), M, N, a.shape[1], a.data_ptr(), a.stride(0), b.data_ptr(),
-                                   b.stride(0), out.data_ptr(), out.stride(0))
-        rc = _lib.lib().packed_gemm(None, args + (_lib.GEMM_TAIL_STATIC if _scope.static_b else _lib.GEMM_TAIL), current_stream_ptr())
+        rc = _lib.lib().packed_gemm(None, _packed_plain_args(a, b, out), current_stream_ptr())
         if rc:
             _lib.check(rc)
         return out
@@ -260,7 +259,7 @@ def gemm_add_norm(a: torch.Tensor, b: torch.Tensor, residual: torch.Tensor, weig
     epi = _lib.AddEpilogue(residual.data_ptr(), residual.stride(0), weight.data_ptr(), scaled.data_ptr(), ssq.data_ptr())
     args = _plain_args(a, b, h)
     args.epilogue = _lib.EPILOGUE_ADD
-    args.epilogue_args = ctypes.cast(ctypes.pointer(epi), ctypes.c_void_p)
+    args.epilogue_args = ctypes.addressof(epi)
     _lib.check(_lib.lib().oob_gemm(None, args, current_stream_ptr()))
     return RowSums(scaled, ssq, eps), h
 
@@ -295,13 +294,12 @@ def gemm_swiglu(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = 
         raise ValueError("this problem is not split over K, so the epilogue has no kernel to run in")
     if fused is False:
         return silu_mul(gemm(a, b, max_ctas=max_ctas), out)
-    epi = _lib.SwigluEpilogue()
-    epi.F = F
+    epi = _lib.SwigluEpilogue(F)
     args = _plain_args(a, b, out)
     _set_row_sums(args, sums)
     args.max_ctas = max_ctas
     args.epilogue = _lib.EPILOGUE_SWIGLU if can_fuse else _lib.EPILOGUE_SWIGLU_TILE
-    args.epilogue_args = ctypes.cast(ctypes.pointer(epi), ctypes.c_void_p)
+    args.epilogue_args = ctypes.addressof(epi)
     rc = _lib.lib().oob_gemm(None, args, current_stream_ptr())
     if rc == _lib.ERR_UNSUPPORTED and not can_fuse and sums is a:  # no kernel that has the sums may or can apply it: two kernels
         dense = silu_mul(gemm(a, b, max_ctas=max_ctas), out if out.is_contiguous() else None)

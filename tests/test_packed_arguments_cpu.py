@@ -11,6 +11,15 @@ def test_packed_norm_arguments():
     assert [getattr(a, f) for f, _ in a._fields_] == values
 
 
+def test_packed_model_arguments():
+    for structure, pack, values in (
+            (_lib.RopeArgs, _lib.ROPE_ARGS, [1, 2, 3, 4, 5, 6, 7 << 40, 8 << 40, 9 << 40, 10 << 40, 11 << 40, 12, 13, 14 << 40, 15 << 40, 16 << 40, 17]),
+            (_lib.AttnDecodeArgs, _lib.ATTN_ARGS, [1, 2, 3, 4, 5 << 40, 6 << 40, 7 << 40, 8 << 40, 9, 10, 11 << 40, 12 << 40, 13, 0.25, 14, 15,
+                                                   16 << 40, 1])):
+        a = structure.from_buffer_copy(pack.pack(*values))
+        assert [getattr(a, f) for f, _ in a._fields_] == values
+
+
 def test_packed_plain_gemm_arguments():
     values = [0, 1, 16, 7168, 8192, 2 << 40, 8200, 3 << 40, 8208, 4 << 40, 7176]
     for tail, static in ((_lib.GEMM_TAIL, 0), (_lib.GEMM_TAIL_STATIC, 1)):
