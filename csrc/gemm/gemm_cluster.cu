@@ -3,7 +3,7 @@
 // of a decode step or of a short mixed batch: what bounds it is the time to read B once, plus whatever happens before the
 // first and after the last byte.
 //
-// A CTA goes through 64 elements of K in 0.17 - 0.27 us (the chain load - multiply - release of its issuing threads), so that
+// A CTA goes through 64 elements of K in 0.11 - 0.15 us (the chain load - multiply - release of its issuing threads), so that
 // neither few CTAs nor long K ranges reach the memory's rate.  128-row weight tiles are therefore computed by S CTAs, each over 1/S
 // of K; a cost model on the host picks S and the token blocks.
 //
@@ -25,8 +25,8 @@
 //   RoPE + KV  query and key heads are rotated, queries go to q_out, keys and values into the layer's cache
 //
 // Measured on B200, bf16, in a chain of launches (before: fp32 partial tiles through memory and a second kernel that sums
-// them): 16 x 7168 x 8192 23.1 us (26.5), 16 x 8192 x 3584 13.3 (18.2), 8 x 8192 x 1024 6.9 (10.6), 8 x 1280 x 8192 7.8 (14.3),
-// 64 x 7168 x 8192 24.4 (29.6), 128 x 4096 x 4096 13.4, 512 x 1280 x 8192 17.4 (21.6).
+// them): 16 x 7168 x 8192 22.2 us (26.5), 32 x 8192 x 3584 12.8 (18.2 with 16 rows), 8 x 8192 x 1024 6.9 (10.6), 8 x 1280 x 8192 7.8 (14.3),
+// 128 x 7168 x 8192 24.7 (27.5), 64 x 7168 x 8192 24.4 (29.6), 128 x 4096 x 4096 13.4, 512 x 1280 x 8192 17.4 (21.6).
 //
 // Roles: warp 0 loads weights, warp 1 issues the MMAs, warp 2 loads activations (one thread each), warps 2-5 drain TMEM; all six
 // warps take part in the reduction.  A cluster handles tiles c, c + G, ... one after the other; normally the grid covers all tiles, a CTA
@@ -54,8 +54,8 @@ constexpr int kRowsW = 128;                  // weight rows of a CTA (the instru
 constexpr int kRowBytes = kTileK * 2;        // 128: one row of a stage
 constexpr int kMaxTokens = 256;              // per instruction (its N)
 constexpr int kMaxTileTokens = 384;          // per tile: what its fp32 sums leave of an SM's shared memory; more rows are cut into blocks
-// Up to this many tokens a stage holds 128 elements of K: half the waits and commits per byte (one CTA, 16 tokens: 0.17 us per
-// 64 elements instead of 0.24; 64 tokens: 0.20 instead of 0.25).  With more tokens it would leave too few stages
+// Up to this many tokens a stage holds 128 elements of K: half the waits and commits per byte (one CTA, 16 tokens: 0.107 us per
+// 64 elements, 128 tokens with 64 elements a stage 0.142).  With more tokens it would leave too few stages
 // (128 x 7168 x 8192 27.1 us with 64 elements and 27.6 with 128, 128 x 8192 x 3584 split four ways 17.6 and 22.8).
 constexpr int kWideTokens = 64;
 constexpr int kThreadsC = 192;

@@ -4,7 +4,8 @@ Every linear layer is this library's tcgen05 GEMM; each transformer layer has tw
 (``o_proj`` and ``down_proj``) whose all-reduce is fused with the residual add and the following RMSNorm, i.e. 160
 all-reduces per token step for the 80-layer 70B configuration.  A decode step of a layer is seven kernels of this
 library: QKV GEMM with RoPE + KV-cache write, grouped-query decode attention over the static cache (head size 128),
-output GEMM, all-reduce + residual + RMSNorm, gate/up GEMM with SwiGLU, down GEMM, all-reduce + residual + RMSNorm.
+output GEMM, all-reduce + residual + RMSNorm, gate/up GEMM with SwiGLU, down GEMM, all-reduce + residual + RMSNorm; on one
+GPU it is five, the projections carrying the residual and the norm themselves.
 Prefill attention uses PyTorch's causal ``scaled_dot_product_attention`` (the reference has no attention kernels;
 it only replaces the tensor-parallel communication of a served model).  The decode step has static shapes (the
 position is a device tensor) and is replayed from one CUDA graph.

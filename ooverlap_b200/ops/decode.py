@@ -3,7 +3,7 @@ attention over a static cache.
 
 Capability parity: the reference leaves the model's own ops to vLLM
 (patches/vllm/v0.25.0/vllm/model_executor/models/qwen2.py); this library's serving path needs them so that one
-decode step is a fixed sequence of kernels (seven per transformer layer) that a CUDA graph replays.
+decode step is a fixed sequence of kernels (seven per transformer layer, five on one GPU) that a CUDA graph replays.
 """
 from __future__ import annotations
 

@@ -86,7 +86,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
     summed in split order), 1 turns it off; 0 leaves it to the kernel that the shape takes (few rows or few tiles: the
     weight-streaming kernel, else the two-SM kernel; the tiled kernels split by shape where both are ruled out).
 
-    ``pair`` selects the two-SM kernel (tiles of 256 rows and 128 to 256 columns computed by CTA pairs with
+    ``pair`` selects the two-SM kernel (tiles of 256 rows and 128 to 512 columns computed by CTA pairs with
     ``tcgen05.mma.cta_group::2``; each CTA stages half of the B block): 0 uses it for problems with more than 128 rows that
     the weight-streaming kernel is not expected to compute faster, 1 whenever the problem is unsplit, -1 never.
 
