@@ -219,7 +219,7 @@ typedef struct {
                    kernel before it on the stream still runs.  0 = B may be that kernel's output */
   const float* row_ssq; /* plain mode, M <= 128: row m of the product is multiplied by 1 / sqrt(s / K + row_eps), s = the sum over
                            row_parts of row_ssq[part * M + m] (the sums that OOB_EPILOGUE_ADD writes); null = not */
-  int row_parts;
+  int row_parts;        /* ceil(K / 128) */
   float row_eps;
 } oob_gemm_args_t;
 #define OOB_EPILOGUE_NONE 0

@@ -290,7 +290,7 @@ cudaError_t launch_gemm(const CommCtx& ctx, const GemmArgs& args, cudaStream_t s
     // What the weight-streaming kernel alone can do.
     if (a.epilogue == kGemmEpilogueAdd || a.row_ssq != nullptr) {
       if (a.epilogue != 0 && a.epilogue_args == nullptr) return cudaErrorInvalidValue;
-      if (a.row_ssq != nullptr && a.row_parts < 1) return cudaErrorInvalidValue;
+      if (a.row_ssq != nullptr && a.row_parts != (a.K + 127) / 128) return cudaErrorInvalidValue;
       if (a.epilogue == kGemmEpilogueAdd) {
         const auto& add = *static_cast<const oob_gemm_epilogue_add_t*>(a.epilogue_args);
         const uintptr_t align = reinterpret_cast<uintptr_t>(add.residual) | reinterpret_cast<uintptr_t>(add.norm_weight) |

@@ -1073,6 +1073,9 @@ int oob_gemm(oob_comm* c, const oob_gemm_args_t* a, void* stream) {
   g.row_ssq = a->row_ssq;
   g.row_parts = a->row_parts;
   g.row_eps = a->row_eps;
+  // The kernel reads row_parts x M sums: one part for every 128 columns of A, as the epilogue that writes them leaves them.
+  if (a->row_ssq != nullptr && (a->K <= 0 || a->row_parts != (a->K + 127) / 128 || (reinterpret_cast<uintptr_t>(a->row_ssq) & 3)))
+    return set_error(OOB_ERR_INVALID, "row sums of squares: one part for every 128 elements of K, 4-byte aligned");
   g.epilogue = a->epilogue;
   g.epilogue_args = a->epilogue_args;
   if (a->epilogue != OOB_EPILOGUE_NONE) {

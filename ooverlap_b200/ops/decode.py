@@ -79,12 +79,12 @@ def gemm_rope_kv_write(x: torch.Tensor, wqkv: torch.Tensor, B: int, T: int, head
     done from the fp32 sums by the kernel that has them (the weight-streaming kernel, or the one that sums the splits);
     otherwise (or with ``fused=False``) the GEMM is followed by :func:`rope_kv_write`.  ``x`` may be a ``RowSums`` (see
     ``gemm_add_norm``).  Returns the rotated queries, [B*T, heads * hd]."""
-    from .gemm import RowSums, _check_operands, _plain_args, _set_row_sums, gemm, gemm_plan_splits
+    from .gemm import RowSums, _check_operands, _plain_args, _scaled_rows, _set_row_sums, gemm, gemm_plan_splits
     sums = x
     if isinstance(x, RowSums):
         if fused is False:
             raise ValueError("row sums need the kernel that this call rules out")
-        x = x.scaled
+        x = _scaled_rows(x)
     _check_operands(x, wqkv)
     M, N, K = x.shape[0], wqkv.shape[0], x.shape[1]
     if M != B * T:

@@ -234,6 +234,15 @@ class RowSums(NamedTuple):
     eps: float
 
 
+def _scaled_rows(x: RowSums) -> torch.Tensor:
+    """``x.scaled``, once ``x.ssq`` is seen to belong to it.  The kernel reads ``ssq`` as dense ``[ceil(K / 128), M]`` fp32: for some of
+    the rows, slices of both tensors are only that when the sums have been copied (``ssq[:, rows].contiguous()``)."""
+    want = ((x.scaled.shape[1] + 127) // 128, x.scaled.shape[0]) if x.scaled.dim() == 2 else ()
+    if x.ssq.dtype != torch.float32 or x.ssq.shape != want or x.ssq.device != x.scaled.device or not x.ssq.is_contiguous():
+        raise ValueError(f"row sums must be a contiguous fp32 tensor {list(want)} beside the [M, K] rows that they belong to")
+    return x.scaled
+
+
 def _set_row_sums(args: _lib.GemmArgs, x) -> None:
     if isinstance(x, RowSums):
         args.row_ssq, args.row_parts, args.row_eps = x.ssq.data_ptr(), x.ssq.shape[0], x.eps
@@ -279,7 +288,7 @@ def gemm_swiglu(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = 
     if isinstance(a, RowSums):
         if max_ctas or fused is False:
             raise ValueError("row sums need the kernel that this call rules out")
-        a = a.scaled
+        a = _scaled_rows(a)
     _check_operands(a, b)
     M, N = a.shape[0], b.shape[0]
     if N % 16 != 0:
