@@ -1030,6 +1030,9 @@ int oob_fused_norm(oob_comm* c, int algo, const oob_norm_args_t* a, int max_ctas
 int oob_gemm(oob_comm* c, const oob_gemm_args_t* a, void* stream) {
   if (a == nullptr) return set_error(OOB_ERR_INVALID, "null argument");
   if (a->dtype != OOB_F16 && a->dtype != OOB_BF16) return set_error(OOB_ERR_INVALID, "GEMM dtype must be fp16 or bf16");
+  const bool row_norms = a->row_ssq != nullptr || a->epilogue == OOB_EPILOGUE_ADD;
+  if (row_norms && a->mode != OOB_GEMM_PLAIN)
+    return set_error(OOB_ERR_INVALID, "row sums of squares and the Add epilogue apply to the plain GEMM only");
   CommCtx ctx{};
   if (c != nullptr) {
     int rc = check_comm(c);
@@ -1076,6 +1079,11 @@ int oob_gemm(oob_comm* c, const oob_gemm_args_t* a, void* stream) {
   // The kernel reads row_parts x M sums: one part for every 128 columns of A, as the epilogue that writes them leaves them.
   if (a->row_ssq != nullptr && (a->K <= 0 || a->row_parts != (a->K + 127) / 128 || (reinterpret_cast<uintptr_t>(a->row_ssq) & 3)))
     return set_error(OOB_ERR_INVALID, "row sums of squares: one part for every 128 elements of K, 4-byte aligned");
+  // One kernel does this, and it writes neither record: what it would have to drop is refused.
+  if (row_norms && (a->trace != nullptr || a->order != nullptr || a->gemv > 0 || a->stream_k > 0 || a->splitk_reduce != 0 || a->pair > 0 ||
+                    a->skinny < 0))
+    return set_error(OOB_ERR_UNSUPPORTED, "row sums of squares and the Add epilogue are for the weight-streaming kernel: no trace, tile order, "
+                                          "gemv, stream_k, splitk_reduce or pair, and skinny not negative");
   g.epilogue = a->epilogue;
   g.epilogue_args = a->epilogue_args;
   if (a->epilogue != OOB_EPILOGUE_NONE) {
@@ -1104,8 +1112,12 @@ int oob_gemm(oob_comm* c, const oob_gemm_args_t* a, void* stream) {
         return set_error(OOB_ERR_INVALID, "RoPE epilogue: bad cache geometry or alignment");
       if (r->pos_dev == nullptr && (r->pos0 < 0 || r->pos0 + r->T > r->max_len))
         return set_error(OOB_ERR_INVALID, "RoPE epilogue: positions outside the cache");
+    } else if (a->epilogue == OOB_EPILOGUE_ADD) {
+      // Rows of C that overlap would be written twice; rows of the residual are only read and may be one row for all.
+      if (a->ldc < a->N || static_cast<const oob_gemm_epilogue_add_t*>(a->epilogue_args)->ld_residual < 0)
+        return set_error(OOB_ERR_INVALID, "Add epilogue: ldc >= N, ld_residual >= 0");
     } else {
-      if (a->epilogue != OOB_EPILOGUE_ADD) return set_error(OOB_ERR_INVALID, "unknown epilogue");
+      return set_error(OOB_ERR_INVALID, "unknown epilogue");
     }
   }
   g.splitk_ws = nullptr;
@@ -1140,8 +1152,8 @@ int oob_gemm(oob_comm* c, const oob_gemm_args_t* a, void* stream) {
   }
   if (e == cudaErrorNotSupported && (a->epilogue == OOB_EPILOGUE_ADD || a->row_ssq != nullptr)) {
     (void)cudaGetLastError();
-    return set_error(OOB_ERR_UNSUPPORTED, "row sums of squares are for the weight-streaming kernel: at most 128 rows, and neither "
-                                          "OOB_GEMM_SKINNY=0 nor an argument may rule it out");
+    return set_error(OOB_ERR_UNSUPPORTED, "row sums of squares are for the weight-streaming kernel: at most 128 rows, and "
+                                          "OOB_GEMM_SKINNY=0 rules it out");
   }
   if (e == cudaErrorNotSupported && a->epilogue == OOB_EPILOGUE_SWIGLU_TILE) {
     (void)cudaGetLastError();

@@ -260,8 +260,9 @@ def gemm_add_norm(a: torch.Tensor, b: torch.Tensor, residual: torch.Tensor, weig
     if M > DEFERRED_NORM_MAX_ROWS or N % 8 != 0:
         raise ValueError(f"at most {DEFERRED_NORM_MAX_ROWS} rows, and columns in multiples of 8")
     if residual.shape != (M, N) or residual.dtype != a.dtype or residual.stride(1) != 1 or residual.stride(0) % 4 != 0 \
-            or weight.shape != (N,) or weight.dtype != a.dtype or not weight.is_contiguous():
-        raise ValueError("residual must be [M, N] with unit column stride and weight [N], both of the operands' dtype")
+            or weight.shape != (N,) or weight.dtype != a.dtype or not weight.is_contiguous() or residual.device != a.device \
+            or weight.device != a.device:
+        raise ValueError("residual must be [M, N] with unit column stride and weight [N], both of the operands' dtype and device")
     h = torch.empty((M, N), dtype=a.dtype, device=a.device)
     scaled = torch.empty_like(h)
     ssq = torch.empty(((N + 127) // 128, M), dtype=torch.float32, device=a.device)
