@@ -226,7 +226,8 @@ class LlamaTP:
                         q = rope_kv_write(qkv, B, T, self.h_local, self.kv_local, kc, vc, self.rope_cos32, self.rope_sin32,
                                           pos, batch0=batch0)
                     if decode and hd == 128:
-                        att = attn_decode(q.view(B, self.h_local, hd), kc, vc, pos, batch0=batch0)
+                        # The projection just before wrote this step's key; the others are of earlier steps.
+                        att = attn_decode(q.view(B, self.h_local, hd), kc, vc, pos, batch0=batch0, cache_ready=True)
                     elif decode:
                         att = F.scaled_dot_product_attention(q.view(B, 1, self.h_local, hd).transpose(1, 2), kc[sl], vc[sl],
                                                              attn_mask=attn_mask, enable_gqa=True)

@@ -16,7 +16,6 @@ import torch
 from .. import _lib
 from ..utils.dtypes import dtype_code
 from ..utils.stream import current_stream_ptr as _stream
-from .gemm import _scope
 
 
 def rope_tables(max_len: int, head_dim: int, theta: float, device) -> tuple[torch.Tensor, torch.Tensor]:
@@ -128,14 +127,18 @@ def silu_mul(gu: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tens
 
 def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, pos, *, batch0: int = 0,
                 scale: Optional[float] = None, out: Optional[torch.Tensor] = None, splits: int = 0,
-                len_bound: int = 0) -> torch.Tensor:
+                len_bound: int = 0, cache_ready: bool = False) -> torch.Tensor:
     """One decode step of grouped-query attention: ``q`` is [B, heads, 128], the cache is
     [batch, kv_heads, max_len, 128] and keys ``0 .. pos`` of sequences ``batch0 .. batch0 + B - 1`` are attended
     (``pos``: int or one-element device ``int64`` tensor, the index of the newest key).  Returns [B, heads * 128].
 
     The CTAs of a cluster share the keys of one (sequence, KV head) by the length found on the device; ``splits`` > 1 adds
     that many clusters, whose results a second kernel merges.  0 picks both from ``B * kv_heads`` and ``len_bound`` (an
-    upper bound of the context length of this and any replayed launch; default ``max_len``)."""
+    upper bound of the context length of this and any replayed launch; default ``max_len``).
+
+    ``cache_ready`` promises that neither the call before this one on the stream nor, in a chain of this library's kernels, one of
+    those before it writes a position on the device or a key or value other than the newest of each sequence: they are then
+    loaded while the kernel before still runs.  Not so behind a call that appends several tokens."""
     if q.dim() != 3 or q.shape[2] != 128 or not q.is_contiguous():
         raise ValueError("q must be a contiguous [B, heads, 128] tensor")
     B, H, hd = q.shape
@@ -168,7 +171,7 @@ def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, p
     a = _lib.AttnDecodeArgs.from_buffer_copy(_lib.ATTN_ARGS.pack(
         dtype_code(q.dtype), B, H, KV, q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), k_cache.stride(0), max_len, batch0,
         out.data_ptr(), pos_dev, length, scale if scale is not None else 1.0 / math.sqrt(hd), splits, bound,
-        ws.data_ptr() if ws is not None else 0, _scope.static_b))
+        ws.data_ptr() if ws is not None else 0, cache_ready))
     _lib.check(lib.oob_attn_decode(ctypes.byref(a), _stream()))
     return out
 

@@ -32,8 +32,7 @@ def static_weights():
     """GEMMs that this thread launches in this block take their ``b`` to be a weight: neither the kernel before the call on the
     stream nor, in a chain of this library's kernels, one of those before it writes ``b``.  The weight-streaming kernel then
     loads its first weights while the kernel before it still runs.  Elsewhere ``b`` may be any tensor, also the result of
-    the call just before.  ``attn_decode`` takes a position on the device and the cache up to the newest key the same way: only the
-    newest key and value are that kernel's."""
+    the call just before.  The promise is about weights alone: see ``attn_decode`` for its cache."""
     before = _scope.static_b
     _scope.static_b = True
     try:

@@ -49,6 +49,31 @@ def test_weights_loaded_ahead(rows, hidden, ffn, dtype):
         assert (a.double() - b.double()).norm() <= 4 * eps * a.double().norm()
 
 
+@pytest.mark.parametrize("tokens,ctx", [(3, 3), (17, 40), (33, 600)])
+def test_the_promise_about_weights_says_nothing_about_the_cache(tokens, ctx):
+    """A projection that appends several tokens, and attention right behind it, in one block of static weights."""
+    torch.manual_seed(ctx)
+    b, heads, kv, hd, max_len, hidden = 3, 8, 1, 128, 1024, 512
+    x = torch.randn(b * tokens, hidden, device="cuda").bfloat16()
+    w = (torch.randn((heads + 2 * kv) * hd, hidden, device="cuda") / hidden ** 0.5).bfloat16()
+    cos, sin = rope_tables(max_len, hd, 10000.0, "cuda")
+    first = torch.full((1,), ctx - tokens, dtype=torch.long, device="cuda")
+    last = torch.full((1,), ctx - 1, dtype=torch.long, device="cuda")
+    cache = torch.randn(2, b, kv, max_len, hd, device="cuda").bfloat16()
+    cache[:, :, :, ctx - tokens:] = float("nan")
+    kc, vc = cache.clone()
+    q = gemm_rope_kv_write(x, w, b, tokens, heads, kv, kc, vc, cos, sin, first)
+    newest = q.view(b, tokens, heads, hd)[:, -1].contiguous()
+    want = attn_decode_reference(newest, kc, vc, ctx - 1)
+    for _ in range(5):
+        kc, vc = cache.clone()
+        torch.cuda.synchronize()
+        with static_weights():
+            gemm_rope_kv_write(x, w, b, tokens, heads, kv, kc, vc, cos, sin, first)
+            got = attn_decode(newest, kc, vc, last)
+        assert (got.double() - want.double()).norm() < 2 * 2.0 ** -8 * want.double().norm()
+
+
 @pytest.mark.parametrize("ctx", [1, 2, 16, 17, 64, 65, 200, 1000])
 @pytest.mark.parametrize("b,heads,kv", [(1, 8, 1), (3, 16, 1), (40, 8, 2)])
 def test_cache_read_ahead_of_the_newest_key(ctx, b, heads, kv):
@@ -67,8 +92,7 @@ def test_cache_read_ahead_of_the_newest_key(ctx, b, heads, kv):
         torch.cuda.synchronize()
         with static_weights() if ahead else contextlib.nullcontext():
             q = gemm_rope_kv_write(x, w, b, 1, heads, kv, kc, vc, cos, sin, pos)
-        with static_weights() if ahead else contextlib.nullcontext():
-            out.append((attn_decode(q.view(b, heads, hd), kc, vc, pos), q))
+        out.append((attn_decode(q.view(b, heads, hd), kc, vc, pos, cache_ready=ahead), q))
     assert torch.equal(out[1][0], out[2][0])
     want = attn_decode_reference(out[1][1].view(b, heads, hd), kc, vc, ctx - 1)
     assert (out[1][0].double() - want.double()).norm() < 2 * 2.0 ** -8 * want.double().norm()
