@@ -13,8 +13,8 @@ namespace gemm_pair {
 // accumulator (256x256 fp32), so the size depends on the pair count only.
 constexpr int kSkMaxPairs = 80;               // >= 74 pairs of a 148-SM part
 constexpr int kSkMaxTiles = 2 * kSkMaxPairs;  // tiles of a tail
-constexpr int kSkWarps = 8;                   // epilogue warps of a CTA that park and add
-constexpr size_t kSkFlagBytes = 16384;        // kSkMaxTiles x 2 CTAs x kSkWarps x 4 bytes, rounded up
+constexpr int kSkWarps = 4;                   // epilogue warps of a CTA that park and add
+constexpr size_t kSkFlagBytes = 8192;         // kSkMaxTiles x 2 CTAs x kSkWarps x 4 bytes, rounded up
 constexpr size_t kSkSlotBytes = size_t(256) * 256 * 4;
 constexpr size_t kSkWorkspaceBytes = kSkFlagBytes + size_t(kSkMaxPairs) * kSkSlotBytes;
 
