@@ -87,6 +87,7 @@ struct ParamsC {
   int num_kb, num_tiles, clusters;  // num_kb: pipeline stages' worth of K (sub * 64 elements each)
   int sub;
   int S;  // CTAs (pairs) that share the K range of a tile
+  int per_sm;  // CTAs of an SM (the host's)
   int stages, stage_bytes, work_bytes;  // work_bytes: pipeline buffers or partial sums, whichever is larger
   int smem_bytes;
   uint32_t tmem_cols;
@@ -250,7 +251,9 @@ __device__ __forceinline__ void emit(const ParamsC& p, int m, int n, const float
 // units are dealt out over the CTAs of the cluster, then over the threads, and TB units x S copies of independent loads are
 // in flight per thread.  `n_first`: first output column of the tile.
 // All threads of the CTA call `read_done` together, once, when the last copies have been read and before the last results are
-// written: the cluster barrier behind it would otherwise wait for those stores (0.6 us).
+// written: the cluster barrier behind it would otherwise wait for those stores (35 x 2304 x 1536 5.4 us, 5.8 behind them).  Not so where a
+// plain launch takes several turns: inside the loop it keeps a turn's loads from being issued among the stores of the turn before
+// (250 x 8192 x 3584 20.7 us, 20.4 behind the loop; 128 x 3896 x 608 7.8 and 7.4).
 template <typename T, int EPI, int S, bool PAIR, typename F>
 __device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base, int rank, int m_first, int n_first, int rows,
                                             long long pos_base, const float* scale, F read_done) {
@@ -265,7 +268,7 @@ __device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base
   const int u_first = EPI == kEpiAdd ? rows * rank / S * upt : units * rank / S;
   const int u1 = EPI == kEpiAdd ? rows * (rank + 1) / S * upt : units * (rank + 1) / S;
   const int turns = (u1 - u_first + kThreadsC * TB - 1) / (kThreadsC * TB);  // the same for all threads
-  for (int turn = 0; turn < turns; ++turn) {
+  auto take = [&](int turn, auto last) {
     const int u0 = u_first + turn * kThreadsC * TB + int(threadIdx.x);
     float4 v[TB][kParts][S];
     RopeUnit rope[TB];
@@ -304,7 +307,7 @@ __device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base
         }
       }
     }
-    if (turn + 1 == turns) read_done();
+    if (last) read_done();
     if (p.row_ssq != nullptr) {
 #pragma unroll
       for (int i = 0; i < TB; ++i) {
@@ -334,18 +337,29 @@ __device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base
         for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
         if ((threadIdx.x & 31) == 0) p.add.ssq[size_t(n_first / kRowsW) * p.M + row] = ss;
       }
-      continue;
+      return;
     }
 #pragma unroll
     for (int i = 0; i < TB; ++i)
       if (u0 + i * kThreadsC < u1) emit<T, EPI>(p, m_first + m[i], n_first + c[i], s[i][0], s[i][kParts - 1], rope[i]);
+  };
+  if constexpr (EPI != kEpiPlain) {
+    for (int turn = 0; turn < turns; ++turn) take(turn, turn + 1 == turns);
+    if (turns == 0) read_done();
+  } else if (turns == 1) {
+    take(0, std::true_type{});
+  } else {
+    for (int turn = 0; turn < turns; ++turn) take(turn, std::false_type{});
+    read_done();
   }
-  if (turns == 0) read_done();
 }
 
-// SUB: 64-element boxes of K in a pipeline stage.
-template <typename T, int EPI, bool PAIR, int SUB>
-__global__ void __launch_bounds__(kThreadsC)
+// SUB: 64-element boxes of K in a pipeline stage.  RES: CTAs of an SM that the registers leave room for, 0 = what the compiler makes of it.
+// That is so few registers (50) for a plain launch's sums that the loads of a turn wait for each other; with three CTAs 80 - 90
+// (256 x 3456 x 4544 18.8 us, 17.9), with four 70 - 80 (143 x 1024 x 7680 17.7 us, 16.4 with three), which only the plans take that
+// place four on an SM (16 x 64000 x 512 14.4 us, 16.8 on three).
+template <typename T, int EPI, bool PAIR, int SUB, int RES>
+__global__ void __launch_bounds__(kThreadsC, RES)
     gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                         const __grid_constant__ ParamsC p, DeviceStatus* status) {
   constexpr int FMT = PackTraits<T>::kDType == kBF16 ? 1 : 0;
@@ -606,9 +620,9 @@ __global__ void __launch_bounds__(kThreadsC)
   }
 }
 
-template <typename T, int EPI, bool PAIR, int SUB>
+template <typename T, int EPI, bool PAIR, int SUB, int RES>
 cudaError_t launch_pair(const GemmArgs& a, ParamsC& p, DeviceStatus* status, cudaStream_t stream, TmapFn make_tmap) {
-  auto kernel = gemm_cluster_kernel<T, EPI, PAIR, SUB>;
+  auto kernel = gemm_cluster_kernel<T, EPI, PAIR, SUB, RES>;
   const int size = PAIR ? 2 * p.S : p.S;  // CTAs of a cluster
   static std::atomic<uint64_t> attr_set_mask{0};
   int dev = 0;
@@ -643,9 +657,15 @@ cudaError_t launch_pair(const GemmArgs& a, ParamsC& p, DeviceStatus* status, cud
 
 template <typename T, int EPI>
 cudaError_t launch_epi(const GemmArgs& a, ParamsC& p, bool pair, DeviceStatus* status, cudaStream_t stream, TmapFn make_tmap) {
-  if (pair) return launch_pair<T, EPI, true, 1>(a, p, status, stream, make_tmap);
-  return p.sub == 2 ? launch_pair<T, EPI, false, 2>(a, p, status, stream, make_tmap)
-                    : launch_pair<T, EPI, false, 1>(a, p, status, stream, make_tmap);
+  constexpr int kRes = EPI == kEpiPlain ? 3 : 0;
+  if (pair) return launch_pair<T, EPI, true, 1, kRes>(a, p, status, stream, make_tmap);
+  if constexpr (EPI == kEpiPlain) {
+    if (p.per_sm > kRes)
+      return p.sub == 2 ? launch_pair<T, EPI, false, 2, 4>(a, p, status, stream, make_tmap)
+                        : launch_pair<T, EPI, false, 1, 4>(a, p, status, stream, make_tmap);
+  }
+  return p.sub == 2 ? launch_pair<T, EPI, false, 2, kRes>(a, p, status, stream, make_tmap)
+                    : launch_pair<T, EPI, false, 1, kRes>(a, p, status, stream, make_tmap);
 }
 
 template <typename T>
@@ -903,6 +923,7 @@ cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStr
   p.Mp = pl.n_mma * pl.nj;
   p.m_blocks = pl.m_blocks;
   p.S = pl.S;
+  p.per_sm = pl.per_sm;
   p.num_tiles = tile_count(a.N, pl);
   p.stage_bytes = pl.sub * (kRowsW + p.Mp / P) * kRowBytes;
   p.stages = pl.stages;
