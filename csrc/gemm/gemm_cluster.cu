@@ -760,18 +760,19 @@ int cluster_slots(int sms, int size, int per_sm) {
 
 // Microseconds a plan takes: rounds of clusters, each as long as its K blocks at the pace of one CTA or of the tensor cores of an
 // SM (cycles a block grow with the tokens), at the memory's rate for the weights or at L2's for all operands, whichever is
-// slowest; then draining the sums, reading the other CTAs' sums, and the fixed cost of a launch.  `ragged`: rows start off a
-// 128-byte line, and a row of a box touches two.
+// slowest; then draining the sums, reading the other CTAs' sums, and the fixed cost of a launch.  A row of a box that starts off a
+// 128-byte line touches two (`line`), one that starts off a 32-byte sector one more of these (`sector`); the pace of one CTA with stages of
+// many tokens suffers most (`pace_sector`: 103 x 5504 x 6728 split two ways 28.2 us, three ways 21.1, which were taken for the slower).
 // The constants are fitted to timings for the choice they make, so that one need not be the rate that it stands for.  Up to 128 rows to
 // 16000 timings of every K split (1930 shapes of 3 - 128 rows, N and K of 512 - 8192): 3.3 % off the best plan on average, 4.8 % with
 // the other set.  Above, the set against which the two-SM kernel is weighed.
 struct CostC {
-  double wide, wide_tokens, pace, pace_tokens, mma, l2, hbm, drain, reduce, round, alone, cluster, eight, split, ragged;
+  double wide, wide_tokens, pace, pace_tokens, mma, l2, hbm, drain, reduce, round, alone, cluster, eight, split, line, sector, pace_sector;
 };
-constexpr CostC kFewRows = {0.153, 0.00061, 0.17, 0.00028, 1140.0, 11.8e6, 6.4e6, 0.0117, 2.84e6, 1.85, 2.52, 3.06, 2.6, 0.105, 1.29};
-constexpr CostC kMoreRows = {0.165, 0.0005, 0.235, 0.0002, 1850.0, 11.5e6, 6.4e6, 0.015, 3.0e6, 2.0, 3.4, 3.8, 2.0, 0.08, 1.45};
+constexpr CostC kFewRows = {0.153, 0.00061, 0.17, 0.00028, 1140.0, 11.8e6, 6.4e6, 0.0117, 2.84e6, 1.85, 2.52, 3.06, 2.6, 0.105, 1.29, 1.29, 1.8};
+constexpr CostC kMoreRows = {0.165, 0.0005, 0.235, 0.0002, 1850.0, 11.5e6, 6.4e6, 0.015, 3.0e6, 2.0, 3.4, 3.8, 2.0, 0.08, 1.16, 1.45, 1.45};
 
-double plan_cost(int M, int N, int num_kb, int sms, bool ragged, const PlanC& pl) {
+double plan_cost(int M, int N, int num_kb, int sms, RowStart start, const PlanC& pl) {
   const CostC& c = M <= kTileM ? kFewRows : kMoreRows;
   const int P = pl.pair ? 2 : 1, Mp = pl.n_mma * pl.nj, size = P * pl.S;
   const int clusters = tile_count(N, pl), slots = cluster_slots(sms, size, pl.per_sm);
@@ -780,8 +781,8 @@ double plan_cost(int M, int N, int num_kb, int sms, bool ragged, const PlanC& pl
   const double share = live > sms ? live / sms : 1.0;
   const double kb = double((num_kb + pl.S - 1) / pl.S);
   const double w = kRowsW * kRowBytes, x = double(Mp) / P * kRowBytes;
-  const double lines = ragged ? c.ragged : 1.0;
-  double t = lines * kb * (pl.sub == 2 ? c.wide + c.wide_tokens * Mp : c.pace + c.pace_tokens * Mp);
+  const double lines = start == kOnLine ? 1.0 : start == kOnSector ? c.line : c.sector;
+  double t = (start == kOffSector && Mp > kWideTokens ? c.pace_sector : lines) * kb * (pl.sub == 2 ? c.wide + c.wide_tokens * Mp : c.pace + c.pace_tokens * Mp);
   const double mma = share * kb * 2.0 * Mp / c.mma, l2 = lines * live * kb * (w + x) / c.l2, hbm = live * kb * w / pl.m_blocks / c.hbm;
   if (mma > t) t = mma;
   if (l2 > t) t = l2;
@@ -819,7 +820,7 @@ bool plan(int M, int N, int K, int sms, int pair, int fix_s, bool ahead, PlanC* 
         if (fix_s > 0 ? pl.S != fix_s : (num_kb < 4 * pl.S && pl.S > 1)) continue;
         if (!size_cta(N, num_kb, sms, &pl)) continue;
         // (with more rows the plans are compared as if rows started on a line: the set was fitted so)
-        double c = plan_cost(M, N, num_kb, sms, M <= kTileM && K % kTileK != 0, pl);
+        double c = plan_cost(M, N, num_kb, sms, M <= kTileM ? row_start(K) : kOnLine, pl);
         if (ahead) c -= ring_us(N, num_kb, sms, pl);
         if (!found || c < *cost) {
           found = true;
@@ -864,7 +865,7 @@ bool gemm_cluster_supported(const GemmArgs& a) {
 // Whether this kernel is expected to be faster than the persistent two-SM kernel, which overlaps a tile's epilogue with the next
 // tile and needs no sum of parts, but deals out 256-row tiles: with fewer than three rounds of those, what they leave
 // idle or compute on padding is often more than this kernel's fixed cost.  Its estimate is taken a tenth lower,
-// which fits its present pace: over 1611 shapes of more than 128 rows the choice is then 3.1 % slower than the best one on average.
+// which fits its present pace: over 467 shapes of more than 128 rows the choice is then 0.9 % slower than the best one on average.
 // Both sides measured, bf16 on B200: 512 x 1280 x 8192 17.4 here and 29.6 us there, 200 x 4096 x 4096 15.0 and 18.1, 512 x 2048 x 2048
 // 12.0 and 11.9; 1037 x 4104 x 2056 27.2 and 23.0, 768 x 7168 x 8192 71.5 and 64.7, 512 x 8192 x 8192 53.8 and 51.0, 2048 x 2048 x 2048
 // 20.5 and 17.5.
@@ -883,7 +884,7 @@ bool gemm_cluster_preferred(const GemmArgs& a) {
   if (static_cast<long long>((a.M + 2 * kTileM - 1) / (2 * kTileM)) * ((a.N + kTileN - 1) / kTileN) > 3ll * pairs) return false;
   const double two_sm = pair_cut(kGemmPlain, a.M, a.N, a.K, pairs, a.stream_k, swiglu, false, false).us;
   const Planned& c = planned(a.M, a.N, a.K, a.pair, 0, false);
-  return c.ok && 0.9 * plan_cost(a.M, a.N, (a.K + kTileK - 1) / kTileK, sm_count(), a.K % kTileK != 0, c.pl) < two_sm;
+  return c.ok && 0.9 * plan_cost(a.M, a.N, (a.K + kTileK - 1) / kTileK, sm_count(), row_start(a.K), c.pl) < two_sm;
 }
 
 cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStream_t stream, gemm_detail::TmapFn make_tmap) {

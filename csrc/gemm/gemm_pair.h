@@ -144,6 +144,10 @@ int pair_streamk_auto(int tiles, int pairs, int num_kb, long long operand_bytes)
 // that share it; both 0 when a tail is not possible.
 void pair_streamk_plan(int tiles, int pairs, int num_kb, int* sk_tiles, int* sk_pairs);
 
+// Where the rows of dense 16-bit operands with K elements begin: all on a 128-byte line, all on a 32-byte sector, or neither.
+enum RowStart { kOnLine, kOnSector, kOffSector };
+inline RowStart row_start(int K) { return K % 64 == 0 ? kOnLine : K % 16 == 0 ? kOnSector : kOffSector; }
+
 // How a problem is cut into tiles on `pairs` pairs: 256 columns with or without a stream-K tail or, in plain launches that do
 // not ask for a tail, another width where it is expected to be faster.  Up to 256 columns the two accumulators alternate between
 // tiles; a wider tile takes both at once, which brings fewer operand bytes per product and leaves the drain of a tile to be

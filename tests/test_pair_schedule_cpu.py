@@ -120,6 +120,27 @@ def test_auto_rule_picks_a_tail_only_where_it_pays():
     assert not _tail(PLAIN, 2048, 8192, 512)
 
 
+def tile_columns(M, N, K, pairs=74):
+    """Columns of a tile: both accumulators where a pair takes two neighbouring ones in one item."""
+    items = schedule(PLAIN, M, N, K, pairs, 0)
+    assert not any(item[6] >= 0 for item in items)
+    joined = max(sum(1 for i in items if i[:2] == first[:2]) for first in items[:2])
+    return joined * columns(PLAIN, M, N, K, pairs, 0)
+
+
+def test_the_widths_that_were_measured_faster():
+    # rows that start off a 128-byte line, but on a sector, cost a tenth more and not half: no wide tile to spare a round
+    assert tile_columns(3983, 1648, 1808) == 192 and tile_columns(3769, 1424, 3040) == 160
+    # off a sector they cost more than half: one round of wide tiles
+    assert tile_columns(1037, 4104, 2056) == 320
+    # many rounds: the power cap, not the last round, decides
+    assert tile_columns(8192, 14336, 8192) == 256 and tile_columns(4096, 28672, 8192) == 256
+    assert tile_columns(8192, 8192, 4096) == 256 and tile_columns(8192, 8192, 6144) == 256
+    assert tile_columns(8192, 8192, 7168) == 512 and tile_columns(16384, 8192, 8192) == 512
+    # ... unless the wide tiles leave more of a round idle
+    assert tile_columns(4096, 14336, 8192) == 256
+
+
 def test_all_gather_keeps_whole_columns_and_the_tail():
     # the chunk flags of an all-gather count 256-column tiles: a tail is the only way to fill the last wave
     assert _tail(AG, 4096, 3584, 8192) and _tail(AG, 2048, 8192, 8192)
