@@ -101,7 +101,7 @@ def main() -> int:
     out["items_by_gemm_ctas"] = int(gemm_rows[:, 5].sum())
     out["comm_cta_wait_us_med"] = round(statistics.median([int(v) / 1e3 for v in comm_rows[:, 6]]), 1) if len(comm_rows) else None
     if getattr(op, "order_buffer", None) is not None:
-        rec = tile_order(op.order_buffer)
+        rec = tile_order(op.order_buffer, in_sequence=False)
         if rec:
             # Tile-order record of the two-SM kernel: when each 128-row half-tile was published to its reducer.
             out["half_tiles_published"] = len(rec)

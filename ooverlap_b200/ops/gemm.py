@@ -79,7 +79,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
 
     ``order`` (two-SM kernel): an int64 CUDA tensor ``[2 * tiles, 2]`` (``tiles`` = 256x256 tiles of the output) that
     the kernel fills with the tile-order record: per 128-row half of every tile the globaltimer nanoseconds at which
-    it was stored and ``pair << 32 | index in the pair's sequence``; see :func:`tile_order`.
+    it was stored and ``pair << 32 | index in the pair's sequence``; see :func:`tile_order`.  The record is of 256-column tiles:
+    a call with one runs on these whatever width it would take without.
 
     ``splits`` > 1 splits K over that many CTAs per output tile (fp32 partials in the library's workspace,
     summed in split order), 1 turns it off; 0 leaves it to the kernel that the shape takes (few rows or few tiles: the
@@ -155,20 +156,33 @@ def check_order_buffer(order: torch.Tensor, M: int, N: int) -> None:
         raise ValueError(f"order must be a contiguous int64 CUDA tensor of at least {2 * tiles} x 2 words")
 
 
-def tile_order(order: torch.Tensor) -> list:
+def tile_order(order: torch.Tensor, in_sequence: bool = True) -> list:
     """Decodes a tile-order record into a list of dicts sorted by completion time: ``unit`` (2 * tile's number in the
     schedule + CTA of the pair), ``t_us`` (microseconds after the first completion), ``pair`` and ``index`` (the
     tile's position in that pair's own sequence).  Halves the kernel never wrote (rows past M) are left out.
 
+    The CTAs of a pair store their halves on their own, and one may be a tile ahead of the other.  ``in_sequence``: such a half counts as
+    complete when the tiles before it in its pair's sequence are, so that the list follows every pair's sequence; False
+    gives the times as they were stamped.
+
     Capability parity: the reference records in which order its GEMM finishes tiles to derive reorder hints
     (tool/search.py, the tile-order capture of src/gemm/gemm_with_signal_sm90.h); here the schedule is fixed by the
     kernel (PairSched) and the record shows how the hardware actually ran it."""
-    rows = order.detach().cpu().tolist()
-    done = [(t, u, w) for u, (t, w) in enumerate(rows) if t > 0]
+    done = [(t, u, int(w >> 32), int(w & 0xFFFFFFFF)) for u, (t, w) in enumerate(order.detach().cpu().tolist()) if t > 0]
     if not done:
         return []
-    t0 = min(t for t, _, _ in done)
-    return [dict(unit=u, t_us=(t - t0) / 1e3, pair=int(w >> 32), index=int(w & 0xFFFFFFFF)) for t, u, w in sorted(done)]
+    if in_sequence:
+        seen = {}  # pair -> (index, latest time of the tiles up to it, the same of those before it)
+        done.sort(key=lambda d: (d[2], d[3]))
+        for i, (t, u, pair, index) in enumerate(done):
+            last, upto, before = seen.get(pair, (index, 0, 0))
+            if index != last:
+                before = upto
+            done[i] = (max(t, before), u, pair, index)
+            seen[pair] = (index, max(upto, t), before)
+    t0 = min(d[0] for d in done)
+    return [dict(unit=u, t_us=(t - t0) / 1e3, pair=pair, index=index)
+            for t, u, pair, index in sorted(done, key=lambda d: (d[0], d[3], d[1]))]
 
 
 def stable_tile_waves(records, wave: int) -> dict:
