@@ -24,7 +24,7 @@ from typing import Optional
 import torch
 import torch.nn.functional as F
 
-from ..ops import (DEFERRED_NORM_MAX_ROWS, attn_decode, fused_allreduce_rmsnorm, gemm, gemm_add_norm, gemm_rope_kv_write, gemm_swiglu, rmsnorm, rope_kv_write,
+from ..ops import (attn_decode, fused_allreduce_rmsnorm, gemm, gemm_add_norm, gemm_rope_kv_write, gemm_swiglu, rmsnorm, rope_kv_write,
                    rope_tables, silu_mul, static_weights)
 from ..utils.config import env_flag, env_int
 from ..utils.tracing import nvtx_range
@@ -59,6 +59,14 @@ LLAMA3_70B = LlamaConfig()
 LLAMA3_8B = LlamaConfig(layers=32, hidden=4096, heads=32, kv_heads=8, ffn=14336)
 TINY = LlamaConfig(layers=2, hidden=512, heads=8, kv_heads=2, ffn=1024, vocab=1024)
 TINY128 = LlamaConfig(layers=2, hidden=1024, heads=8, kv_heads=2, ffn=2048, vocab=1024)  # head size 128
+
+
+# Rows up to which norms are folded into the projections around them.  Microseconds a layer of a decode step, folded and with norm
+# kernels, on the 70B configuration's shard at TP 8 / the 8B / the whole 70B configuration: one row 59.0 and 60.8 / 94.7 and 98.9 / 302 and 314
+# (where the CUDA-core kernel would take the gate/up projection), 32 rows 61.8 and 63.6 / 104.6 and 105.3 / 298 and 299, 64 rows 68.8
+# and 68.9 / 114.1 and 115.2 / 318 and 319; 96 rows 73.5 and 71.6 / 113.4 and 111.7 / 364 and 362, 128 rows 84.4 and 78.4 / 129.7 and 124.3 / 391
+# and 387.
+DEFERRED_NORM_ROWS = 64
 
 
 def _apply_rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:
@@ -210,7 +218,7 @@ class LlamaTP:
         h = self.embed[tokens.reshape(-1)]  # [B*T, hidden]  residual stream
         x = self._norm(h, self.layers[0]["norm1"])
         sl = slice(batch0, batch0 + B)
-        deferred = self.deferred_norm and B * T <= DEFERRED_NORM_MAX_ROWS
+        deferred = self.deferred_norm and B * T <= DEFERRED_NORM_ROWS
         for li, layer in enumerate(self.layers):
             with nvtx_range("layer"):
                 if ours and self.fused_epilogues:
