@@ -658,7 +658,11 @@ cudaError_t launch_pair(const GemmArgs& a, ParamsC& p, DeviceStatus* status, cud
 template <typename T, int EPI>
 cudaError_t launch_epi(const GemmArgs& a, ParamsC& p, bool pair, DeviceStatus* status, cudaStream_t stream, TmapFn make_tmap) {
   constexpr int kRes = EPI == kEpiPlain ? 3 : 0;
-  if (pair) return launch_pair<T, EPI, true, 1, kRes>(a, p, status, stream, make_tmap);
+  if constexpr (EPI == kEpiAdd) {  // at most 128 rows, which no pair takes; a pair's second tile may lie past N, and has no sums to write
+    if (pair) return cudaErrorInvalidValue;
+  } else {
+    if (pair) return launch_pair<T, EPI, true, 1, kRes>(a, p, status, stream, make_tmap);
+  }
   if constexpr (EPI == kEpiPlain) {
     if (p.per_sm > kRes)
       return p.sub == 2 ? launch_pair<T, EPI, false, 2, 4>(a, p, status, stream, make_tmap)

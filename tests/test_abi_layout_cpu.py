@@ -14,7 +14,7 @@ sys.path.insert(0, ROOT)
 
 PAIRS = [("oob_comm_info_t", "CommInfo"), ("oob_device_status_t", "DeviceStatus"), ("oob_norm_args_t", "NormArgs"),
          ("oob_gemm_args_t", "GemmArgs"), ("oob_rope_args_t", "RopeArgs"), ("oob_attn_decode_args_t", "AttnDecodeArgs"),
-         ("oob_gemm_epilogue_swiglu_t", "SwigluEpilogue")]
+         ("oob_gemm_epilogue_swiglu_t", "SwigluEpilogue"), ("oob_gemm_epilogue_add_t", "AddEpilogue")]
 
 
 @pytest.mark.skipif(shutil.which("g++") is None, reason="needs a host C++ compiler")
