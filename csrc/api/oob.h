@@ -228,7 +228,9 @@ typedef struct {
 #define OOB_EPILOGUE_SWIGLU_TILE 3 /* as 1, for any problem: applied where a GEMM tile is written.  OOB_ERR_UNSUPPORTED where no
                                       kernel may (pair) or should (one row of a large weight): then oob_gemm + oob_silu_mul */
 #define OOB_EPILOGUE_ADD 4 /* M <= 128, N % 8 == 0: C = round(A B^T) + residual, scaled_out = C * norm_weight, and per 128 columns the
-                              sums of the squares of C's rows.  OOB_ERR_UNSUPPORTED where the weight-streaming kernel may not run */
+                              sums of the squares of C's rows; ldc >= N.  OOB_ERR_UNSUPPORTED, as with row_ssq, where the
+                              weight-streaming kernel may not run and with what it does not do: trace, order, gemv, stream_k,
+                              splitk_reduce, pair = 1, skinny = -1 */
 typedef struct {
   const void* residual;    /* [M, N], row stride ld_residual (a multiple of 4 elements, 8-byte aligned) */
   int ld_residual;

@@ -45,7 +45,10 @@ def env_flag(name: str, default: bool = False) -> bool:
 #   OOB_GEMM_GEMV=0 / 1        plain GEMM, CUDA-core streaming kernel: 0 = never by default, 1 = for every M <= 4
 #                              (unset: one row of a small or a very large weight matrix, two rows of a tiny one)
 #   OOB_SPLITK_REDUCE_MIN_M=n  split-K: sum inside the GEMM kernel below n rows (default 1: always the second kernel)
+#   OOB_FUSED_PAIR=0           fused GEMM + collective ops: never the two-SM kernel by default
 #   OOB_FUSED_EPILOGUES=0      model runner: RoPE + cache write and SwiGLU as kernels of their own behind the GEMM
+#   OOB_DEFERRED_NORM=0        model runner, one GPU: RMSNorm kernels also between the projections of a few rows, which otherwise
+#                              carry the norms (ops.gemm_add_norm)
 #   OOB_PREFILL_CHUNKS=n       model runner, prefill: row-parallel GEMM in n slabs overlapped with the all-reduce + norm
 #   OOB_PREFILL_CHUNK_MIN_ROWS from how many tokens on (default 4096)
 #   OOB_NVTX=1                 NVTX ranges around the model runner's layers (utils/tracing.py)
