@@ -92,7 +92,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
 
     ``stream_k`` (two-SM kernel): when the tile count is not a multiple of the pair count, the last wave and the
     remainder are cut along K into equal ranges, one per pair, so that no pair idles; pairs that compute part of a tile
-    park fp32 accumulators in a library-owned workspace and the part that arrives last sums them in pair order
+    park fp32 accumulators in a library-owned workspace and the pair with the first part sums them in pair order
     (bit-reproducible).  0 uses it when the idle share would exceed 3 % of the run and neither whole tiles nor narrower
     ones are expected to be faster, 1 whenever there is a remainder, -1 never.
 
