@@ -15,7 +15,7 @@ FORMS = [
     (768, 1728, 1032, 5, 384, 3),
     (520, 1128, 1032, 3, 384, 3),     # rows past M, K off a block
     (1000, 2016, 1032, 5, 448, 4),
-    (1000, 2019, 1032, 5, 448, 4),    # rows of C at any 2-byte boundary: no vector stores
+    (300, 1339, 1032, 2, 448, 3),     # rows of C at any 2-byte boundary: no vector stores
     (1280, 1784, 1032, 5, 448, 4),
     (1000, 2304, 1032, 5, 512, 4),
     (1280, 2040, 1032, 5, 512, 4),
@@ -24,6 +24,8 @@ FORMS = [
     (2304, 1024, 2048, 2, 256, 18),   # ... four: many rounds of long tiles
     (2304, 152, 3392, 1, 160, 9),
     (2200, 1443, 4096, 5, 256, 11),
+    (2200, 1446, 4096, 5, 256, 11),   # rows of C on 4 bytes
+    (300, 1914, 1032, 5, 384, 2),
 ]
 
 
@@ -55,3 +57,23 @@ def test_every_form_has_the_bits_of_the_one_sm_kernel(M, N, K, pairs, width, rou
     wide = torch.full((M, N + 24), 7.0, device="cuda", dtype=dtype)
     gemm(a, b, out=wide[:, :N], **how)
     assert torch.equal(wide[:, :N], want) and (wide[:, N:] == 7.0).all()
+
+
+@pytest.mark.parametrize("N", [1026, 1027, 1030, 1279])
+def test_a_tail_writes_rows_off_a_vector(N):
+    """The pair that owns a tile of the tail adds the parts and writes; against 64 bits and bit by bit between calls."""
+    from ooverlap_b200.ops import gemm
+    M, K, pairs = 700, 4096, 7
+    assert any(item[6] >= 0 for item in schedule(PLAIN, M, N, K, pairs, 1))
+    g = torch.Generator(device="cuda").manual_seed(N)
+    a = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+    b = (torch.randn(N, K, device="cuda", generator=g) / K ** 0.5).bfloat16()
+    exact = a.double() @ b.double().t()
+    outs = []
+    for _ in range(2):
+        wide = torch.full((M, N + 24), 7.0, device="cuda", dtype=torch.bfloat16)
+        gemm(a, b, out=wide[:, :N], splits=1, pair=1, stream_k=1, max_ctas=2 * pairs)
+        assert (wide[:, N:] == 7.0).all()
+        outs.append(wide[:, :N])
+    # one rounding to the output type
+    assert torch.equal(*outs) and (outs[0].double() - exact).norm() <= 2.0 ** -8 * exact.norm()
