@@ -38,6 +38,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <limits>
 #include <type_traits>
 
 #include "../api/oob.h"
@@ -98,6 +99,7 @@ struct ParamsC {
   const float* row_ssq;
   int row_parts;
   float row_eps, inv_k;
+  float nan;  // see settle
   oob_gemm_epilogue_add_t add;
 };
 
@@ -119,6 +121,12 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
                : "r"(addr)
                : "memory");
   return v;
+}
+// Waits for the loads that `x` comes from.  A CTA may end when its peers have arrived at the last cluster barrier, and a load from it that
+// is still under way then faults; nothing but its use makes an instruction wait for a load, and one whose result goes nowhere (past the
+// last column) is not waited for.  `nan` is no constant to the compiler, and equal to nothing: the store never happens.
+__device__ __forceinline__ void settle(float x, float nan, uint32_t smem_addr) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.f32 p, %0, %1;\n\t@p st.shared.f32 [%2], %0;\n\t}" ::"f"(x), "f"(nan), "r"(smem_addr) : "memory");
 }
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -250,10 +258,10 @@ __device__ __forceinline__ void emit(const ParamsC& p, int m, int n, const float
 // Sums the S partial copies of this CTA's share of a tile and writes them.  A unit is four output columns of a token; the
 // units are dealt out over the CTAs of the cluster, then over the threads, and TB units x S copies of independent loads are
 // in flight per thread.  `n_first`: first output column of the tile.
-// All threads of the CTA call `read_done` together, once, when the last copies have been read and before the last results are
-// written: the cluster barrier behind it would otherwise wait for those stores (35 x 2304 x 1536 5.4 us, 5.8 behind them).  Not so where a
-// plain launch takes several turns: inside the loop it keeps a turn's loads from being issued among the stores of the turn before
-// (250 x 8192 x 3584 20.7 us, 20.4 behind the loop; 128 x 3896 x 608 7.8 and 7.4).
+// All threads of the CTA call `read_done` together, once, when the last copies have been read (each turn waits for its loads).  Where one
+// turn reads them all that is before the results are written: the cluster barrier behind it would otherwise wait for those stores
+// (35 x 2304 x 1536 5.4 us, 5.8 behind them).  Not so where a plain or SwiGLU launch takes several turns: inside the loop it keeps a turn's
+// loads from being issued among the stores of the turn before (250 x 8192 x 3584 20.7 us, 20.4 behind the loop; 128 x 3896 x 608 7.8 and 7.4).
 template <typename T, int EPI, int S, bool PAIR, typename F>
 __device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base, int rank, int m_first, int n_first, int rows,
                                             long long pos_base, const float* scale, F read_done) {
@@ -276,7 +284,8 @@ __device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base
     int m[TB], c[TB];
 #pragma unroll
     for (int i = 0; i < TB; ++i) {
-      const int u = u0 + i * kThreadsC < u1 ? u0 + i * kThreadsC : u_first;  // past the end: re-read a live unit, result unused
+      const bool live = u0 + i * kThreadsC < u1;
+      const int u = live ? u0 + i * kThreadsC : u_first;
       m[i] = u / upt;
       c[i] = (u - m[i] * upt) * 4;
       if constexpr (EPI == kEpiRopeKv) rope[i] = rope_unit(p, m_first + m[i], n_first + c[i], pos_base);
@@ -290,7 +299,10 @@ __device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base
 #pragma unroll
       for (int h = 0; h < kParts; ++h)
 #pragma unroll
-        for (int r = 0; r < S; ++r) v[i][h][r] = ld_cluster_f4(base[r] + uint32_t(m[i] * kRowsW + h * (kRowsW / 2) + c[i]) * 4u);
+        for (int r = 0; r < S; ++r) {
+          v[i][h][r] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (live) v[i][h][r] = ld_cluster_f4(base[r] + uint32_t(m[i] * kRowsW + h * (kRowsW / 2) + c[i]) * 4u);
+        }
     }
     float4 s[TB][kParts];
 #pragma unroll
@@ -307,6 +319,10 @@ __device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base
         }
       }
     }
+#pragma unroll
+    for (int i = 0; i < TB; ++i)
+#pragma unroll
+      for (int h = 0; h < kParts; ++h) settle(s[i][h].x, p.nan, smem_base);
     if (last) read_done();
     if (p.row_ssq != nullptr) {
 #pragma unroll
@@ -343,7 +359,7 @@ __device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base
     for (int i = 0; i < TB; ++i)
       if (u0 + i * kThreadsC < u1) emit<T, EPI>(p, m_first + m[i], n_first + c[i], s[i][0], s[i][kParts - 1], rope[i]);
   };
-  if constexpr (EPI != kEpiPlain) {
+  if constexpr (EPI == kEpiRopeKv || EPI == kEpiAdd) {
     for (int turn = 0; turn < turns; ++turn) take(turn, turn + 1 == turns);
     if (turns == 0) read_done();
   } else if (turns == 1) {
@@ -657,13 +673,14 @@ cudaError_t launch_pair(const GemmArgs& a, ParamsC& p, DeviceStatus* status, cud
 
 template <typename T, int EPI>
 cudaError_t launch_epi(const GemmArgs& a, ParamsC& p, bool pair, DeviceStatus* status, cudaStream_t stream, TmapFn make_tmap) {
-  constexpr int kRes = EPI == kEpiPlain ? 3 : 0;
+  constexpr bool kBound = EPI == kEpiPlain || EPI == kEpiSwiglu;  // the others read more, of weights with at most two tiles for every SM
+  constexpr int kRes = kBound ? 3 : 0;
   if constexpr (EPI == kEpiAdd) {  // at most 128 rows, which no pair takes; a pair's second tile may lie past N, and has no sums to write
     if (pair) return cudaErrorInvalidValue;
   } else {
     if (pair) return launch_pair<T, EPI, true, 1, kRes>(a, p, status, stream, make_tmap);
   }
-  if constexpr (EPI == kEpiPlain) {
+  if constexpr (kBound) {
     if (p.per_sm > kRes)
       return p.sub == 2 ? launch_pair<T, EPI, false, 2, 4>(a, p, status, stream, make_tmap)
                         : launch_pair<T, EPI, false, 1, 4>(a, p, status, stream, make_tmap);
@@ -922,6 +939,7 @@ cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStr
   p.row_parts = a.row_parts;
   p.row_eps = a.row_eps;
   p.inv_k = 1.f / static_cast<float>(a.K);
+  p.nan = std::numeric_limits<float>::quiet_NaN();
   if (a.epilogue == kEpiRopeKv) p.rope = *static_cast<const oob_rope_args_t*>(a.epilogue_args);
   p.n_mma = pl.n_mma;
   p.nj = pl.nj;

@@ -216,6 +216,7 @@ struct AttnParams {
   int max_len, batch0;
   int splits;
   float scale_log2;
+  float nan;   // see the merge over the cluster
   bool ahead;  // the position and the keys and values before the newest may be read before the kernels this one depends on are done
 };
 
@@ -491,8 +492,13 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
         acc += f * v[r];
         l_tot += f * l[r];
       }
-      // All parts are read: the barrier need not wait for the stores of the last result.
-      if (g + S >= G) attn_cluster_arrive();
+      // All parts are read: the barrier need not wait for the stores of the last result.  A peer may end behind it, and a load from it
+      // that is still under way then faults; what makes an instruction wait for a load is its use.  No value equals the NaN, which is
+      // no constant to the compiler: the stores never happen.
+      if (g + S >= G) {
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.f32 p, %0, %2;\n\t@p st.shared.f32 [%3], %0;\n\tsetp.eq.f32 p, %1, %2;\n\t@p st.shared.f32 [%3], %1;\n\t}" ::"f"(acc), "f"(l_tot), "f"(p.nan), "r"(cm_a) : "memory");
+        attn_cluster_arrive();
+      }
       deliver(g, acc, m_tot, l_tot);
     }
     attn_cluster_wait();  // the peers have read this CTA's part
@@ -755,6 +761,7 @@ int oob_attn_decode(const oob_attn_decode_args_t* a, void* stream) {
   p.batch0 = a->batch0;
   p.splits = splits;
   p.scale_log2 = a->scale * 1.4426950408889634f;
+  p.nan = NAN;
   p.ahead = a->ahead != 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   AttnSlots slots = attn_slots();
