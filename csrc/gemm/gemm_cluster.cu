@@ -781,17 +781,22 @@ int cluster_slots(int sms, int size, int per_sm) {
 
 // Microseconds a plan takes: rounds of clusters, each as long as its K blocks at the pace of one CTA or of the tensor cores of an
 // SM (cycles a block grow with the tokens), at the memory's rate for the weights or at L2's for all operands, whichever is
-// slowest; then draining the sums, reading the other CTAs' sums, and the fixed cost of a launch.  A row of a box that starts off a
-// 128-byte line touches two (`line`), one that starts off a 32-byte sector one more of these (`sector`); the pace of one CTA with stages of
-// many tokens suffers most (`pace_sector`: 103 x 5504 x 6728 split two ways 28.2 us, three ways 21.1, which were taken for the slower).
+// slowest; then draining the sums, reading the other CTAs' sums, writing a CTA's share of C, and the fixed cost of a launch.  A
+// row of a box that starts off a 128-byte line touches two (`line`), one that starts off a 32-byte sector one more of these
+// (`sector`); the pace of one CTA with stages of many tokens suffers most (`pace_sector`: 103 x 5504 x 6728 split two ways 28.2 us,
+// three ways 21.1, which were taken for the slower).
 // The constants are fitted to timings for the choice they make, so that one need not be the rate that it stands for.  Up to 128 rows to
 // 16000 timings of every K split (1930 shapes of 3 - 128 rows, N and K of 512 - 8192): 3.3 % off the best plan on average, 4.8 % with
-// the other set.  Above, the set against which the two-SM kernel is weighed.
+// the other set.  `write`, `alone`, the paces and `pace_sector` once more to the kernel with whole loads before its last barrier: of
+// 461 shapes 1.5 % off on average, 1.8 % before; too few were split where K is short.  340 other shapes whose split this changed
+// (SwiGLU in 80) take 0.97 of the time, 124 x 1248 x 560 SwiGLU 8.2 us on two CTAs against 9.4 on one; the worst 38 x 7552 x 512, 6.2
+// against 5.3.  Above, the set against which the two-SM kernel is weighed.
 struct CostC {
-  double wide, wide_tokens, pace, pace_tokens, mma, l2, hbm, drain, reduce, round, alone, cluster, eight, split, line, sector, pace_sector;
+  double wide, wide_tokens, pace, pace_tokens, mma, l2, hbm, drain, write, reduce, round, alone, cluster, eight, split, line, sector,
+      pace_sector;
 };
-constexpr CostC kFewRows = {0.153, 0.00061, 0.17, 0.00028, 1140.0, 11.8e6, 6.4e6, 0.0117, 2.84e6, 1.85, 2.52, 3.06, 2.6, 0.105, 1.29, 1.29, 1.8};
-constexpr CostC kMoreRows = {0.165, 0.0005, 0.235, 0.0002, 1850.0, 11.5e6, 6.4e6, 0.015, 3.0e6, 2.0, 3.4, 3.8, 2.0, 0.08, 1.16, 1.45, 1.45};
+constexpr CostC kFewRows = {0.153, 0.00061, 0.18, 0.0004, 1140.0, 11.8e6, 6.4e6, 0.0117, 0.01, 2.84e6, 1.85, 3.1, 3.06, 2.6, 0.105, 1.29, 1.29, 1.6};
+constexpr CostC kMoreRows = {0.165, 0.0005, 0.235, 0.0002, 1850.0, 11.5e6, 6.4e6, 0.015, 0.0, 3.0e6, 2.0, 3.4, 3.8, 2.0, 0.08, 1.16, 1.45, 1.45};
 
 double plan_cost(int M, int N, int num_kb, int sms, RowStart start, const PlanC& pl) {
   const CostC& c = M <= kTileM ? kFewRows : kMoreRows;
@@ -808,7 +813,7 @@ double plan_cost(int M, int N, int num_kb, int sms, RowStart start, const PlanC&
   if (mma > t) t = mma;
   if (l2 > t) t = l2;
   if (hbm > t) t = hbm;
-  t += c.drain * Mp + live * Mp * kRowsW * 4.0 * (pl.S - 1) / pl.S / c.reduce;
+  t += c.drain * Mp + c.write * Mp / pl.S + live * Mp * kRowsW * 4.0 * (pl.S - 1) / pl.S / c.reduce;
   return rounds * t + (rounds - 1) * c.round + (size > 1 ? c.cluster : c.alone) + (size == 8 && Mp > 128 ? c.eight : 0.0) +
          c.split * (pl.S - 1);
 }
