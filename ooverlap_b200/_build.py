@@ -2,7 +2,9 @@
 
 Every source under ``csrc/`` is compiled with
 ``-gencode arch=compute_100a,code=sm_100a`` into ``build/obj`` and linked into
-``ooverlap_b200/lib/libooverlap_b200.so`` (plus the ``oob_topology`` CLI).  A
+``ooverlap_b200/lib/libooverlap_b200.so`` (plus the ``oob_topology`` CLI, and
+``_fast_ops.so``, the Python entries of the small ops, built against the
+installed PyTorch).  A
 stamp file holding a hash of the sources and flags makes the step a no-op when
 nothing changed, so a machine that receives the tree with the built library
 does not rebuild it.
@@ -13,10 +15,13 @@ src/CMakeLists.txt:169-683) for compute_90a only.
 from __future__ import annotations
 
 import hashlib
+import importlib.metadata
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -26,6 +31,7 @@ OBJ = ROOT / "build" / "obj"
 LIB_DIR = Path(__file__).resolve().parent / "lib"
 LIB = LIB_DIR / "libooverlap_b200.so"
 CLI = LIB_DIR / "oob_topology"
+FAST = LIB_DIR / "_fast_ops.so"
 STAMP = LIB_DIR / "build.stamp"
 
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -41,7 +47,7 @@ def _nvcc() -> str:
 
 
 def _sources() -> list[Path]:
-    srcs = sorted(p for p in CSRC.rglob("*") if p.suffix in (".cu", ".cpp") and "cli" not in p.parts)
+    srcs = sorted(p for p in CSRC.rglob("*") if p.suffix in (".cu", ".cpp") and not {"cli", "python"} & set(p.parts))
     return srcs
 
 
@@ -52,6 +58,7 @@ def _all_inputs() -> list[Path]:
 def source_hash() -> str:
     h = hashlib.sha256()
     h.update(" ".join(ARCH_FLAGS + COMMON).encode())
+    h.update(f"{importlib.metadata.version('torch')} {sys.implementation.cache_tag}".encode())
     for p in _all_inputs():
         h.update(str(p.relative_to(ROOT)).encode())
         h.update(p.read_bytes())
@@ -59,7 +66,19 @@ def source_hash() -> str:
 
 
 def is_current() -> bool:
-    return LIB.exists() and STAMP.exists() and STAMP.read_text().strip() == source_hash()
+    return LIB.exists() and FAST.exists() and STAMP.exists() and STAMP.read_text().strip() == source_hash()
+
+
+def _build_fast() -> None:
+    torch = Path(importlib.util.find_spec("torch").submodule_search_locations[0])
+    cuda = Path(_nvcc()).resolve().parent.parent
+    include = [torch / "include", torch / "include/torch/csrc/api/include", cuda / "include", sysconfig.get_paths()["include"]]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", *(f"-I{p}" for p in include),
+           str(CSRC / "python" / "fast_ops.cpp"), "-o", str(FAST), f"-L{torch / 'lib'}", f"-L{LIB_DIR}", "-ltorch_python", "-ltorch",
+           "-ltorch_cpu", "-lc10_cuda", "-lc10", "-looverlap_b200", "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed for {CSRC / 'python' / 'fast_ops.cpp'}:\n{res.stdout}\n{res.stderr}")
 
 
 def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> Path:
@@ -94,6 +113,7 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
     res = subprocess.run(cli, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"CLI link failed:\n{res.stdout}\n{res.stderr}")
+    _build_fast()
     STAMP.write_text(source_hash() + "\n")
     return LIB
 

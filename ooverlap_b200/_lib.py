@@ -12,6 +12,7 @@ Capability parity: the reference exposes its C++ through two pybind11 modules
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import struct
 import threading
 from ctypes import (POINTER, Structure, byref, c_char_p, c_float, c_int, c_int64, c_uint, c_uint64, c_void_p)
@@ -123,6 +124,7 @@ GEMM_TAIL_STATIC = bytes(GemmArgs(b_static=1))[GEMM_HEAD.size:]
 
 _lock = threading.Lock()
 _lib = None
+_fast = None
 
 
 def _declare(lib) -> None:
@@ -206,6 +208,35 @@ def lib():
                 _declare(handle)
                 _lib = handle
     return _lib
+
+
+_real_lib = lib
+
+
+class _NoFast:
+    """Answers every call with None: the Python implementation goes on."""
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
+_no_fast = _NoFast()
+
+
+def fast():
+    """The module of native Python entries (csrc/python/fast_ops.cpp).  They would pass by a stand-in for the library that has been put in
+    the place of ``lib``: then none is used."""
+    global _fast
+    if lib is not _real_lib:
+        return _no_fast
+    if _fast is None:
+        lib()
+        with _lock:
+            if _fast is None:
+                spec = importlib.util.spec_from_file_location("ooverlap_b200.lib._fast_ops", _build.FAST)
+                module = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(module)
+                _fast = module
+    return _fast
 
 
 def last_error() -> str:

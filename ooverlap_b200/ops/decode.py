@@ -14,6 +14,8 @@ from typing import Optional
 import torch
 
 from .. import _lib
+from . import solutions
+from .gemm import RowSums, _check_operands, _plain_args, _scaled_rows, _scope, _set_row_sums, gemm, gemm_plan_splits
 from ..utils.dtypes import dtype_code
 from ..utils.stream import current_stream_ptr as _stream
 
@@ -78,7 +80,10 @@ def gemm_rope_kv_write(x: torch.Tensor, wqkv: torch.Tensor, B: int, T: int, head
     done from the fp32 sums by the kernel that has them (the weight-streaming kernel, or the one that sums the splits);
     otherwise (or with ``fused=False``) the GEMM is followed by :func:`rope_kv_write`.  ``x`` may be a ``RowSums`` (see
     ``gemm_add_norm``).  Returns the rotated queries, [B*T, heads * hd]."""
-    from .gemm import RowSums, _check_operands, _plain_args, _scaled_rows, _set_row_sums, gemm, gemm_plan_splits
+    if q_out is None and fused is None and solutions.no_gemm_table():
+        done = _lib.fast().gemm_rope_kv_write(x, wqkv, B, T, heads, kv_heads, k_cache, v_cache, cos, sin, pos, batch0, _scope.static_b)
+        if done is not None:
+            return done
     sums = x
     if isinstance(x, RowSums):
         if fused is False:
@@ -139,6 +144,10 @@ def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, p
     ``cache_ready`` promises that neither the call before this one on the stream nor, in a chain of this library's kernels, one of
     those before it writes a position on the device or a key or value other than the newest of each sequence: they are then
     loaded while the kernel before still runs.  Not so behind a call that appends several tokens."""
+    if scale is None and out is None:
+        done = _lib.fast().attn_decode(q, k_cache, v_cache, pos, batch0, splits, len_bound, cache_ready)
+        if done is not None:
+            return done
     if q.dim() != 3 or q.shape[2] != 128 or not q.is_contiguous():
         raise ValueError("q must be a contiguous [B, heads, 128] tensor")
     B, H, hd = q.shape

@@ -109,6 +109,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None, *
     ``gemv`` = 1 uses the CUDA-core streaming kernel for ``M <= 4`` (a warp per weight row, no tensor cores, no
     split-K hand-off); 0 uses it where it measured faster (one row of a small or a very large weight,
     two rows of a tiny one), -1 never."""
+    if out is None and order is None and not (max_ctas or splits or pair or skinny or splitk_reduce or gemv or stream_k) \
+            and solutions.no_gemm_table():
+        done = _lib.fast().gemm(a, b, _scope.static_b)
+        if done is not None:
+            return done
     _check_operands(a, b)
     M, N = a.shape[0], b.shape[0]
     if out is None:
@@ -297,6 +302,10 @@ def gemm_swiglu(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = 
     by the stand-alone SwiGLU kernel.  ``fused=True`` insists on a problem that the tiled kernels would split over K (every
     decode-step shape) and raises otherwise.  ``a`` may be a :class:`RowSums` (see
     :func:`gemm_add_norm`)."""
+    if out is None and fused is None and not max_ctas:
+        done = _lib.fast().gemm_swiglu(a, b, _scope.static_b)
+        if done is not None:
+            return done
     from .decode import silu_mul
     sums = a
     if isinstance(a, RowSums):

@@ -60,6 +60,13 @@ def gemm_key(M: int, N: int, K: int, dtype: str) -> str:
     return f"gemm:{M}x{N}x{K}:{dtype}"
 
 
+def no_gemm_table() -> bool:
+    """Whether there is no table for :func:`lookup_gemm` to look into."""
+    if _gemm_path is None:
+        lookup_gemm(0, 0, 0, "")
+    return not _gemm_path
+
+
 def lookup_gemm(M: int, N: int, K: int, dtype: str) -> Optional[dict]:
     """The profiled configuration of a plain GEMM shape (written by ``ooverlap_b200.bench.gemm_profile``): the file
     named by ``OOB_GEMM_SOLUTIONS``, else the packaged ``policy/gemm_solutions.json``; ``OOB_GEMM_SOLUTIONS=none`` turns
