@@ -124,6 +124,13 @@ __device__ __forceinline__ void prefetch_tmap(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
 }
 
+// A box of a tensor map into L2.  Nothing waits for it, and it changes nothing that a program can see: it may be asked for before the
+// kernels that may still write the box are done.
+__device__ __forceinline__ void tma_prefetch_2d(const void* tmap, int32_t x, int32_t y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y)
+               : "memory");
+}
+
 // x is the innermost (contiguous) coordinate; x * elem_size must be a
 // multiple of 16 bytes.
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, uint64_t* bar, int32_t x,

@@ -59,6 +59,12 @@ constexpr int kMaxTileTokens = 384;          // per tile: what its fp32 sums lea
 // 64 elements, 128 tokens with 64 elements a stage 0.142).  With more tokens it would leave too few stages
 // (128 x 7168 x 8192 27.1 us with 64 elements and 27.6 with 128, 128 x 8192 x 3584 split four ways 17.6 and 22.8).
 constexpr int kWideTokens = 64;
+// The first weights of a CTA are fetched into L2 while the kernel before this one ends (0.7 us from its end to the return of the wait for
+// it, then 1.4 us to weights from memory and 0.8 to weights from L2).  All of them where K is short, 16 x 2048 x 2048 5.4 -> 4.9 us, 1 x 2048 x
+// 2048 5.2 -> 4.7, 32 x 8192 x 1024 6.6 -> 6.25; else two wide stages, 32 x 8192 x 3584 12.4 -> 12.15, 64 x 7168 x 8192 24.4 -> 24.1.  More
+// of them takes memory's time from the kernel before and gains nothing here (16 stages: 64 x 7168 x 8192 26.4); stages of many tokens gain
+// nothing from two (100 x 2048 x 2048 7.44 -> 7.6, with all eight 7.35).
+constexpr int kFetchAll = 8, kFetchSome = 2;
 constexpr int kThreadsC = 192;
 constexpr int kMaxStagesC = 12;
 constexpr int kMaxCluster = 8;               // portable cluster size
@@ -100,6 +106,7 @@ struct ParamsC {
   int row_parts;
   float row_eps, inv_k;
   float nan;  // see settle
+  int fetch;  // stages of weights that each CTA fetches into L2 before the wait for earlier kernels (see kFetchAll)
   oob_gemm_epilogue_add_t add;
 };
 
@@ -427,6 +434,19 @@ __global__ void __launch_bounds__(kThreadsC, RES)
   ptx::griddep_launch_dependents();
   // Static weights are not behind that wait: their warp fills the ring at once, and waits when it has loaded its first tile.
   bool waited = !(p.w_static && warp == 0);
+  // Other weights may still be written by the kernel before: they are fetched into L2, which keeps up with such a write, and no further.
+  if (warp == 0 && p.fetch > 0 && ptx::elect_one()) {
+    const int tile = cluster / p.m_blocks * P + member;
+    const int w_row = EPI == kEpiSwiglu ? tile * (kRowsW / 2) : tile * kRowsW;
+    const int kbe = min(kb1, kb0 + p.fetch);
+    for (int kb = kb0; kb < kbe; ++kb)
+#pragma unroll
+      for (int h = 0; h < SUB; ++h) {
+        ptx::tma_prefetch_2d(&tmap_w, (kb * SUB + h) * kTileK, w_row);
+        if constexpr (EPI == kEpiSwiglu) ptx::tma_prefetch_2d(&tmap_w, (kb * SUB + h) * kTileK, p.F + w_row);
+      }
+  }
+  __syncwarp();
   if (waited) ptx::griddep_wait();
   long long pos_base = 0;
   auto load_pos = [&]() { return p.rope.pos_dev != nullptr ? *p.rope.pos_dev : static_cast<long long>(p.rope.pos0); };
@@ -946,6 +966,8 @@ cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStr
   p.inv_k = 1.f / static_cast<float>(a.K);
   p.nan = std::numeric_limits<float>::quiet_NaN();
   if (a.epilogue == kEpiRopeKv) p.rope = *static_cast<const oob_rope_args_t*>(a.epilogue_args);
+  const int steps = (p.num_kb + pl.S - 1) / pl.S;
+  p.fetch = a.b_static ? 0 : steps <= kFetchAll ? steps : pl.sub == 2 ? kFetchSome : 0;
   p.n_mma = pl.n_mma;
   p.nj = pl.nj;
   p.Mp = pl.n_mma * pl.nj;
