@@ -163,6 +163,7 @@ constexpr int kMaxAttnCluster = 8;                 // portable cluster size
 constexpr int kAttnStages = 3;                     // tiles of K and V in flight or in use per warp (96 KiB per CTA, two per SM)
 constexpr int kWarpBufBytes = kAttnStages * 2 * kKvTileBytes;
 __host__ __device__ constexpr int attn_smem_bytes() { return kAttnWarps * kWarpBufBytes; }
+constexpr int kMergeStride = kHD + 8;              // fp32 words of a row of a warp's result: eight rows start in different banks
 constexpr int kPartialStride = kHD + 2;            // fp32 words of one partial result: 128 values, max, sum
 
 template <typename T>
@@ -235,11 +236,18 @@ __device__ __forceinline__ void attn_cluster_sync() {
 // The two halves of attn_cluster_sync.
 __device__ __forceinline__ void attn_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void attn_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ float ld_cluster_f32(uint32_t smem_addr, uint32_t rank) {
+__device__ __forceinline__ float2 ld_cluster_f2(uint32_t smem_addr, uint32_t rank) {
   uint32_t a;
-  float v;
+  float2 v;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t smem_addr, uint32_t rank) {
+  uint32_t a;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
   return v;
 }
 
@@ -249,7 +257,7 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t smem_addr, uint32_t ran
 template <typename T, int S>
 __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams p) {
   constexpr int STAGES = kAttnStages;
-  static_assert(attn_smem_bytes() >= (kAttnWarps + 1) * 16 * (kHD + 2) * 4, "merge buffers");
+  static_assert(attn_smem_bytes() >= (kAttnWarps * 16 * kMergeStride + 16 * (kHD + 2)) * 4, "merge buffers");
   extern __shared__ __align__(128) uint8_t attn_smem[];
   const int part = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -407,100 +415,107 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
     l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 1);
     l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 2);
   }
-  __syncthreads();  // all warps are done with their tile buffers: reuse shared memory for the merge
 
-  // ---- merge over the warps: [warp][16 rows][128] fp32 values, [warp][16] max, [warp][16] sum, then the CTA's result
-  // in the same form with one "warp".  A warp or CTA without keys has max = -inf and contributes nothing.
-  float* mo = reinterpret_cast<float*>(attn_smem);
-  float* mm = mo + kAttnWarps * 16 * kHD;
-  float* ml = mm + kAttnWarps * 16;
-  float* co = ml + kAttnWarps * 16;
-  float* cm = co + 16 * kHD;
-  float* cl = cm + 16;
-#pragma unroll
-  for (int nb = 0; nb < 16; ++nb) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-      if (row0 + h * 8 < G)
-        *reinterpret_cast<float2*>(&mo[(warp * 16 + row0 + h * 8) * kHD + nb * 8 + colp]) = make_float2(o[nb][2 * h], o[nb][2 * h + 1]);
-  }
+  // ---- merge over the warps.  Every warp scales its own values to the largest maximum of a head before it stores them, so that what is
+  // left is a sum.  A warp or CTA without keys has max = -inf and contributes nothing.  What bounds a short context is this tail: 3 - 4 us of
+  // 5 - 9 when one thread a dimension went through the heads one by one, 8-way bank conflicts in front (1 sequence, 500 keys
+  // 4.7 -> 4.1 us, 16 x 2000 keys 8.4 -> 7.3, 20 x 3000 keys with 16 heads 14.2 -> 11.3).
+  __shared__ float warp_max[kAttnWarps * 16], warp_sum[kAttnWarps * 16];
   if ((lane & 3) == 0) {
-    mm[warp * 16 + row0] = m_run[0];
-    mm[warp * 16 + row0 + 8] = m_run[1];
-    ml[warp * 16 + row0] = l_run[0];
-    ml[warp * 16 + row0 + 8] = l_run[1];
+    warp_max[warp * 16 + row0] = m_run[0];
+    warp_max[warp * 16 + row0 + 8] = m_run[1];
+  }
+  __syncthreads();  // all warps are done with their tile buffers: shared memory is reused from here on
+  float* mo = reinterpret_cast<float*>(attn_smem);   // [warp][16][kMergeStride]
+  float* co = mo + kAttnWarps * 16 * kMergeStride;   // the CTA's result: [16][kHD], then (max, sum) of each head
+  float* cml = co + 16 * kHD;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int row = row0 + h * 8;
+    float m_tot = warp_max[row];
+#pragma unroll
+    for (int w = 1; w < kAttnWarps; ++w) m_tot = fmaxf(m_tot, warp_max[w * 16 + row]);
+    const float f = m_run[h] == -INFINITY ? 0.f : exp2f(m_run[h] - m_tot);
+    if ((lane & 3) == 0) warp_sum[warp * 16 + row] = f * l_run[h];
+    if (row < G) {
+      float* dst = mo + (warp * 16 + row) * kMergeStride + colp;
+#pragma unroll
+      for (int nb = 0; nb < 16; ++nb) *reinterpret_cast<float2*>(dst + nb * 8) = make_float2(f * o[nb][2 * h], f * o[nb][2 * h + 1]);
+    }
   }
   __syncthreads();
-  const int d = threadIdx.x;  // 128 threads = 128 dims
-  auto deliver = [&](int g, float acc, float m_tot, float l_tot) {
+  // A unit is four dimensions of a head.
+  auto deliver = [&](int u, const float4& acc, float m_tot, float l_tot) {
+    const int g = u >> 5, d = (u & 31) * 4;
     const long long hrow = static_cast<long long>(b) * p.H + h0 + g;
     if (p.splits == 1) {
-      static_cast<T*>(p.out)[hrow * kHD + d] = to_out<T>(acc / l_tot);
+      *reinterpret_cast<uint2*>(static_cast<T*>(p.out) + hrow * kHD + d) =
+          make_uint2(Cvt<T>::pack(acc.x / l_tot, acc.y / l_tot), Cvt<T>::pack(acc.z / l_tot, acc.w / l_tot));
     } else {
       float* w = p.ws + (hrow * p.splits + part / S) * kPartialStride;
-      w[d] = acc;
-      if (d == 0) {
-        w[kHD] = m_tot;
-        w[kHD + 1] = l_tot;
-      }
+      *reinterpret_cast<float2*>(w + d) = make_float2(acc.x, acc.y);
+      *reinterpret_cast<float2*>(w + d + 2) = make_float2(acc.z, acc.w);
+      if (d == 0) *reinterpret_cast<float2*>(w + kHD) = make_float2(m_tot, l_tot);
     }
   };
-  for (int g = 0; g < G; ++g) {
-    float m_tot = -INFINITY;
+  for (int u = threadIdx.x; u < G * 32; u += kAttnThreads) {
+    const int g = u >> 5;
+    const float* src = mo + g * kMergeStride + (u & 31) * 4;
+    float4 acc = *reinterpret_cast<const float4*>(src);
+    float l_tot = warp_sum[g], m_tot = warp_max[g];
 #pragma unroll
-    for (int w = 0; w < kAttnWarps; ++w) m_tot = fmaxf(m_tot, mm[w * 16 + g]);
-    float acc = 0.f, l_tot = 0.f;
-#pragma unroll
-    for (int w = 0; w < kAttnWarps; ++w) {
-      const float mw = mm[w * 16 + g];
-      const float f = mw == -INFINITY ? 0.f : exp2f(mw - m_tot);
-      acc += f * mo[(w * 16 + g) * kHD + d];
-      l_tot += f * ml[w * 16 + g];
+    for (int w = 1; w < kAttnWarps; ++w) {
+      const float4 v = *reinterpret_cast<const float4*>(src + w * 16 * kMergeStride);
+      acc = make_float4(acc.x + v.x, acc.y + v.y, acc.z + v.z, acc.w + v.w);
+      l_tot += warp_sum[w * 16 + g];
+      m_tot = fmaxf(m_tot, warp_max[w * 16 + g]);
     }
     if constexpr (S == 1) {
-      deliver(g, acc, m_tot, l_tot);
+      deliver(u, acc, m_tot, l_tot);
     } else {
-      co[g * kHD + d] = acc;
-      if (d == 0) {
-        cm[g] = m_tot;
-        cl[g] = l_tot;
-      }
+      *reinterpret_cast<float4*>(co + u * 4) = acc;
+      if ((u & 31) == 0) *reinterpret_cast<float2*>(cml + g * 2) = make_float2(m_tot, l_tot);
     }
   }
   if constexpr (S > 1) {
-    // ---- merge over the cluster through distributed shared memory: CTA r takes query heads r, r + S, ... ----
+    // ---- merge over the cluster through distributed shared memory: the units are dealt out to its CTAs ----
     const int rank = part % S;
-    const uint32_t co_a = static_cast<uint32_t>(__cvta_generic_to_shared(co));
-    const uint32_t cm_a = static_cast<uint32_t>(__cvta_generic_to_shared(cm)), cl_a = static_cast<uint32_t>(__cvta_generic_to_shared(cl));
+    const uint32_t co_a = static_cast<uint32_t>(__cvta_generic_to_shared(co)), cml_a = static_cast<uint32_t>(__cvta_generic_to_shared(cml));
     attn_cluster_sync();
-    if (rank >= G) attn_cluster_arrive();
-    for (int g = rank; g < G; g += S) {
-      float m[S], l[S], v[S];
+    const int u1 = G * 32 * (rank + 1) / S, u_first = G * 32 * rank / S;
+    const int turns = (u1 - u_first + kAttnThreads - 1) / kAttnThreads;  // at least one: G >= 1, S <= 8
+    for (int turn = 0; turn < turns; ++turn) {
+      const int u = u_first + turn * kAttnThreads + int(threadIdx.x);
+      const bool live = u < u1;
+      float4 v[S], acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      float2 ml[S];
+      float m_tot = -INFINITY, l_tot = 0.f;
+      if (live) {
 #pragma unroll
-      for (int r = 0; r < S; ++r) {
-        m[r] = ld_cluster_f32(cm_a + g * 4, r);
-        l[r] = ld_cluster_f32(cl_a + g * 4, r);
-        v[r] = ld_cluster_f32(co_a + (g * kHD + d) * 4, r);
-      }
-      float m_tot = m[0];
+        for (int r = 0; r < S; ++r) {
+          ml[r] = ld_cluster_f2(cml_a + (u >> 5) * 8, r);
+          v[r] = ld_cluster_f4(co_a + u * 16, r);
+        }
 #pragma unroll
-      for (int r = 1; r < S; ++r) m_tot = fmaxf(m_tot, m[r]);
-      float acc = 0.f, l_tot = 0.f;
+        for (int r = 0; r < S; ++r) m_tot = fmaxf(m_tot, ml[r].x);
 #pragma unroll
-      for (int r = 0; r < S; ++r) {
-        const float f = m[r] == -INFINITY ? 0.f : exp2f(m[r] - m_tot);
-        acc += f * v[r];
-        l_tot += f * l[r];
+        for (int r = 0; r < S; ++r) {
+          const float f = ml[r].x == -INFINITY ? 0.f : exp2f(ml[r].x - m_tot);
+          acc = make_float4(acc.x + f * v[r].x, acc.y + f * v[r].y, acc.z + f * v[r].z, acc.w + f * v[r].w);
+          l_tot += f * ml[r].y;
+        }
       }
       // All parts are read: the barrier need not wait for the stores of the last result.  A peer may end behind it, and a load from it
       // that is still under way then faults; what makes an instruction wait for a load is its use.  No value equals the NaN, which is
       // no constant to the compiler: the stores never happen.
-      if (g + S >= G) {
-        asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.f32 p, %0, %2;\n\t@p st.shared.f32 [%3], %0;\n\tsetp.eq.f32 p, %1, %2;\n\t@p st.shared.f32 [%3], %1;\n\t}" ::"f"(acc), "f"(l_tot), "f"(p.nan), "r"(cm_a) : "memory");
+      if (turn + 1 == turns) {
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.f32 p, %0, %2;\n\t@p st.shared.f32 [%3], %0;\n\tsetp.eq.f32 p, %1, %2;\n\t@p st.shared.f32 [%3], %1;\n\t}" ::"f"(acc.x), "f"(l_tot), "f"(p.nan), "r"(cml_a) : "memory");
+        __syncwarp();
         attn_cluster_arrive();
       }
-      deliver(g, acc, m_tot, l_tot);
+      if (live) deliver(u, acc, m_tot, l_tot);
     }
+    __syncwarp();
     attn_cluster_wait();  // the peers have read this CTA's part
   }
 }
