@@ -161,9 +161,13 @@ constexpr int kRowBytes = kHD * 2;                 // 256
 constexpr int kKvTileBytes = kTileKeys * kRowBytes;  // 4 KiB
 constexpr int kMaxAttnCluster = 8;                 // portable cluster size
 constexpr int kAttnStages = 3;                     // tiles of K and V in flight or in use per warp (96 KiB per CTA, two per SM)
-constexpr int kWarpBufBytes = kAttnStages * 2 * kKvTileBytes;
-__host__ __device__ constexpr int attn_smem_bytes() { return kAttnWarps * kWarpBufBytes; }
-constexpr int kMergeStride = kHD + 8;              // fp32 words of a row of a warp's result: eight rows start in different banks
+// Where no SM gets two CTAs anyway, and CTAs alone or in pairs (64 x 300 keys 5.5 -> 5.15 us; clusters of eight gain nothing, fewer of
+// them fit the device, and they start later: 1 x 4000 keys 6.9 and 7.15).
+constexpr int kAttnDeepStages = 6;
+__host__ __device__ constexpr int attn_warp_bytes(int stages) { return stages * 2 * kKvTileBytes; }
+__host__ __device__ constexpr int attn_smem_bytes(int stages) { return kAttnWarps * attn_warp_bytes(stages); }
+// fp32 words of a head's row of a warp's result: the rows that are stored together start in different banks.
+__host__ __device__ constexpr int merge_stride(bool few) { return few ? kHD + 4 : kHD + 8; }
 constexpr int kPartialStride = kHD + 2;            // fp32 words of one partial result: 128 values, max, sum
 
 template <typename T>
@@ -191,6 +195,12 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t add
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(addr));
+}
+// Rows and columns of an 8 x 8 matrix of 16-bit values change places.
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t a) {
+  uint32_t d;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
+  return d;
 }
 __device__ __forceinline__ void cp_async_16(uint32_t smem_addr, const void* gptr) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr), "l"(gptr) : "memory");
@@ -254,11 +264,20 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t smem_addr, uint32_t ran
 // Grid: (splits * S, KV, B) in clusters of S along x.  The keys of one (sequence, KV head) are dealt out in 16-key tiles
 // to the splits * S CTAs from the length the kernel finds on the device, so that a cache that is mostly empty, or a
 // length just past a multiple of anything, leaves no CTA with more than one tile per warp over its share.
-template <typename T, int S>
+//
+// What bounds a warp is the chain of a tile: with eight tiles a warp and nothing else on its SM a tile of 16 keys took 0.53 us, as long as with
+// twice as many loads in flight.  So all fragments of a tile are read before the first instruction that needs one, and the maximum
+// over the warp is taken, and values rescaled, only for a tile that has a new one.  FEW, up to eight heads a KV head: the keys are the 16
+// rows of the instruction and the heads its eight columns, half the instructions, exponentials and accumulators of the layout with
+// heads as rows, of which half would be zero; the probabilities are transposed in registers.  Microseconds before, after: 1 x 4000 keys
+// 7.65, 7.25; 16 x 2000 7.3, 6.9; 64 x 300 6.0, 5.2; 2 x 8000 with 8 KV heads 15.9, 14.9; 256 x 1900 41.5, 40.9; 16 heads a KV head,
+// 20 x 3000 11.35, 11.2.  (A maximum raised only by scores that exceed it by eight was another 2 % faster, and 10 % further from 64-bit
+// results: the largest probabilities are then no longer exactly one.)
+template <typename T, int S, int STAGES, bool FEW>
 __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams p) {
-  constexpr int STAGES = kAttnStages;
-  static_assert(attn_smem_bytes() >= (kAttnWarps * 16 * kMergeStride + 16 * (kHD + 2)) * 4, "merge buffers");
+  static_assert(attn_smem_bytes(STAGES) >= (kAttnWarps * 16 * merge_stride(FEW) + 16 * (kHD + 2)) * 4, "merge buffers");
   extern __shared__ __align__(128) uint8_t attn_smem[];
+  constexpr int kMergeStride = merge_stride(FEW);
   const int part = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = p.G;
@@ -274,7 +293,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
 
   const T* kbase = static_cast<const T*>(p.k) + (p.batch0 + b) * p.batch_stride + static_cast<long long>(kvh) * p.max_len * kHD;
   const T* vbase = static_cast<const T*>(p.v) + (p.batch0 + b) * p.batch_stride + static_cast<long long>(kvh) * p.max_len * kHD;
-  const uint32_t wbuf_u32 = static_cast<uint32_t>(__cvta_generic_to_shared(attn_smem + warp * kWarpBufBytes));
+  const uint32_t wbuf_u32 = static_cast<uint32_t>(__cvta_generic_to_shared(attn_smem + warp * attn_warp_bytes(STAGES)));
   // The warps take the CTA's tiles in turn.
   const int my_tiles = t1 - t0 > warp ? (t1 - t0 - warp + kAttnWarps - 1) / kAttnWarps : 0;
 
@@ -290,9 +309,10 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
     }
   };
 
-  float o[16][4];
+  constexpr int kAcc = FEW ? 8 : 16;
+  float o[kAcc][4];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+  for (int i = 0; i < kAcc; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
 
   // One commit group per tile slot, empty when there is no tile: the group count is then the same for every warp
@@ -312,10 +332,17 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
   }
   if (!waited) ptx::griddep_wait();
 
-  // ---- Q fragments (A operand, 16 x 128; rows >= G are zero) ----
+  // ---- Q fragments (16 x 128, the A operand; FEW: 128 x 8, the B operand; heads >= G are zero) ----
   const int row0 = lane >> 2, colp = (lane & 3) * 2;
-  uint32_t qa[8][4];
-  {
+  uint32_t qa[8][FEW ? 2 : 4];
+  if constexpr (FEW) {
+    const T* qb = static_cast<const T*>(p.q) + (static_cast<long long>(b) * p.H + h0) * kHD;
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+      qa[ks][0] = row0 < G ? *reinterpret_cast<const uint32_t*>(qb + row0 * kHD + ks * 16 + colp) : 0u;
+      qa[ks][1] = row0 < G ? *reinterpret_cast<const uint32_t*>(qb + row0 * kHD + ks * 16 + colp + 8) : 0u;
+    }
+  } else {
     const T* qb = static_cast<const T*>(p.q) + (static_cast<long long>(b) * p.H + h0) * kHD;
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
@@ -337,22 +364,75 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
     const uint32_t ks = wbuf_u32 + stage * 2 * kKvTileBytes, vs = ks + kKvTileBytes;
     if (++stage == STAGES) stage = 0;
 
+    if constexpr (FEW) {
+      // ---- S^T = K Q^T: 16 keys x 8 heads, in two sums (each instruction waits for the one before it) ----
+      float sa[4] = {0.f, 0.f, 0.f, 0.f}, sb[4] = {0.f, 0.f, 0.f, 0.f};
+      const int mat = lane >> 3;
+      uint32_t kf[8][4], vf[8][4];
+#pragma unroll
+      for (int kp = 0; kp < 8; ++kp) ldmatrix_x4(kf[kp], ks + kv_off((mat & 1) * 8 + (lane & 7), kp * 2 + (mat >> 1)));
+#pragma unroll
+      for (int dt = 0; dt < 8; ++dt) ldmatrix_x4_trans(vf[dt], vs + kv_off((mat >> 1) * 8 + (lane & 7), dt * 2 + (mat & 1)));
+#pragma unroll
+      for (int kp = 0; kp < 8; kp += 2) {
+        mma_16816<T>(sa, kf[kp], qa[kp][0], qa[kp][1]);
+        mma_16816<T>(sb, kf[kp + 1], qa[kp + 1][0], qa[kp + 1][1]);
+      }
+      // ---- mask, online softmax: a thread has keys row0 and row0 + 8 of heads colp and colp + 1 ----
+      float s[4], m_use[2];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[e] = key0 + row0 + (e >> 1) * 8 < L ? (sa[e] + sb[e]) * p.scale_log2 : -INFINITY;
+      if (__any_sync(0xffffffffu, fmaxf(s[0], s[2]) > m_run[0] || fmaxf(s[1], s[3]) > m_run[1])) {
+        float tmax[2] = {fmaxf(s[0], s[2]), fmaxf(s[1], s[3])}, corr[2];
+#pragma unroll
+        for (int x = 4; x < 32; x <<= 1)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) tmax[h] = fmaxf(tmax[h], __shfl_xor_sync(0xffffffffu, tmax[h], x));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float m_new = fmaxf(m_run[h], tmax[h]);
+          corr[h] = exp2f(m_run[h] - (m_new == -INFINITY ? 0.f : m_new));  // 0 when nothing has been seen yet
+          m_run[h] = m_new;
+          l_run[h] *= corr[h];
+        }
+#pragma unroll
+        for (int i2 = 0; i2 < kAcc; ++i2) {
+          o[i2][0] *= corr[0];
+          o[i2][1] *= corr[1];
+          o[i2][2] *= corr[0];
+          o[i2][3] *= corr[1];
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        m_use[h] = m_run[h] == -INFINITY ? 0.f : m_run[h];
+        s[h] = exp2f(s[h] - m_use[h]);
+        s[h + 2] = exp2f(s[h + 2] - m_use[h]);
+        l_run[h] += s[h] + s[h + 2];
+      }
+      // ---- O^T += V^T P^T ----
+      const uint32_t p0 = transpose_8x8(Cvt<T>::pack(s[0], s[1])), p1 = transpose_8x8(Cvt<T>::pack(s[2], s[3]));
+#pragma unroll
+      for (int dt = 0; dt < 8; ++dt) mma_16816<T>(o[dt], vf[dt], p0, p1);
+    } else {
     // ---- S = Q K^T for 16 keys ----
     float s[2][4];
 #pragma unroll
     for (int nb = 0; nb < 2; ++nb) s[nb][0] = s[nb][1] = s[nb][2] = s[nb][3] = 0.f;
+    uint32_t f[8][4];
+#pragma unroll
+    for (int i2 = 0; i2 < 8; ++i2) ldmatrix_x4(f[i2], ks + kv_off((i2 & 1) * 8 + (lane & 7), (i2 >> 1) * 4 + (lane >> 3)));
 #pragma unroll
     for (int kp = 0; kp < 4; ++kp) {
 #pragma unroll
-      for (int nb = 0; nb < 2; ++nb) {
-        uint32_t r[4];
-        ldmatrix_x4(r, ks + kv_off(nb * 8 + (lane & 7), kp * 4 + (lane >> 3)));
-        mma_16816<T>(s[nb], qa[2 * kp], r[0], r[1]);
-        mma_16816<T>(s[nb], qa[2 * kp + 1], r[2], r[3]);
-      }
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb) mma_16816<T>(s[nb], qa[2 * kp + h], f[kp * 2 + nb][h * 2], f[kp * 2 + nb][h * 2 + 1]);
     }
+#pragma unroll
+    for (int dp = 0; dp < 8; ++dp) ldmatrix_x4_trans(f[dp], vs + kv_off(((lane >> 3) & 1) * 8 + (lane & 7), dp * 2 + (lane >> 4)));
     // ---- mask, online softmax ----
-    float tmax[2] = {-INFINITY, -INFINITY};
+    float tmax[2] = {-INFINITY, -INFINITY}, m_use[2];
 #pragma unroll
     for (int nb = 0; nb < 2; ++nb) {
 #pragma unroll
@@ -363,17 +443,27 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
         tmax[e >> 1] = fmaxf(tmax[e >> 1], v);
       }
     }
-    float corr[2], m_use[2];
+    if (__any_sync(0xffffffffu, tmax[0] > m_run[0] || tmax[1] > m_run[1])) {
+      float corr[2];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      tmax[h] = fmaxf(tmax[h], __shfl_xor_sync(0xffffffffu, tmax[h], 1));
-      tmax[h] = fmaxf(tmax[h], __shfl_xor_sync(0xffffffffu, tmax[h], 2));
-      const float m_new = fmaxf(m_run[h], tmax[h]);
-      m_use[h] = m_new == -INFINITY ? 0.f : m_new;
-      corr[h] = exp2f(m_run[h] - m_use[h]);  // 0 when nothing has been seen yet
-      m_run[h] = m_new;
-      l_run[h] *= corr[h];
+      for (int h = 0; h < 2; ++h) {
+        tmax[h] = fmaxf(tmax[h], __shfl_xor_sync(0xffffffffu, tmax[h], 1));
+        tmax[h] = fmaxf(tmax[h], __shfl_xor_sync(0xffffffffu, tmax[h], 2));
+        const float m_new = fmaxf(m_run[h], tmax[h]);
+        corr[h] = exp2f(m_run[h] - (m_new == -INFINITY ? 0.f : m_new));  // 0 when nothing has been seen yet
+        m_run[h] = m_new;
+        l_run[h] *= corr[h];
+      }
+#pragma unroll
+      for (int i2 = 0; i2 < kAcc; ++i2) {
+        o[i2][0] *= corr[0];
+        o[i2][1] *= corr[0];
+        o[i2][2] *= corr[1];
+        o[i2][3] *= corr[1];
+      }
     }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) m_use[h] = m_run[h] == -INFINITY ? 0.f : m_run[h];
 #pragma unroll
     for (int nb = 0; nb < 2; ++nb) {
 #pragma unroll
@@ -381,16 +471,6 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
         const float pv = exp2f(s[nb][e] - m_use[e >> 1]);
         s[nb][e] = pv;
         l_run[e >> 1] += pv;
-      }
-    }
-    // After the first few tiles a new maximum is rare: the 64 products are skipped when every factor is one.
-    if (__any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f)) {
-#pragma unroll
-      for (int i2 = 0; i2 < 16; ++i2) {
-        o[i2][0] *= corr[0];
-        o[i2][1] *= corr[0];
-        o[i2][2] *= corr[1];
-        o[i2][3] *= corr[1];
       }
     }
     // ---- O += P V ----
@@ -401,29 +481,29 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
     pa[3] = Cvt<T>::pack(s[1][2], s[1][3]);
 #pragma unroll
     for (int dp = 0; dp < 8; ++dp) {
-      uint32_t r[4];
-      const int j = lane >> 3;
-      ldmatrix_x4_trans(r, vs + kv_off((j & 1) * 8 + (lane & 7), dp * 2 + (j >> 1)));
-      mma_16816<T>(o[2 * dp], pa, r[0], r[1]);
-      mma_16816<T>(o[2 * dp + 1], pa, r[2], r[3]);
+      mma_16816<T>(o[2 * dp], pa, f[dp][0], f[dp][1]);
+      mma_16816<T>(o[2 * dp + 1], pa, f[dp][2], f[dp][3]);
+    }
     }
     __syncwarp();  // every lane is done with this stage before the next iteration's copies overwrite it
   }
   cp_async_wait<0>();
+  // A thread's two heads, and whether it speaks for them.
+  const int head0 = FEW ? colp : row0, head_step = FEW ? 1 : 8;
+  const bool speaks = FEW ? lane < 4 : (lane & 3) == 0;
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 1);
-    l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 2);
-  }
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int x = FEW ? 4 : 1; x < (FEW ? 32 : 4); x <<= 1) l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], x);
 
   // ---- merge over the warps.  Every warp scales its own values to the largest maximum of a head before it stores them, so that what is
   // left is a sum.  A warp or CTA without keys has max = -inf and contributes nothing.  What bounds a short context is this tail: 3 - 4 us of
   // 5 - 9 when one thread a dimension went through the heads one by one, 8-way bank conflicts in front (1 sequence, 500 keys
   // 4.7 -> 4.1 us, 16 x 2000 keys 8.4 -> 7.3, 20 x 3000 keys with 16 heads 14.2 -> 11.3).
   __shared__ float warp_max[kAttnWarps * 16], warp_sum[kAttnWarps * 16];
-  if ((lane & 3) == 0) {
-    warp_max[warp * 16 + row0] = m_run[0];
-    warp_max[warp * 16 + row0 + 8] = m_run[1];
+  if (speaks) {
+    warp_max[warp * 16 + head0] = m_run[0];
+    warp_max[warp * 16 + head0 + head_step] = m_run[1];
   }
   __syncthreads();  // all warps are done with their tile buffers: shared memory is reused from here on
   float* mo = reinterpret_cast<float*>(attn_smem);   // [warp][16][kMergeStride]
@@ -431,13 +511,22 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
   float* cml = co + 16 * kHD;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    const int row = row0 + h * 8;
+    const int row = head0 + h * head_step;
     float m_tot = warp_max[row];
 #pragma unroll
     for (int w = 1; w < kAttnWarps; ++w) m_tot = fmaxf(m_tot, warp_max[w * 16 + row]);
     const float f = m_run[h] == -INFINITY ? 0.f : exp2f(m_run[h] - m_tot);
-    if ((lane & 3) == 0) warp_sum[warp * 16 + row] = f * l_run[h];
-    if (row < G) {
+    if (speaks) warp_sum[warp * 16 + row] = f * l_run[h];
+    if constexpr (FEW) {
+      if (row < G) {
+        float* dst = mo + (warp * 16 + row) * kMergeStride + row0;
+#pragma unroll
+        for (int dt = 0; dt < 8; ++dt) {
+          dst[dt * 16] = f * o[dt][h];
+          dst[dt * 16 + 8] = f * o[dt][h + 2];
+        }
+      }
+    } else if (row < G) {
       float* dst = mo + (warp * 16 + row) * kMergeStride + colp;
 #pragma unroll
       for (int nb = 0; nb < 16; ++nb) *reinterpret_cast<float2*>(dst + nb * 8) = make_float2(f * o[nb][2 * h], f * o[nb][2 * h + 1]);
@@ -541,29 +630,33 @@ __global__ void attn_combine_kernel(const float* ws, void* out, int splits) {
   static_cast<T*>(out)[hrow * kHD + d] = to_out<T>(acc / l_tot);
 }
 
-template <typename T, int S>
+template <typename T, int S, int STAGES, bool FEW>
 cudaError_t launch_attn_s(const AttnParams& p, cudaStream_t stream) {
   static std::atomic<uint64_t> attr_done{0};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!(attr_done.load(std::memory_order_relaxed) >> (dev & 63) & 1)) {
-    cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         attn_smem_bytes());
+    cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<T, S, STAGES, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         attn_smem_bytes(STAGES));
     if (e != cudaSuccess) return e;
     attr_done.fetch_or(uint64_t(1) << (dev & 63), std::memory_order_relaxed);
   }
-  return launch_pdl(attn_decode_kernel<T, S>, dim3(p.splits * S, p.KV, p.B), kAttnThreads, attn_smem_bytes(), stream, S, p);
+  return launch_pdl(attn_decode_kernel<T, S, STAGES, FEW>, dim3(p.splits * S, p.KV, p.B), kAttnThreads, attn_smem_bytes(STAGES), stream, S, p);
 }
 
 template <typename T>
-cudaError_t launch_attn(const AttnParams& p, int cluster, cudaStream_t stream) {
-  cudaError_t e;
-  switch (cluster) {
-    case 1: e = launch_attn_s<T, 1>(p, stream); break;
-    case 2: e = launch_attn_s<T, 2>(p, stream); break;
-    case 4: e = launch_attn_s<T, 4>(p, stream); break;
-    default: e = launch_attn_s<T, 8>(p, stream); break;
-  }
+cudaError_t launch_attn(const AttnParams& p, int cluster, bool deep, cudaStream_t stream) {
+  constexpr int A = kAttnStages, D = kAttnDeepStages;
+  auto size = [&](auto few) {
+    constexpr bool F = decltype(few)::value;
+    switch (cluster) {
+      case 1: return deep ? launch_attn_s<T, 1, D, F>(p, stream) : launch_attn_s<T, 1, A, F>(p, stream);
+      case 2: return deep ? launch_attn_s<T, 2, D, F>(p, stream) : launch_attn_s<T, 2, A, F>(p, stream);
+      case 4: return launch_attn_s<T, 4, A, F>(p, stream);
+      default: return launch_attn_s<T, 8, A, F>(p, stream);
+    }
+  };
+  cudaError_t e = p.G <= 8 ? size(std::true_type{}) : size(std::false_type{});
   if (e != cudaSuccess) return e;
   if (p.splits > 1) e = launch_pdl(attn_combine_kernel<T>, dim3(p.B * p.H), kHD, 0, stream, 1, p.ws, p.out, p.splits);
   return e;
@@ -573,18 +666,19 @@ cudaError_t launch_attn(const AttnParams& p, int cluster, cudaStream_t stream) {
 // may differ from one GPU to the next: the device is asked.
 struct AttnSlots {
   int n[4];
+  int deep[2];  // of the kernel with kAttnDeepStages, alone and in pairs
 };
 
-template <typename T, int S>
+template <typename T, int S, int STAGES, bool FEW = true>
 int attn_slots_of() {
-  if (cudaFuncSetAttribute(attn_decode_kernel<T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem_bytes()) != cudaSuccess) {
+  if (cudaFuncSetAttribute(attn_decode_kernel<T, S, STAGES, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem_bytes(STAGES)) != cudaSuccess) {
     (void)cudaGetLastError();
     return 0;
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(S * 2 * 148);
   cfg.blockDim = dim3(kAttnThreads);
-  cfg.dynamicSmemBytes = attn_smem_bytes();
+  cfg.dynamicSmemBytes = attn_smem_bytes(STAGES);
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = S;
@@ -593,7 +687,7 @@ int attn_slots_of() {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, attn_decode_kernel<T, S>, &cfg) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&clusters, attn_decode_kernel<T, S, STAGES, FEW>, &cfg) != cudaSuccess) {
     (void)cudaGetLastError();
     return 0;
   }
@@ -611,9 +705,11 @@ AttnSlots attn_slots() {
   AttnSlots& s = cached[dev & 63];
   if (!have[dev & 63]) {
     s.n[0] = 2 * 148;
-    s.n[1] = attn_slots_of<__nv_bfloat16, 2>();
-    s.n[2] = attn_slots_of<__nv_bfloat16, 4>();
-    s.n[3] = attn_slots_of<__nv_bfloat16, 8>();
+    s.n[1] = attn_slots_of<__nv_bfloat16, 2, kAttnStages>();
+    s.n[2] = attn_slots_of<__nv_bfloat16, 4, kAttnStages>();
+    s.n[3] = attn_slots_of<__nv_bfloat16, 8, kAttnStages>();
+    s.deep[0] = 148;
+    s.deep[1] = attn_slots_of<__nv_bfloat16, 2, kAttnDeepStages>();
     have[dev & 63] = true;
   }
   return s;
@@ -784,7 +880,8 @@ int oob_attn_decode(const oob_attn_decode_args_t* a, void* stream) {
   // the GPU then wait for the last ones (2 x 30000 keys on 8 KV heads 48 - 55 us in eights, 45 in fours; alone both 44).
   if (splits > 1) slots.n[3] -= slots.n[3] / 4;
   const int cluster = attn_cluster_size(static_cast<long long>(a->B) * a->KV * splits, (bound + splits - 1) / splits, slots);
-  cudaError_t e = a->dtype == OOB_BF16 ? launch_attn<__nv_bfloat16>(p, cluster, s) : launch_attn<__half>(p, cluster, s);
+  const bool deep = cluster <= 2 && static_cast<long long>(a->B) * a->KV * splits * cluster <= slots.deep[cluster - 1];
+  cudaError_t e = a->dtype == OOB_BF16 ? launch_attn<__nv_bfloat16>(p, cluster, deep, s) : launch_attn<__half>(p, cluster, deep, s);
   if (e != cudaSuccess) return cuda_fail(e, "attn_decode launch");
   return OOB_OK;
 }
