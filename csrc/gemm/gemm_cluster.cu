@@ -37,6 +37,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <limits>
 #include <type_traits>
@@ -67,6 +68,7 @@ constexpr int kWideTokens = 64;
 constexpr int kFetchAll = 8, kFetchSome = 2;
 constexpr int kThreadsC = 192;
 constexpr int kMaxStagesC = 12;
+constexpr int kSpreadRows = 32;              // rows, from which on a block of so many tokens is weighed
 constexpr int kMaxCluster = 8;               // portable cluster size
 constexpr int kMaxScaledRows = 128;           // rows that may carry a sum of squares (ParamsC::row_ssq)
 constexpr int kCtlBytes = 256 + kMaxScaledRows * 4;
@@ -791,9 +793,43 @@ bool size_cta(int N, int num_kb, int sms, PlanC* pl) {
   return false;
 }
 
-// Clusters of `size` CTAs that run at once with `per_sm` CTAs on an SM.  A cluster lives in one GPC (about 18 SMs on this
-// part, some have fewer).
-int cluster_slots(int sms, int size, int per_sm) {
+// Clusters of `size` CTAs that run at once with `per_sm` CTAs on an SM.  A cluster lives in one GPC (about 18 SMs on this part, some have
+// fewer, and not the same on every GPU): the device is asked, and its answers are kept.  One cluster too many is a second round of them
+// (SwiGLU 116 x 1024 x 5624 on 16 clusters of seven, of which 15 run at once: 17.9 us, 11.0).  Without a device, one B200's answers.
+int device_slots(int size, int per_sm) {
+  static const int b200[4][9] = {{0, 148, 74, 45, 33, 26, 22, 15, 15}, {0, 296, 148, 93, 71, 56, 45, 37, 33},
+                                 {0, 444, 222, 142, 104, 82, 71, 56, 48}, {0, 592, 296, 187, 142, 112, 93, 78, 71}};
+  static std::atomic<int> cached[64][4][9];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return b200[per_sm - 1][size];
+  }
+  std::atomic<int>& slot = cached[dev & 63][per_sm - 1][size];
+  int n = slot.load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  auto kernel = gemm_cluster_kernel<__nv_bfloat16, kEpiPlain, false, 1, 4>;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(size * 1024);
+  cfg.blockDim = dim3(kThreadsC);
+  cfg.dynamicSmemBytes = per_sm == 1 ? kSmemLimit : 228 * 1024 / per_sm - 1024;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = size;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+    (void)cudaGetLastError();
+    return b200[per_sm - 1][size];
+  }
+  slot.store(n, std::memory_order_relaxed);
+  return n;
+}
+// What the plans of few rows were fitted with.
+int rough_slots(int sms, int size, int per_sm) {
   if (size <= 2) return sms * per_sm / size;
   if (size > 4 && per_sm == 1) return size == 8 ? 12 : 16;
   return 8 * (18 * per_sm / size);
@@ -805,23 +841,28 @@ int cluster_slots(int sms, int size, int per_sm) {
 // row of a box that starts off a 128-byte line touches two (`line`), one that starts off a 32-byte sector one more of these
 // (`sector`); the pace of one CTA with stages of many tokens suffers most (`pace_sector`: 103 x 5504 x 6728 split two ways 28.2 us,
 // three ways 21.1, which were taken for the slower).
-// The constants are fitted to timings for the choice they make, so that one need not be the rate that it stands for.  Up to 128 rows to
-// 16000 timings of every K split (1930 shapes of 3 - 128 rows, N and K of 512 - 8192): 3.3 % off the best plan on average, 4.8 % with
-// the other set.  `write`, `alone`, the paces and `pace_sector` once more to the kernel with whole loads before its last barrier: of
-// 461 shapes 1.5 % off on average, 1.8 % before; too few were split where K is short.  340 other shapes whose split this changed
-// (SwiGLU in 80) take 0.97 of the time, 124 x 1248 x 560 SwiGLU 8.2 us on two CTAs against 9.4 on one; the worst 38 x 7552 x 512, 6.2
-// against 5.3.  Above, the set against which the two-SM kernel is weighed.
+// The constants are fitted to timings for the choice they make, so that one need not be the rate that it stands for.  Few rows (one token
+// block): 16000 timings of every K split (1930 shapes of 3 - 128 rows, N and K of 512 - 8192), 3.3 % off the best plan on average; `write`,
+// `alone`, the paces and `pace_sector` once more to 461 shapes.  Some and more rows, where blocks of fewer tokens than 128 are weighed too: 1223
+// shapes of 33 - 128 and 867 of 129 - 1500 rows, every block count and split.  The choice is 2.3 % off the best plan there (8 % with blocks
+// of 128 tokens only: 128 x 4096 x 4096 12.3 us, 11.75 in two blocks and two splits) and 2.6 % off the best of both kernels (8.1 %: 256 x
+// 4096 x 4096 17.0, 13.2; 1500 x 1000 x 4000 17.2, 16.2).
 struct CostC {
-  double wide, wide_tokens, pace, pace_tokens, mma, l2, hbm, drain, write, reduce, round, alone, cluster, eight, split, line, sector,
+  double wide, wide_tokens, pace, pace_tokens, mma, l2, hbm, drain, write, reduce, round, alone, cluster, eight, split, five, line, sector,
       pace_sector;
 };
-constexpr CostC kFewRows = {0.153, 0.00061, 0.18, 0.0004, 1140.0, 11.8e6, 6.4e6, 0.0117, 0.01, 2.84e6, 1.85, 3.1, 3.06, 2.6, 0.105, 1.29, 1.29, 1.6};
-constexpr CostC kMoreRows = {0.165, 0.0005, 0.235, 0.0002, 1850.0, 11.5e6, 6.4e6, 0.015, 0.0, 3.0e6, 2.0, 3.4, 3.8, 2.0, 0.08, 1.16, 1.45, 1.45};
+constexpr CostC kFewRows = {0.153, 0.00061, 0.18, 0.0004, 1140.0, 11.8e6, 6.4e6, 0.0117, 0.01, 2.84e6, 1.85, 3.1, 3.06, 2.6, 0.105, 0.0, 1.29, 1.29, 1.6};
+constexpr CostC kSomeRows = {0.2026, 0.00328, 0.0705, 0.00486, 1e9, 6.11e6, 67e6, 0.00018, 0.0176, 0.537e6, 0.478, 1.093, 1.525, 42.0, 0.0036, 0.376, 1.854, 3.133, 3.016};
+constexpr CostC kMoreRows = {0.0121, 0.00226, 0.1137, 0.000385, 2164.0, 19.1e6, 1e9, 0.000434, 0.025, 1.87e6, 3.86, 1.539, 1.881, 0.01, 0.0878, 0.04, 1.246, 1.95, 1.866};
 
-double plan_cost(int M, int N, int num_kb, int sms, RowStart start, const PlanC& pl) {
-  const CostC& c = M <= kTileM ? kFewRows : kMoreRows;
+// Blocks of fewer tokens than 128 are weighed where more than 32 rows may be cut: row sums and the Add epilogue need one block, and static
+// weights of few rows are planned for what their rings hold.
+bool spread_rows(int M, bool ahead, bool one_block) { return M > kSpreadRows && !one_block && (M > kTileM || !ahead); }
+
+double plan_cost(int M, int N, int num_kb, int sms, RowStart start, bool spread, const PlanC& pl) {
+  const CostC& c = M > kTileM ? kMoreRows : spread ? kSomeRows : kFewRows;
   const int P = pl.pair ? 2 : 1, Mp = pl.n_mma * pl.nj, size = P * pl.S;
-  const int clusters = tile_count(N, pl), slots = cluster_slots(sms, size, pl.per_sm);
+  const int clusters = tile_count(N, pl), slots = &c == &kFewRows ? rough_slots(sms, size, pl.per_sm) : device_slots(size, pl.per_sm);
   const int rounds = (clusters + slots - 1) / slots;
   const double live = double(clusters < slots ? clusters : slots) * size;  // CTAs at once
   const double share = live > sms ? live / sms : 1.0;
@@ -835,24 +876,26 @@ double plan_cost(int M, int N, int num_kb, int sms, RowStart start, const PlanC&
   if (hbm > t) t = hbm;
   t += c.drain * Mp + c.write * Mp / pl.S + live * Mp * kRowsW * 4.0 * (pl.S - 1) / pl.S / c.reduce;
   return rounds * t + (rounds - 1) * c.round + (size > 1 ? c.cluster : c.alone) + (size == 8 && Mp > 128 ? c.eight : 0.0) +
-         c.split * (pl.S - 1);
+         c.split * (pl.S - 1) + (pl.S >= 5 ? c.five : 0.0);
 }
 
 // What static weights save: the rings are filled while the kernel before ends.  Plans with more CTAs hold more (32 x 8192 x 3584 in a
 // decode step 13.3 us on 128 CTAs, 14.3 on 64, which were taken for faster).
 double ring_us(int N, int num_kb, int sms, const PlanC& pl) {
-  const int clusters = tile_count(N, pl), size = (pl.pair ? 2 : 1) * pl.S, slots = cluster_slots(sms, size, pl.per_sm);
+  const int clusters = tile_count(N, pl), size = (pl.pair ? 2 : 1) * pl.S, slots = rough_slots(sms, size, pl.per_sm);
   const double live = double(clusters < slots ? clusters : slots) * size;
   return live * pl.stages * pl.sub * kRowsW * kRowBytes / 6.05e6;
 }
 
 // The cheapest cut of a problem.  `fix_s` > 0 fixes the K split, `pair` is as in GemmArgs; `ahead`: static weights.
-bool plan(int M, int N, int K, int sms, int pair, int fix_s, bool ahead, PlanC* out, double* cost) {
+bool plan(int M, int N, int K, int sms, int pair, int fix_s, bool ahead, bool spread, PlanC* out, double* cost) {
   const int num_kb = (K + kTileK - 1) / kTileK;
   if (N <= kRowsW) pair = -1;  // one weight tile is no pair
   bool found = false;
   int last = 0;
-  for (int blocks = (M + kMaxTileTokens - 1) / kMaxTileTokens; blocks <= (M + 127) / 128; ++blocks) {
+  int most_blocks = (M + 127) / 128;
+  if (spread) most_blocks = std::max(most_blocks, std::min((M + kSpreadRows - 1) / kSpreadRows, 10));
+  for (int blocks = (M + kMaxTileTokens - 1) / kMaxTileTokens; blocks <= most_blocks; ++blocks) {
     PlanC pl{};
     token_tile(M, blocks, &pl);
     const int Mp = pl.n_mma * pl.nj;
@@ -865,8 +908,7 @@ bool plan(int M, int N, int K, int sms, int pair, int fix_s, bool ahead, PlanC* 
       for (pl.S = 1; pl.S <= kMaxCluster / (two ? 2 : 1); ++pl.S) {
         if (fix_s > 0 ? pl.S != fix_s : (num_kb < 4 * pl.S && pl.S > 1)) continue;
         if (!size_cta(N, num_kb, sms, &pl)) continue;
-        // (with more rows the plans are compared as if rows started on a line: the set was fitted so)
-        double c = plan_cost(M, N, num_kb, sms, M <= kTileM ? row_start(K) : kOnLine, pl);
+        double c = plan_cost(M, N, num_kb, sms, row_start(K), spread, pl);
         if (ahead) c -= ring_us(N, num_kb, sms, pl);
         if (!found || c < *cost) {
           found = true;
@@ -886,9 +928,9 @@ struct Planned {
   PlanC pl;
   double cost;
 };
-const Planned& planned(int M, int N, int K, int pair, int fix_s, bool ahead) {
+const Planned& planned(int M, int N, int K, int pair, int fix_s, bool ahead, bool one_block) {
   static thread_local Planned cache[64];
-  const int flags = 1 | (pair > 0 ? 2 : pair < 0 ? 1 : 0) << 1 | (ahead ? 1 : 0) << 3 | fix_s << 4;
+  const int flags = 1 | (pair > 0 ? 2 : pair < 0 ? 1 : 0) << 1 | (ahead ? 1 : 0) << 3 | fix_s << 4 | (one_block ? 1 : 0) << 12;
   Planned& c = cache[(static_cast<unsigned>(M) * 2654435761u ^ static_cast<unsigned>(N) * 40503u ^ static_cast<unsigned>(K) * 97u ^
                       static_cast<unsigned>(flags) * 7u) >> 8 & 63u];
   if (c.M != M || c.N != N || c.K != K || c.flags != flags) {
@@ -896,7 +938,7 @@ const Planned& planned(int M, int N, int K, int pair, int fix_s, bool ahead) {
     c.N = N;
     c.K = K;
     c.flags = flags;
-    c.ok = plan(M, N, K, sm_count(), pair, fix_s, ahead, &c.pl, &c.cost);
+    c.ok = plan(M, N, K, sm_count(), pair, fix_s, ahead, spread_rows(M, ahead, one_block), &c.pl, &c.cost);
   }
   return c;
 }
@@ -910,8 +952,8 @@ bool gemm_cluster_supported(const GemmArgs& a) {
 
 // Whether this kernel is expected to be faster than the persistent two-SM kernel, which overlaps a tile's epilogue with the next
 // tile and needs no sum of parts, but deals out 256-row tiles: with fewer than three rounds of those, what they leave
-// idle or compute on padding is often more than this kernel's fixed cost.  Its estimate is taken a tenth lower,
-// which fits its present pace: over 467 shapes of more than 128 rows the choice is then 0.9 % slower than the best one on average.
+// idle or compute on padding is often more than this kernel's fixed cost.  Its estimate is taken times 1.14, as it was when the constants
+// of its plans were fitted to the choice of both (see CostC).
 // Both sides measured, bf16 on B200: 512 x 1280 x 8192 17.4 here and 29.6 us there, 200 x 4096 x 4096 15.0 and 18.1, 512 x 2048 x 2048
 // 12.0 and 11.9; 1037 x 4104 x 2056 27.2 and 23.0, 768 x 7168 x 8192 71.5 and 64.7, 512 x 8192 x 8192 53.8 and 51.0, 2048 x 2048 x 2048
 // 20.5 and 17.5.
@@ -929,8 +971,8 @@ bool gemm_cluster_preferred(const GemmArgs& a) {
   const int pairs = sm_count() / 2;
   if (static_cast<long long>((a.M + 2 * kTileM - 1) / (2 * kTileM)) * ((a.N + kTileN - 1) / kTileN) > 3ll * pairs) return false;
   const double two_sm = pair_cut(kGemmPlain, a.M, a.N, a.K, pairs, a.stream_k, swiglu, false, false).us;
-  const Planned& c = planned(a.M, a.N, a.K, a.pair, 0, false);
-  return c.ok && 0.9 * plan_cost(a.M, a.N, (a.K + kTileK - 1) / kTileK, sm_count(), row_start(a.K), c.pl) < two_sm;
+  const Planned& c = planned(a.M, a.N, a.K, a.pair, 0, false, false);
+  return c.ok && 1.14 * c.cost < two_sm;
 }
 
 cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStream_t stream, gemm_detail::TmapFn make_tmap) {
@@ -945,7 +987,8 @@ cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStr
     if (fix_s == 0) fix_s = 1;
     if (fix_s > a.max_ctas) fix_s = a.max_ctas;
   }
-  const Planned& chosen = planned(a.M, a.N, a.K, a.max_ctas > 0 ? -1 : a.pair, fix_s, a.b_static != 0);
+  const Planned& chosen = planned(a.M, a.N, a.K, a.max_ctas > 0 ? -1 : a.pair, fix_s, a.b_static != 0,
+                                  a.row_ssq != nullptr || a.epilogue == kGemmEpilogueAdd);
   if (!chosen.ok) return cudaErrorInvalidValue;
   const PlanC pl = chosen.pl;
   const int P = pl.pair ? 2 : 1;
