@@ -66,6 +66,11 @@ constexpr int kWideTokens = 64;
 // of them takes memory's time from the kernel before and gains nothing here (16 stages: 64 x 7168 x 8192 26.4); stages of many tokens gain
 // nothing from two (100 x 2048 x 2048 7.44 -> 7.6, with all eight 7.35).
 constexpr int kFetchAll = 8, kFetchSome = 2;
+// With one token block a launch reads every weight once.  Where they cannot be expected to be in L2 the next time (a third of it, or
+// a weight of a chain of layers), they are the first to leave it: 16 x 7168 x 8192 21.9 -> 20.9 us, 64 x 7168 x 8192 24.1 -> 22.9, 24 x 16000 x
+// 4096 23.0 -> 22.0, 32 x 8192 x 3584 12.15 -> 11.7, a layer of a decode step of 32 sequences 60.1 -> 55.0.  Weights that do stay there lose: a
+// layer of 88 MB that is used again and again 40.1 -> 43.9, 16 x 1024 x 1024 4.0 -> 4.3.
+constexpr long long kOnceBytes = 40ll << 20, kOnceStaticBytes = 8ll << 20;
 constexpr int kThreadsC = 192;
 constexpr int kMaxStagesC = 12;
 constexpr int kSpreadRows = 32;              // rows, from which on a block of so many tokens is weighed
@@ -108,6 +113,7 @@ struct ParamsC {
   int row_parts;
   float row_eps, inv_k;
   float nan;  // see settle
+  bool once;  // which kernel the host takes
   int fetch;  // stages of weights that each CTA fetches into L2 before the wait for earlier kernels (see kFetchAll)
   oob_gemm_epilogue_add_t add;
 };
@@ -169,9 +175,17 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t mask) {
       : "memory");
 }
 
-template <bool PAIR>
-__device__ __forceinline__ void load_box(void* smem_dst, const void* tmap, uint32_t bar, int32_t x, int32_t y) {
-  if constexpr (PAIR) {
+// ONCE: `policy` says how the box is kept in L2.
+template <bool PAIR, bool ONCE = false>
+__device__ __forceinline__ void load_box(void* smem_dst, const void* tmap, uint32_t bar, int32_t x, int32_t y, uint64_t policy = 0) {
+  if constexpr (ONCE) {
+    static_assert(!PAIR, "a pair's weights are read by every token block");
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
+        :
+        : "r"(ptx::smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(x), "r"(y), "l"(policy)
+        : "memory");
+  } else if constexpr (PAIR) {
     tma_load_2d_pair(smem_dst, tmap, bar, x, y);
   } else {
     asm volatile(
@@ -383,7 +397,8 @@ __device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base
 // That is so few registers (50) for a plain launch's sums that the loads of a turn wait for each other; with three CTAs 80 - 90
 // (256 x 3456 x 4544 18.8 us, 17.9), with four 70 - 80 (143 x 1024 x 7680 17.7 us, 16.4 with three), which only the plans take that
 // place four on an SM (16 x 64000 x 512 14.4 us, 16.8 on three).
-template <typename T, int EPI, bool PAIR, int SUB, int RES>
+// ONCE: see kOnceBytes (a kernel of its own: the policy beside the loop costs small launches 1 - 5 %).
+template <typename T, int EPI, bool PAIR, int SUB, int RES, bool ONCE>
 __global__ void __launch_bounds__(kThreadsC, RES)
     gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                         const __grid_constant__ ParamsC p, DeviceStatus* status) {
@@ -436,6 +451,8 @@ __global__ void __launch_bounds__(kThreadsC, RES)
   ptx::griddep_launch_dependents();
   // Static weights are not behind that wait: their warp fills the ring at once, and waits when it has loaded its first tile.
   bool waited = !(p.w_static && warp == 0);
+  uint64_t once_policy = 0;
+  if constexpr (ONCE) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(once_policy));
   // Other weights may still be written by the kernel before: they are fetched into L2, which keeps up with such a write, and no further.
   if (warp == 0 && p.fetch > 0 && ptx::elect_one()) {
     const int tile = cluster / p.m_blocks * P + member;
@@ -495,8 +512,8 @@ __global__ void __launch_bounds__(kThreadsC, RES)
         for (int h = 0; h < SUB; ++h) {
           const int k = (kb * SUB + h) * kTileK;  // past K: the box is filled with zeros
           if constexpr (W) {
-            load_box<PAIR>(sw + h * w_bytes, &tmap_w, full, k, w_row);
-            if constexpr (EPI == kEpiSwiglu) load_box<PAIR>(sw + h * w_bytes + w_bytes / 2, &tmap_w, full, k, p.F + w_row);
+            load_box<PAIR, ONCE>(sw + h * w_bytes, &tmap_w, full, k, w_row, once_policy);
+            if constexpr (EPI == kEpiSwiglu) load_box<PAIR, ONCE>(sw + h * w_bytes + w_bytes / 2, &tmap_w, full, k, p.F + w_row, once_policy);
           } else {
             uint8_t* sx = sw + SUB * w_bytes + h * (x_bytes / SUB);
 #pragma unroll
@@ -511,7 +528,9 @@ __global__ void __launch_bounds__(kThreadsC, RES)
       }
     };
     if (warp == 0) {
-      if (ptx::elect_one()) produce(std::true_type{}, One{});
+      if (ptx::elect_one()) {
+        produce(std::true_type{}, One{});
+      }
     } else if (warp == 2) {
       if (ptx::elect_one()) {
         if (SUB == 1 && p.n_mma == 2) {  // a wide stage holds one instruction's tokens
@@ -658,9 +677,9 @@ __global__ void __launch_bounds__(kThreadsC, RES)
   }
 }
 
-template <typename T, int EPI, bool PAIR, int SUB, int RES>
+template <typename T, int EPI, bool PAIR, int SUB, int RES, bool ONCE = false>
 cudaError_t launch_pair(const GemmArgs& a, ParamsC& p, DeviceStatus* status, cudaStream_t stream, TmapFn make_tmap) {
-  auto kernel = gemm_cluster_kernel<T, EPI, PAIR, SUB, RES>;
+  auto kernel = gemm_cluster_kernel<T, EPI, PAIR, SUB, RES, ONCE>;
   const int size = PAIR ? 2 * p.S : p.S;  // CTAs of a cluster
   static std::atomic<uint64_t> attr_set_mask{0};
   int dev = 0;
@@ -702,13 +721,17 @@ cudaError_t launch_epi(const GemmArgs& a, ParamsC& p, bool pair, DeviceStatus* s
   } else {
     if (pair) return launch_pair<T, EPI, true, 1, kRes>(a, p, status, stream, make_tmap);
   }
-  if constexpr (kBound) {
-    if (p.per_sm > kRes)
-      return p.sub == 2 ? launch_pair<T, EPI, false, 2, 4>(a, p, status, stream, make_tmap)
-                        : launch_pair<T, EPI, false, 1, 4>(a, p, status, stream, make_tmap);
-  }
-  return p.sub == 2 ? launch_pair<T, EPI, false, 2, kRes>(a, p, status, stream, make_tmap)
-                    : launch_pair<T, EPI, false, 1, kRes>(a, p, status, stream, make_tmap);
+  auto launch = [&](auto once) {
+    constexpr bool O = decltype(once)::value;
+    if constexpr (kBound) {
+      if (p.per_sm > kRes)
+        return p.sub == 2 ? launch_pair<T, EPI, false, 2, 4, O>(a, p, status, stream, make_tmap)
+                          : launch_pair<T, EPI, false, 1, 4, O>(a, p, status, stream, make_tmap);
+    }
+    return p.sub == 2 ? launch_pair<T, EPI, false, 2, kRes, O>(a, p, status, stream, make_tmap)
+                      : launch_pair<T, EPI, false, 1, kRes, O>(a, p, status, stream, make_tmap);
+  };
+  return p.once ? launch(std::true_type{}) : launch(std::false_type{});
 }
 
 template <typename T>
@@ -808,7 +831,7 @@ int device_slots(int size, int per_sm) {
   std::atomic<int>& slot = cached[dev & 63][per_sm - 1][size];
   int n = slot.load(std::memory_order_relaxed);
   if (n > 0) return n;
-  auto kernel = gemm_cluster_kernel<__nv_bfloat16, kEpiPlain, false, 1, 4>;
+  auto kernel = gemm_cluster_kernel<__nv_bfloat16, kEpiPlain, false, 1, 4, false>;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(size * 1024);
   cfg.blockDim = dim3(kThreadsC);
@@ -1009,6 +1032,7 @@ cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStr
   p.inv_k = 1.f / static_cast<float>(a.K);
   p.nan = std::numeric_limits<float>::quiet_NaN();
   if (a.epilogue == kEpiRopeKv) p.rope = *static_cast<const oob_rope_args_t*>(a.epilogue_args);
+  p.once = pl.m_blocks == 1 && 2ll * a.N * a.K >= (a.b_static ? kOnceStaticBytes : kOnceBytes);
   const int steps = (p.num_kb + pl.S - 1) / pl.S;
   p.fetch = a.b_static ? 0 : steps <= kFetchAll ? steps : pl.sub == 2 ? kFetchSome : 0;
   p.n_mma = pl.n_mma;
