@@ -159,6 +159,10 @@ constexpr int kAttnWarps = 4;
 constexpr int kAttnThreads = kAttnWarps * 32;
 constexpr int kRowBytes = kHD * 2;                 // 256
 constexpr int kKvTileBytes = kTileKeys * kRowBytes;  // 4 KiB
+// Keys and values are read once, and from here on (three such caches do not fit it) the next call does not find them in L2: they leave it
+// first.  256 x 1900 keys 40.7 -> 40.3 us, 2 x 8000 with 8 KV heads 14.9 -> 14.65, 32 x 500 with 8 13.1 -> 12.8, 100 x 700 with 2 14.3 -> 14.0.  A kernel
+// of its own, chosen by the bound of the length: a policy in a register costs short contexts 1 - 4 %.
+constexpr long long kOnceBytes = 48ll << 20;
 constexpr int kMaxAttnCluster = 8;                 // portable cluster size
 constexpr int kAttnStages = 3;                     // tiles of K and V in flight or in use per warp (96 KiB per CTA, two per SM)
 // Where no SM gets two CTAs anyway, and CTAs alone or in pairs (64 x 300 keys 5.5 -> 5.15 us; clusters of eight gain nothing, fewer of
@@ -202,8 +206,13 @@ __device__ __forceinline__ uint32_t transpose_8x8(uint32_t a) {
   asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
   return d;
 }
-__device__ __forceinline__ void cp_async_16(uint32_t smem_addr, const void* gptr) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr), "l"(gptr) : "memory");
+template <bool ONCE>
+__device__ __forceinline__ void cp_async_16(uint32_t smem_addr, const void* gptr, uint64_t policy) {
+  if constexpr (ONCE) {
+    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(smem_addr), "l"(gptr), "l"(policy) : "memory");
+  } else {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr), "l"(gptr) : "memory");
+  }
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -273,7 +282,7 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t smem_addr, uint32_t ran
 // 7.65, 7.25; 16 x 2000 7.3, 6.9; 64 x 300 6.0, 5.2; 2 x 8000 with 8 KV heads 15.9, 14.9; 256 x 1900 41.5, 40.9; 16 heads a KV head,
 // 20 x 3000 11.35, 11.2.  (A maximum raised only by scores that exceed it by eight was another 2 % faster, and 10 % further from 64-bit
 // results: the largest probabilities are then no longer exactly one.)
-template <typename T, int S, int STAGES, bool FEW>
+template <typename T, int S, int STAGES, bool FEW, bool ONCE>
 __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams p) {
   static_assert(attn_smem_bytes(STAGES) >= (kAttnWarps * 16 * merge_stride(FEW) + 16 * (kHD + 2)) * 4, "merge buffers");
   extern __shared__ __align__(128) uint8_t attn_smem[];
@@ -297,6 +306,8 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
   // The warps take the CTA's tiles in turn.
   const int my_tiles = t1 - t0 > warp ? (t1 - t0 - warp + kAttnWarps - 1) / kAttnWarps : 0;
 
+  [[maybe_unused]] uint64_t policy = 0;
+  if constexpr (ONCE) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
   auto issue_tile = [&](int i, int stage) {
     const int key0 = (t0 + warp + i * kAttnWarps) * kTileKeys;
     const uint32_t ks = wbuf_u32 + stage * 2 * kKvTileBytes, vs = ks + kKvTileBytes;
@@ -304,8 +315,8 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
     for (int j = 0; j < kKvTileBytes / 512; ++j) {
       const int r = j * 2 + (lane >> 4), c = lane & 15;  // 16 units of 16 bytes per key row
       const int key = min(key0 + r, L - 1);  // masked later; the address stays inside the written part of the cache
-      cp_async_16(ks + kv_off(r, c), kbase + static_cast<long long>(key) * kHD + c * 8);
-      cp_async_16(vs + kv_off(r, c), vbase + static_cast<long long>(key) * kHD + c * 8);
+      cp_async_16<ONCE>(ks + kv_off(r, c), kbase + static_cast<long long>(key) * kHD + c * 8, policy);
+      cp_async_16<ONCE>(vs + kv_off(r, c), vbase + static_cast<long long>(key) * kHD + c * 8, policy);
     }
   };
 
@@ -655,33 +666,34 @@ __global__ void attn_combine_kernel(const float* ws, void* out, int splits) {
   static_cast<T*>(out)[hrow * kHD + d] = to_out<T>(acc / l_tot);
 }
 
-template <typename T, int S, int STAGES, bool FEW>
+template <typename T, int S, int STAGES, bool FEW, bool ONCE>
 cudaError_t launch_attn_s(const AttnParams& p, cudaStream_t stream) {
   static std::atomic<uint64_t> attr_done{0};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!(attr_done.load(std::memory_order_relaxed) >> (dev & 63) & 1)) {
-    cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<T, S, STAGES, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<T, S, STAGES, FEW, ONCE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          attn_smem_bytes(STAGES));
     if (e != cudaSuccess) return e;
     attr_done.fetch_or(uint64_t(1) << (dev & 63), std::memory_order_relaxed);
   }
-  return launch_pdl(attn_decode_kernel<T, S, STAGES, FEW>, dim3(p.splits * S, p.KV, p.B), kAttnThreads, attn_smem_bytes(STAGES), stream, S, p);
+  return launch_pdl(attn_decode_kernel<T, S, STAGES, FEW, ONCE>, dim3(p.splits * S, p.KV, p.B), kAttnThreads, attn_smem_bytes(STAGES), stream, S, p);
 }
 
 template <typename T>
-cudaError_t launch_attn(const AttnParams& p, int cluster, bool deep, cudaStream_t stream) {
+cudaError_t launch_attn(const AttnParams& p, int cluster, bool deep, bool once, cudaStream_t stream) {
   constexpr int A = kAttnStages, D = kAttnDeepStages;
-  auto size = [&](auto few) {
-    constexpr bool F = decltype(few)::value;
+  auto size = [&](auto few, auto read_once) {
+    constexpr bool F = decltype(few)::value, O = decltype(read_once)::value;
     switch (cluster) {
-      case 1: return deep ? launch_attn_s<T, 1, D, F>(p, stream) : launch_attn_s<T, 1, A, F>(p, stream);
-      case 2: return deep ? launch_attn_s<T, 2, D, F>(p, stream) : launch_attn_s<T, 2, A, F>(p, stream);
-      case 4: return launch_attn_s<T, 4, A, F>(p, stream);
-      default: return launch_attn_s<T, 8, A, F>(p, stream);
+      case 1: return deep ? launch_attn_s<T, 1, D, F, O>(p, stream) : launch_attn_s<T, 1, A, F, O>(p, stream);
+      case 2: return deep ? launch_attn_s<T, 2, D, F, O>(p, stream) : launch_attn_s<T, 2, A, F, O>(p, stream);
+      case 4: return launch_attn_s<T, 4, A, F, O>(p, stream);
+      default: return launch_attn_s<T, 8, A, F, O>(p, stream);
     }
   };
-  cudaError_t e = p.G <= 8 ? size(std::true_type{}) : size(std::false_type{});
+  cudaError_t e = p.G <= 8 ? (once ? size(std::true_type{}, std::true_type{}) : size(std::true_type{}, std::false_type{}))
+                           : (once ? size(std::false_type{}, std::true_type{}) : size(std::false_type{}, std::false_type{}));
   if (e != cudaSuccess) return e;
   if (p.splits > 1) e = launch_pdl(attn_combine_kernel<T>, dim3(p.B * p.H), kHD, 0, stream, 1, p.ws, p.out, p.splits);
   return e;
@@ -694,9 +706,9 @@ struct AttnSlots {
   int deep[2];  // of the kernel with kAttnDeepStages, alone and in pairs
 };
 
-template <typename T, int S, int STAGES, bool FEW = true>
+template <typename T, int S, int STAGES, bool FEW = true, bool ONCE = false>
 int attn_slots_of() {
-  if (cudaFuncSetAttribute(attn_decode_kernel<T, S, STAGES, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem_bytes(STAGES)) != cudaSuccess) {
+  if (cudaFuncSetAttribute(attn_decode_kernel<T, S, STAGES, FEW, ONCE>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem_bytes(STAGES)) != cudaSuccess) {
     (void)cudaGetLastError();
     return 0;
   }
@@ -712,7 +724,7 @@ int attn_slots_of() {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, attn_decode_kernel<T, S, STAGES, FEW>, &cfg) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&clusters, attn_decode_kernel<T, S, STAGES, FEW, ONCE>, &cfg) != cudaSuccess) {
     (void)cudaGetLastError();
     return 0;
   }
@@ -905,8 +917,9 @@ int oob_attn_decode(const oob_attn_decode_args_t* a, void* stream) {
   // the GPU then wait for the last ones (2 x 30000 keys on 8 KV heads 48 - 55 us in eights, 45 in fours; alone both 44).
   if (splits > 1) slots.n[3] -= slots.n[3] / 4;
   const int cluster = attn_cluster_size(static_cast<long long>(a->B) * a->KV * splits, (bound + splits - 1) / splits, slots);
+  const bool once = static_cast<long long>(a->B) * a->KV * bound * (4 * kHD) >= kOnceBytes;
   const bool deep = cluster <= 2 && static_cast<long long>(a->B) * a->KV * splits * cluster <= slots.deep[cluster - 1];
-  cudaError_t e = a->dtype == OOB_BF16 ? launch_attn<__nv_bfloat16>(p, cluster, deep, s) : launch_attn<__half>(p, cluster, deep, s);
+  cudaError_t e = a->dtype == OOB_BF16 ? launch_attn<__nv_bfloat16>(p, cluster, deep, once, s) : launch_attn<__half>(p, cluster, deep, once, s);
   if (e != cudaSuccess) return cuda_fail(e, "attn_decode launch");
   return OOB_OK;
 }
