@@ -1,7 +1,7 @@
 // The single-GPU ops as Python calls them, for the calls that ask for nothing: checks, output and launch in one native call.
 //
 // Why: the kernel of a small call is done before Python has prepared the next.  On the host such a call took, in Python and with this
-// (B200 box, microseconds): residual + RMSNorm of 4 x 1024 7.6 and 4.9, GEMM of 16 x 1024 x 1024 9.6 and 4.4, SwiGLU projection 11.7 and
+// (B200, microseconds): residual + RMSNorm of 4 x 1024 7.6 and 4.9, GEMM of 16 x 1024 x 1024 9.6 and 4.4, SwiGLU projection 11.7 and
 // 4.4, QKV projection 15.6 and 4.6, decode attention 11.0 and 4.4; the launch itself takes 2.3 of these, an output 0.9.
 //
 // Every function answers None for a call that is not plainly of that kind (an option set, another type, layout, device or number of
