@@ -53,7 +53,7 @@ typedef struct {
   float scale;        /* softmax scale (1/sqrt(128) for standard attention) */
   int splits;         /* clusters of CTAs per (sequence, KV head) along the keys; 0 = choose from B * KV and len_bound */
   int len_bound;      /* upper bound of the context length for this launch (chooses clusters and splits); 0 = max_len */
-  float* workspace;   /* fp32, oob_attn_decode_workspace_bytes(B, H, splits) bytes; may be NULL when splits == 1 */
+  float* workspace;   /* fp32, oob_attn_decode_workspace_bytes(B, H, splits) bytes on a multiple of four; may be NULL when splits == 1 */
   int ahead;          /* 1 = nothing that this call could overtake writes *pos_dev or a key or value before the newest: they may be
                          read while the kernel before it on the stream still runs */
 } oob_attn_decode_args_t;

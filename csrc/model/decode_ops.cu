@@ -229,6 +229,7 @@ struct AttnParams {
   const void* v;
   void* out;
   float* ws;
+  bool ws_pairs;  // the workspace, which is on four bytes, stands on eight (and with it every part, of 65 pairs): two floats an access
   const long long* pos_dev;
   int len;
   int B, H, KV, G;
@@ -553,9 +554,20 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
           make_uint2(Cvt<T>::pack(acc.x / l_tot, acc.y / l_tot), Cvt<T>::pack(acc.z / l_tot, acc.w / l_tot));
     } else {
       float* w = p.ws + (hrow * p.splits + part / S) * kPartialStride;
-      *reinterpret_cast<float2*>(w + d) = make_float2(acc.x, acc.y);
-      *reinterpret_cast<float2*>(w + d + 2) = make_float2(acc.z, acc.w);
-      if (d == 0) *reinterpret_cast<float2*>(w + kHD) = make_float2(m_tot, l_tot);
+      if (p.ws_pairs) {
+        *reinterpret_cast<float2*>(w + d) = make_float2(acc.x, acc.y);
+        *reinterpret_cast<float2*>(w + d + 2) = make_float2(acc.z, acc.w);
+        if (d == 0) *reinterpret_cast<float2*>(w + kHD) = make_float2(m_tot, l_tot);
+      } else {
+        w[d] = acc.x;
+        w[d + 1] = acc.y;
+        w[d + 2] = acc.z;
+        w[d + 3] = acc.w;
+        if (d == 0) {
+          w[kHD] = m_tot;
+          w[kHD + 1] = l_tot;
+        }
+      }
     }
   };
   for (int u = threadIdx.x; u < G * 32; u += kAttnThreads) {
@@ -620,8 +632,8 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
   }
 }
 
-// Merges the key chunks of one (sequence, head): grid = B * H, 128 threads.
-template <typename T>
+// Merges the key chunks of one (sequence, head): grid = B * H, 128 threads.  PAIRS: see AttnParams::ws_pairs.
+template <typename T, bool PAIRS>
 __global__ void attn_combine_kernel(const float* ws, void* out, int splits) {
   const long long hrow = blockIdx.x;
   const int d = threadIdx.x;
@@ -635,7 +647,14 @@ __global__ void attn_combine_kernel(const float* ws, void* out, int splits) {
   for (int s0 = 0; s0 < splits; s0 += 32) {
     const int n = min(splits - s0, 32);
     float2 ml = make_float2(-INFINITY, 0.f);
-    if (lane < n) ml = *reinterpret_cast<const float2*>(w + (s0 + lane) * kPartialStride + kHD);
+    if (lane < n) {
+      const float* p = w + (s0 + lane) * kPartialStride + kHD;
+      if constexpr (PAIRS) {
+        ml = *reinterpret_cast<const float2*>(p);
+      } else {
+        ml = make_float2(p[0], p[1]);
+      }
+    }
     float v[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = i < n ? w[(s0 + i) * kPartialStride + d] : 0.f;
@@ -695,7 +714,7 @@ cudaError_t launch_attn(const AttnParams& p, int cluster, bool deep, bool once, 
   cudaError_t e = p.G <= 8 ? (once ? size(std::true_type{}, std::true_type{}) : size(std::true_type{}, std::false_type{}))
                            : (once ? size(std::false_type{}, std::true_type{}) : size(std::false_type{}, std::false_type{}));
   if (e != cudaSuccess) return e;
-  if (p.splits > 1) e = launch_pdl(attn_combine_kernel<T>, dim3(p.B * p.H), kHD, 0, stream, 1, p.ws, p.out, p.splits);
+  if (p.splits > 1) e = launch_pdl(p.ws_pairs ? attn_combine_kernel<T, true> : attn_combine_kernel<T, false>, dim3(p.B * p.H), kHD, 0, stream, 1, p.ws, p.out, p.splits);
   return e;
 }
 
@@ -892,12 +911,14 @@ int oob_attn_decode(const oob_attn_decode_args_t* a, void* stream) {
   int splits = a->splits > 0 ? a->splits : oob_attn_decode_auto_splits(a->B, a->KV, bound);
   if (splits > 65535) return set_error(OOB_ERR_INVALID, "too many splits");
   if (splits > 1 && a->workspace == nullptr) return set_error(OOB_ERR_INVALID, "splits > 1 need a workspace");
+  if (splits > 1 && (reinterpret_cast<uintptr_t>(a->workspace) & 3)) return set_error(OOB_ERR_INVALID, "the workspace holds floats: four-byte aligned");
   AttnParams p{};
   p.q = a->q;
   p.k = a->k_cache;
   p.v = a->v_cache;
   p.out = a->out;
   p.ws = a->workspace;
+  p.ws_pairs = (reinterpret_cast<uintptr_t>(a->workspace) & 7) == 0;
   p.pos_dev = reinterpret_cast<const long long*>(a->pos_dev);
   p.len = a->len;
   p.B = a->B;

@@ -39,3 +39,12 @@ def test_overlapping_split_calls_have_partial_results_of_their_own(monkeypatch):
     need = rec.oob_attn_decode_workspace_bytes(2, 8, 4)
     assert len(rec.pointers) == 2 and all(rec.pointers)
     assert abs(rec.pointers[0] - rec.pointers[1]) >= need
+
+
+def test_a_workspace_off_four_bytes_is_refused_by_the_host():
+    import ctypes
+
+    from ooverlap_b200 import _lib
+    a = _lib.AttnDecodeArgs(_lib.BF16, 1, 8, 1, 1 << 20, 1 << 20, 1 << 20, 64 * 128, 64, 0, 1 << 20, None, 64, 0.1, 2, 64, (1 << 20) + 2, 0)
+    assert _lib.lib().oob_attn_decode(ctypes.byref(a), None) == _lib.ERR_INVALID
+    assert "workspace" in _lib.last_error()
