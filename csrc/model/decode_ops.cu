@@ -661,8 +661,10 @@ __global__ void attn_combine_kernel(const float* ws, void* out, int splits) {
     float m_new = fmaxf(m_tot, ml.x);
 #pragma unroll
     for (int x = 16; x > 0; x >>= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, x));
-    const float f = ml.x == -INFINITY ? 0.f : exp2f(ml.x - m_new);  // 0: a part without keys
-    float l = f * ml.y;
+    // A part without keys may hold anything; one whose factor underflows has values, and a NaN or infinity among them is passed on.
+    const unsigned some = __ballot_sync(0xffffffffu, ml.x != -INFINITY);
+    const float f = ml.x == -INFINITY ? 0.f : exp2f(ml.x - m_new);
+    float l = ml.x == -INFINITY ? 0.f : f * ml.y;
 #pragma unroll
     for (int x = 16; x > 0; x >>= 1) l += __shfl_xor_sync(0xffffffffu, l, x);
     if (s0 > 0) {
@@ -674,7 +676,7 @@ __global__ void attn_combine_kernel(const float* ws, void* out, int splits) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const float fi = __shfl_sync(0xffffffffu, f, (i0 + i) & 31);
-        if (i0 + i < n && fi != 0.f) acc += fi * v[i];  // a part without keys may hold anything
+        if (i0 + i < n && (some >> ((i0 + i) & 31) & 1)) acc += fi * v[i];
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i) v[i] = i0 + 8 + i < n ? w[(s0 + i0 + 8 + i) * kPartialStride + d] : 0.f;
