@@ -273,7 +273,7 @@ PyObject* py_attn_decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
       kc->sizes() != vc->sizes() || kc->strides() != vc->strides())
     return none();
   oob_attn_decode_args_t a{};
-  if (!whole(args[4], &a.batch0) || !whole(args[5], &a.splits) || !whole(args[6], &a.len_bound) || a.batch0 < 0 || a.splits < 0 ||
+  if (!PyBool_Check(args[7]) || !whole(args[4], &a.batch0) || !whole(args[5], &a.splits) || !whole(args[6], &a.len_bound) || a.batch0 < 0 || a.splits < 0 ||
       a.len_bound < 0)
     return none();
   const int64_t B = q->size(0), H = q->size(1), KV = kc->size(1), max_len = kc->size(2);

@@ -302,7 +302,7 @@ def gemm_swiglu(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = 
     by the stand-alone SwiGLU kernel.  ``fused=True`` insists on a problem that the tiled kernels would split over K (every
     decode-step shape) and raises otherwise.  ``a`` may be a :class:`RowSums` (see
     :func:`gemm_add_norm`)."""
-    if out is None and fused is None and not max_ctas:
+    if out is None and fused is None and max_ctas == 0:
         done = _lib.fast().gemm_swiglu(a, b, _scope.static_b)
         if done is not None:
             return done

@@ -30,7 +30,7 @@ def rmsnorm_reference(x: torch.Tensor, weight: torch.Tensor, eps: float,
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, residual: Optional[torch.Tensor] = None,
             *, out: Optional[torch.Tensor] = None, residual_out: Optional[torch.Tensor] = None, max_ctas: int = 0):
     """Local ``y = rmsnorm(x + residual) * weight`` (no communication).  Returns ``y`` or ``(y, residual_out)``."""
-    if out is None and residual_out is None and not max_ctas:
+    if out is None and residual_out is None and max_ctas == 0:
         done = _lib.fast().rmsnorm(x, weight, eps, residual)
         if done is not None:
             return done

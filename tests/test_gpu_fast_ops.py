@@ -144,3 +144,13 @@ def test_under_inference_mode_and_capture(monkeypatch):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, want) and torch.equal(other, want)
+
+
+def test_options_given_in_another_type(monkeypatch):
+    """``None`` for a number of CTAs is refused as by the library's argument types, and a promise that is not a bool is still one."""
+    a, b, w = _rand(4, 64), _rand(64, 64), _rand(64)
+    for call in (lambda: rmsnorm(a, w, max_ctas=None), lambda: gemm_swiglu(a, b, max_ctas=None)):
+        with pytest.raises(Exception):
+            call()
+    q, kc = _rand(1, 2, 128), _rand(1, 2, 16, 128)
+    _same(*_both(monkeypatch, lambda: attn_decode(q, kc, kc, 3, cache_ready=1), "attn_decode", taken=False))
