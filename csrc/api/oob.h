@@ -297,6 +297,10 @@ int oob_pad_counter_count(void);
 int oob_test_pair_schedule(int mode, int M, int N, int K, int pairs, int stream_k, int world, int rank, int* out, int cap);
 /* Columns of an accumulator of that schedule (rows: 256); a pair may take two neighbouring ones in one item. */
 int oob_test_pair_tile_columns(int mode, int M, int N, int K, int pairs, int stream_k);
+/* Test hook (host only): how the weight-streaming GEMM cuts a problem, five integers: token blocks, tokens of a block (padded),
+ * 1 = CTA pairs, K splits, CTAs that share an SM.  `pair` and `splits` are as in oob_gemm_args_t, `one_block`: row sums or
+ * the Add epilogue.  -1: it cannot. */
+int oob_test_gemm_cluster_plan(int M, int N, int K, int pair, int splits, int b_static, int one_block, int* out);
 
 /* Test hook: the local norm of oob_fused_norm(NULL, OOB_NORM_LOCAL, ...) whose waits for the rows of its ring run out at
  * once, so that every row takes the way of a row that arrives late. */

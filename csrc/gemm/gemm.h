@@ -37,6 +37,8 @@ enum TraceSlot : int {
 constexpr int kGemmEpilogueSwigluTile = 3;
 constexpr int kGemmEpilogueAdd = 4;
 constexpr int kGemmClusterMaxRows = 4096;  // rows the weight-streaming kernel (gemm_cluster.cu) accepts
+// How that kernel cuts a problem: token blocks, tokens of a block, pairs, K splits, CTAs an SM.
+bool gemm_cluster_plan(int M, int N, int K, int pair, int splits, bool b_static, bool one_block, int out[5]);
 
 // All matrices are 16-bit (fp16 or bf16), A is [M, K] row-major with leading
 // dimension lda, B is [N, K] row-major (the layout of a torch Linear weight)

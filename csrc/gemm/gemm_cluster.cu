@@ -816,40 +816,15 @@ bool size_cta(int N, int num_kb, int sms, PlanC* pl) {
   return false;
 }
 
-// Clusters of `size` CTAs that run at once with `per_sm` CTAs on an SM.  A cluster lives in one GPC (about 18 SMs on this part, some have
-// fewer, and not the same on every GPU): the device is asked, and its answers are kept.  One cluster too many is a second round of them
-// (SwiGLU 116 x 1024 x 5624 on 16 clusters of seven, of which 15 run at once: 17.9 us, 11.0).  Without a device, one B200's answers.
-int device_slots(int size, int per_sm) {
-  static const int b200[4][9] = {{0, 148, 74, 45, 33, 26, 22, 15, 15}, {0, 296, 148, 93, 71, 56, 45, 37, 33},
-                                 {0, 444, 222, 142, 104, 82, 71, 56, 48}, {0, 592, 296, 187, 142, 112, 93, 78, 71}};
-  static std::atomic<int> cached[64][4][9];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return b200[per_sm - 1][size];
-  }
-  std::atomic<int>& slot = cached[dev & 63][per_sm - 1][size];
-  int n = slot.load(std::memory_order_relaxed);
-  if (n > 0) return n;
-  auto kernel = gemm_cluster_kernel<__nv_bfloat16, kEpiPlain, false, 1, 4, false>;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(size * 1024);
-  cfg.blockDim = dim3(kThreadsC);
-  cfg.dynamicSmemBytes = per_sm == 1 ? kSmemLimit : 228 * 1024 / per_sm - 1024;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = size;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
-    (void)cudaGetLastError();
-    return b200[per_sm - 1][size];
-  }
-  slot.store(n, std::memory_order_relaxed);
-  return n;
+// Clusters of `size` CTAs that run at once with `per_sm` CTAs on an SM, as a B200 answers (cudaOccupancyMaxActiveClusters).  A cluster lives
+// in one GPC, about 18 SMs on this part, some have fewer, and not the same on every GPU.  One cluster too many is a second round of them
+// (SwiGLU 116 x 1024 x 5624 on 16 clusters of seven, of which 15 run at once: 17.9 us, 11.0).  A table all the same, and not a question to the
+// device: a plan has the K split in it, and with that the order of the sums, so that a call has the same bits on every GPU of a group, and
+// plans can be kept by sizes alone.
+int cluster_slots(int size, int per_sm) {
+  static const int b200[4][kMaxCluster + 1] = {{0, 148, 74, 45, 33, 26, 22, 15, 15}, {0, 296, 148, 93, 71, 56, 45, 37, 33},
+                                               {0, 444, 222, 142, 104, 82, 71, 56, 48}, {0, 592, 296, 187, 142, 112, 93, 78, 71}};
+  return b200[per_sm - 1][size];
 }
 // What the plans of few rows were fitted with.
 int rough_slots(int sms, int size, int per_sm) {
@@ -885,7 +860,7 @@ bool spread_rows(int M, bool ahead, bool one_block) { return M > kSpreadRows && 
 double plan_cost(int M, int N, int num_kb, int sms, RowStart start, bool spread, const PlanC& pl) {
   const CostC& c = M > kTileM ? kMoreRows : spread ? kSomeRows : kFewRows;
   const int P = pl.pair ? 2 : 1, Mp = pl.n_mma * pl.nj, size = P * pl.S;
-  const int clusters = tile_count(N, pl), slots = &c == &kFewRows ? rough_slots(sms, size, pl.per_sm) : device_slots(size, pl.per_sm);
+  const int clusters = tile_count(N, pl), slots = &c == &kFewRows ? rough_slots(sms, size, pl.per_sm) : cluster_slots(size, pl.per_sm);
   const int rounds = (clusters + slots - 1) / slots;
   const double live = double(clusters < slots ? clusters : slots) * size;  // CTAs at once
   const double share = live > sms ? live / sms : 1.0;
@@ -996,6 +971,17 @@ bool gemm_cluster_preferred(const GemmArgs& a) {
   const double two_sm = pair_cut(kGemmPlain, a.M, a.N, a.K, pairs, a.stream_k, swiglu, false, false).us;
   const Planned& c = planned(a.M, a.N, a.K, a.pair, 0, false, false);
   return c.ok && 1.14 * c.cost < two_sm;
+}
+
+bool gemm_cluster_plan(int M, int N, int K, int pair, int splits, bool b_static, bool one_block, int out[5]) {
+  const gemm_cluster::Planned& c = gemm_cluster::planned(M, N, K, pair, splits, b_static, one_block);
+  if (!c.ok) return false;
+  out[0] = c.pl.m_blocks;
+  out[1] = c.pl.n_mma * c.pl.nj;
+  out[2] = c.pl.pair;
+  out[3] = c.pl.S;
+  out[4] = c.pl.per_sm;
+  return true;
 }
 
 cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStream_t stream, gemm_detail::TmapFn make_tmap) {

@@ -1193,6 +1193,11 @@ int oob_test_pair_tile_columns(int mode, int M, int N, int K, int pairs, int str
   return pair_cut(mode, M, N, K, pairs, stream_k, false, false, false).tile_n;
 }
 
+int oob_test_gemm_cluster_plan(int M, int N, int K, int pair, int splits, int b_static, int one_block, int* out) {
+  if (M <= 0 || M > kGemmClusterMaxRows || N <= 0 || K <= 0 || splits < 0 || splits > 8 || out == nullptr) return -1;
+  return gemm_cluster_plan(M, N, K, pair, splits, b_static != 0, one_block != 0, out) ? 0 : -1;
+}
+
 uint64_t oob_gemm_splitk_bytes(int M, int N, int K, int max_ctas, int splits) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   return gemm_splitk_bytes(M, N, K, max_ctas, splits);

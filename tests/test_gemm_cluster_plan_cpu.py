@@ -1,0 +1,77 @@
+"""How the weight-streaming GEMM cuts a problem.  The K split decides the order of the sums, so a plan follows from the sizes and from
+nothing that differs from one GPU, thread or process to the next."""
+import ctypes
+import os
+import random
+import threading
+
+import pytest
+import torch
+
+from ooverlap_b200 import _lib
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def plan(M, N, K, pair=0, splits=0, b_static=0, one_block=0):
+    out = (ctypes.c_int * 5)()
+    assert _lib.lib().oob_test_gemm_cluster_plan(M, N, K, pair, splits, b_static, one_block, out) == 0
+    return tuple(out)
+
+
+def shapes(n, seed):
+    rng = random.Random(seed)
+    return [(int(2 ** rng.uniform(0, 12)), 8 * rng.randint(8, 1024), 8 * rng.randint(8, 1024)) for _ in range(n)]
+
+
+# Token blocks, tokens of a block, pairs, K splits, CTAs an SM: shapes whose clusters come close to what a GPU runs at once, where one
+# cluster fewer has another K split.
+PINNED = {(154, 5568, 2584): (1, 160, 1, 3, 1), (116, 1024, 5624): (2, 64, 0, 6, 1), (512, 1280, 8192): (3, 176, 1, 4, 1),
+          (16, 7168, 8192): (1, 16, 0, 2, 1), (64, 7168, 8192): (1, 64, 0, 2, 1)}
+
+
+def check_pinned():
+    for shape, want in PINNED.items():
+        assert plan(*shape) == want, shape
+
+
+def test_pinned_plans_without_a_device():
+    check_pinned()
+
+
+@pytest.mark.gpu
+def test_pinned_plans_on_a_device():
+    torch.zeros(1, device="cuda")
+    check_pinned()
+
+
+def test_planning_asks_no_device():
+    with open(os.path.join(ROOT, "csrc", "gemm", "gemm_cluster.cu")) as f:
+        assert "cudaOccupancy" not in f.read().replace("(cudaOccupancyMaxActiveClusters)", "")
+
+
+def test_threads_agree():
+    want = [plan(*s) for s in shapes(400, 1)]
+    got = {}
+
+    def other(i):
+        order = list(enumerate(shapes(400, 1)))
+        random.Random(i).shuffle(order)
+        got[i] = [p for _, p in sorted((j, plan(*s)) for j, s in order)]
+
+    threads = [threading.Thread(target=other, args=(i,)) for i in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert all(got[i] == want for i in range(3))
+
+
+def test_plans_are_sound():
+    for M, N, K in shapes(600, 2):
+        blocks, tokens, pair, S, per_sm = plan(M, N, K)
+        assert tokens % 16 == 0 and blocks * tokens >= M > (blocks - 1) * tokens and tokens <= 384
+        assert 1 <= S * (2 if pair else 1) <= 8 and 1 <= per_sm <= 4
+        if M <= 128:
+            assert plan(M, N, K, one_block=1)[0] == 1
+        assert plan(M, N, K, splits=1)[3] == 1
