@@ -60,12 +60,13 @@ constexpr int kMaxTileTokens = 384;          // per tile: what its fp32 sums lea
 // 64 elements, 128 tokens with 64 elements a stage 0.142).  With more tokens it would leave too few stages
 // (128 x 7168 x 8192 27.1 us with 64 elements and 27.6 with 128, 128 x 8192 x 3584 split four ways 17.6 and 22.8).
 constexpr int kWideTokens = 64;
-// The first weights of a CTA are fetched into L2 while the kernel before this one ends (0.7 us from its end to the return of the wait for
-// it, then 1.4 us to weights from memory and 0.8 to weights from L2).  All of them where K is short, 16 x 2048 x 2048 5.4 -> 4.9 us, 1 x 2048 x
-// 2048 5.2 -> 4.7, 32 x 8192 x 1024 6.6 -> 6.25; else two wide stages, 32 x 8192 x 3584 12.4 -> 12.15, 64 x 7168 x 8192 24.4 -> 24.1.  More
-// of them takes memory's time from the kernel before and gains nothing here (16 stages: 64 x 7168 x 8192 26.4); stages of many tokens gain
-// nothing from two (100 x 2048 x 2048 7.44 -> 7.6, with all eight 7.35).
-constexpr int kFetchAll = 8, kFetchSome = 2;
+// The first stage of a CTA's weights is fetched into L2 while the kernel before this one ends (0.7 us from its end to the return of the wait for
+// it, then 1.4 us to weights from memory and 0.8 to weights from L2), where the weight is large enough not to be in L2 as a matter of course and
+// its rows start on a line.  One stage: over 728 shapes of 1 - 64 rows in a chain of calls on weights from memory 0.984 of the time, 3 of 330 more than
+// 2 % slower, on weights from L2 1.002.  All of up to eight stages: 0.973 and 1.018, 43 and 130 shapes slower, by up to 13 %: many CTAs' loads wait behind
+// what is fetched.  Weights of less than kFetchBytes are slower by up to 6 % where they are in L2 (1024 x 2048, 16 rows 4.26 -> 4.48 us); rows off a
+// line, whose boxes are two lines a row, are slower from memory as well (40 x 2736 x 1880 6.7 -> 7.3, 54 x 4800 x 3032 with SwiGLU 10.7 -> 11.9).
+constexpr long long kFetchBytes = 8ll << 20;
 // With one token block a launch reads every weight once.  Where they cannot be expected to be in L2 the next time (a third of it, or
 // a weight of a chain of layers), they are the first to leave it: 16 x 7168 x 8192 21.9 -> 20.9 us, 64 x 7168 x 8192 24.1 -> 22.9, 24 x 16000 x
 // 4096 23.0 -> 22.0, 32 x 8192 x 3584 12.15 -> 11.7, a layer of a decode step of 32 sequences 60.1 -> 55.0.  Weights that do stay there lose: a
@@ -114,7 +115,7 @@ struct ParamsC {
   float row_eps, inv_k;
   float nan;  // see settle
   bool once;  // which kernel the host takes
-  int fetch;  // stages of weights that each CTA fetches into L2 before the wait for earlier kernels (see kFetchAll)
+  bool fetch;  // the first stage of weights is fetched into L2 before the wait for earlier kernels (see kFetchBytes)
   oob_gemm_epilogue_add_t add;
 };
 
@@ -454,16 +455,13 @@ __global__ void __launch_bounds__(kThreadsC, RES)
   uint64_t once_policy = 0;
   if constexpr (ONCE) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(once_policy));
   // Other weights may still be written by the kernel before: they are fetched into L2, which keeps up with such a write, and no further.
-  if (warp == 0 && p.fetch > 0 && ptx::elect_one()) {
-    const int tile = cluster / p.m_blocks * P + member;
-    const int w_row = EPI == kEpiSwiglu ? tile * (kRowsW / 2) : tile * kRowsW;
-    const int kbe = min(kb1, kb0 + p.fetch);
-    for (int kb = kb0; kb < kbe; ++kb)
+  if (warp == 0 && p.fetch && ptx::elect_one()) {
+    const int w_row = (cluster / p.m_blocks * P + member) * (EPI == kEpiSwiglu ? kRowsW / 2 : kRowsW);
 #pragma unroll
-      for (int h = 0; h < SUB; ++h) {
-        ptx::tma_prefetch_2d(&tmap_w, (kb * SUB + h) * kTileK, w_row);
-        if constexpr (EPI == kEpiSwiglu) ptx::tma_prefetch_2d(&tmap_w, (kb * SUB + h) * kTileK, p.F + w_row);
-      }
+    for (int h = 0; h < SUB; ++h) {
+      ptx::tma_prefetch_2d(&tmap_w, (kb0 * SUB + h) * kTileK, w_row);
+      if constexpr (EPI == kEpiSwiglu) ptx::tma_prefetch_2d(&tmap_w, (kb0 * SUB + h) * kTileK, p.F + w_row);
+    }
   }
   __syncwarp();
   if (waited) ptx::griddep_wait();
@@ -1019,8 +1017,7 @@ cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStr
   p.nan = std::numeric_limits<float>::quiet_NaN();
   if (a.epilogue == kEpiRopeKv) p.rope = *static_cast<const oob_rope_args_t*>(a.epilogue_args);
   p.once = pl.m_blocks == 1 && 2ll * a.N * a.K >= (a.b_static ? kOnceStaticBytes : kOnceBytes);
-  const int steps = (p.num_kb + pl.S - 1) / pl.S;
-  p.fetch = a.b_static ? 0 : steps <= kFetchAll ? steps : pl.sub == 2 ? kFetchSome : 0;
+  p.fetch = !a.b_static && a.ldb % kTileK == 0 && (reinterpret_cast<uintptr_t>(a.B) & 127) == 0 && 2ll * a.N * a.K >= kFetchBytes;
   p.n_mma = pl.n_mma;
   p.nj = pl.nj;
   p.Mp = pl.n_mma * pl.nj;
