@@ -301,6 +301,9 @@ int oob_test_pair_tile_columns(int mode, int M, int N, int K, int pairs, int str
  * 1 = CTA pairs, K splits, CTAs that share an SM.  `pair` and `splits` are as in oob_gemm_args_t, `one_block`: row sums or
  * the Add epilogue.  -1: it cannot. */
 int oob_test_gemm_cluster_plan(int M, int N, int K, int pair, int splits, int b_static, int one_block, int* out);
+/* Test hook: the most bytes of local memory (spilled registers) a thread of that GEMM's kernels has; `epilogue` 0 none, 1 SwiGLU, 2 RoPE + cache write,
+ * 3 residual + norm weight.  -1: no device. */
+int oob_test_gemm_cluster_local_bytes(int epilogue, int dtype);
 
 /* Test hook: the local norm of oob_fused_norm(NULL, OOB_NORM_LOCAL, ...) whose waits for the rows of its ring run out at
  * once, so that every row takes the way of a row that arrives late. */

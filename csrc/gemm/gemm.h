@@ -39,6 +39,8 @@ constexpr int kGemmEpilogueAdd = 4;
 constexpr int kGemmClusterMaxRows = 4096;  // rows the weight-streaming kernel (gemm_cluster.cu) accepts
 // How that kernel cuts a problem: token blocks, tokens of a block, pairs, K splits, CTAs an SM.
 bool gemm_cluster_plan(int M, int N, int K, int pair, int splits, bool b_static, bool one_block, int out[5]);
+// The most bytes of registers that a thread of its kernels spills, by epilogue (0 - 3: none, SwiGLU, RoPE + cache, Add); -1: no device.
+int gemm_cluster_local_bytes(int epilogue, int fmt);
 
 // All matrices are 16-bit (fp16 or bf16), A is [M, K] row-major with leading
 // dimension lda, B is [N, K] row-major (the layout of a torch Linear weight)

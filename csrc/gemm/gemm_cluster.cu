@@ -395,7 +395,7 @@ __device__ __forceinline__ void reduce_tile(const ParamsC& p, uint32_t smem_base
 }
 
 // SUB: 64-element boxes of K in a pipeline stage.  RES: CTAs of an SM that the registers leave room for, 0 = what the compiler makes of it.
-// That is so few registers (50) for a plain launch's sums that the loads of a turn wait for each other; with three CTAs 80 - 90
+// For a plain launch's sums that is so few registers (50) that the loads of a turn wait for each other; with three CTAs 80 - 96
 // (256 x 3456 x 4544 18.8 us, 17.9), with four 70 - 80 (143 x 1024 x 7680 17.7 us, 16.4 with three), which only the plans take that
 // place four on an SM (16 x 64000 x 512 14.4 us, 16.8 on three).
 // ONCE: see kOnceBytes (a kernel of its own: the policy beside the loop costs small launches 1 - 5 %).
@@ -455,7 +455,8 @@ __global__ void __launch_bounds__(kThreadsC, RES)
   uint64_t once_policy = 0;
   if constexpr (ONCE) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(once_policy));
   // Other weights may still be written by the kernel before: they are fetched into L2, which keeps up with such a write, and no further.
-  if (warp == 0 && p.fetch && ptx::elect_one()) {
+  // (Not where four CTAs share an SM: its few registers spill 12 - 28 bytes of 80.)
+  if (RES < 4 && warp == 0 && p.fetch && ptx::elect_one()) {
     const int w_row = (cluster / p.m_blocks * P + member) * (EPI == kEpiSwiglu ? kRowsW / 2 : kRowsW);
 #pragma unroll
     for (int h = 0; h < SUB; ++h) {
@@ -710,10 +711,14 @@ cudaError_t launch_pair(const GemmArgs& a, ParamsC& p, DeviceStatus* status, cud
   return cudaLaunchKernelEx(&cfg, kernel, tw, tx, p, status);
 }
 
+// RES of the kernels that are not asked for four CTAs an SM.  The Add epilogue holds a turn's loads in 132 - 141 registers; with three CTAs it spills 250 - 350
+// bytes and takes 1.066 times as long, 72 shapes of 1 - 128 rows.
+constexpr int residents(int epi) { return epi == kEpiPlain || epi == kEpiSwiglu ? 3 : epi == kEpiAdd ? 2 : 0; }
+
 template <typename T, int EPI>
 cudaError_t launch_epi(const GemmArgs& a, ParamsC& p, bool pair, DeviceStatus* status, cudaStream_t stream, TmapFn make_tmap) {
   constexpr bool kBound = EPI == kEpiPlain || EPI == kEpiSwiglu;  // the others read more, of weights with at most two tiles for every SM
-  constexpr int kRes = kBound ? 3 : 0;
+  constexpr int kRes = residents(EPI);
   if constexpr (EPI == kEpiAdd) {  // at most 128 rows, which no pair takes; a pair's second tile may lie past N, and has no sums to write
     if (pair) return cudaErrorInvalidValue;
   } else {
@@ -741,6 +746,34 @@ cudaError_t launch_fmt(const GemmArgs& a, ParamsC& p, bool pair, DeviceStatus* s
     case kGemmEpilogueAdd: return launch_epi<T, kEpiAdd>(a, p, pair, status, stream, make_tmap);
     default: return launch_epi<T, kEpiPlain>(a, p, pair, status, stream, make_tmap);
   }
+}
+
+// The most bytes of local memory (spilled registers) that a thread of any of the kernels has on the current device, -1 on an error.
+template <typename T, int EPI>
+int local_bytes() {
+  int most = 0;
+  auto look = [&](auto kernel) {
+    cudaFuncAttributes attr{};
+    if (most < 0 || cudaFuncGetAttributes(&attr, kernel) != cudaSuccess) {
+      (void)cudaGetLastError();
+      most = -1;
+    } else {
+      most = std::max(most, static_cast<int>(attr.localSizeBytes));
+    }
+  };
+  constexpr int R = residents(EPI);
+  look(gemm_cluster_kernel<T, EPI, false, 1, R, false>);
+  look(gemm_cluster_kernel<T, EPI, false, 2, R, false>);
+  look(gemm_cluster_kernel<T, EPI, false, 1, R, true>);
+  look(gemm_cluster_kernel<T, EPI, false, 2, R, true>);
+  if constexpr (EPI != kEpiAdd) look(gemm_cluster_kernel<T, EPI, true, 1, R, false>);
+  if constexpr (EPI == kEpiPlain || EPI == kEpiSwiglu) {
+    look(gemm_cluster_kernel<T, EPI, false, 1, 4, false>);
+    look(gemm_cluster_kernel<T, EPI, false, 2, 4, false>);
+    look(gemm_cluster_kernel<T, EPI, false, 1, 4, true>);
+    look(gemm_cluster_kernel<T, EPI, false, 2, 4, true>);
+  }
+  return most;
 }
 
 }  // namespace gemm_cluster
@@ -969,6 +1002,20 @@ bool gemm_cluster_preferred(const GemmArgs& a) {
   const double two_sm = pair_cut(kGemmPlain, a.M, a.N, a.K, pairs, a.stream_k, swiglu, false, false).us;
   const Planned& c = planned(a.M, a.N, a.K, a.pair, 0, false, false);
   return c.ok && 1.14 * c.cost < two_sm;
+}
+
+int gemm_cluster_local_bytes(int epilogue, int fmt) {
+  using namespace gemm_cluster;
+  auto of = [&](auto t) {
+    using T = decltype(t);
+    switch (epilogue) {
+      case kEpiPlain: return local_bytes<T, kEpiPlain>();
+      case kEpiSwiglu: return local_bytes<T, kEpiSwiglu>();
+      case kEpiRopeKv: return local_bytes<T, kEpiRopeKv>();
+      default: return local_bytes<T, kEpiAdd>();
+    }
+  };
+  return fmt == 1 ? of(__nv_bfloat16()) : of(__half());
 }
 
 bool gemm_cluster_plan(int M, int N, int K, int pair, int splits, bool b_static, bool one_block, int out[5]) {

@@ -1198,6 +1198,8 @@ int oob_test_gemm_cluster_plan(int M, int N, int K, int pair, int splits, int b_
   return gemm_cluster_plan(M, N, K, pair, splits, b_static != 0, one_block != 0, out) ? 0 : -1;
 }
 
+int oob_test_gemm_cluster_local_bytes(int epilogue, int dtype) { return gemm_cluster_local_bytes(epilogue, dtype == OOB_BF16 ? 1 : 0); }
+
 uint64_t oob_gemm_splitk_bytes(int M, int N, int K, int max_ctas, int splits) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   return gemm_splitk_bytes(M, N, K, max_ctas, splits);

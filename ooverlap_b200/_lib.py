@@ -170,6 +170,7 @@ def _declare(lib) -> None:
     lib.oob_test_pair_schedule.argtypes = [c_int] * 8 + [POINTER(c_int), c_int]
     lib.oob_test_pair_tile_columns.argtypes = [c_int] * 6
     lib.oob_test_gemm_cluster_plan.argtypes = [c_int] * 7 + [POINTER(c_int)]
+    lib.oob_test_gemm_cluster_local_bytes.argtypes = [c_int, c_int]
     lib.oob_gemm_reserve_workspace.argtypes = [c_uint64]
     lib.oob_gemm_splitk_bytes.argtypes = [c_int, c_int, c_int, c_int, c_int]
     lib.oob_gemm_splitk_bytes.restype = c_uint64

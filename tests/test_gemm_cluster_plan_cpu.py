@@ -75,3 +75,13 @@ def test_plans_are_sound():
         if M <= 128:
             assert plan(M, N, K, one_block=1)[0] == 1
         assert plan(M, N, K, splits=1)[3] == 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [_lib.F16, _lib.BF16])
+@pytest.mark.parametrize("epilogue", [0, 1, 2, 3])
+def test_no_kernel_spills_its_sums(epilogue, dtype):
+    """Loads of a turn wait for each other where a thread has too few registers for its sums.  (The SwiGLU kernels have 32 bytes of arrays that are
+    indexed.)"""
+    torch.zeros(1, device="cuda")
+    assert _lib.lib().oob_test_gemm_cluster_local_bytes(epilogue, dtype) == (32 if epilogue == 1 else 0)
