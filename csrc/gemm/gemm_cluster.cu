@@ -74,7 +74,10 @@ constexpr long long kFetchBytes = 8ll << 20;
 constexpr long long kOnceBytes = 40ll << 20, kOnceStaticBytes = 8ll << 20;
 constexpr int kThreadsC = 192;
 constexpr int kMaxStagesC = 12;
-constexpr int kSpreadRows = 32;              // rows, from which on a block of so many tokens is weighed
+constexpr int kSpreadRows = 32, kSpreadMost = 1500;  // rows between which blocks of fewer tokens than 128 are weighed, down to the first
+constexpr int kSpreadBlocks = 10;            // as far as they were timed
+constexpr double kSpreadGain[2] = {0.82, 0.943};  // up to 128 rows and above, see planned
+constexpr double kSpreadTwoSm = 1.235;       // see gemm_cluster_preferred
 constexpr int kMaxCluster = 8;               // portable cluster size
 constexpr int kMaxScaledRows = 128;           // rows that may carry a sum of squares (ParamsC::row_ssq)
 constexpr int kCtlBytes = 256 + kMaxScaledRows * 4;
@@ -870,28 +873,30 @@ int rough_slots(int sms, int size, int per_sm) {
 // row of a box that starts off a 128-byte line touches two (`line`), one that starts off a 32-byte sector one more of these
 // (`sector`); the pace of one CTA with stages of many tokens suffers most (`pace_sector`: 103 x 5504 x 6728 split two ways 28.2 us,
 // three ways 21.1, which were taken for the slower).
-// The constants are fitted to timings for the choice they make, so that one need not be the rate that it stands for.  Few rows (one token
-// block): 16000 timings of every K split (1930 shapes of 3 - 128 rows, N and K of 512 - 8192), 3.3 % off the best plan on average; `write`,
-// `alone`, the paces and `pace_sector` once more to 461 shapes.  Some and more rows, where blocks of fewer tokens than 128 are weighed too: 1223
-// shapes of 33 - 128 and 867 of 129 - 1500 rows, every block count and split.  The choice is 2.3 % off the best plan there (8 % with blocks
-// of 128 tokens only: 128 x 4096 x 4096 12.3 us, 11.75 in two blocks and two splits) and 2.6 % off the best of both kernels (8.1 %: 256 x
-// 4096 x 4096 17.0, 13.2; 1500 x 1000 x 4000 17.2, 16.2).
+// The constants are fitted to timings for the choice they make, so that one need not be the rate that it stands for; kNone takes a limit
+// out.  kFewRows (up to 128 rows): 16000 timings of every K split (1930 shapes of 3 - 128 rows, N and K of 512 - 8192), 3.3 % off the best plan on
+// average; `write`, `alone`, the paces and `pace_sector` once more to 461 shapes.  kMoreRows: the set against which the two-SM kernel is weighed.
+// Both were fitted to blocks of 128 tokens and more.
+// kSpreadSome (33 - 128 rows) and kSpreadMore (129 - 1500) tell where blocks of 32 tokens and more beat these, see planned: only the quotient of two
+// estimates of one set is used, and its constants are no rates.  Fitted to 1223 and 867 timed shapes, every split of up to ten blocks.
 struct CostC {
   double wide, wide_tokens, pace, pace_tokens, mma, l2, hbm, drain, write, reduce, round, alone, cluster, eight, split, five, line, sector,
       pace_sector;
 };
+constexpr double kNone = 1e30;
 constexpr CostC kFewRows = {0.153, 0.00061, 0.18, 0.0004, 1140.0, 11.8e6, 6.4e6, 0.0117, 0.01, 2.84e6, 1.85, 3.1, 3.06, 2.6, 0.105, 0.0, 1.29, 1.29, 1.6};
-constexpr CostC kSomeRows = {0.2026, 0.00328, 0.0705, 0.00486, 1e9, 6.11e6, 67e6, 0.00018, 0.0176, 0.537e6, 0.478, 1.093, 1.525, 42.0, 0.0036, 0.376, 1.854, 3.133, 3.016};
-constexpr CostC kMoreRows = {0.0121, 0.00226, 0.1137, 0.000385, 2164.0, 19.1e6, 1e9, 0.000434, 0.025, 1.87e6, 3.86, 1.539, 1.881, 0.01, 0.0878, 0.04, 1.246, 1.95, 1.866};
+constexpr CostC kMoreRows = {0.165, 0.0005, 0.235, 0.0002, 1850.0, 11.5e6, 6.4e6, 0.015, 0.0, 3.0e6, 2.0, 3.4, 3.8, 2.0, 0.08, 0.0, 1.16, 1.45, 1.45};
+constexpr CostC kSpreadSome = {0.185, 0.00294, 0.0018, 0.0038, kNone, 7.92e6, 6.69e6, 0.0, 0.066, 0.381e6, 2.95, 0.27, 0.054, 0.0, 0.188, 0.036, 2.21, 2.70, 2.52};
+constexpr CostC kSpreadMore = {0.0036, 0.0026, 0.082, 0.000745, 2080.0, 17.8e6, kNone, 0.0, 0.0303, 1.415e6, 22.6, 0.574, 0.715, 0.095, 0.0, 0.01, 2.04, 2.81, 2.79};
 
-// Blocks of fewer tokens than 128 are weighed where more than 32 rows may be cut: row sums and the Add epilogue need one block, and static
-// weights of few rows are planned for what their rings hold.
-bool spread_rows(int M, bool ahead, bool one_block) { return M > kSpreadRows && !one_block && (M > kTileM || !ahead); }
+// Blocks of fewer tokens than 128 are weighed in the range that they were timed in (150 shapes of 1501 - 4096 rows: 0.995 of the time with them, as many
+// faster as slower), where the rows may be cut: row sums and the Add epilogue need one block, and static weights of few rows are
+// planned for what their rings hold.
+bool spread_rows(int M, bool ahead, bool one_block) { return M > kSpreadRows && M <= kSpreadMost && !one_block && (M > kTileM || !ahead); }
 
-double plan_cost(int M, int N, int num_kb, int sms, RowStart start, bool spread, const PlanC& pl) {
-  const CostC& c = M > kTileM ? kMoreRows : spread ? kSomeRows : kFewRows;
+double plan_cost(const CostC& c, int N, int num_kb, RowStart start, const PlanC& pl, int slots, int sms) {
   const int P = pl.pair ? 2 : 1, Mp = pl.n_mma * pl.nj, size = P * pl.S;
-  const int clusters = tile_count(N, pl), slots = &c == &kFewRows ? rough_slots(sms, size, pl.per_sm) : cluster_slots(size, pl.per_sm);
+  const int clusters = tile_count(N, pl);
   const int rounds = (clusters + slots - 1) / slots;
   const double live = double(clusters < slots ? clusters : slots) * size;  // CTAs at once
   const double share = live > sms ? live / sms : 1.0;
@@ -907,6 +912,16 @@ double plan_cost(int M, int N, int num_kb, int sms, RowStart start, bool spread,
   return rounds * t + (rounds - 1) * c.round + (size > 1 ? c.cluster : c.alone) + (size == 8 && Mp > 128 ? c.eight : 0.0) +
          c.split * (pl.S - 1) + (pl.S >= 5 ? c.five : 0.0);
 }
+// With blocks of 128 tokens and more.
+double whole_cost(int M, int N, int K, RowStart start, int sms, const PlanC& pl) {
+  const int num_kb = (K + kTileK - 1) / kTileK, size = (pl.pair ? 2 : 1) * pl.S;
+  return plan_cost(M <= kTileM ? kFewRows : kMoreRows, N, num_kb, start, pl, rough_slots(sms, size, pl.per_sm), sms);
+}
+// With blocks of any size.
+double spread_cost(int M, int N, int K, int sms, const PlanC& pl) {
+  const int num_kb = (K + kTileK - 1) / kTileK, size = (pl.pair ? 2 : 1) * pl.S;
+  return plan_cost(M <= kTileM ? kSpreadSome : kSpreadMore, N, num_kb, row_start(K), pl, cluster_slots(size, pl.per_sm), sms);
+}
 
 // What static weights save: the rings are filled while the kernel before ends.  Plans with more CTAs hold more (32 x 8192 x 3584 in a
 // decode step 13.3 us on 128 CTAs, 14.3 on 64, which were taken for faster).
@@ -916,14 +931,15 @@ double ring_us(int N, int num_kb, int sms, const PlanC& pl) {
   return live * pl.stages * pl.sub * kRowsW * kRowBytes / 6.05e6;
 }
 
-// The cheapest cut of a problem.  `fix_s` > 0 fixes the K split, `pair` is as in GemmArgs; `ahead`: static weights.
+// The cheapest cut of a problem into blocks of 128 tokens and more, or of any size (`spread`).  `fix_s` > 0 fixes the K split, `pair` is as
+// in GemmArgs; `ahead`: static weights.
 bool plan(int M, int N, int K, int sms, int pair, int fix_s, bool ahead, bool spread, PlanC* out, double* cost) {
   const int num_kb = (K + kTileK - 1) / kTileK;
   if (N <= kRowsW) pair = -1;  // one weight tile is no pair
   bool found = false;
   int last = 0;
   int most_blocks = (M + 127) / 128;
-  if (spread) most_blocks = std::max(most_blocks, std::min((M + kSpreadRows - 1) / kSpreadRows, 10));
+  if (spread) most_blocks = std::max(most_blocks, std::min((M + kSpreadRows - 1) / kSpreadRows, kSpreadBlocks));
   for (int blocks = (M + kMaxTileTokens - 1) / kMaxTileTokens; blocks <= most_blocks; ++blocks) {
     PlanC pl{};
     token_tile(M, blocks, &pl);
@@ -937,7 +953,8 @@ bool plan(int M, int N, int K, int sms, int pair, int fix_s, bool ahead, bool sp
       for (pl.S = 1; pl.S <= kMaxCluster / (two ? 2 : 1); ++pl.S) {
         if (fix_s > 0 ? pl.S != fix_s : (num_kb < 4 * pl.S && pl.S > 1)) continue;
         if (!size_cta(N, num_kb, sms, &pl)) continue;
-        double c = plan_cost(M, N, num_kb, sms, row_start(K), spread, pl);
+        // (with more rows the plans of whole blocks are compared as if rows started on a line: the set was fitted so)
+        double c = spread ? spread_cost(M, N, K, sms, pl) : whole_cost(M, N, K, M <= kTileM ? row_start(K) : kOnLine, sms, pl);
         if (ahead) c -= ring_us(N, num_kb, sms, pl);
         if (!found || c < *cost) {
           found = true;
@@ -953,10 +970,15 @@ bool plan(int M, int N, int K, int sms, int pair, int fix_s, bool ahead, bool sp
 // Plans depend on sizes alone; the last ones of a thread are kept (a model's layers repeat a handful of shapes).
 struct Planned {
   int M, N, K, flags;
-  bool ok;
+  bool ok, spread;  // spread: cut into blocks of any size
   PlanC pl;
-  double cost;
+  double whole_us, spread_us;  // estimates (without what static weights save): of the cut into whole blocks, of the spread one
 };
+// A spread cut is taken where its estimate is kSpreadGain of that of whole blocks, which the sets were fitted with: first of all to be no slower.
+// Over the 2090 timed shapes 0.952 of the time of whole blocks, 15 more than 3 % slower (a fit to the smallest mean time, where the cheaper estimate is
+// taken: 0.946, and 98 slower, 432 x 4048 x 4136 21.5 -> 24.6 us among them).
+// 340 other shapes of 33 - 1500 rows, against the code with whole blocks alone: plain 0.955, SwiGLU 0.93, QKV with rotation and cache write 0.97 of
+// the time, 16 more than 3 % slower (46 with the cheaper estimate).
 const Planned& planned(int M, int N, int K, int pair, int fix_s, bool ahead, bool one_block) {
   static thread_local Planned cache[64];
   const int flags = 1 | (pair > 0 ? 2 : pair < 0 ? 1 : 0) << 1 | (ahead ? 1 : 0) << 3 | fix_s << 4 | (one_block ? 1 : 0) << 12;
@@ -967,7 +989,19 @@ const Planned& planned(int M, int N, int K, int pair, int fix_s, bool ahead, boo
     c.N = N;
     c.K = K;
     c.flags = flags;
-    c.ok = plan(M, N, K, sm_count(), pair, fix_s, ahead, spread_rows(M, ahead, one_block), &c.pl, &c.cost);
+    const int sms = sm_count();
+    double us;
+    c.spread = false;
+    c.ok = plan(M, N, K, sms, pair, fix_s, ahead, false, &c.pl, &us);
+    c.whole_us = c.ok ? whole_cost(M, N, K, row_start(K), sms, c.pl) : kNone;
+    PlanC other;
+    if (spread_rows(M, ahead, one_block) && plan(M, N, K, sms, pair, fix_s, ahead, true, &other, &us)) {
+      c.spread_us = spread_cost(M, N, K, sms, other);
+      if (!c.ok || c.spread_us < kSpreadGain[M > kTileM] * spread_cost(M, N, K, sms, c.pl)) {
+        c.ok = c.spread = true;
+        c.pl = other;
+      }
+    }
   }
   return c;
 }
@@ -981,8 +1015,9 @@ bool gemm_cluster_supported(const GemmArgs& a) {
 
 // Whether this kernel is expected to be faster than the persistent two-SM kernel, which overlaps a tile's epilogue with the next
 // tile and needs no sum of parts, but deals out 256-row tiles: with fewer than three rounds of those, what they leave
-// idle or compute on padding is often more than this kernel's fixed cost.  Its estimate is taken times 1.14, as it was when the constants
-// of its plans were fitted to the choice of both (see CostC).
+// idle or compute on padding is often more than this kernel's fixed cost.  The estimate of whole blocks is taken a tenth lower, which
+// fits its present pace (over 467 shapes of more than 128 rows the choice is then 0.9 % slower than the best one on average), that of a spread
+// cut times kSpreadTwoSm, as it was when its constants were fitted.
 // Both sides measured, bf16 on B200: 512 x 1280 x 8192 17.4 here and 29.6 us there, 200 x 4096 x 4096 15.0 and 18.1, 512 x 2048 x 2048
 // 12.0 and 11.9; 1037 x 4104 x 2056 27.2 and 23.0, 768 x 7168 x 8192 71.5 and 64.7, 512 x 8192 x 8192 53.8 and 51.0, 2048 x 2048 x 2048
 // 20.5 and 17.5.
@@ -1001,7 +1036,7 @@ bool gemm_cluster_preferred(const GemmArgs& a) {
   if (static_cast<long long>((a.M + 2 * kTileM - 1) / (2 * kTileM)) * ((a.N + kTileN - 1) / kTileN) > 3ll * pairs) return false;
   const double two_sm = pair_cut(kGemmPlain, a.M, a.N, a.K, pairs, a.stream_k, swiglu, false, false).us;
   const Planned& c = planned(a.M, a.N, a.K, a.pair, 0, false, false);
-  return c.ok && 1.14 * c.cost < two_sm;
+  return c.ok && (0.9 * c.whole_us < two_sm || (c.spread && kSpreadTwoSm * c.spread_us < two_sm));
 }
 
 int gemm_cluster_local_bytes(int epilogue, int fmt) {

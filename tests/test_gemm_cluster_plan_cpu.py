@@ -26,8 +26,8 @@ def shapes(n, seed):
 
 # Token blocks, tokens of a block, pairs, K splits, CTAs an SM: shapes whose clusters come close to what a GPU runs at once, where one
 # cluster fewer has another K split.
-PINNED = {(154, 5568, 2584): (1, 160, 1, 3, 1), (116, 1024, 5624): (2, 64, 0, 6, 1), (512, 1280, 8192): (3, 176, 1, 4, 1),
-          (16, 7168, 8192): (1, 16, 0, 2, 1), (64, 7168, 8192): (1, 64, 0, 2, 1)}
+PINNED = {(154, 5568, 2584): (1, 160, 1, 3, 1), (116, 1024, 5624): (1, 128, 0, 8, 1), (512, 1280, 8192): (3, 176, 1, 3, 1),
+          (256, 4096, 4096): (2, 128, 0, 2, 1), (100, 2048, 2048): (4, 32, 0, 2, 1), (16, 7168, 8192): (1, 16, 0, 2, 1)}
 
 
 def check_pinned():
