@@ -216,7 +216,8 @@ typedef struct {
                    2 * tile's number in the schedule + CTA of the pair): [0] globaltimer ns at which the half was
                    complete (fused AR / RS: published to its reducer), [1] = pair << 32 | index in the pair's sequence */
   int b_static; /* plain mode: 1 = nothing that this call could overtake writes B (weights): the kernel may read B while the
-                   kernel before it on the stream still runs.  0 = B may be that kernel's output */
+                   kernel before it on the stream still runs.  2 = that, and B is one of a chain of weights that L2 does not hold
+                   together.  0 = B may be that kernel's output */
   const float* row_ssq; /* plain mode, M <= 128: row m of the product is multiplied by 1 / sqrt(s / K + row_eps), s = the sum over
                            row_parts of row_ssq[part * M + m] (the sums that OOB_EPILOGUE_ADD writes); null = not */
   int row_parts;        /* ceil(K / 128) */
@@ -297,8 +298,8 @@ int oob_pad_counter_count(void);
 int oob_test_pair_schedule(int mode, int M, int N, int K, int pairs, int stream_k, int world, int rank, int* out, int cap);
 /* Columns of an accumulator of that schedule (rows: 256); a pair may take two neighbouring ones in one item. */
 int oob_test_pair_tile_columns(int mode, int M, int N, int K, int pairs, int stream_k);
-/* Test hook (host only): how the weight-streaming GEMM cuts a problem, five integers: token blocks, tokens of a block (padded),
- * 1 = CTA pairs, K splits, CTAs that share an SM.  `pair` and `splits` are as in oob_gemm_args_t, `one_block`: row sums or
+/* Test hook (host only): how the weight-streaming GEMM cuts a problem, six integers: token blocks, tokens of a block (padded),
+ * 1 = CTA pairs, K splits, CTAs that share an SM, 1 = the weights leave L2 first.  `pair` and `splits` are as in oob_gemm_args_t, `one_block`: row sums or
  * the Add epilogue.  -1: it cannot. */
 int oob_test_gemm_cluster_plan(int M, int N, int K, int pair, int splits, int b_static, int one_block, int* out);
 /* Test hook: the most bytes of local memory (spilled registers) a thread of that GEMM's kernels has; `epilogue` 0 none, 1 SwiGLU, 2 RoPE + cache write,

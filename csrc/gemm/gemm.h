@@ -37,8 +37,8 @@ enum TraceSlot : int {
 constexpr int kGemmEpilogueSwigluTile = 3;
 constexpr int kGemmEpilogueAdd = 4;
 constexpr int kGemmClusterMaxRows = 4096;  // rows the weight-streaming kernel (gemm_cluster.cu) accepts
-// How that kernel cuts a problem: token blocks, tokens of a block, pairs, K splits, CTAs an SM.
-bool gemm_cluster_plan(int M, int N, int K, int pair, int splits, bool b_static, bool one_block, int out[5]);
+// How that kernel cuts a problem: token blocks, tokens of a block, pairs, K splits, CTAs an SM, and whether the weights leave L2 first.
+bool gemm_cluster_plan(int M, int N, int K, int pair, int splits, int b_static, bool one_block, int out[6]);
 // The most bytes of registers that a thread of its kernels spills, by epilogue (0 - 3: none, SwiGLU, RoPE + cache, Add); -1: no device.
 int gemm_cluster_local_bytes(int epilogue, int fmt);
 

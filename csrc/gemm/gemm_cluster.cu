@@ -67,11 +67,14 @@ constexpr int kWideTokens = 64;
 // what is fetched.  Weights of less than kFetchBytes are slower by up to 6 % where they are in L2 (1024 x 2048, 16 rows 4.26 -> 4.48 us); rows off a
 // line, whose boxes are two lines a row, are slower from memory as well (40 x 2736 x 1880 6.7 -> 7.3, 54 x 4800 x 3032 with SwiGLU 10.7 -> 11.9).
 constexpr long long kFetchBytes = 8ll << 20;
-// With one token block a launch reads every weight once.  Where they cannot be expected to be in L2 the next time (a third of it, or
-// a weight of a chain of layers), they are the first to leave it: 16 x 7168 x 8192 21.9 -> 20.9 us, 64 x 7168 x 8192 24.1 -> 22.9, 24 x 16000 x
-// 4096 23.0 -> 22.0, 32 x 8192 x 3584 12.15 -> 11.7, a layer of a decode step of 32 sequences 60.1 -> 55.0.  Weights that do stay there lose: a
-// layer of 88 MB that is used again and again 40.1 -> 43.9, 16 x 1024 x 1024 4.0 -> 4.3.
-constexpr long long kOnceBytes = 40ll << 20, kOnceStaticBytes = 8ll << 20;
+// With one token block a launch reads every weight once, and weights that will not be in L2 the next time leave it first: they then drive out neither
+// what is read again nor what has just been written.  One weight used again and again is in L2 up to some 80 MB (two thirds of it: both dies hold
+// some lines).  16 / 64 rows, K = 8192, one weight in repeated calls, default and evict-first: 72 MB 10.5 and 10.9 / 12.2 and 12.3 us, 80 MB
+// 16.9 and 16.8 / 12.7 and 12.85, 96 MB 19.5 and 19.1 / 20.6 and 19.4, 112 MB 20.7 and 19.8 / 22.3 and 22.1, 200 MB 35.3 and 34.5 / 38.1 and
+// 37.1; three weights in turn, 48 MB 12.7 and 12.3, 24 MB 7.1 and 8.1.  So from kOnceBytes on for a single call, and below only where the caller says that
+// the weights are part of a chain that L2 does not hold (a layer of a decode step of 32 sequences 60.1 -> 55.0 us; but four weights of 32 MB in turn 8.25
+// -> 8.9): weights of kOnceChainBytes and more, smaller ones gain nothing.
+constexpr long long kOnceBytes = 96ll << 20, kOnceChainBytes = 8ll << 20;
 constexpr int kThreadsC = 192;
 constexpr int kMaxStagesC = 12;
 constexpr int kSpreadRows = 32, kSpreadMost = 1500;  // rows between which blocks of fewer tokens than 128 are weighed, down to the first
@@ -967,6 +970,11 @@ bool plan(int M, int N, int K, int sms, int pair, int fix_s, bool ahead, bool sp
   return found;
 }
 
+// Whether the weights are loaded so that they leave L2 first.
+bool read_once(int N, int K, const PlanC& pl, int b_static) {
+  return pl.m_blocks == 1 && 2ll * N * K >= (b_static == 2 ? kOnceChainBytes : kOnceBytes);
+}
+
 // Plans depend on sizes alone; the last ones of a thread are kept (a model's layers repeat a handful of shapes).
 struct Planned {
   int M, N, K, flags;
@@ -1053,14 +1061,15 @@ int gemm_cluster_local_bytes(int epilogue, int fmt) {
   return fmt == 1 ? of(__nv_bfloat16()) : of(__half());
 }
 
-bool gemm_cluster_plan(int M, int N, int K, int pair, int splits, bool b_static, bool one_block, int out[5]) {
-  const gemm_cluster::Planned& c = gemm_cluster::planned(M, N, K, pair, splits, b_static, one_block);
+bool gemm_cluster_plan(int M, int N, int K, int pair, int splits, int b_static, bool one_block, int out[6]) {
+  const gemm_cluster::Planned& c = gemm_cluster::planned(M, N, K, pair, splits, b_static != 0, one_block);
   if (!c.ok) return false;
   out[0] = c.pl.m_blocks;
   out[1] = c.pl.n_mma * c.pl.nj;
   out[2] = c.pl.pair;
   out[3] = c.pl.S;
   out[4] = c.pl.per_sm;
+  out[5] = gemm_cluster::read_once(N, K, c.pl, b_static);
   return true;
 }
 
@@ -1098,7 +1107,7 @@ cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStr
   p.inv_k = 1.f / static_cast<float>(a.K);
   p.nan = std::numeric_limits<float>::quiet_NaN();
   if (a.epilogue == kEpiRopeKv) p.rope = *static_cast<const oob_rope_args_t*>(a.epilogue_args);
-  p.once = pl.m_blocks == 1 && 2ll * a.N * a.K >= (a.b_static ? kOnceStaticBytes : kOnceBytes);
+  p.once = read_once(a.N, a.K, pl, a.b_static);
   p.fetch = !a.b_static && a.ldb % kTileK == 0 && (reinterpret_cast<uintptr_t>(a.B) & 127) == 0 && 2ll * a.N * a.K >= kFetchBytes;
   p.n_mma = pl.n_mma;
   p.nj = pl.nj;

@@ -82,6 +82,13 @@ bool whole(PyObject* o, int* v) {
   return true;
 }
 
+// What is promised about B (oob_gemm_args_t::b_static); anything else: nothing.
+int promise(PyObject* o) {
+  int v = 0;
+  if (PyBool_Check(o)) return o == Py_True;
+  return whole(o, &v) && v >= 0 && v <= 2 ? v : 0;
+}
+
 // The operands of a GEMM that the kernels take as they are; false: not for this path.
 bool operands(const at::Tensor& a, const at::Tensor& b, int b_static, oob_gemm_args_t* g) {
   if (!half(a) || a.scalar_type() != b.scalar_type() || a.dim() != 2 || b.dim() != 2) return false;
@@ -151,7 +158,7 @@ PyObject* py_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 3 || modes_on() || !device(args[0], &dev)) return none();
   const at::Tensor *a = plain(args[0], dev), *b = plain(args[1], dev);
   oob_gemm_args_t g;
-  if (a == nullptr || b == nullptr || !operands(*a, *b, args[2] == Py_True, &g)) return none();
+  if (a == nullptr || b == nullptr || !operands(*a, *b, promise(args[2]), &g)) return none();
   at::Tensor out;
   int rc;
   {
@@ -172,7 +179,7 @@ PyObject* py_gemm_swiglu(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 3 || modes_on() || !device(args[0], &dev)) return none();
   const at::Tensor *a = plain(args[0], dev), *b = plain(args[1], dev);
   oob_gemm_args_t g;
-  if (a == nullptr || b == nullptr || !operands(*a, *b, args[2] == Py_True, &g) || g.N % 16 != 0) return none();
+  if (a == nullptr || b == nullptr || !operands(*a, *b, promise(args[2]), &g) || g.N % 16 != 0) return none();
   at::Tensor out;
   int rc;
   bool split;
@@ -202,7 +209,7 @@ PyObject* py_gemm_rope_kv_write(PyObject*, PyObject* const* args, Py_ssize_t n) 
                    *cos = plain(args[8], dev), *sin = plain(args[9], dev), *pos = nullptr;
   oob_gemm_args_t g;
   if (x == nullptr || w == nullptr || kc == nullptr || vc == nullptr || cos == nullptr || sin == nullptr ||
-      !operands(*x, *w, args[12] == Py_True, &g))
+      !operands(*x, *w, promise(args[12]), &g))
     return none();
   oob_rope_args_t r{};
   if (!whole(args[2], &r.B) || !whole(args[3], &r.T) || !whole(args[4], &r.H) || !whole(args[5], &r.KV) || !whole(args[11], &r.batch0) ||

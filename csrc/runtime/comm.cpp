@@ -1195,7 +1195,7 @@ int oob_test_pair_tile_columns(int mode, int M, int N, int K, int pairs, int str
 
 int oob_test_gemm_cluster_plan(int M, int N, int K, int pair, int splits, int b_static, int one_block, int* out) {
   if (M <= 0 || M > kGemmClusterMaxRows || N <= 0 || K <= 0 || splits < 0 || splits > 8 || out == nullptr) return -1;
-  return gemm_cluster_plan(M, N, K, pair, splits, b_static != 0, one_block != 0, out) ? 0 : -1;
+  return gemm_cluster_plan(M, N, K, pair, splits, b_static, one_block != 0, out) ? 0 : -1;
 }
 
 int oob_test_gemm_cluster_local_bytes(int epilogue, int dtype) { return gemm_cluster_local_bytes(epilogue, dtype == OOB_BF16 ? 1 : 0); }

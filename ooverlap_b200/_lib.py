@@ -117,10 +117,11 @@ def packer(structure) -> struct.Struct:
 NORM_ARGS = packer(NormArgs)
 ROPE_ARGS = packer(RopeArgs)
 ATTN_ARGS = packer(AttnDecodeArgs)
-# GemmArgs: the fields every plain call sets, and the rest with nothing asked for, with and without static weights.
+# GemmArgs: the fields every plain call sets, and the rest with nothing asked for, by what is promised about the weights.
 GEMM_HEAD = struct.Struct("@iiiiiPiPiPi")
 GEMM_TAIL = bytes(ctypes.sizeof(GemmArgs) - GEMM_HEAD.size)
 GEMM_TAIL_STATIC = bytes(GemmArgs(b_static=1))[GEMM_HEAD.size:]
+GEMM_TAIL_CHAIN = bytes(GemmArgs(b_static=2))[GEMM_HEAD.size:]
 
 _lock = threading.Lock()
 _lib = None

@@ -21,20 +21,23 @@ from ..utils.stream import current_stream_ptr
 
 
 class _Scope(threading.local):
-    static_b = False
+    static_b = 0  # GemmArgs.b_static
 
 
 _scope = _Scope()
 
 
 @contextlib.contextmanager
-def static_weights():
+def static_weights(*, beyond_l2: bool = False):
     """GEMMs that this thread launches in this block take their ``b`` to be a weight: neither the kernel before the call on the
     stream nor, in a chain of this library's kernels, one of those before it writes ``b``.  The weight-streaming kernel then
     loads its first weights while the kernel before it still runs.  Elsewhere ``b`` may be any tensor, also the result of
-    the call just before.  The promise is about weights alone: see ``attn_decode`` for its cache."""
+    the call just before.  The promise is about weights alone: see ``attn_decode`` for its cache.
+
+    ``beyond_l2``: the weights of the block, used again and again, are more together than L2 holds (from some 100 MB on).  Those of 8 MB and
+    more then leave it first, which keeps activations and keys in it; without, only weights that are too large by themselves do."""
     before = _scope.static_b
-    _scope.static_b = True
+    _scope.static_b = 2 if beyond_l2 else 1
     try:
         yield
     finally:
@@ -60,12 +63,15 @@ def fill_gemm_args(args: _lib.GemmArgs, a: torch.Tensor, b: torch.Tensor) -> Non
     args.B, args.ldb = b.data_ptr(), b.stride(0)
 
 
+_TAILS = (_lib.GEMM_TAIL, _lib.GEMM_TAIL_STATIC, _lib.GEMM_TAIL_CHAIN)
+
+
 def _packed_plain_args(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor) -> bytes:
     """The arguments of a call that asks for nothing, packed in one step: a third of the time of assigning them one by one (0.17 and
     0.75 us)."""
     return _lib.GEMM_HEAD.pack(_lib.GEMM_PLAIN, dtype_code(a.dtype), a.shape[0], b.shape[0], a.shape[1], a.data_ptr(), a.stride(0),
                                b.data_ptr(), b.stride(0), out.data_ptr(), out.stride(0)
-                               ) + (_lib.GEMM_TAIL_STATIC if _scope.static_b else _lib.GEMM_TAIL)
+                               ) + _TAILS[_scope.static_b]
 
 
 def _plain_args(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor) -> _lib.GemmArgs:

@@ -14,9 +14,15 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def plan(M, N, K, pair=0, splits=0, b_static=0, one_block=0):
-    out = (ctypes.c_int * 5)()
+    out = (ctypes.c_int * 6)()
     assert _lib.lib().oob_test_gemm_cluster_plan(M, N, K, pair, splits, b_static, one_block, out) == 0
-    return tuple(out)
+    return tuple(out)[:5]
+
+
+def leaves_l2_first(M, N, K, b_static=0):
+    out = (ctypes.c_int * 6)()
+    assert _lib.lib().oob_test_gemm_cluster_plan(M, N, K, 0, 0, b_static, 0, out) == 0
+    return bool(out[5])
 
 
 def shapes(n, seed):
@@ -75,6 +81,29 @@ def test_plans_are_sound():
         if M <= 128:
             assert plan(M, N, K, one_block=1)[0] == 1
         assert plan(M, N, K, splits=1)[3] == 1
+
+
+def test_weights_that_stay_in_l2_are_kept_there():
+    """A weight of up to some 80 MB that is used again and again is in L2 the next time, whether it is promised not to be written or not; only
+    the caller knows that it is one of many."""
+    for mb, alone in ((4, False), (16, False), (48, False), (72, False), (95, False), (97, True), (200, True)):
+        N = mb * (1 << 20) // (2 * 4096)
+        assert leaves_l2_first(16, N, 4096) == alone and leaves_l2_first(16, N, 4096, 1) == alone, mb
+        assert leaves_l2_first(16, N, 4096, 2) == (mb >= 8), mb
+    assert not leaves_l2_first(1000, 16384, 4096)  # several token blocks read it
+
+
+def test_a_model_says_that_its_weights_exceed_l2():
+    from ooverlap_b200.models import llama
+    from ooverlap_b200.ops.gemm import _scope
+    m = llama.LlamaTP(llama.TINY, None, dtype=torch.bfloat16, device=torch.device("cpu"), max_batch=8, max_len=16)
+    assert m.weight_bytes == sum(w.numel() * 2 for layer in m.layers for k, w in layer.items() if k.startswith("w")) + 2 * m.lm_head.numel()
+    seen = []
+    m._forward = lambda *a: seen.append(_scope.static_b)
+    for mb, rows, want in ((8, 8, 1), (95, 8, 1), (96, 8, 2), (100, 1, 1), (128, 1, 2)):
+        m.weight_bytes = mb << 20
+        m.forward(torch.zeros(rows, 1, dtype=torch.long), 0)
+        assert seen.pop() == want and not _scope.static_b
 
 
 @pytest.mark.gpu
