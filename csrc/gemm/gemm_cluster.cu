@@ -66,7 +66,8 @@ constexpr int kWideTokens = 64;
 // 2 % slower, on weights from L2 1.002.  All of up to eight stages: 0.973 and 1.018, 43 and 130 shapes slower, by up to 13 %: many CTAs' loads wait behind
 // what is fetched.  Weights of less than kFetchBytes are slower by up to 6 % where they are in L2 (1024 x 2048, 16 rows 4.26 -> 4.48 us); rows off a
 // line, whose boxes are two lines a row, are slower from memory as well (40 x 2736 x 1880 6.7 -> 7.3, 54 x 4800 x 3032 with SwiGLU 10.7 -> 11.9).
-constexpr long long kFetchBytes = 8ll << 20;
+// From kFetchTwoBytes on two stages: 16 x 8192 x 4096 13.5 -> 13.3 us, 64 x 8192 x 4096 14.0 -> 13.8; 16 x 7168 x 8192 21.3 -> 20.95.
+constexpr long long kFetchBytes = 8ll << 20, kFetchTwoBytes = 32ll << 20;
 // With one token block a launch reads every weight once, and weights that will not be in L2 the next time leave it first: they then drive out neither
 // what is read again nor what has just been written.  One weight used again and again is in L2 up to some 80 MB (two thirds of it: both dies hold
 // some lines).  16 / 64 rows, K = 8192, one weight in repeated calls, default and evict-first: 72 MB 10.5 and 10.9 / 12.2 and 12.3 us, 80 MB
@@ -121,7 +122,7 @@ struct ParamsC {
   float row_eps, inv_k;
   float nan;  // see settle
   bool once;  // which kernel the host takes
-  bool fetch;  // the first stage of weights is fetched into L2 before the wait for earlier kernels (see kFetchBytes)
+  int fetch;  // stages of weights, at most two, that a CTA fetches into L2 before the wait for earlier kernels (see kFetchBytes)
   oob_gemm_epilogue_add_t add;
 };
 
@@ -462,13 +463,14 @@ __global__ void __launch_bounds__(kThreadsC, RES)
   if constexpr (ONCE) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(once_policy));
   // Other weights may still be written by the kernel before: they are fetched into L2, which keeps up with such a write, and no further.
   // (Not where four CTAs share an SM: its few registers spill 12 - 28 bytes of 80.)
-  if (RES < 4 && warp == 0 && p.fetch && ptx::elect_one()) {
+  if (RES < 4 && warp == 0 && p.fetch > 0 && ptx::elect_one()) {
     const int w_row = (cluster / p.m_blocks * P + member) * (EPI == kEpiSwiglu ? kRowsW / 2 : kRowsW);
+    for (int kb = kb0; kb < min(kb1, kb0 + p.fetch); ++kb)
 #pragma unroll
-    for (int h = 0; h < SUB; ++h) {
-      ptx::tma_prefetch_2d(&tmap_w, (kb0 * SUB + h) * kTileK, w_row);
-      if constexpr (EPI == kEpiSwiglu) ptx::tma_prefetch_2d(&tmap_w, (kb0 * SUB + h) * kTileK, p.F + w_row);
-    }
+      for (int h = 0; h < SUB; ++h) {
+        ptx::tma_prefetch_2d(&tmap_w, (kb * SUB + h) * kTileK, w_row);
+        if constexpr (EPI == kEpiSwiglu) ptx::tma_prefetch_2d(&tmap_w, (kb * SUB + h) * kTileK, p.F + w_row);
+      }
   }
   __syncwarp();
   if (waited) ptx::griddep_wait();
@@ -1108,7 +1110,9 @@ cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStr
   p.nan = std::numeric_limits<float>::quiet_NaN();
   if (a.epilogue == kEpiRopeKv) p.rope = *static_cast<const oob_rope_args_t*>(a.epilogue_args);
   p.once = read_once(a.N, a.K, pl, a.b_static);
-  p.fetch = !a.b_static && a.ldb % kTileK == 0 && (reinterpret_cast<uintptr_t>(a.B) & 127) == 0 && 2ll * a.N * a.K >= kFetchBytes;
+  const long long weights = 2ll * a.N * a.K;
+  const bool on_line = a.ldb % kTileK == 0 && (reinterpret_cast<uintptr_t>(a.B) & 127) == 0;
+  p.fetch = a.b_static || !on_line || weights < kFetchBytes ? 0 : weights < kFetchTwoBytes ? 1 : 2;
   p.n_mma = pl.n_mma;
   p.nj = pl.nj;
   p.Mp = pl.n_mma * pl.nj;
