@@ -89,6 +89,11 @@ constexpr int kSmemLimit = 227 * 1024;
 
 enum { kEpiPlain = 0, kEpiSwiglu = 1, kEpiRopeKv = 2, kEpiAdd = 3 };
 
+// The fetch is paid for in registers of the sums, 4 - 6 a thread.  Where four CTAs share an SM they would be spilled, 12 - 28 bytes of 80; in the SwiGLU kernels they
+// cost what it gives (1 - 32 rows, weights in L2 1.02, from memory 1.00) but for weights that leave L2 first (16 x 7168 x 8192 21.8 -> 20.9 us, 16 x 28672 x 4096
+// 40.0 -> 37.7).
+constexpr bool fetches(int epi, int res, bool once) { return res < 4 && (epi != kEpiSwiglu || once); }
+
 struct CtlC {
   uint64_t full[kMaxStagesC];
   uint64_t empty[kMaxStagesC];
@@ -462,15 +467,16 @@ __global__ void __launch_bounds__(kThreadsC, RES)
   uint64_t once_policy = 0;
   if constexpr (ONCE) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(once_policy));
   // Other weights may still be written by the kernel before: they are fetched into L2, which keeps up with such a write, and no further.
-  // (Not where four CTAs share an SM: its few registers spill 12 - 28 bytes of 80.)
-  if (RES < 4 && warp == 0 && p.fetch > 0 && ptx::elect_one()) {
-    const int w_row = (cluster / p.m_blocks * P + member) * (EPI == kEpiSwiglu ? kRowsW / 2 : kRowsW);
-    for (int kb = kb0; kb < min(kb1, kb0 + p.fetch); ++kb)
+  if constexpr (fetches(EPI, RES, ONCE)) {
+    if (warp == 0 && p.fetch > 0 && ptx::elect_one()) {
+      const int w_row = (cluster / p.m_blocks * P + member) * (EPI == kEpiSwiglu ? kRowsW / 2 : kRowsW);
+      for (int kb = kb0; kb < min(kb1, kb0 + p.fetch); ++kb)
 #pragma unroll
-      for (int h = 0; h < SUB; ++h) {
-        ptx::tma_prefetch_2d(&tmap_w, (kb * SUB + h) * kTileK, w_row);
-        if constexpr (EPI == kEpiSwiglu) ptx::tma_prefetch_2d(&tmap_w, (kb * SUB + h) * kTileK, p.F + w_row);
-      }
+        for (int h = 0; h < SUB; ++h) {
+          ptx::tma_prefetch_2d(&tmap_w, (kb * SUB + h) * kTileK, w_row);
+          if constexpr (EPI == kEpiSwiglu) ptx::tma_prefetch_2d(&tmap_w, (kb * SUB + h) * kTileK, p.F + w_row);
+        }
+    }
   }
   __syncwarp();
   if (waited) ptx::griddep_wait();
