@@ -159,10 +159,12 @@ constexpr int kAttnWarps = 4;
 constexpr int kAttnThreads = kAttnWarps * 32;
 constexpr int kRowBytes = kHD * 2;                 // 256
 constexpr int kKvTileBytes = kTileKeys * kRowBytes;  // 4 KiB
-// Keys and values are read once, and from here on (three such caches do not fit it) the next call does not find them in L2: they leave it
-// first.  256 x 1900 keys 40.7 -> 40.3 us, 2 x 8000 with 8 KV heads 14.9 -> 14.65, 32 x 500 with 8 13.1 -> 12.8, 100 x 700 with 2 14.3 -> 14.0.  A kernel
-// of its own, chosen by the bound of the length: a policy in a register costs short contexts 1 - 4 %.
-constexpr long long kOnceBytes = 48ll << 20;
+// Keys and values are read once; those that the next call will not find in L2 leave it first.  A cache that is read again and again is found there up to 100 MB, so
+// that this is for the live keys of a call from here on: 256 x 1024 keys (128 MB) 23.4 -> 22.8 us, 256 x 1900 40.7 -> 40.3; but 80 MB of them, 256 x 640,
+// 10.35 -> 12.3, and in a cache of five times the length 10.5 -> 13.9.  The host knows a bound of the length and takes a kernel of its own by it (the
+// policy in a register costs short contexts 1 - 4 %), which looks at the length and has loads of both kinds (a normal policy for the short ones instead: up to
+// 5 % slower).  Not with more than eight heads a KV head: no gain (40 x 6553 keys 26.7, 27.0).
+constexpr long long kOnceBytes = 128ll << 20;
 constexpr int kMaxAttnCluster = 8;                 // portable cluster size
 constexpr int kAttnStages = 3;                     // tiles of K and V in flight or in use per warp (96 KiB per CTA, two per SM)
 // Where no SM gets two CTAs anyway, and CTAs alone or in pairs (64 x 300 keys 5.5 -> 5.15 us; clusters of eight gain nothing, fewer of
@@ -236,6 +238,7 @@ struct AttnParams {
   long long batch_stride;
   int max_len, batch0;
   int splits;
+  int once_len;  // of the kernel with ONCE: the length from which on keys and values leave L2 first (see kOnceBytes)
   float scale_log2;
   float nan;   // see the merge over the cluster
   bool ahead;  // the position and the keys and values before the newest may be read before the kernels this one depends on are done
@@ -308,6 +311,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
   const int my_tiles = t1 - t0 > warp ? (t1 - t0 - warp + kAttnWarps - 1) / kAttnWarps : 0;
 
   [[maybe_unused]] uint64_t policy = 0;
+  [[maybe_unused]] const bool first = ONCE && L >= p.once_len;
   if constexpr (ONCE) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
   auto issue_tile = [&](int i, int stage) {
     const int key0 = (t0 + warp + i * kAttnWarps) * kTileKeys;
@@ -316,8 +320,13 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
     for (int j = 0; j < kKvTileBytes / 512; ++j) {
       const int r = j * 2 + (lane >> 4), c = lane & 15;  // 16 units of 16 bytes per key row
       const int key = min(key0 + r, L - 1);  // masked later; the address stays inside the written part of the cache
-      cp_async_16<ONCE>(ks + kv_off(r, c), kbase + static_cast<long long>(key) * kHD + c * 8, policy);
-      cp_async_16<ONCE>(vs + kv_off(r, c), vbase + static_cast<long long>(key) * kHD + c * 8, policy);
+      if (ONCE && first) {
+        cp_async_16<true>(ks + kv_off(r, c), kbase + static_cast<long long>(key) * kHD + c * 8, policy);
+        cp_async_16<true>(vs + kv_off(r, c), vbase + static_cast<long long>(key) * kHD + c * 8, policy);
+      } else {
+        cp_async_16<false>(ks + kv_off(r, c), kbase + static_cast<long long>(key) * kHD + c * 8, policy);
+        cp_async_16<false>(vs + kv_off(r, c), vbase + static_cast<long long>(key) * kHD + c * 8, policy);
+      }
     }
   };
 
@@ -713,8 +722,9 @@ cudaError_t launch_attn(const AttnParams& p, int cluster, bool deep, bool once, 
       default: return launch_attn_s<T, 8, A, F, O>(p, stream);
     }
   };
-  cudaError_t e = p.G <= 8 ? (once ? size(std::true_type{}, std::true_type{}) : size(std::true_type{}, std::false_type{}))
-                           : (once ? size(std::false_type{}, std::true_type{}) : size(std::false_type{}, std::false_type{}));
+  cudaError_t e = p.G > 8 ? size(std::false_type{}, std::false_type{})
+                  : once  ? size(std::true_type{}, std::true_type{})
+                          : size(std::true_type{}, std::false_type{});
   if (e != cudaSuccess) return e;
   if (p.splits > 1) e = launch_pdl(p.ws_pairs ? attn_combine_kernel<T, true> : attn_combine_kernel<T, false>, dim3(p.B * p.H), kHD, 0, stream, 1, p.ws, p.out, p.splits);
   return e;
@@ -940,7 +950,9 @@ int oob_attn_decode(const oob_attn_decode_args_t* a, void* stream) {
   // the GPU then wait for the last ones (2 x 30000 keys on 8 KV heads 48 - 55 us in eights, 45 in fours; alone both 44).
   if (splits > 1) slots.n[3] -= slots.n[3] / 4;
   const int cluster = attn_cluster_size(static_cast<long long>(a->B) * a->KV * splits, (bound + splits - 1) / splits, slots);
-  const bool once = static_cast<long long>(a->B) * a->KV * bound * (4 * kHD) >= kOnceBytes;
+  const long long key_bytes = static_cast<long long>(a->B) * a->KV * (4 * kHD);  // of one key and value of all sequences
+  const bool once = key_bytes * bound >= kOnceBytes;
+  p.once_len = static_cast<int>((kOnceBytes + key_bytes - 1) / key_bytes);
   const bool deep = cluster <= 2 && static_cast<long long>(a->B) * a->KV * splits * cluster <= slots.deep[cluster - 1];
   cudaError_t e = a->dtype == OOB_BF16 ? launch_attn<__nv_bfloat16>(p, cluster, deep, once, s) : launch_attn<__half>(p, cluster, deep, once, s);
   if (e != cudaSuccess) return cuda_fail(e, "attn_decode launch");
