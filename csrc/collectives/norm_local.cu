@@ -41,15 +41,26 @@ struct LocalNorm {
   uint32_t polls;  // of a wait for a row
 };
 
-// Rows are read once, and what is written instead of them is read next: they are the first to leave L2 (residual + norm of 16384 x 8192 182.6 us,
-// 181.5 so; 4096 x 8192 47.9, 47.1; 6000 x 5120 45.3, 43.3; rows that stay in L2 are not slower).
+// Rows are read once.  In a call that moves more than L2 holds they leave it first: what is written instead of them is read next (residual + norm of 16384 x 8192
+// 182.6 us, 181.5 so; 6000 x 5120 45.3, 43.3; 6144 x 8192 without residual 40.5, 38.2).  In smaller calls rows may be in L2 the next time, and what they
+// came from may be read again: 3072 x 4096 with residual, the same rows again and again, 11.5, 13.6; 6144 x 4096 without 15.8, 17.6.
+constexpr long long kOnceBytesN = 160ll << 20;  // rows read and written
+// A kernel of its own: chosen row by row, by the thread that asks for the rows, 32768 x 1024 with residual took 51.5 us and not 49.9.
+template <bool ONCE>
 __device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  uint64_t policy;
-  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
-               :
-               : "r"(ptx::smem_u32(smem_dst)), "l"(src), "r"(bytes), "r"(ptx::smem_u32(bar)), "l"(policy)
-               : "memory");
+  if constexpr (ONCE) {
+    uint64_t policy;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+                 :
+                 : "r"(ptx::smem_u32(smem_dst)), "l"(src), "r"(bytes), "r"(ptx::smem_u32(bar)), "l"(policy)
+                 : "memory");
+  } else {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :
+                 : "r"(ptx::smem_u32(smem_dst)), "l"(src), "r"(bytes), "r"(ptx::smem_u32(bar))
+                 : "memory");
+  }
 }
 
 __device__ __forceinline__ float warp_sum(float v) {
@@ -129,8 +140,8 @@ __device__ __forceinline__ void finish_rows(const LocalNorm& a, int row, bool su
   }
 }
 
-// PPT: 16-byte packs per thread and row.
-template <typename T, int PPT>
+// PPT: 16-byte packs per thread and row.  ONCE: see kOnceBytesN.
+template <typename T, int PPT, bool ONCE>
 __global__ void __launch_bounds__(kThreadsN, PPT <= 2 ? 5 : PPT <= 4 ? 3 : 1) norm_stream_kernel(const __grid_constant__ LocalNorm a) {
   using PT = PackTraits<T>;
   extern __shared__ __align__(128) uint8_t smem[];
@@ -145,8 +156,8 @@ __global__ void __launch_bounds__(kThreadsN, PPT <= 2 ? 5 : PPT <= 4 ? 3 : 1) no
   auto issue = [&](int row, int stage) {
     uint8_t* dst = smem + size_t(stage) * stage_bytes;
     ptx::mbar_arrive_expect_tx(&full[stage], stage_bytes);
-    bulk_load(dst, a.x + size_t(row) * row_bytes, row_bytes, &full[stage]);
-    if (a.res != nullptr) bulk_load(dst + row_bytes, a.res + size_t(row) * row_bytes, row_bytes, &full[stage]);
+    bulk_load<ONCE>(dst, a.x + size_t(row) * row_bytes, row_bytes, &full[stage]);
+    if (a.res != nullptr) bulk_load<ONCE>(dst + row_bytes, a.res + size_t(row) * row_bytes, row_bytes, &full[stage]);
   };
   if (threadIdx.x == 0) {
     abort_word = 0;
@@ -297,9 +308,9 @@ cudaError_t launch(void (*kernel)(LocalNorm), int grid, int threads, int smem, c
   return cudaLaunchKernelEx(&cfg, kernel, n);
 }
 
-template <typename T, int PPT>
-cudaError_t launch_stream(LocalNorm n, int max_ctas, cudaStream_t stream) {
-  auto kernel = norm_stream_kernel<T, PPT>;
+template <typename T, int PPT, bool ONCE>
+cudaError_t launch_stream_of(LocalNorm n, int max_ctas, cudaStream_t stream) {
+  auto kernel = norm_stream_kernel<T, PPT, ONCE>;
   static std::atomic<uint64_t> attr_set{0};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -322,6 +333,12 @@ cudaError_t launch_stream(LocalNorm n, int max_ctas, cudaStream_t stream) {
   if (grid > max_ctas) grid = max_ctas;
   if (grid > n.rows) grid = n.rows;
   return launch(kernel, grid, kThreadsN, smem, n, stream);
+}
+
+template <typename T, int PPT>
+cudaError_t launch_stream(const LocalNorm& n, int max_ctas, cudaStream_t stream) {
+  const long long bytes = 2ll * n.rows * n.hidden * (2 + (n.res != nullptr ? 1 : 0) + (n.ro != nullptr ? 1 : 0));
+  return bytes >= kOnceBytesN ? launch_stream_of<T, PPT, true>(n, max_ctas, stream) : launch_stream_of<T, PPT, false>(n, max_ctas, stream);
 }
 
 template <typename T>
