@@ -15,6 +15,7 @@ import ctypes
 import importlib.util
 import struct
 import threading
+import warnings
 from ctypes import (POINTER, Structure, byref, c_char_p, c_float, c_int, c_int64, c_uint, c_uint64, c_void_p)
 
 from . import _build
@@ -226,8 +227,8 @@ _no_fast = _NoFast()
 
 
 def fast():
-    """The module of native Python entries (csrc/python/fast_ops.cpp).  They would pass by a stand-in for the library that has been put in
-    the place of ``lib``: then none is used."""
+    """The module of native Python entries (csrc/python/fast_ops.cpp), or what answers in its place where it cannot be built or loaded.  They
+    would pass by a stand-in for the library that has been put in the place of ``lib``: then none is used."""
     global _fast
     if lib is not _real_lib:
         return _no_fast
@@ -235,11 +236,21 @@ def fast():
         lib()
         with _lock:
             if _fast is None:
-                spec = importlib.util.spec_from_file_location("ooverlap_b200.lib._fast_ops", _build.FAST)
-                module = importlib.util.module_from_spec(spec)
-                spec.loader.exec_module(module)
-                _fast = module
+                _fast = _load_fast()
     return _fast
+
+
+def _load_fast():
+    if not (_build.fast_is_current() or _build.build_fast()):
+        return _no_fast
+    try:
+        spec = importlib.util.spec_from_file_location("ooverlap_b200.lib._fast_ops", _build.FAST)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        return module
+    except ImportError as e:
+        warnings.warn(f"the native Python entries cannot be loaded, the Python implementations are used: {e}", RuntimeWarning, stacklevel=3)
+        return _no_fast
 
 
 def last_error() -> str:
