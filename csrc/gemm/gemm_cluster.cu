@@ -25,8 +25,8 @@
 //   RoPE + KV  query and key heads are rotated, queries go to q_out, keys and values into the layer's cache
 //
 // Measured on B200, bf16, in a chain of launches (before: fp32 partial tiles through memory and a second kernel that sums
-// them): 16 x 7168 x 8192 22.2 us (26.5), 32 x 8192 x 3584 12.8 (18.2 with 16 rows), 8 x 8192 x 1024 6.9 (10.6), 8 x 1280 x 8192 7.8 (14.3),
-// 128 x 7168 x 8192 24.7 (27.5), 64 x 7168 x 8192 24.4 (29.6), 128 x 4096 x 4096 13.4, 512 x 1280 x 8192 17.4 (21.6).
+// them): 16 x 7168 x 8192 20.6 us (26.5), 32 x 8192 x 3584 12.2 (18.2 with 16 rows), 8 x 8192 x 1024 6.1 (10.6), 8 x 1280 x 8192 7.4 (14.3),
+// 128 x 7168 x 8192 24.0 (27.5), 64 x 7168 x 8192 22.9 (29.6), 128 x 4096 x 4096 12.2, 512 x 1280 x 8192 17.5 (21.6).
 //
 // Roles: warp 0 loads weights, warp 1 issues the MMAs, warp 2 loads activations (one thread each), warps 2-5 drain TMEM; all six
 // warps take part in the reduction.  A cluster handles tiles c, c + G, ... one after the other; normally the grid covers all tiles, a CTA
@@ -541,9 +541,7 @@ __global__ void __launch_bounds__(kThreadsC, RES)
       }
     };
     if (warp == 0) {
-      if (ptx::elect_one()) {
-        produce(std::true_type{}, One{});
-      }
+      if (ptx::elect_one()) produce(std::true_type{}, One{});
     } else if (warp == 2) {
       if (ptx::elect_one()) {
         if (SUB == 1 && p.n_mma == 2) {  // a wide stage holds one instruction's tokens
@@ -1034,9 +1032,9 @@ bool gemm_cluster_supported(const GemmArgs& a) {
 // idle or compute on padding is often more than this kernel's fixed cost.  The estimate of whole blocks is taken a tenth lower, which
 // fits its present pace (over 467 shapes of more than 128 rows the choice is then 0.9 % slower than the best one on average), that of a spread
 // cut times kSpreadTwoSm, as it was when its constants were fitted.
-// Both sides measured, bf16 on B200: 512 x 1280 x 8192 17.4 here and 29.6 us there, 200 x 4096 x 4096 15.0 and 18.1, 512 x 2048 x 2048
-// 12.0 and 11.9; 1037 x 4104 x 2056 27.2 and 23.0, 768 x 7168 x 8192 71.5 and 64.7, 512 x 8192 x 8192 53.8 and 51.0, 2048 x 2048 x 2048
-// 20.5 and 17.5.
+// Both sides measured, bf16 on B200: 512 x 1280 x 8192 17.5 here and 26.6 us there, 200 x 4096 x 4096 12.6 and 16.4, 512 x 2048 x 2048
+// 9.4 and 10.3; 1037 x 4104 x 2056 24.3 and 22.2, 768 x 7168 x 8192 70.5 and 63.6, 512 x 8192 x 8192 61.9 and 50.9, 2048 x 2048 x 2048
+// 25.6 and 16.8.
 bool gemm_cluster_preferred(const GemmArgs& a) {
   using namespace gemm_cluster;
   // Up to 128 rows the alternative is the one-SM kernel, persistent from the first tile to the last, on 256 weight rows a tile.

@@ -2,10 +2,10 @@
 // and grouped-query decode attention over a static cache.
 //
 // The attention kernel is bound by reading the cache once: a CTA handles one (sequence, KV head, key chunk); its
-// four warps take 16-key tiles in turn (cp.async, three stages, per-warp buffers, XOR-swizzled rows), compute
-// scores for all query heads of the KV group at once on the tensor cores (the <= 16 query heads are the M rows of
-// m16n8k16 MMAs -- too few rows for a tcgen05 tile, which needs 64), keep an online softmax per row and accumulate
-// P*V in fp32.  The warps' partial results are merged through shared memory, those of the up to eight CTAs of a cluster
+// four warps take 16-key tiles in turn (cp.async, three stages or six, per-warp buffers, XOR-swizzled rows), compute
+// scores for all query heads of the KV group at once on the tensor cores (m16n8k16: up to eight query heads are its columns and the
+// keys its rows, nine to sixteen are its rows -- too few for a tcgen05 tile, which needs 64), keep an online softmax per head and
+// accumulate P*V in fp32.  The warps' partial results are merged through shared memory, those of the up to eight CTAs of a cluster
 // through distributed shared memory; only few long sequences are cut further, and a second small kernel then merges.
 //
 // Capability parity: none of these exist in the reference (it delegates the model to vLLM,
@@ -436,75 +436,75 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
 #pragma unroll
       for (int dt = 0; dt < 8; ++dt) mma_16816<T>(o[dt], vf[dt], p0, p1);
     } else {
-    // ---- S = Q K^T for 16 keys ----
-    float s[2][4];
+      // ---- S = Q K^T for 16 keys ----
+      float s[2][4];
 #pragma unroll
-    for (int nb = 0; nb < 2; ++nb) s[nb][0] = s[nb][1] = s[nb][2] = s[nb][3] = 0.f;
-    uint32_t f[8][4];
+      for (int nb = 0; nb < 2; ++nb) s[nb][0] = s[nb][1] = s[nb][2] = s[nb][3] = 0.f;
+      uint32_t f[8][4];
 #pragma unroll
-    for (int i2 = 0; i2 < 8; ++i2) ldmatrix_x4(f[i2], ks + kv_off((i2 & 1) * 8 + (lane & 7), (i2 >> 1) * 4 + (lane >> 3)));
+      for (int i2 = 0; i2 < 8; ++i2) ldmatrix_x4(f[i2], ks + kv_off((i2 & 1) * 8 + (lane & 7), (i2 >> 1) * 4 + (lane >> 3)));
 #pragma unroll
-    for (int kp = 0; kp < 4; ++kp) {
+      for (int kp = 0; kp < 4; ++kp) {
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int nb = 0; nb < 2; ++nb) mma_16816<T>(s[nb], qa[2 * kp + h], f[kp * 2 + nb][h * 2], f[kp * 2 + nb][h * 2 + 1]);
-    }
-#pragma unroll
-    for (int dp = 0; dp < 8; ++dp) ldmatrix_x4_trans(f[dp], vs + kv_off(((lane >> 3) & 1) * 8 + (lane & 7), dp * 2 + (lane >> 4)));
-    // ---- mask, online softmax ----
-    float tmax[2] = {-INFINITY, -INFINITY}, m_use[2];
-#pragma unroll
-    for (int nb = 0; nb < 2; ++nb) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int key = key0 + nb * 8 + colp + (e & 1);
-        const float v = key < L ? s[nb][e] * p.scale_log2 : -INFINITY;
-        s[nb][e] = v;
-        tmax[e >> 1] = fmaxf(tmax[e >> 1], v);
-      }
-    }
-    if (__any_sync(0xffffffffu, tmax[0] > m_run[0] || tmax[1] > m_run[1])) {
-      float corr[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        tmax[h] = fmaxf(tmax[h], __shfl_xor_sync(0xffffffffu, tmax[h], 1));
-        tmax[h] = fmaxf(tmax[h], __shfl_xor_sync(0xffffffffu, tmax[h], 2));
-        const float m_new = fmaxf(m_run[h], tmax[h]);
-        corr[h] = exp2f(m_run[h] - (m_new == -INFINITY ? 0.f : m_new));  // 0 when nothing has been seen yet
-        m_run[h] = m_new;
-        l_run[h] *= corr[h];
+          for (int nb = 0; nb < 2; ++nb) mma_16816<T>(s[nb], qa[2 * kp + h], f[kp * 2 + nb][h * 2], f[kp * 2 + nb][h * 2 + 1]);
       }
 #pragma unroll
-      for (int i2 = 0; i2 < kAcc; ++i2) {
-        o[i2][0] *= corr[0];
-        o[i2][1] *= corr[0];
-        o[i2][2] *= corr[1];
-        o[i2][3] *= corr[1];
+      for (int dp = 0; dp < 8; ++dp) ldmatrix_x4_trans(f[dp], vs + kv_off(((lane >> 3) & 1) * 8 + (lane & 7), dp * 2 + (lane >> 4)));
+      // ---- mask, online softmax ----
+      float tmax[2] = {-INFINITY, -INFINITY}, m_use[2];
+#pragma unroll
+      for (int nb = 0; nb < 2; ++nb) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int key = key0 + nb * 8 + colp + (e & 1);
+          const float v = key < L ? s[nb][e] * p.scale_log2 : -INFINITY;
+          s[nb][e] = v;
+          tmax[e >> 1] = fmaxf(tmax[e >> 1], v);
+        }
       }
-    }
+      if (__any_sync(0xffffffffu, tmax[0] > m_run[0] || tmax[1] > m_run[1])) {
+        float corr[2];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) m_use[h] = m_run[h] == -INFINITY ? 0.f : m_run[h];
+        for (int h = 0; h < 2; ++h) {
+          tmax[h] = fmaxf(tmax[h], __shfl_xor_sync(0xffffffffu, tmax[h], 1));
+          tmax[h] = fmaxf(tmax[h], __shfl_xor_sync(0xffffffffu, tmax[h], 2));
+          const float m_new = fmaxf(m_run[h], tmax[h]);
+          corr[h] = exp2f(m_run[h] - (m_new == -INFINITY ? 0.f : m_new));  // 0 when nothing has been seen yet
+          m_run[h] = m_new;
+          l_run[h] *= corr[h];
+        }
 #pragma unroll
-    for (int nb = 0; nb < 2; ++nb) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float pv = exp2f(s[nb][e] - m_use[e >> 1]);
-        s[nb][e] = pv;
-        l_run[e >> 1] += pv;
+        for (int i2 = 0; i2 < kAcc; ++i2) {
+          o[i2][0] *= corr[0];
+          o[i2][1] *= corr[0];
+          o[i2][2] *= corr[1];
+          o[i2][3] *= corr[1];
+        }
       }
-    }
-    // ---- O += P V ----
-    uint32_t pa[4];
-    pa[0] = Cvt<T>::pack(s[0][0], s[0][1]);
-    pa[1] = Cvt<T>::pack(s[0][2], s[0][3]);
-    pa[2] = Cvt<T>::pack(s[1][0], s[1][1]);
-    pa[3] = Cvt<T>::pack(s[1][2], s[1][3]);
 #pragma unroll
-    for (int dp = 0; dp < 8; ++dp) {
-      mma_16816<T>(o[2 * dp], pa, f[dp][0], f[dp][1]);
-      mma_16816<T>(o[2 * dp + 1], pa, f[dp][2], f[dp][3]);
-    }
+      for (int h = 0; h < 2; ++h) m_use[h] = m_run[h] == -INFINITY ? 0.f : m_run[h];
+#pragma unroll
+      for (int nb = 0; nb < 2; ++nb) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float pv = exp2f(s[nb][e] - m_use[e >> 1]);
+          s[nb][e] = pv;
+          l_run[e >> 1] += pv;
+        }
+      }
+      // ---- O += P V ----
+      uint32_t pa[4];
+      pa[0] = Cvt<T>::pack(s[0][0], s[0][1]);
+      pa[1] = Cvt<T>::pack(s[0][2], s[0][3]);
+      pa[2] = Cvt<T>::pack(s[1][0], s[1][1]);
+      pa[3] = Cvt<T>::pack(s[1][2], s[1][3]);
+#pragma unroll
+      for (int dp = 0; dp < 8; ++dp) {
+        mma_16816<T>(o[2 * dp], pa, f[dp][0], f[dp][1]);
+        mma_16816<T>(o[2 * dp + 1], pa, f[dp][2], f[dp][3]);
+      }
     }
     __syncwarp();  // every lane is done with this stage before the next iteration's copies overwrite it
   }
@@ -799,8 +799,10 @@ double attn_cost_ns(long long items, int s, int slots, double len) {
 
 // CTAs of a cluster that share the keys of one (sequence, KV head).  The host knows a bound of the length, not the length, so a
 // size is weighed at the bound and at a third of it, each against one CTA: a cluster that gains little on a full cache loses
-// several times over on a short context, where all it adds is CTAs.  Timed with every size over 1057 combinations of batch,
-// heads, bound and length on B200, this choice is 0.3 % off the best one at full caches and 4 % over all lengths.  The rule that
+// several times over on a short context, where all it adds is CTAs.  The constants of attn_cost_ns were fitted to the kernel before this one,
+// whose merges took 0.5 - 3 us longer (0.3 % off the best size at full caches).  With this one, every size timed over 171 combinations of batch, heads,
+// bound and length on B200, the choice is 2.9 % off the best size at full caches (11 of 57 more than 3 %, most of them of less than 500 keys, where more CTAs
+// would pay), 0.7 % at a third and 14 % at a thirtieth of the bound (20 sequences with 16 heads, 59 of 1974 keys 5.9 us, 3.8 without clusters).  The rule that
 // looked at whole rounds at the bound only took four CTAs for 300 items of a 2048-key cache with 16 keys in it (20.3 us, 5.6 with
 // one) and for 600 items with 500 keys in it (68.5, 33.5).
 int attn_cluster_size(long long items, int len_bound, const AttnSlots& slots) {
