@@ -65,7 +65,8 @@ constexpr int kWideTokens = 64;
 // its rows start on a line.  One stage: over 728 shapes of 1 - 64 rows in a chain of calls on weights from memory 0.984 of the time, 3 of 330 more than
 // 2 % slower, on weights from L2 1.002.  All of up to eight stages: 0.973 and 1.018, 43 and 130 shapes slower, by up to 13 %: many CTAs' loads wait behind
 // what is fetched.  Weights of less than kFetchBytes are slower by up to 6 % where they are in L2 (1024 x 2048, 16 rows 4.26 -> 4.48 us); rows off a
-// line, whose boxes are two lines a row, are slower from memory as well (40 x 2736 x 1880 6.7 -> 7.3, 54 x 4800 x 3032 with SwiGLU 10.7 -> 11.9).
+// line, whose boxes are two lines a row, are slower from memory as well (40 x 2736 x 1880 6.7 -> 7.3, 54 x 4800 x 3032 with SwiGLU 10.7 -> 11.9) but for
+// weights that leave L2 first (three weights of 99 - 119 MB, 3 - 100 rows: 0.95 - 0.99 of the time).
 // From kFetchTwoBytes on two stages: 16 x 8192 x 4096 13.5 -> 13.3 us, 64 x 8192 x 4096 14.0 -> 13.8; 16 x 7168 x 8192 21.3 -> 20.95.
 constexpr long long kFetchBytes = 8ll << 20, kFetchTwoBytes = 32ll << 20;
 // With one token block a launch reads every weight once, and weights that will not be in L2 the next time leave it first: they then drive out neither
@@ -1116,7 +1117,7 @@ cudaError_t launch_gemm_cluster(const GemmArgs& a, DeviceStatus* status, cudaStr
   p.once = read_once(a.N, a.K, pl, a.b_static);
   const long long weights = 2ll * a.N * a.K;
   const bool on_line = a.ldb % kTileK == 0 && (reinterpret_cast<uintptr_t>(a.B) & 127) == 0;
-  p.fetch = a.b_static || !on_line || weights < kFetchBytes ? 0 : weights < kFetchTwoBytes ? 1 : 2;
+  p.fetch = a.b_static || weights < (on_line ? kFetchBytes : kOnceBytes) ? 0 : weights < kFetchTwoBytes ? 1 : 2;
   p.n_mma = pl.n_mma;
   p.nj = pl.nj;
   p.Mp = pl.n_mma * pl.nj;
