@@ -70,13 +70,12 @@ constexpr int kWideTokens = 64;
 // From kFetchTwoBytes on two stages: 16 x 8192 x 4096 13.5 -> 13.3 us, 64 x 8192 x 4096 14.0 -> 13.8; 16 x 7168 x 8192 21.3 -> 20.95.
 constexpr long long kFetchBytes = 8ll << 20, kFetchTwoBytes = 32ll << 20;
 // With one token block a launch reads every weight once, and weights that will not be in L2 the next time leave it first: they then drive out neither
-// what is read again nor what has just been written.  One weight used again and again is in L2 up to some 80 MB (two thirds of it: both dies hold
-// some lines).  16 / 64 rows, K = 8192, one weight in repeated calls, default and evict-first: 72 MB 10.5 and 10.9 / 12.2 and 12.3 us, 80 MB
-// 16.9 and 16.8 / 12.7 and 12.85, 96 MB 19.5 and 19.1 / 20.6 and 19.4, 112 MB 20.7 and 19.8 / 22.3 and 22.1, 200 MB 35.3 and 34.5 / 38.1 and
-// 37.1; three weights in turn, 48 MB 12.7 and 12.3, 24 MB 7.1 and 8.1.  So from kOnceBytes on for a single call, and below only where the caller says that
-// the weights are part of a chain that L2 does not hold (a layer of a decode step of 32 sequences 60.1 -> 55.0 us; but four weights of 32 MB in turn 8.25
-// -> 8.9): weights of kOnceChainBytes and more, smaller ones gain nothing.
-constexpr long long kOnceBytes = 96ll << 20, kOnceChainBytes = 8ll << 20;
+// what is read again nor what has just been written.  One weight used again and again is in L2 up to some 70 MB (more than half of it: both dies hold
+// some lines).  Time with such loads to time without, 3 - 64 rows, K of 4096 and 8192, one weight in repeated calls / two / three in turn: 40 MB 1.00 / 1.08 /
+// 0.95, 56 MB 1.03 / 0.95 / 0.96, 72 MB 1.03 / 0.93 / 0.95, 80 MB 0.99 / 0.97 / 0.95, 96 MB 0.97 / 0.97 / 0.97, 112 MB 0.94 / 0.95 / 0.95.  So from kOnceBytes on for a
+// single call, and below only where the caller says that the weights are part of a chain that L2 does not hold (a layer of a decode step of 32 sequences
+// 60.1 -> 55.0 us; but four weights of 32 MB in turn 8.25 -> 8.9): weights of kOnceChainBytes and more, smaller ones gain nothing.
+constexpr long long kOnceBytes = 80ll << 20, kOnceChainBytes = 8ll << 20;
 constexpr int kThreadsC = 192;
 constexpr int kMaxStagesC = 12;
 constexpr int kSpreadRows = 32, kSpreadMost = 1500;  // rows between which blocks of fewer tokens than 128 are weighed, down to the first

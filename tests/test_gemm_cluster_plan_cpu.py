@@ -84,9 +84,9 @@ def test_plans_are_sound():
 
 
 def test_weights_that_stay_in_l2_are_kept_there():
-    """A weight of up to some 80 MB that is used again and again is in L2 the next time, whether it is promised not to be written or not; only
+    """A weight of up to some 70 MB that is used again and again is in L2 the next time, whether it is promised not to be written or not; only
     the caller knows that it is one of many."""
-    for mb, alone in ((4, False), (16, False), (48, False), (72, False), (95, False), (97, True), (200, True)):
+    for mb, alone in ((4, False), (16, False), (48, False), (72, False), (79, False), (81, True), (200, True)):
         N = mb * (1 << 20) // (2 * 4096)
         assert leaves_l2_first(16, N, 4096) == alone and leaves_l2_first(16, N, 4096, 1) == alone, mb
         assert leaves_l2_first(16, N, 4096, 2) == (mb >= 8), mb
