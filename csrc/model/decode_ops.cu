@@ -316,17 +316,24 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_decode_kernel(AttnParams
   auto issue_tile = [&](int i, int stage) {
     const int key0 = (t0 + warp + i * kAttnWarps) * kTileKeys;
     const uint32_t ks = wbuf_u32 + stage * 2 * kKvTileBytes, vs = ks + kKvTileBytes;
+    auto copy = [&](auto leaves_first) {
+      constexpr bool H = decltype(leaves_first)::value;
 #pragma unroll
-    for (int j = 0; j < kKvTileBytes / 512; ++j) {
-      const int r = j * 2 + (lane >> 4), c = lane & 15;  // 16 units of 16 bytes per key row
-      const int key = min(key0 + r, L - 1);  // masked later; the address stays inside the written part of the cache
-      if (ONCE && first) {
-        cp_async_16<true>(ks + kv_off(r, c), kbase + static_cast<long long>(key) * kHD + c * 8, policy);
-        cp_async_16<true>(vs + kv_off(r, c), vbase + static_cast<long long>(key) * kHD + c * 8, policy);
-      } else {
-        cp_async_16<false>(ks + kv_off(r, c), kbase + static_cast<long long>(key) * kHD + c * 8, policy);
-        cp_async_16<false>(vs + kv_off(r, c), vbase + static_cast<long long>(key) * kHD + c * 8, policy);
+      for (int j = 0; j < kKvTileBytes / 512; ++j) {
+        const int r = j * 2 + (lane >> 4), c = lane & 15;  // 16 units of 16 bytes per key row
+        const int key = min(key0 + r, L - 1);  // masked later; the address stays inside the written part of the cache
+        cp_async_16<H>(ks + kv_off(r, c), kbase + static_cast<long long>(key) * kHD + c * 8, policy);
+        cp_async_16<H>(vs + kv_off(r, c), vbase + static_cast<long long>(key) * kHD + c * 8, policy);
       }
+    };
+    if constexpr (ONCE) {
+      if (first) {
+        copy(std::true_type{});
+      } else {
+        copy(std::false_type{});
+      }
+    } else {
+      copy(std::false_type{});
     }
   };
 
